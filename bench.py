@@ -168,7 +168,8 @@ def run_ours(args, rank, world, device):
         cu.collision()
         cu.forcing_resident(ALPHA, BETA)
 
-    cu.set_overlap(args.overlap)
+    if args.overlap:
+        cu.set_overlap(True)
     for _ in range(args.warmup):
         device_step()
     cu.synchronize()

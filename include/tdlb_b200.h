@@ -251,8 +251,8 @@ int tdlb_checkpoint_read(tdlb_handle h, const char* dir, const char* unit_name);
 
 /* Step-kernel variant: cells per thread (1, 2 or 4 -- float2 / float4
  * traffic). Default: 1 for FP32 storage; for 16-bit storage 4 with Simple
- * streaming, 2 with Esotwist (the fastest on B200 at 400^3 for each). Split steps (tdlb_set_overlap) need
- * one cell per thread. FP32
+ * streaming, 2 with Esotwist (the fastest on B200 at 400^3 for each). FP32
+ * steps split (tdlb_set_overlap) at one cell per thread only. FP32
  * storage: all variants compute identical results; 16-bit storage: 2 and 4
  * cells per thread use packed FP32x2 arithmetic (results within FP32
  * rounding). A residual box works with every variant (its own launches run
@@ -274,11 +274,10 @@ int tdlb_set_l2_prefetch(tdlb_handle h, int on);
  * deviation, the FP32 residual of its rounding, so these locations are
  * stored exactly: the stirred tank's velocity error against FP64 comes
  * mostly from the 16-bit rounding in the impeller's swept volume. The box
- * costs 72 (Esotwist) or 144 (Simple) bytes of device memory per box cell,
- * plus 76 bytes of scratch per cell of the 32-cell chunks within one cell of
- * it, and traffic only there: a step with a box adds two launches over those
- * chunks (they are stepped with the residuals before the plain launch and
- * committed after it) and never splits (tdlb_set_overlap).
+ * costs 72 (Esotwist) or 144 (Simple) bytes of device memory per box cell
+ * and traffic only there: a step with a box steps the cells near it (the
+ * groups of 32 along z that reach within one cell of it) in a launch of
+ * their own, with the residuals, and leaves them out of the others.
  * tdlb_attach_rushton sets it over the blades' swept volume with a 4-cell
  * margin, unless a box was set (or removed) with this call; an empty box
  * (i1 <= i0) removes it. Requires 16-bit storage (TDLB_EINVAL), a lattice
@@ -289,22 +288,20 @@ int tdlb_set_residual_box(tdlb_handle h, int64_t i0, int64_t i1, int64_t j0, int
 /* The current box as {i0, i1, j0, j1, k0, k1} (all zero: none). */
 int tdlb_get_residual_box(tdlb_handle h, int64_t* box6);
 
-/* Split steps. mode 0 (default): off; 1: on when the inner chunks hold at
- * most 60 % of the lattice (large tanks; a small one is mostly stencil
- * cells); 2: on whenever possible. With resident markers (tdlb_set_markers
- * or tdlb_attach_rushton) and one cell per thread, a step runs as two launches:
- * the cells outside every marker stencil (the "outer" chunks, which read no
- * force) on the handle's stream, and the stencil cells and their neighbours
- * (the "inner" chunks) on a second stream, after the forcing pass. The
- * previous step's forcing pass then runs while the outer cells of the next
- * step are computed. Every cell computes what the single launch computes,
- * so results are bit-identical with overlap on and off. Measured on B200
- * at 400^3 (Rushton tank): whole steps 0-4 % faster, because the two
- * launches over scattered chunks lose most of what the overlap hides, hence
- * off by default. A step with a residual box (tdlb_set_residual_box) runs
- * unsplit. Entry points other
- * than tdlb_collision, tdlb_forcing_resident, tdlb_rotate_impeller and
- * tdlb_step first order the handle's stream after that second stream. */
+/* Split steps. With resident markers (tdlb_set_markers or
+ * tdlb_attach_rushton) a step can run as two launches: the cells outside every
+ * marker stencil (the "outer" ones, which read no force) on an internal
+ * stream, and the stencil cells and their neighbours (the "inner" ones), in
+ * words of 32 cells along y, on the handle's stream after the forcing pass.
+ * The outer cells of a step then run beside the previous step's forcing
+ * pass. Every cell computes what the single launch computes, so results are
+ * bit-identical with and without. mode 0: off; 1: on when the inner words
+ * hold at most 60 % of the lattice; 2: on whenever possible. Until this is
+ * called, as 1 for lattices of at least 2^19 cells (below, the second launch
+ * costs more than it hides). FP32 storage needs one cell per thread; a step
+ * under stream capture is never split. The handle's stream waits for the
+ * outer launch at the end of each step, so work queued there afterwards sees
+ * the whole step. */
 int tdlb_set_overlap(tdlb_handle h, int mode);
 
 /* Order the handle's stream (tdlb_get_stream) after every queued step and
@@ -312,8 +309,9 @@ int tdlb_set_overlap(tdlb_handle h, int mode);
 int tdlb_join(tdlb_handle h);
 
 /* Per-cell flags (interior cells in (i, j, k) order) of the split-step zone:
- * 1 where the cell belongs to an inner chunk. TDLB_ESTATE when the handle
- * does not split its steps (see tdlb_set_overlap). */
+ * 1 where the cell belongs to an inner word. TDLB_ESTATE when tdlb_set_overlap
+ * has not turned split steps on, the handle cannot split them, or the step
+ * kernel takes several cells per thread. */
 int tdlb_read_zone(tdlb_handle h, uint8_t* flags);
 
 /* Step-kernel timing: when on, every step-kernel launch (both launches of a

@@ -101,13 +101,13 @@ __device__ __forceinline__ void prefetch_chunk(const TankStep& ts, unsigned q0) 
     const Dims& g = ts.g;
     const long long e0 = (long long)q0 * V, e1 = e0 + (long long)NT * V;
     if (d == NQ) return prefetch_span(ts.Nu, 4, g.plane, e0, e1);
-    const long long rs = (long long)g.ny * g.kp;
+    const long long rs = (long long)g.nz * g.jp;
     long long sh;
     if (ESO) {
         const int sg = ts.even ? -1 : 1;
-        sh = (sg * cx_of(d) > 0 ? rs : 0) + (sg * cy_of(d) > 0 ? g.kp : 0);
+        sh = (sg * cx_of(d) > 0 ? rs : 0) + (sg * cz_of(d) > 0 ? g.jp : 0);
     } else {
-        sh = -(cx_of(d) * rs + cy_of(d) * g.kp);
+        sh = -(cx_of(d) * rs + cz_of(d) * g.jp);
     }
     prefetch_span(ts.A.p[d], (int)sizeof(S), g.plane, e0 + sh - 1, e1 + sh + 1);
 }
@@ -130,7 +130,7 @@ __global__ void __launch_bounds__(NT, (ESO ? kEsotwistBlocksPerSM<V> : 4) * 128 
         __syncthreads();
         stage<NT>(ts, tanks + wk.x);
         __syncthreads();
-        const unsigned nquads = (unsigned)ts.g.nx * (unsigned)ts.g.ny * (unsigned)(ts.g.kp / V);
+        const unsigned nquads = (unsigned)ts.g.nx * (unsigned)ts.g.nz * (unsigned)(ts.g.jp / V);
         for (int c = 0; c < kBatchChunks; c++) {
             const unsigned t0 = (unsigned)wk.y + (unsigned)(c * NT);
             if (t0 >= nquads) break;   // uniform over the block
@@ -284,6 +284,14 @@ int bguard(tdlb_batch_s* b, F&& fn) {
 int storage_of(const tdlb_batch_s* b) { return b->storage; }
 bool eso_of(const tdlb_batch_s* b) { return b->streaming == TDLB_STREAMING_ESOTWIST; }
 
+// Cells per thread of the fused launch: the batch's shape, or the widest that
+// every tank's rows take (16-bit storage is built for 1 and 4).
+int width_of(const tdlb_batch_s* b) {
+    int v = b->vec;
+    for (const tdlb_lattice* h : b->tanks) v = std::min(v, tdlb::vector_width(h->g, v));
+    return v == 2 && b->storage != TDLB_STORAGE_FP32 ? 1 : v;
+}
+
 // Upload `items` into `w` (the stream is idle: callers synchronise first).
 void put(WorkList& w, const std::vector<int2>& items) {
     if ((int)items.size() > w.cap) {
@@ -307,7 +315,7 @@ void drop(WorkList& w) {
 void assign_groups(tdlb_batch_s* b) {
     std::vector<int> order(b->tanks.size());
     for (size_t t = 0; t < order.size(); t++) order[t] = (int)t;
-    auto cells = [&](int t) { return b->tanks[(size_t)t]->g.rows() * (long long)b->tanks[(size_t)t]->g.nz; };
+    auto cells = [&](int t) { return b->tanks[(size_t)t]->g.cells(); };
     std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return cells(x) > cells(y); });
     long long sum[2] = {0, 0};
     b->grp[0].tanks.clear();
@@ -331,11 +339,12 @@ cudaError_t quiesce(tdlb_batch_s* b) {
 // Fused-step work lists for the current shape: (tank, first quad) per item,
 // for every tank and per group.
 void build_work(tdlb_batch_s* b) {
+    const int vec = width_of(b);
     auto items = [&](const std::vector<int>& ts) {
         std::vector<int2> w;
         for (int t : ts) {
             const Dims& g = b->tanks[(size_t)t]->g;
-            const long long nq = g.rows() * (g.kp / b->vec);
+            const long long nq = g.rows() * (g.jp / vec);
             for (long long q = 0; q < nq; q += (long long)b->threads * tdlb::kBatchChunks) w.push_back(make_int2(t, (int)q));
         }
         return w;
@@ -360,8 +369,14 @@ void build_ibm_work(tdlb_batch_s* b) {
         for (int t : G.tanks) {
             const tdlb_lattice* h = b->tanks[(size_t)t];
             if (!h->markers_set) continue;
-            const int ncell = (int)h->cells.cell_e.size();
-            for (int c = 0; c < ncell; c += 256) cells.push_back(make_int2(t, c));
+            const int places = std::max(h->max_cells, h->max_big);
+            for (int p = 0; p < places; p += 8)
+                for (int jg = 0; jg < h->g.ny; jg += 32) {
+                    bool any = false;   // a tile past every plane's cells is left out
+                    for (int j = jg; j < std::min(jg + 32, h->g.ny); j++)
+                        any = any || h->cells.plane_cell[(size_t)j + 1] - h->cells.plane_cell[(size_t)j] > p;
+                    if (any) cells.push_back(make_int2(t, (p / 8) << 10 | jg / 32));
+                }
             for (int q = 0; q < h->n_markers - h->n0; q += 128) tails.push_back(make_int2(t, q));
             for (long long wd = 0; wd < h->mask_words; wd += tdlb::kMaskCopyWords) copies.push_back(make_int2(t, (int)wd));
             for (int s = 0; s < h->n_small; s++) small.push_back(make_int2(t, h->h_plane_list[(size_t)s]));
@@ -413,9 +428,10 @@ void advance_step_state(tdlb_lattice* h) {
 // it starts, within its item.
 void launch_fused(tdlb_batch_s* b, const TankStep* d_views, const WorkList& work, int* counter, cudaStream_t st) {
     if (work.n == 0) return;
-    const tdlb::BatchFn fn = tdlb::batch_kernel(storage_of(b), eso_of(b), b->vec, b->threads);
+    const int vec = width_of(b);
+    const tdlb::BatchFn fn = tdlb::batch_kernel(storage_of(b), eso_of(b), vec, b->threads);
     const int grid = b->bps > 0 ? std::min(work.n, b->sms * b->bps) : work.n;
-    const int ahead = std::max(1, tdlb::kBatchPrefetchCells / (b->threads * b->vec));
+    const int ahead = std::max(1, tdlb::kBatchPrefetchCells / (b->threads * vec));
     fn<<<grid, b->threads, 0, st>>>(d_views, work.d, work.n, counter, ahead);
     TDLB_BCK(cudaGetLastError());
 }
@@ -685,7 +701,7 @@ void eager_step(tdlb_batch_s* b, float alpha, float beta) {
 // its key is unchanged (the views, tables and rotors it reads are device
 // arrays rewritten before every run).
 std::vector<uintptr_t> graph_key(const tdlb_batch_s* b, int P) {
-    std::vector<uintptr_t> k = {(uintptr_t)P, b->tanks.size(), (uintptr_t)b->vec, (uintptr_t)b->threads,
+    std::vector<uintptr_t> k = {(uintptr_t)P, b->tanks.size(), (uintptr_t)width_of(b), (uintptr_t)b->threads,
                                 (uintptr_t)b->bps, (uintptr_t)b->d_steps, (uintptr_t)b->d_ibm,
                                 (uintptr_t)b->d_rotors, (uintptr_t)b->d_step};
     for (const BatchGroup& G : b->grp) {
@@ -762,7 +778,7 @@ cudaGraphExec_t graph_for(tdlb_batch_s* b, int P, int& kernels) {
         if (h->markers_set) h->pass -= 2 * P;
     // every kernel but the fused launch (forcing passes, rotations) keeps the
     // high priority of the streams it was captured from
-    cudaError_t pe = prioritise_nodes(g, (const void*)tdlb::batch_kernel(storage_of(b), eso_of(b), b->vec, b->threads),
+    cudaError_t pe = prioritise_nodes(g, (const void*)tdlb::batch_kernel(storage_of(b), eso_of(b), width_of(b), b->threads),
                                       b->ibm_priority);
     cudaGraphExec_t ge = nullptr;
     const cudaError_t ie = pe != cudaSuccess ? pe : cudaGraphInstantiateWithFlags(&ge, g, cudaGraphInstantiateFlagUseNodePriority);

@@ -51,11 +51,9 @@ template <typename S>
 __global__ void __launch_bounds__(256) k_ckpt_q_out(Planes A, Dims g, int mode, int even, CollideParams p, int esotwist,
                                                     float* __restrict__ out) {
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= g.rows() * g.nz) return;
-    const int k = (int)(t % g.nz);
-    const long long row = t / g.nz;
-    const int j = (int)(row % g.ny);
-    const int i = (int)(row / g.ny);
+    if (t >= g.cells()) return;
+    int i, j, k;
+    g.cell(t, i, j, k);
     float m[NQ];
     state_moments18<S>(A, g, mode, even, p, i, j, k, m);
     if (!esotwist) {
@@ -76,14 +74,12 @@ __global__ void __launch_bounds__(256) k_ckpt_f_out(const float4* __restrict__ F
                                                     const float* __restrict__ Nu, Dims g, float* __restrict__ f3,
                                                     float* __restrict__ nu) {
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= g.rows() * g.nz) return;
-    const int k = (int)(t % g.nz);
-    const long long row = t / g.nz;
-    const int j = (int)(row % g.ny);
-    const int i = (int)(row / g.ny);
-    const long long e = row * g.kp + k;
+    if (t >= g.cells()) return;
+    int i, j, k;
+    g.cell(t, i, j, k);
+    const long long e = g.at(i, j, k);
     const long long o = ghost_index(g, i, j, k);
-    const bool on = (mask[row * g.kw + (k >> 5)] >> (k & 31)) & 1u;
+    const bool on = (mask[g.word(i, j, k)] >> (j & 31)) & 1u;
     const float4 v = F[e];
     f3[3 * o] = on ? v.x : 0.f;
     f3[3 * o + 1] = on ? v.y : 0.f;
@@ -96,13 +92,11 @@ __global__ void __launch_bounds__(256) k_ckpt_f_out(const float4* __restrict__ F
 // of the stored parity for Esotwist).
 __global__ void __launch_bounds__(256) k_ckpt_q_in(const float* __restrict__ in, Planes A, Dims g) {
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= g.rows() * g.nz) return;
-    const int k = (int)(t % g.nz);
-    const long long row = t / g.nz;
-    const int j = (int)(row % g.ny);
-    const int i = (int)(row / g.ny);
+    if (t >= g.cells()) return;
+    int i, j, k;
+    g.cell(t, i, j, k);
     const float* q = in + ghost_index(g, i, j, k) * NQ;
-    const long long e = row * g.kp + k;
+    const long long e = g.at(i, j, k);
 #pragma unroll
     for (int s = 0; s < NQ; s++) A.p[s][e] = q[s];
 }
@@ -114,17 +108,17 @@ __global__ void __launch_bounds__(256) k_ckpt_f_in(const float* __restrict__ f3,
                                                    float4* __restrict__ F, float* __restrict__ Nu,
                                                    uint32_t* __restrict__ mask) {
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= g.rows() * g.kw) return;
-    const long long row = t / g.kw;
-    const int w = (int)(t - row * g.kw);
-    const int j = (int)(row % g.ny);
-    const int i = (int)(row / g.ny);
+    if (t >= g.rows() * g.jw) return;
+    const long long row = t / g.jw;
+    const int w = (int)(t - row * g.jw);
+    const int i = (int)(row / g.nz);
+    const int k = (int)(row - (long long)i * g.nz);
     uint32_t bits = 0;
     for (int b = 0; b < 32; b++) {
-        const int k = w * 32 + b;
-        if (k >= g.kp) break;
-        const long long e = row * g.kp + k;
-        if (k >= g.nz) {
+        const int j = w * 32 + b;
+        if (j >= g.jp) break;
+        const long long e = row * g.jp + j;
+        if (j >= g.ny) {
             F[e] = make_float4(0.f, 0.f, 0.f, 0.f);
             Nu[e] = 0.f;
             continue;
@@ -158,8 +152,7 @@ int cguard(tdlb_lattice* h, F&& fn) {
     if (!h) return TDLB_EINVAL;
     try {
         cudaSetDevice(h->device);
-        const cudaError_t je = tdlb_rt::join_side(h);   // after every queued step and forcing pass
-        if (je != cudaSuccess) throw CFail{TDLB_ECUDA, std::string("join: ") + cudaGetErrorString(je)};
+        tdlb_rt::fence(h);
         fn();
         return TDLB_OK;
     } catch (const CFail& f) {
@@ -367,7 +360,7 @@ int tdlb_checkpoint_write(tdlb_handle h, const char* dir, const char* unit_name,
         Scratch sc;
         TDLB_CCK(cudaMalloc(&sc.dev, (size_t)ng * tdlb::NQ * sizeof(float)));
         TDLB_CCK(cudaHostAlloc((void**)&sc.pin, kStage, cudaHostAllocDefault));
-        const long long cells = g.rows() * g.nz;
+        const long long cells = g.cells();
         const int eso = h->cfg.streaming == TDLB_STREAMING_ESOTWIST;
         // Q
         TDLB_CCK(cudaMemsetAsync(sc.dev, 0, (size_t)ng * tdlb::NQ * sizeof(float), h->stream));
@@ -441,14 +434,14 @@ int tdlb_checkpoint_read(tdlb_handle h, const char* dir, const char* unit_name) 
         Scratch sc;
         TDLB_CCK(cudaMalloc(&sc.dev, (size_t)ng * tdlb::NQ * sizeof(float)));
         TDLB_CCK(cudaHostAlloc((void**)&sc.pin, kStage, cudaHostAllocDefault));
-        const long long cells = g.rows() * g.nz;
+        const long long cells = g.cells();
         read_device(grid_file(sdir, id, unit, "Q"), sc.dev, (size_t)ng * tdlb::NQ * sizeof(float), h->stream, sc.pin);
         tdlb::k_ckpt_q_in<<<blocks(cells), 256, 0, h->stream>>>(sc.dev, h->planes(h->bufA), g);
         TDLB_CCK(cudaGetLastError());
         read_device(grid_file(sdir, id, unit, "F"), sc.dev, (size_t)ng * 3 * sizeof(float), h->stream, sc.pin);
         read_device(grid_file(sdir, id, unit, "Nu"), sc.dev + 3 * ng, (size_t)ng * sizeof(float), h->stream, sc.pin);
         TDLB_CCK(cudaMemsetAsync(h->mask, 0, (size_t)2 * h->mask_words * sizeof(uint32_t), h->stream));
-        tdlb::k_ckpt_f_in<<<blocks(g.rows() * g.kw), 256, 0, h->stream>>>(sc.dev, sc.dev + 3 * ng, g,
+        tdlb::k_ckpt_f_in<<<blocks(g.rows() * g.jw), 256, 0, h->stream>>>(sc.dev, sc.dev + 3 * ng, g,
                                                                           reinterpret_cast<float4*>(h->F), h->Nu, h->mask);
         TDLB_CCK(cudaGetLastError());
         TDLB_CCK(cudaStreamSynchronize(h->stream));

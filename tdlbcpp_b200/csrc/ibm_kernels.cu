@@ -82,7 +82,7 @@ template <typename S>
 __device__ __forceinline__ void cell_moments4(const Planes& A, int mode, int even, const Dims& g, int i, int j, int k,
                                               const CollideParams& p, float* m4, const ResidualBox& rb) {
     if (mode == 1) {
-        const long long e = ((long long)i * g.ny + j) * g.kp + k;
+        const long long e = g.at(i, j, k);
 #pragma unroll
         for (int s = 0; s < 4; s++) m4[s] = ld_state<S>(A.p[s], e);
         return;
@@ -94,7 +94,7 @@ __device__ __forceinline__ void cell_moments4(const Planes& A, int mode, int eve
         for (int d = 0; d < NQ; d++) {
             const int si = i - cx_of(d), sj = j - cy_of(d), sk = k - cz_of(d);
             const bool in = (unsigned)si < (unsigned)g.nx && (unsigned)sj < (unsigned)g.ny && (unsigned)sk < (unsigned)g.nz;
-            const long long src = in ? ((long long)si * g.ny + sj) * g.kp + sk : ((long long)i * g.ny + j) * g.kp + k;
+            const long long src = in ? g.at(si, sj, sk) : g.at(i, j, k);
             q[d] = ld_state<S>(A.p[d], src) + (Storage<S>::deviation ? (is_face(d) ? p.wface : p.wedge) : 0.f);
         }
         if (near_box) {   // residual box: the exact deviations
@@ -117,7 +117,7 @@ __device__ __forceinline__ void cell_moments4(const Planes& A, int mode, int eve
         const int s = even ? d : (d ^ 1);
         const int sg = even ? -1 : 1;
         const bool oi = sg * cx_of(s) > 0, oj = sg * cy_of(s) > 0, ok = sg * cz_of(s) > 0;
-        q[d] = ld_state<S>(A.p[s], ((long long)(oi ? i1 : i) * g.ny + (oj ? j1 : j)) * g.kp + (ok ? k1 : k)) +
+        q[d] = ld_state<S>(A.p[s], g.at(oi ? i1 : i, oj ? j1 : j, ok ? k1 : k)) +
                (mode == 2 && Storage<S>::deviation ? (is_face(d) ? p.wface : p.wedge) : 0.f);
     }
     if (mode == 2 && near_box) {   // residual box: the exact deviations
@@ -155,43 +155,93 @@ __global__ void k_ibm_prepare(IbmArgs a, float* __restrict__ prep) {
 }
 
 // Per pass: rho and momentum of every unique stencil cell of the first
-// segment (cells sorted by row, so neighbouring threads pull neighbouring
-// cells), and the F each cell starts the pass with (zero unless the previous
+// segment, and the F each cell starts the pass with (zero unless the previous
 // pass touched it, Forcing.hpp:162-174).
 template <typename S>
-__device__ __forceinline__ void ibm_cell(const IbmArgs& a, int c) {
+__device__ __forceinline__ void ibm_cell(const IbmArgs& a, int e, float4& m, float4& f) {
     const Dims& g = a.g;
-    const int e = a.cell_e[c];
-    const int row = e / g.kp;
-    const int k = e - row * g.kp;
-    const int i = row / g.ny;
-    const int j = row - i * g.ny;
+    const int row = e / g.jp;
+    const int j = e - row * g.jp;
+    const int i = row / g.nz;
+    const int k = row - i * g.nz;
     float m4[4];
     cell_moments4<S>(a.A, a.state_mode, a.even, g, i, j, k, a.p, m4, a.rbox);
+    m = make_float4(m4[0], m4[1], m4[2], m4[3]);
+    const bool live = (a.mask_old[(long long)row * g.jw + (j >> 5)] >> (j & 31)) & 1u;
+    f = live ? a.F4[e] : make_float4(0.f, 0.f, 0.f, 0.f);
+}
+__device__ __forceinline__ void put_cell(const IbmArgs& a, int c, const float4 m, const float4 f) {
     const long long C = a.ncell;
-    reinterpret_cast<float4*>(a.cell_m)[c] = make_float4(m4[0], m4[1], m4[2], m4[3]);
-    const bool live = (a.mask_old[(long long)row * g.kw + (k >> 5)] >> (k & 31)) & 1u;
-    const float4 f = live ? a.F4[e] : make_float4(0.f, 0.f, 0.f, 0.f);
+    reinterpret_cast<float4*>(a.cell_m)[c] = m;
     a.cell_F[c] = f.x;
     a.cell_F[C + c] = f.y;
     a.cell_F[2 * C + c] = f.z;
 }
 
-// Cells [first, first + count) of a.cell_order (of the cell list itself
-// when there is no order).
-// copy_mask: the launch also starts mask_new as the first segment's touched
-// flags (mask_static, a multiple of 16 bytes), so that the pass needs no
-// separate copy.
+// The cells of one plane in list order: the big planes (an impeller disk),
+// whose cells fill an (i, k) area of a single j.
 template <typename S>
-__global__ void __launch_bounds__(256) k_ibm_cells(IbmArgs a, int first, int count, int copy_mask) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+__global__ void __launch_bounds__(256) k_ibm_cells_big(IbmArgs a, const int* __restrict__ planes) {
+    const int j = planes[blockIdx.y];
+    const int c = a.plane_cell[j] + (int)(blockIdx.x * blockDim.x + threadIdx.x);
+    if (c >= a.plane_cell[j + 1]) return;
+    float4 m, f;
+    ibm_cell<S>(a, a.cell_e[c], m, f);
+    put_cell(a, c, m, f);
+}
+
+// The cells of 32 consecutive planes, 8 list places of each: place p of plane
+// j is cell plane_cell[j] + p, the places sorted by (i, k). The markers of a
+// tank repeat from plane to plane, so place p is the same (i, k) in
+// neighbouring planes and lanes that run over the planes read whole lines of
+// every population row; a tile in shared memory then turns the results round
+// so that lanes running over the places write the lists (128 bytes of a list
+// per plane). Any list is right; one that does not repeat reads a sector per
+// cell and row. Bound by DRAM bytes: 72 populations + 16 F + 4 index + 28
+// written per cell. Planes with more than skip_above cells belong to
+// k_ibm_cells_big. copy: the launch's threads also start mask_new as the
+// first segment's touched flags (mask_static, a multiple of 16 bytes), so
+// that the pass needs no separate copy.
+constexpr int kCellPlaces = 8;
+struct CellTile {
+    int e[32][kCellPlaces + 1];
+    float4 m[kCellPlaces][33];
+    float4 f[kCellPlaces][33];
+};
+template <typename S>
+__device__ __forceinline__ void ibm_cell_tile(const IbmArgs& a, CellTile& sm, int j0, int p0, int skip_above) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    {
+        const int jj = threadIdx.x / kCellPlaces, p = threadIdx.x % kCellPlaces;
+        int e = -1;
+        if (j0 + jj < a.g.ny) {
+            const int c0 = a.plane_cell[j0 + jj], nc = a.plane_cell[j0 + jj + 1] - c0;
+            if (nc <= skip_above && p0 + p < nc) e = a.cell_e[c0 + p0 + p];
+        }
+        sm.e[jj][p] = e;
+    }
+    __syncthreads();
+    const int e = sm.e[lane][warp];
+    if (e >= 0) {
+        float4 m, f;
+        ibm_cell<S>(a, e, m, f);
+        sm.m[warp][lane] = m;
+        sm.f[warp][lane] = f;
+    }
+    __syncthreads();
+    const int jj = threadIdx.x / kCellPlaces, p = threadIdx.x % kCellPlaces;
+    if (sm.e[jj][p] >= 0) put_cell(a, a.plane_cell[j0 + jj] + p0 + p, sm.m[p][jj], sm.f[p][jj]);
+}
+template <typename S>
+__global__ void __launch_bounds__(32 * kCellPlaces) k_ibm_cells(IbmArgs a, int skip_above, int copy_mask) {
+    __shared__ CellTile sm;
     if (copy_mask) {
         const long long n4 = (long long)(a.mask_bytes / 16);
-        for (long long w = t; w < n4; w += (long long)gridDim.x * blockDim.x)
+        const long long t = ((long long)blockIdx.y * gridDim.x + blockIdx.x) * blockDim.x + threadIdx.x;
+        for (long long w = t; w < n4; w += (long long)gridDim.x * gridDim.y * blockDim.x)
             reinterpret_cast<uint4*>(a.mask_new)[w] = reinterpret_cast<const uint4*>(a.mask_static)[w];
     }
-    if (t >= count) return;
-    ibm_cell<S>(a, a.cell_order ? a.cell_order[first + t] : first + t);
+    ibm_cell_tile<S>(a, sm, (int)blockIdx.x * 32, (int)blockIdx.y * kCellPlaces, skip_above);
 }
 
 // Second segment (the blades): weights and the moments of the 9 stencil
@@ -371,10 +421,8 @@ __device__ __noinline__ void blade_levels_global(const IbmArgs& a, int j, const 
                 const float w = s[(TF_W + c) * cap + t];
                 const int packed = __float_as_int(s[(TF_CELL + c) * cap + t]);
                 const int i2 = packed >> 16, k2 = packed & 0xffff;
-                const long long row = (long long)i2 * g.ny + j;
-                const long long e = row * g.kp + k2;
-                const long long wd = row * g.kw + (k2 >> 5);
-                const uint32_t bit = 1u << (k2 & 31);
+                const long long e = g.at(i2, j, k2), wd = g.word(i2, j, k2);
+                const uint32_t bit = 1u << (j & 31);
                 const bool live = (__ldcg(a.mask_new + wd) & bit) || (a.mask_old[wd] & bit);
                 const float4 v = live ? __ldcg(a.F4 + e) : make_float4(0.f, 0.f, 0.f, 0.f);
                 const float vx = v.x, vy = v.y, vz = v.z;
@@ -393,10 +441,8 @@ __device__ __noinline__ void blade_levels_global(const IbmArgs& a, int j, const 
             for (int c = 0; c < 9; c++) {
                 const int packed = __float_as_int(s[(TF_CELL + c) * cap + t]);
                 const int i2 = packed >> 16, k2 = packed & 0xffff;
-                const long long row = (long long)i2 * g.ny + j;
-                const long long e = row * g.kp + k2;
-                const long long wd = row * g.kw + (k2 >> 5);
-                const uint32_t bit = 1u << (k2 & 31);
+                const long long e = g.at(i2, j, k2), wd = g.word(i2, j, k2);
+                const uint32_t bit = 1u << (j & 31);
                 const bool live = (__ldcg(a.mask_new + wd) & bit) || (a.mask_old[wd] & bit);
                 const float4 v = live ? __ldcg(a.F4 + e) : make_float4(0.f, 0.f, 0.f, 0.f);
                 const float bw = a.beta * s[(TF_W + c) * cap + t];
@@ -477,10 +523,8 @@ __device__ __forceinline__ bool blade_levels_tile(const IbmArgs& a, int j, float
             const int h = h0 + u * THREADS;
             const int key = h < H ? keys[h] : -1;
             const int i2 = key >> 16, k2 = key & 0xffff;
-            const long long row = (long long)i2 * g.ny + j;
-            const long long e = row * g.kp + k2;
-            const long long wd = row * g.kw + (k2 >> 5);
-            const uint32_t bit = 1u << (k2 & 31);
+            const long long e = g.at(i2, j, k2), wd = g.word(i2, j, k2);
+            const uint32_t bit = 1u << (j & 31);
             live[u] = false;
             vx[u] = vy[u] = vz[u] = 0.f;
             if (key >= 0) {
@@ -553,10 +597,8 @@ __device__ __forceinline__ bool blade_levels_tile(const IbmArgs& a, int j, float
         const int key = keys[h];
         if (key < 0) continue;
         const int i2 = key >> 16, k2 = key & 0xffff;
-        const long long row = (long long)i2 * g.ny + j;
-        const long long e = row * g.kp + k2;
-        a.F4[e] = make_float4(hx[h], hy[h], hz[h], 0.f);
-        atomicOr(&a.mask_new[row * g.kw + (k2 >> 5)], 1u << (k2 & 31));
+        a.F4[g.at(i2, j, k2)] = make_float4(hx[h], hy[h], hz[h], 0.f);
+        atomicOr(&a.mask_new[g.word(i2, j, k2)], 1u << (j & 31));
     }
     return true;
 }
@@ -863,17 +905,16 @@ template <typename S>
 __global__ void __launch_bounds__(256) k_reduce_fp64(IbmArgs a, const uint32_t* __restrict__ mask, double* partial) {
     __shared__ double red[4][256];
     const Dims g = a.g;
-    const long long total = g.rows() * g.nz;
+    const long long total = g.cells();
     double acc[4] = {0, 0, 0, 0};
     for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < total;
          t += (long long)gridDim.x * blockDim.x) {
-        const int k = (int)(t % g.nz);
-        const long long row = t / g.nz;
-        const int j = (int)(row % g.ny), i = (int)(row / g.ny);
+        int i, j, k;
+        g.cell(t, i, j, k);
         float m4[4];
         cell_moments4<S>(a.A, a.state_mode, a.even, g, i, j, k, a.p, m4, a.rbox);
-        const long long e = row * g.kp + k;
-        const bool on = (mask[row * g.kw + (k >> 5)] >> (k & 31)) & 1u;
+        const long long e = g.at(i, j, k);
+        const bool on = (mask[g.word(i, j, k)] >> (j & 31)) & 1u;
         acc[0] += m4[0];
         const float4 f = on ? a.F4[e] : make_float4(0.f, 0.f, 0.f, 0.f);
         acc[1] += (double)m4[1] + (on ? 0.5 * (double)f.x : 0.0);
@@ -1014,12 +1055,20 @@ cudaError_t launch_ibm_prepare(const IbmArgs& a, float* prep, const int* mcell, 
 
 cudaError_t launch_ibm(const IbmArgs& a, cudaStream_t st) {
     bool mask_copied = false;
-    auto cells = [&](int first, int count, bool copy_mask, cudaStream_t cs) {
-        if (count <= 0) return;
+    auto cells_small = [&](cudaStream_t cs) {
+        if (a.max_cells <= 0) return;
+        const dim3 grid((unsigned)((a.g.ny + 31) / 32), (unsigned)((a.max_cells + kCellPlaces - 1) / kCellPlaces));
         with_storage(a.storage, [&](auto s) {
-            k_ibm_cells<decltype(s)><<<(count + 255) / 256, 256, 0, cs>>>(a, first, count, copy_mask ? 1 : 0);
+            k_ibm_cells<decltype(s)><<<grid, 32 * kCellPlaces, 0, cs>>>(a, a.smem_cells, 1);
         });
-        mask_copied |= copy_mask;
+        mask_copied = true;
+    };
+    auto cells_big = [&](cudaStream_t cs) {
+        if (a.n_big <= 0) return;
+        const dim3 grid((unsigned)((a.max_big + 255) / 256), (unsigned)a.n_big);
+        with_storage(a.storage, [&](auto s) {
+            k_ibm_cells_big<decltype(s)><<<grid, 256, 0, cs>>>(a, a.plane_list + a.n_small);
+        });
     };
     auto tail = [&](cudaStream_t ts) {
         if (a.n <= a.n0) return;
@@ -1027,7 +1076,7 @@ cudaError_t launch_ibm(const IbmArgs& a, cudaStream_t st) {
         with_storage(a.storage, [&](auto s) { k_ibm_gather_tail<decltype(s)><<<b, 128, 0, ts>>>(a); });
     };
     // mask_new starts as the first segment's (static) touched cells: copied
-    // by the (largest) cells launch, else by a copy; only the blade walk
+    // by the ordinary planes' cells launch, else by a copy; only the blade walk
     // reads or sets mask_new, at the end of the pass.
     // Side stream: the blade markers' gather (which reads only the state and
     // is needed only by the blade walk) and the planes with many cells (an
@@ -1036,13 +1085,11 @@ cudaError_t launch_ibm(const IbmArgs& a, cudaStream_t st) {
     // blocks over the SMs. Handle's stream: the other planes' cells and
     // spread, then, after the side stream, the blade walk.
     cudaError_t err = cudaSuccess;
-    const bool split = a.n_big > 0 && a.cell_order != nullptr;
-    if (!split) cells(0, a.ncell, true, st);   // (before the fork: a big planes' spread reads them)
     err = cudaEventRecord(a.ev_fork, st);
     if (err != cudaSuccess) return err;
     err = cudaStreamWaitEvent(a.side, a.ev_fork, 0);
     if (err != cudaSuccess) return err;
-    if (split) cells(0, a.ncell_big, false, a.side);
+    cells_big(a.side);
     tail(a.side);
     if (a.n_big > 0) {
         k_ibm_spread_bulk<512, 1, false><<<a.n_big, 512, big_bulk_bytes(a.big_tile_cells), a.side>>>(
@@ -1052,7 +1099,7 @@ cudaError_t launch_ibm(const IbmArgs& a, cudaStream_t st) {
     }
     err = cudaEventRecord(a.ev_join, a.side);
     if (err != cudaSuccess) return err;
-    if (split) cells(a.ncell_big, a.ncell - a.ncell_big, true, st);
+    cells_small(st);
     if (!mask_copied) {
         err = cudaMemcpyAsync(a.mask_new, a.mask_static, a.mask_bytes, cudaMemcpyDeviceToDevice, st);
         if (err != cudaSuccess) return err;
@@ -1095,11 +1142,11 @@ __device__ __forceinline__ void stage_args(IbmArgs& dst, const IbmArgs* src) {
 template <typename S>
 __global__ void __launch_bounds__(256) k_ibm_cells_batch(const IbmArgs* __restrict__ args, const int2* __restrict__ work) {
     __shared__ IbmArgs sa;
+    __shared__ CellTile sm;
     const int2 w = work[blockIdx.x];
     stage_args<256>(sa, args + w.x);
     __syncthreads();
-    const int c = w.y + threadIdx.x;
-    if (c < sa.ncell) ibm_cell<S>(sa, c);
+    ibm_cell_tile<S>(sa, sm, (w.y & 0x3ff) * 32, (w.y >> 10) * kCellPlaces, 0x7fffffff);
 }
 
 template <typename S>

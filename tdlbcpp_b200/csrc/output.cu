@@ -64,8 +64,7 @@ __global__ void __launch_bounds__(256) k_vorticity(Planes A, Dims g, int mode, i
         k = cut;
         o = (long long)j * g.nx + i;
     }
-    const long long row = (long long)i * g.ny + j;
-    if (excl && ((excl[row * g.kw + (k >> 5)] >> (k & 31)) & 1u)) {
+    if (excl && ((excl[g.word(i, j, k)] >> (j & 31)) & 1u)) {
         out[o] = -1.f;
         return;
     }
@@ -101,8 +100,7 @@ __global__ void __launch_bounds__(256) k_plane_xz(Planes A, Dims g, int mode, in
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= (long long)g.nx * g.nz) return;
     const int i = (int)(t / g.nz), k = (int)(t - (long long)(t / g.nz) * g.nz);
-    const long long row = (long long)i * g.ny + j;
-    const long long e = row * g.kp + k;
+    const long long e = g.at(i, j, k);
     float* o = out + t * 8;
     float m[NQ];
     if (!esotwist) {
@@ -121,12 +119,12 @@ __global__ void __launch_bounds__(256) k_plane_xz(Planes A, Dims g, int mode, in
             o[s] = m[d];
         }
     }
-    const bool on = (mask[row * g.kw + (k >> 5)] >> (k & 31)) & 1u;
+    const bool on = (mask[g.word(i, j, k)] >> (j & 31)) & 1u;
     const float4 v = F[e];
     o[4] = on ? v.x : 0.f;
     o[5] = on ? v.y : 0.f;
     o[6] = on ? v.z : 0.f;
-    o[7] = excl && ((excl[row * g.kw + (k >> 5)] >> (k & 31)) & 1u) ? 1.f : 0.f;
+    o[7] = excl && ((excl[g.word(i, j, k)] >> (j & 31)) & 1u) ? 1.f : 0.f;
 }
 
 }  // namespace tdlb
@@ -149,8 +147,7 @@ int oguard(tdlb_lattice* h, F&& fn) {
     if (!h) return TDLB_EINVAL;
     try {
         cudaSetDevice(h->device);
-        const cudaError_t je = tdlb_rt::join_side(h);   // after every queued step and forcing pass
-        if (je != cudaSuccess) throw OFail{TDLB_ECUDA, std::string("join: ") + cudaGetErrorString(je)};
+        tdlb_rt::fence(h);
         fn();
         return TDLB_OK;
     } catch (const OFail& f) {
@@ -191,11 +188,10 @@ int tdlb_set_output_exclude(tdlb_handle h, const tdlb_marker* markers, size_t n,
                 throw OFail{TDLB_EINVAL, "marker " + std::to_string(q) + " outside the interior"};
         if (h->h_exclude.empty()) h->h_exclude.assign((size_t)h->mask_words, 0u);
         for (size_t q = 0; q < n; q++) {
-            const long long row = markers[q].i * g.ny + markers[q].j;
-            const int k = (int)markers[q].k;
-            uint32_t& w = h->h_exclude[(size_t)(row * g.kw + (k >> 5))];
-            if (exclude) w |= 1u << (k & 31);
-            else w &= ~(1u << (k & 31));
+            const int j = (int)markers[q].j;
+            uint32_t& w = h->h_exclude[(size_t)g.word((int)markers[q].i, j, (int)markers[q].k)];
+            if (exclude) w |= 1u << (j & 31);
+            else w &= ~(1u << (j & 31));
         }
         if (!h->d_exclude) TDLB_OCK(cudaMalloc(&h->d_exclude, (size_t)h->mask_words * sizeof(uint32_t)));
         TDLB_OCK(cudaMemcpyAsync(h->d_exclude, h->h_exclude.data(), h->h_exclude.size() * sizeof(uint32_t),

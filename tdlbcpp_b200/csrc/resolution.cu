@@ -27,25 +27,24 @@ __global__ void __launch_bounds__(256) k_double_resolution(Planes A, Dims g, int
                                                            const float* __restrict__ nu_old, Planes N, Dims h,
                                                            float* __restrict__ nu_new, int esotwist) {
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= h.rows() * h.nz) return;
-    const int k = (int)(t % h.nz);
-    const long long row = t / h.nz;
-    const int j = (int)(row % h.ny);
-    const int i = (int)(row / h.ny);
+    if (t >= h.cells()) return;
+    int i, j, k;
+    h.cell(t, i, j, k);
+    const long long e = h.at(i, j, k);
     const int pi = i >> 1, pj = j >> 1, pk = k >> 1;
     float m[NQ];
     state_moments18<float>(A, g, mode, even, p, pi, pj, pk, m);
-    nu_new[row * h.kp + k] = nu_old[((long long)pi * g.ny + pj) * g.kp + pk];
+    nu_new[e] = nu_old[g.at(pi, pj, pk)];
     if (!esotwist) {
 #pragma unroll
-        for (int d = 0; d < NQ; d++) N.p[d][row * h.kp + k] = m[d];
+        for (int d = 0; d < NQ; d++) N.p[d][e] = m[d];
         return;
     }
     const int i1 = i + 1 == h.nx ? 0 : i + 1, j1 = j + 1 == h.ny ? 0 : j + 1, k1 = k + 1 == h.nz ? 0 : k + 1;
 #pragma unroll
     for (int d = 0; d < NQ; d++) {
-        const long long li = cx_of(d) < 0 ? i1 : i, lj = cy_of(d) < 0 ? j1 : j, lk = cz_of(d) < 0 ? k1 : k;
-        N.p[even ? d : (d ^ 1)][(li * h.ny + lj) * h.kp + lk] = m[d];
+        const int li = cx_of(d) < 0 ? i1 : i, lj = cy_of(d) < 0 ? j1 : j, lk = cz_of(d) < 0 ? k1 : k;
+        N.p[even ? d : (d ^ 1)][h.at(li, lj, lk)] = m[d];
     }
 }
 
@@ -86,7 +85,7 @@ int tdlb_double_resolution(tdlb_handle h) {
     uint32_t* mask = nullptr;
     try {
         cudaSetDevice(h->device);
-        TDLB_RCK(tdlb_rt::join_side(h));
+        tdlb_rt::fence(h);
         TDLB_RCK(cudaStreamSynchronize(h->stream));   // the old buffers are freed below
         if (!h->initialised) throw RFail{TDLB_ESTATE, "not initialised (tdlb_initialise)"};
         if (h->own_stream) throw RFail{TDLB_ESTATE, "a tank of a batch cannot change size"};
@@ -95,9 +94,9 @@ int tdlb_double_resolution(tdlb_handle h) {
         if ((long long)g.nx * 2 > 32767 || (long long)g.ny * 2 > 32767 || (long long)g.nz * 2 > 32767)
             throw RFail{TDLB_EINVAL, "doubled grid extent above 32767"};
         const Dims n = tdlb::make_dims(g.nx * 2, g.ny * 2, g.nz * 2);
-        if ((long long)n.nx * n.ny * n.kp >= (1LL << 31) - 64)
+        if (n.rows() * n.jp >= tdlb::kMaxPlane)
             throw RFail{TDLB_EINVAL, "doubled lattice too large: one plane must stay below 2^31 elements"};
-        const long long words = round_up_ll((long long)n.nx * n.ny * n.kw, 64);
+        const long long words = round_up_ll(n.rows() * n.jw, 64);
         const bool simple = h->cfg.streaming == TDLB_STREAMING_SIMPLE;
         const size_t pop = (size_t)tdlb::NQ * n.plane * sizeof(float);
         size_t free_b = 0, total_b = 0;
@@ -118,7 +117,7 @@ int tdlb_double_resolution(tdlb_handle h) {
         TDLB_RCK(cudaMemsetAsync(mask, 0, (size_t)2 * words * sizeof(uint32_t), h->stream));
         Planes dst;
         for (int d = 0; d < tdlb::NQ; d++) dst.p[d] = A + (size_t)d * n.plane;
-        const long long cells = n.rows() * n.nz;
+        const long long cells = n.cells();
         tdlb::k_double_resolution<<<(unsigned)((cells + 255) / 256), 256, 0, h->stream>>>(
             h->planes(h->state_buf()), g, h->state_mode(), h->even ? 1 : 0, h->cp, h->Nu, dst, n, Nu, simple ? 0 : 1);
         TDLB_RCK(cudaGetLastError());
@@ -137,7 +136,7 @@ int tdlb_double_resolution(tdlb_handle h) {
     h->mask = mask;
     Dims& g = h->g;
     g = tdlb::make_dims(g.nx * 2, g.ny * 2, g.nz * 2);
-    h->mask_words = round_up_ll((long long)g.nx * g.ny * g.kw, 64);
+    h->mask_words = round_up_ll(g.rows() * g.jw, 64);
     h->cfg.x *= 2;
     h->cfg.y *= 2;
     h->cfg.z *= 2;
@@ -156,8 +155,7 @@ int tdlb_double_resolution(tdlb_handle h) {
     drop(h->d_plane_lv1);
     drop(h->d_plane_cell);
     drop(h->d_plane_list);
-    drop(h->d_cell_order);
-    h->ncell_big = 0;
+    h->max_cells = h->max_big = 0;
     drop(h->d_mask_static);
     drop(h->d_exclude);
     h->h_exclude.clear();
@@ -165,7 +163,7 @@ int tdlb_double_resolution(tdlb_handle h) {
     drop(h->d_rot_xz);
     h->marker_gen++;
     h->resident = false;
-    h->inner_queued = false;
+    tdlb_rt::drop_zone(h);
     h->h_rot_xz.clear();
     return TDLB_OK;
 }

@@ -48,10 +48,10 @@ __global__ void k_fill_uniform_moments(Planes Q, Dims g, float rho) {
 // ---------------------------------------------------------------------------
 static inline unsigned blocks_for(long long n, int threads) { return (unsigned)((n + threads - 1) / threads); }
 
-// Grid of a launch: every quad (part 0) or one warp per listed chunk (1, 2).
+// Grid of a launch: every quad (parts 0 and 1) or those of the listed words.
 static inline unsigned step_blocks(const StepArgs& a, int V) {
-    if (a.part != 0) return blocks_for((long long)a.zone.count * 32, 128);
-    return blocks_for(a.g.rows() * (a.g.kp / V), 128);
+    if (a.part == 2) return blocks_for((long long)a.zone.count * (32 / V), 128);
+    return blocks_for(a.g.rows() * (a.g.jp / V), 128);
 }
 
 template <int V>
@@ -60,7 +60,7 @@ static cudaError_t launch_simple_v(const StepArgs& a, cudaStream_t st) {
 #define TDLB_SIMPLE(LES, FM, COL, PART)                                                                       \
     k_step_simple<float, V, LES, FM, COL, PART><<<grid, block, 0, st>>>(                                   \
         a.A, a.B, a.Nu, a.F, a.mask, a.g, a.p,                                                               \
-        launch_walk<k_step_simple<float, V, LES, FM, COL, PART>, COL && !FM>(a), ResidualBox{}, BoxOut{})
+        launch_walk<k_step_simple<float, V, LES, FM, COL, PART>, COL && !FM>(a))
     if (!a.collide) TDLB_SIMPLE(false, false, false, 0);
     else if (a.from_moments) { if (a.les) TDLB_SIMPLE(true, true, true, 0); else TDLB_SIMPLE(false, true, true, 0); }
     else if constexpr (V == 1) {
@@ -84,12 +84,10 @@ template <int V, bool LES, bool FM, bool COL, int PART>
 static void eso_launch(const StepArgs& a, dim3 grid, cudaStream_t st) {
     if (a.even)
         k_step_esotwist<float, V, LES, FM, COL, true, PART><<<grid, 128, 0, st>>>(
-            a.A, a.Nu, a.F, a.mask, a.g, a.p, launch_walk<k_step_esotwist<float, V, LES, FM, COL, true, PART>, COL && !FM>(a),
-            ResidualBox{}, BoxOut{});
+            a.A, a.Nu, a.F, a.mask, a.g, a.p, launch_walk<k_step_esotwist<float, V, LES, FM, COL, true, PART>, COL && !FM>(a));
     else
         k_step_esotwist<float, V, LES, FM, COL, false, PART><<<grid, 128, 0, st>>>(
-            a.A, a.Nu, a.F, a.mask, a.g, a.p, launch_walk<k_step_esotwist<float, V, LES, FM, COL, false, PART>, COL && !FM>(a),
-            ResidualBox{}, BoxOut{});
+            a.A, a.Nu, a.F, a.mask, a.g, a.p, launch_walk<k_step_esotwist<float, V, LES, FM, COL, false, PART>, COL && !FM>(a));
 }
 
 template <int V>
@@ -115,9 +113,9 @@ static cudaError_t launch_esotwist_v(const StepArgs& a, cudaStream_t st) {
 }
 
 cudaError_t launch_step_simple(const StepArgs& a, cudaStream_t st) {
-    if (a.part != 0 && (a.vec != 1 || a.from_moments || !a.collide)) return cudaErrorInvalidValue;
+    if (a.part != 0 && (a.from_moments || !a.collide)) return cudaErrorInvalidValue;
     if (a.storage != STORE_F32) return launch_step_simple_h16(a, st);
-    if (a.box != 0) return cudaErrorInvalidValue;   // no residual box for FP32 storage
+    if (a.part != 0 && a.vec != 1) return cudaErrorInvalidValue;   // (FP32 parts are built for one cell per thread)
     switch (a.vec) {
         case 1: return launch_simple_v<1>(a, st);
         case 2: return launch_simple_v<2>(a, st);
@@ -126,9 +124,9 @@ cudaError_t launch_step_simple(const StepArgs& a, cudaStream_t st) {
 }
 
 cudaError_t launch_step_esotwist(const StepArgs& a, cudaStream_t st) {
-    if (a.part != 0 && (a.vec != 1 || a.from_moments || !a.collide)) return cudaErrorInvalidValue;
+    if (a.part != 0 && (a.from_moments || !a.collide)) return cudaErrorInvalidValue;
     if (a.storage != STORE_F32) return launch_step_esotwist_h16(a, st);
-    if (a.box != 0) return cudaErrorInvalidValue;   // no residual box for FP32 storage
+    if (a.part != 0 && a.vec != 1) return cudaErrorInvalidValue;
     switch (a.vec) {
         case 1: return launch_esotwist_v<1>(a, st);
         case 2: return launch_esotwist_v<2>(a, st);
@@ -143,7 +141,7 @@ cudaError_t launch_fill_uniform_moments(Planes Q, const Dims& g, float rho, cuda
 
 cudaError_t launch_state_moments(Planes A, Planes M, const Dims& g, int mode, int even, cudaStream_t st, int storage,
                                  const CollideParams& p, const ResidualBox& rb) {
-    const unsigned blocks = blocks_for(g.rows() * g.nz, 256);
+    const unsigned blocks = blocks_for(g.cells(), 256);
     with_storage(storage, [&](auto s) {
         k_state_moments<decltype(s)><<<blocks, 256, 0, st>>>(A, M, g, mode, even, p, rb);
     });

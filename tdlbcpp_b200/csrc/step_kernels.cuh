@@ -11,8 +11,8 @@
 namespace tdlb {
 
 // ---------------------------------------------------------------------------
-// Thread mapping shared by both schemes: V consecutive cells of one row per
-// thread ("quad"), quads numbered row-major over (row, kq); a warp covers 32
+// Thread mapping shared by both schemes: V consecutive cells (along j) of one
+// row per thread ("quad"), quads numbered row-major over (row, jq); a warp covers 32
 // consecutive quads, so neighbouring lanes hold neighbouring cells of the
 // same row except at row ends (where the wall rule or the periodic wrap
 // applies anyway). V in {1, 2, 4}; populations move as float/float2/float4.
@@ -140,39 +140,70 @@ __device__ __forceinline__ float rest_of(int d, const CollideParams& p) {
 }
 
 struct Quad {
-    int i, j, k0;     // cell (i, j, k0 .. k0+V-1)
-    int row;          // i*ny + j
-    int e0;           // element index of (row, k0)
-    bool active;      // k0 < nz (the quad holds at least one cell)
+    int i, k, j0;     // cells (i, j0 .. j0+V-1, k)
+    int row;          // i*nz + k
+    int e0;           // element index of (row, j0)
+    bool active;      // j0 < ny (the quad holds at least one cell)
 };
 
-// MUL_DIV: divide by multiply-high (Dims::by_kp16, by_ny). Measured on B200
+// MUL_DIV: divide by multiply-high (Dims::by_nq, by_nz). Measured on B200
 // at 400^3: 5 % faster for the 16-bit kernels (issue-bound), but 4-11 %
 // slower for the FP32 ones, whose loads the compiler then schedules worse;
 // the FP32 kernels keep the hardware division sequence.
 template <int V, bool MUL_DIV>
 __device__ __forceinline__ Quad quad_of(const Dims& g, int nq, unsigned t) {
     Quad q;
-    const unsigned total = (unsigned)g.nx * (unsigned)g.ny * (unsigned)nq;
+    const unsigned total = (unsigned)g.nx * (unsigned)g.nz * (unsigned)nq;
     const unsigned tc = t < total ? t : total - 1;   // keep spare lanes on a valid quad
-    // tc / nq = (tc / (16 / V)) / (kp / 16), nq = kp / V
-    constexpr unsigned kShift = V == 1 ? 4 : V == 2 ? 3 : V == 4 ? 2 : 1;
-    static_assert(V == 1 || V == 2 || V == 4 || V == 8, "cells per thread");
+    static_assert(V == 1 || V == 2 || V == 4, "cells per thread");
     unsigned row;
     if (MUL_DIV) {
-        row = g.by_kp16.div(tc >> kShift);
-        q.i = (int)g.by_ny.div(row);
+        row = g.by_nq[V >> 1].div(tc);   // V = 1, 2, 4: entries 0, 1, 2
+        q.i = (int)g.by_nz.div(row);
     } else {
         row = tc / (unsigned)nq;
-        q.i = (int)(row / (unsigned)g.ny);
+        q.i = (int)(row / (unsigned)g.nz);
     }
-    const int kq = (int)(tc - row * (unsigned)nq);
+    const int jq = (int)(tc - row * (unsigned)nq);
     q.row = (int)row;
-    q.j = (int)row - q.i * g.ny;
-    q.k0 = kq * V;
-    q.e0 = (int)row * g.kp + q.k0;
-    q.active = t < total && q.k0 < g.nz;
+    q.k = (int)row - q.i * g.nz;
+    q.j0 = jq * V;
+    q.e0 = (int)row * g.jp + q.j0;
+    q.active = t < total && q.j0 < g.ny;
     return q;
+}
+
+// The quad of thread t of a launch (StepPart) and, per cell, whether this launch
+// stores it (ok, V bits). PART 2: SEG = 32 / V consecutive lanes share a word of
+// the list; lanes past the row's end take its last quad, inactive.
+template <int V, bool MUL_DIV, int PART>
+__device__ __forceinline__ Quad part_quad(const Dims& g, const StepPart& part, unsigned t, unsigned& ok) {
+    constexpr unsigned ALL = (1u << V) - 1u;
+    if constexpr (PART != 2) {
+        const Quad q = quad_of<V, MUL_DIV>(g, g.jp / V, t);
+        ok = q.active ? ALL : 0u;
+        if constexpr (PART == 1)
+            if (__ldg(part.skip + (size_t)q.row * g.jw + (q.j0 >> 5))) ok = 0u;
+        return q;
+    } else {
+        constexpr unsigned SEG = 32 / V;
+        const unsigned lw = t / SEG;
+        const int wd = __ldg(part.words + min(lw, (unsigned)part.count - 1u));
+        const unsigned ex = part.except ? __ldg(part.except + wd) : 0u;
+        Quad q;
+        q.row = wd / g.jw;
+        const int j = (wd - q.row * g.jw) * 32 + (int)(t % SEG) * V;
+        q.i = q.row / g.nz;
+        q.k = q.row - q.i * g.nz;
+        q.j0 = min(j, g.jp - V);
+        q.e0 = q.row * g.jp + q.j0;
+        q.active = lw < (unsigned)part.count && j < g.ny;
+        unsigned live = 0u;
+#pragma unroll
+        for (int e = 0; e < V; e++) live |= j + e < g.ny ? 1u << e : 0u;
+        ok = q.active ? live & ~(ex >> (j & 31)) : 0u;
+        return q;
+    }
 }
 
 // FORCE = false: the cells are known to lie outside every immersed-boundary
@@ -185,7 +216,7 @@ __device__ __forceinline__ void collide_quad(float (&f)[NQ][V], const Quad& q, f
     if (!COLLIDE) return;
     float fx[V], fy[V], fz[V];
     const uint32_t bits =
-        FORCE ? (__ldg(mask + (size_t)q.row * g.kw + (q.k0 >> 5)) >> (q.k0 & 31)) & ((1u << V) - 1u) : 0u;
+        FORCE ? (__ldg(mask + (size_t)q.row * g.jw + (q.j0 >> 5)) >> (q.j0 & 31)) & ((1u << V) - 1u) : 0u;
     if (bits) {
 #pragma unroll
         for (int e = 0; e < V; e++) {
@@ -245,18 +276,12 @@ __device__ __forceinline__ void collide_quad(float (&f)[NQ][V], const Quad& q, f
 }
 
 // ---------------------------------------------------------------------------
-// Residual box (16-bit storage, one cell per thread; tdlb::ResidualBox).
-// A step with a box runs three launches:
-//   the box launch (BOX = 2): the 32-cell chunks with a cell near the box,
-//     from a list, with the residuals of their locations (the code below,
-//     inlined), into a scratch array (BoxOut) -- before the plain launch
-//     overwrites their populations (Esotwist) and their Nu, which the LES
-//     collision reads;
-//   the plain launch: every cell, without residuals;
-//   k_box_commit: the box chunks' exact outputs over the plain ones, with the
-//     residuals of the locations inside the box.
-// The plain kernel so stays as it is. f holds the cell's 18 values in
-// direction order.
+// Residual box (16-bit storage; tdlb::ResidualBox). A step with a box steps the
+// cells of a list with k_box_step: with the residuals of their locations
+// added on reading and kept on writing. The other launches of the step leave
+// those cells out (StepPart::except): a cell's locations are its own alone,
+// so the launches do not meet. f holds the cell's 18 values in direction
+// order.
 // ---------------------------------------------------------------------------
 // Simple: add the residuals of the source locations inside the box (x - c_d,
 // or the cell itself where x - c_d is off the lattice).
@@ -296,44 +321,41 @@ __device__ __forceinline__ void box_read_eso(const ResidualBox& rb, int i, int j
 // All loads of a thread are issued as one straight-line batch (no branch
 // between them), so the 18 population fetches of a quad are in flight
 // together. V = 1 pulls every population directly from x - c_d. V > 1 loads
-// aligned vectors of the upstream rows and moves k-shifted values between
+// aligned vectors of the upstream rows and moves j-shifted values between
 // lanes with shuffles; the values a lane cannot get from a neighbour (warp
 // edges) and the own values the wall rule needs at row ends come from
 // scalar loads issued in the same batch (in bounds for every lane; the ones
 // a lane does not need hit L1).
 // ---------------------------------------------------------------------------
-template <typename S, int V, bool LES, bool FROM_MOMENTS, bool COLLIDE, bool FORCE = true, int BOX = 0>
+template <typename S, int V, bool LES, bool FROM_MOMENTS, bool COLLIDE, int PART = 0>
 __device__ __forceinline__ void simple_quad(const Planes& A, const Planes& B, float* __restrict__ Nu,
                                             const float4* __restrict__ F, const uint32_t* __restrict__ mask,
                                             const Dims& g, const CollideParams& p, unsigned t,
-                                            const ResidualBox rr = ResidualBox{}, const BoxOut out = BoxOut{}) {
+                                            const StepPart& part = StepPart{}) {
     static_assert(!(Storage<S>::deviation && FROM_MOMENTS), "16-bit state always holds populations");
-    static_assert(BOX == 0 || (Storage<S>::deviation && V == 1), "the residual box serves 16-bit storage, one cell per thread");
-    const int nq = g.kp / V;
-    const Quad q = quad_of<V, sizeof(S) == 2>(g, nq, t);
-    const int lane = threadIdx.x & 31;
-    const int rs = g.ny * g.kp;   // elements per i step
-    const bool i_lo = q.i == 0, i_hi = q.i == g.nx - 1, j_lo = q.j == 0, j_hi = q.j == g.ny - 1;
-    const bool k_first = q.k0 == 0, k_last = q.k0 + V >= g.nz;
+    constexpr int SEG = PART == 2 ? 32 / V : 32;   // lanes that hold consecutive quads
+    constexpr unsigned ALL = (1u << V) - 1u;
+    unsigned ok;
+    const Quad q = part_quad<V, sizeof(S) == 2, PART>(g, part, t, ok);
+    const int lane = threadIdx.x & (SEG - 1);
+    const int rs = g.nz * g.jp;   // elements per i step
+    const bool i_lo = q.i == 0, i_hi = q.i == g.nx - 1, k_lo = q.k == 0, k_hi = q.k == g.nz - 1;
+    const bool j_first = q.j0 == 0, j_last = q.j0 + V >= g.ny;
     float f[NQ][V];
     if (FROM_MOMENTS) {
 #pragma unroll
         for (int d = 0; d < NQ; d++) pload<S, V, true>(A.p[d], q.e0, f[d]);
     } else if (V == 1) {
         // direct (unaligned) read-only loads: the texture path serves the
-        // k-shifted rows better here than aligned loads plus lane shuffles
+        // j-shifted rows better here than aligned loads plus lane shuffles
 #pragma unroll
         for (int d = 0; d < NQ; d++) {
             const int cx = cx_of(d), cy = cy_of(d), cz = cz_of(d);
             // upstream cell x - c_d; off the lattice -> the cell keeps its own value
-            const bool in = !((cx > 0 && i_lo) || (cx < 0 && i_hi) || (cy > 0 && j_lo) || (cy < 0 && j_hi) ||
-                              (cz > 0 && k_first) || (cz < 0 && k_last));
-            const int off = in ? -(cx * rs + cy * g.kp + cz) : 0;
+            const bool in = !((cx > 0 && i_lo) || (cx < 0 && i_hi) || (cz > 0 && k_lo) || (cz < 0 && k_hi) ||
+                              (cy > 0 && j_first) || (cy < 0 && j_last));
+            const int off = in ? -(cx * rs + cz * g.jp + cy) : 0;
             f[d][0] = pload1<S, true>(A.p[d], q.e0 + off);
-        }
-        if constexpr (BOX == 2) {
-            // residual box: the exact deviation of every source location inside it
-            if (q.active && rr.near(q.i, q.j, q.k0)) box_pull_simple(rr, q.i, q.j, q.k0, g, f);
         }
     } else {
         float hal[NQ], own[NQ];
@@ -341,40 +363,40 @@ __device__ __forceinline__ void simple_quad(const Planes& A, const Planes& B, fl
 #pragma unroll
         for (int d = 0; d < NQ; d++) {
             const int cx = cx_of(d), cy = cy_of(d), cz = cz_of(d);
-            const bool row_ok = !((cx > 0 && i_lo) || (cx < 0 && i_hi) || (cy > 0 && j_lo) || (cy < 0 && j_hi));
-            const int soff = row_ok ? -(cx * rs + cy * g.kp) : 0;
+            const bool row_ok = !((cx > 0 && i_lo) || (cx < 0 && i_hi) || (cz > 0 && k_lo) || (cz < 0 && k_hi));
+            const int soff = row_ok ? -(cx * rs + cz * g.jp) : 0;
             const int src = q.e0 + soff;
             pload<S, V, true>(A.p[d], src, f[d]);
-            if (cz > 0) {
-                hal[d] = pload1<S, true>(A.p[d], (lane == 0 && !k_first) ? src - 1 : src);
-                own[d] = (cx != 0 || cy != 0) ? pload1<S, true>(A.p[d], q.e0) : 0.f;
-            } else if (cz < 0) {
-                hal[d] = pload1<S, true>(A.p[d], (lane == 31 && !k_last) ? src + V : src);
-                int le = g.nz - 1 - q.k0;
+            if (cy > 0) {
+                hal[d] = pload1<S, true>(A.p[d], (lane == 0 && !j_first) ? src - 1 : src);
+                own[d] = (cx != 0 || cz != 0) ? pload1<S, true>(A.p[d], q.e0) : 0.f;
+            } else if (cy < 0) {
+                hal[d] = pload1<S, true>(A.p[d], (lane == SEG - 1 && !j_last) ? src + V : src);
+                int le = g.ny - 1 - q.j0;
                 le = le < 0 ? 0 : (le > V - 1 ? V - 1 : le);
-                own[d] = (cx != 0 || cy != 0) ? pload1<S, true>(A.p[d], q.e0 + le) : 0.f;
+                own[d] = (cx != 0 || cz != 0) ? pload1<S, true>(A.p[d], q.e0 + le) : 0.f;
             }
         }
-        // batch 2: shift along k
+        // batch 2: shift along j
 #pragma unroll
         for (int d = 0; d < NQ; d++) {
             const int cx = cx_of(d), cy = cy_of(d), cz = cz_of(d);
-            const bool row_ok = !((cx > 0 && i_lo) || (cx < 0 && i_hi) || (cy > 0 && j_lo) || (cy < 0 && j_hi));
-            if (cz > 0) {                          // source k - 1
+            const bool row_ok = !((cx > 0 && i_lo) || (cx < 0 && i_hi) || (cz > 0 && k_lo) || (cz < 0 && k_hi));
+            if (cy > 0) {                          // source j - 1
                 float left = __shfl_up_sync(FULL, f[d][V - 1], 1);
                 if (lane == 0) left = hal[d];
-                const float own0 = (cx != 0 || cy != 0) ? own[d] : f[d][0];
+                const float own0 = (cx != 0 || cz != 0) ? own[d] : f[d][0];
                 if (row_ok) {
 #pragma unroll
                     for (int e = V - 1; e > 0; e--) f[d][e] = f[d][e - 1];
-                    f[d][0] = k_first ? own0 : left;
+                    f[d][0] = j_first ? own0 : left;
                 }
-            } else if (cz < 0) {                   // source k + 1
+            } else if (cy < 0) {                   // source j + 1
                 float right = __shfl_down_sync(FULL, f[d][0], 1);
-                if (lane == 31) right = hal[d];
-                const int le = g.nz - 1 - q.k0;   // element of the row's last cell when k_last
+                if (lane == SEG - 1) right = hal[d];
+                const int le = g.ny - 1 - q.j0;   // element of the row's last cell when j_last
                 float ownl = own[d];
-                if (cx == 0 && cy == 0) {
+                if (cx == 0 && cz == 0) {
 #pragma unroll
                     for (int e = 0; e < V; e++)
                         if (e == le) ownl = f[d][e];
@@ -383,7 +405,7 @@ __device__ __forceinline__ void simple_quad(const Planes& A, const Planes& B, fl
 #pragma unroll
                     for (int e = 0; e < V - 1; e++) f[d][e] = f[d][e + 1];
                     f[d][V - 1] = right;
-                    if (k_last) {
+                    if (j_last) {
 #pragma unroll
                         for (int e = 0; e < V; e++)
                             if (e == le) f[d][e] = ownl;
@@ -396,18 +418,19 @@ __device__ __forceinline__ void simple_quad(const Planes& A, const Planes& B, fl
     // 16-bit storage: approximate reciprocals and square root (measured on
     // B200 at 400^3: FP16 step 1.28 -> 1.19 ms; the Esotwist kernel, which
     // keeps IEEE rounding, measured slower with them, 1.38 -> 1.47 ms)
-    collide_quad<V, LES, COLLIDE, Storage<S>::deviation, FORCE, Storage<S>::deviation>(f, q, Nu, F, mask, g,
-                                                                                       p, FROM_MOMENTS, nu);
-    if constexpr (BOX == 2) {
-        // box launch: the exact outputs and Nu to the scratch array (entry
-        // blockIdx.x * 128 + threadIdx.x of the chunk list)
-        const long long o = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    collide_quad<V, LES, COLLIDE, Storage<S>::deviation, PART != 1, Storage<S>::deviation>(f, q, Nu, F, mask, g,
+                                                                                           p, FROM_MOMENTS, nu);
+    if (!ok) return;
+    if (PART == 2 && ok != ALL) {
 #pragma unroll
-        for (int d = 0; d < NQ; d++) out.v[(long long)d * out.n + o] = f[d][0];
-        out.v[(long long)NQ * out.n + o] = nu[0];
+        for (int e = 0; e < V; e++) {
+            if (!((ok >> e) & 1u)) continue;
+#pragma unroll
+            for (int d = 0; d < NQ; d++) pstore1<S>(B.p[d], q.e0 + e, f[d][e]);
+            if (COLLIDE && LES) Nu[q.e0 + e] = nu[e];
+        }
         return;
     }
-    if (!q.active) return;
 #pragma unroll
     for (int d = 0; d < NQ; d++) pstore<S, V, sizeof(S) == 4>(B.p[d], q.e0, f[d]);
     if constexpr (sizeof(S) == 4) {
@@ -422,63 +445,58 @@ __device__ __forceinline__ void simple_quad(const Planes& A, const Planes& B, fl
 //
 // Slot s of cell x lives at x + o_s, o_s = max(-c_s, 0) (even) or
 // max(+c_s, 0) (odd), +1 wrapping to 0; a cell reads and writes the same 18
-// locations. V = 1 addresses them directly. For V > 1, where o_s has a k
-// component the V locations of a quad are k0+1 .. k0+V: loads take the
-// aligned vector at k0 and the next lane's first element; stores write the
-// aligned vector at k0 holding the previous lane's last value, and the lane
+// locations. V = 1 addresses them directly. For V > 1, where o_s has a j
+// component the V locations of a quad are j0+1 .. j0+V: loads take the
+// aligned vector at j0 and the next lane's first element; stores write the
+// aligned vector at j0 holding the previous lane's last value, and the lane
 // that owns the last cell of a warp (or of a row, where the location wraps to
-// k = 0) stores that one value alone. A __syncwarp() separates every lane's
+// j = 0) stores that one value alone. A __syncwarp() separates every lane's
 // loads from any lane's stores, so a location is always read by its owner
 // before a neighbour overwrites it.
 // ---------------------------------------------------------------------------
-template <typename S, int V, bool LES, bool FROM_MOMENTS, bool COLLIDE, bool EVEN, bool FORCE = true, int BOX = 0>
+template <typename S, int V, bool LES, bool FROM_MOMENTS, bool COLLIDE, bool EVEN, int PART = 0>
 __device__ __forceinline__ void esotwist_quad(const Planes& Q, float* __restrict__ Nu, const float4* __restrict__ F,
                                               const uint32_t* __restrict__ mask, const Dims& g, const CollideParams& p,
-                                              unsigned t, const ResidualBox rb = ResidualBox{},
-                                              const BoxOut out = BoxOut{}) {
+                                              unsigned t, const StepPart& part = StepPart{}) {
     static_assert(!(Storage<S>::deviation && FROM_MOMENTS), "16-bit state always holds populations");
-    static_assert(BOX == 0 || (Storage<S>::deviation && V == 1), "the residual box serves 16-bit storage, one cell per thread");
-    const int nq = g.kp / V;
-    const Quad q = quad_of<V, sizeof(S) == 2>(g, nq, t);
-    const int lane = threadIdx.x & 31;
+    constexpr int SEG = PART == 2 ? 32 / V : 32;   // lanes that hold consecutive quads
+    constexpr unsigned ALL = (1u << V) - 1u;
+    unsigned ok_cells;
+    const Quad q = part_quad<V, sizeof(S) == 2, PART>(g, part, t, ok_cells);
+    const int lane = threadIdx.x & (SEG - 1);
     const int i1 = q.i + 1 == g.nx ? 0 : q.i + 1;
-    const int j1 = q.j + 1 == g.ny ? 0 : q.j + 1;
-    const bool k_last = q.k0 + V >= g.nz;
-    const int last_e = g.nz - 1 - q.k0;   // element holding the row's last cell (if < V)
+    const int k1 = q.k + 1 == g.nz ? 0 : q.k + 1;
+    const bool j_last = q.j0 + V >= g.ny;
+    const int last_e = g.ny - 1 - q.j0;   // element holding the row's last cell (if < V)
     float f[NQ][V];
     if (V == 1) {
-        // Slots with a k offset read element k + 1: every lane loads its own
-        // (aligned) element k and takes k + 1 from the next lane; the lane at
+        // Slots with a j offset read element j + 1: every lane loads its own
+        // (aligned) element j and takes j + 1 from the next lane; the lane at
         // a warp's end or a row's end loads its element itself. (Padding
-        // lanes, k >= nz, load element 0 of their row: in bounds, unused.)
-        const bool row_end = q.k0 == g.nz - 1;
+        // lanes, j >= ny, load element 0 of their row: in bounds, unused.)
+        const bool row_end = q.j0 == g.ny - 1;
         const bool warp_end = lane == 31;
-        const int k1 = (row_end || q.k0 >= g.nz) ? 0 : q.k0 + 1;
+        const int j1 = (row_end || q.j0 >= g.ny) ? 0 : q.j0 + 1;
         float v[NQ], x[NQ];
 #pragma unroll
         for (int s = 0; s < NQ; s++) {
             const int sg = EVEN ? -1 : 1;
             const bool oi = sg * cx_of(s) > 0, oj = sg * cy_of(s) > 0, ok = sg * cz_of(s) > 0;
-            const int base = ((oi ? i1 : q.i) * g.ny + (oj ? j1 : q.j)) * g.kp;
-            v[s] = pload1<S, false>(Q.p[s], base + q.k0);
-            if (ok) x[s] = (warp_end || row_end) ? pload1<S, false>(Q.p[s], base + k1) : 0.f;
+            const int base = ((oi ? i1 : q.i) * g.nz + (ok ? k1 : q.k)) * g.jp;
+            v[s] = pload1<S, false>(Q.p[s], base + q.j0);
+            if (oj) x[s] = (warp_end || row_end) ? pload1<S, false>(Q.p[s], base + j1) : 0.f;
         }
 #pragma unroll
         for (int s = 0; s < NQ; s++) {
             const int sg = EVEN ? -1 : 1;
-            const bool ok = sg * cz_of(s) > 0;
+            const bool oj = sg * cy_of(s) > 0;
             const int d = EVEN ? s : (s ^ 1);
-            if (ok) {
+            if (oj) {
                 const float right = __shfl_down_sync(FULL, v[s], 1);
                 f[d][0] = (warp_end || row_end) ? x[s] : right;
             } else {
                 f[d][0] = v[s];
             }
-        }
-        if constexpr (BOX == 2) {
-            // residual box: the exact deviation of every location inside it
-            // (slot s of this cell lives at cell (li, lj, lk))
-            if (q.active && rb.near(q.i, q.j, q.k0)) box_read_eso<EVEN>(rb, q.i, q.j, q.k0, i1, j1, k1, f);
         }
     } else {
         float hal[NQ], wrap[NQ];
@@ -487,25 +505,25 @@ __device__ __forceinline__ void esotwist_quad(const Planes& Q, float* __restrict
             const int sg = EVEN ? -1 : 1;
             const bool oi = sg * cx_of(s) > 0, oj = sg * cy_of(s) > 0, ok = sg * cz_of(s) > 0;
             const int d = EVEN ? s : (s ^ 1);
-            const int base = ((oi ? i1 : q.i) * g.ny + (oj ? j1 : q.j)) * g.kp;
-            pload<S, V, false>(Q.p[s], base + q.k0, f[d]);
-            if (ok) {
-                hal[s] = pload1<S, false>(Q.p[s], base + ((lane == 31 && !k_last) ? q.k0 + V : q.k0));
+            const int base = ((oi ? i1 : q.i) * g.nz + (ok ? k1 : q.k)) * g.jp;
+            pload<S, V, false>(Q.p[s], base + q.j0, f[d]);
+            if (oj) {
+                hal[s] = pload1<S, false>(Q.p[s], base + ((lane == SEG - 1 && !j_last) ? q.j0 + V : q.j0));
                 wrap[s] = pload1<S, false>(Q.p[s], base);
             }
         }
 #pragma unroll
         for (int s = 0; s < NQ; s++) {
             const int sg = EVEN ? -1 : 1;
-            const bool ok = sg * cz_of(s) > 0;
+            const bool oj = sg * cy_of(s) > 0;
             const int d = EVEN ? s : (s ^ 1);
-            if (!ok) continue;
+            if (!oj) continue;
             float right = __shfl_down_sync(FULL, f[d][0], 1);
-            if (lane == 31) right = hal[s];
+            if (lane == SEG - 1) right = hal[s];
 #pragma unroll
             for (int e = 0; e < V - 1; e++) f[d][e] = f[d][e + 1];
             f[d][V - 1] = right;
-            if (k_last) {                          // k = nz-1 wraps to 0
+            if (j_last) {                          // j = ny-1 wraps to 0
 #pragma unroll
                 for (int e = 0; e < V; e++)
                     if (e == last_e) f[d][e] = wrap[s];
@@ -514,51 +532,52 @@ __device__ __forceinline__ void esotwist_quad(const Planes& Q, float* __restrict
     }
     __syncwarp();
     float nu[V];
-    collide_quad<V, LES, COLLIDE, Storage<S>::deviation, FORCE>(f, q, Nu, F, mask, g, p, FROM_MOMENTS, nu);
-    if constexpr (BOX == 2) {
-        // box launch: the exact outputs, slot by slot, and Nu to the scratch
-        // array (entry blockIdx.x * 128 + threadIdx.x of the chunk list)
-        const long long o = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-#pragma unroll
-        for (int s = 0; s < NQ; s++) out.v[(long long)s * out.n + o] = f[EVEN ? (s ^ 1) : s][0];
-        out.v[(long long)NQ * out.n + o] = nu[0];
-        return;
-    }
+    collide_quad<V, LES, COLLIDE, Storage<S>::deviation, PART != 1>(f, q, Nu, F, mask, g, p, FROM_MOMENTS, nu);
+    // A location of the next cell along j is written by the next lane: bit e of
+    // put: this launch stores the cell before element e.
+    unsigned put = ALL;
+    if constexpr (PART != 0) put = (__shfl_up_sync(FULL, ok_cells, 1) >> (V - 1)) | (ok_cells << 1);
     if (V == 1) {
-        // Slots with a k offset write element k + 1: lane l writes element k
-        // with the value of the previous lane (cell k - 1, same row), so the
+        // Slots with a j offset write element j + 1: lane l writes element j
+        // with the value of the previous lane (cell j - 1, same row), so the
         // warp's store is aligned; the lane at a warp's end or a row's end
-        // writes its own element k + 1 (k = nz - 1: element 0) itself.
-        const bool row_end = q.k0 == g.nz - 1;
+        // writes its own element j + 1 (j = ny - 1: element 0) itself.
+        const bool row_end = q.j0 == g.ny - 1;
         const bool warp_end = lane == 31;
-        const int k1 = (row_end || q.k0 >= g.nz) ? 0 : q.k0 + 1;
+        const int j1 = (row_end || q.j0 >= g.ny) ? 0 : q.j0 + 1;
 #pragma unroll
         for (int s = 0; s < NQ; s++) {
             const int sg = EVEN ? -1 : 1;
             const bool oi = sg * cx_of(s) > 0, oj = sg * cy_of(s) > 0, ok = sg * cz_of(s) > 0;
             const int d = EVEN ? (s ^ 1) : s;
-            const int base = ((oi ? i1 : q.i) * g.ny + (oj ? j1 : q.j)) * g.kp;
-            if (!ok) {
-                if (q.active) pstore1<S>(Q.p[s], base + q.k0, f[d][0]);
+            const int base = ((oi ? i1 : q.i) * g.nz + (ok ? k1 : q.k)) * g.jp;
+            if (!oj) {
+                if (ok_cells) pstore1<S>(Q.p[s], base + q.j0, f[d][0]);
                 continue;
             }
             const float left = __shfl_up_sync(FULL, f[d][0], 1);
-            if (lane > 0 && q.k0 > 0 && q.k0 <= g.nz - 1 && q.active)
-                pstore1<S>(Q.p[s], base + q.k0, left);
-            if (q.active && (warp_end || row_end)) pstore1<S>(Q.p[s], base + k1, f[d][0]);
+            if (lane > 0 && q.j0 > 0 && q.j0 <= g.ny - 1 && q.active && (put & 1u))
+                pstore1<S>(Q.p[s], base + q.j0, left);
+            if (ok_cells && (warp_end || row_end)) pstore1<S>(Q.p[s], base + j1, f[d][0]);
         }
-        if (COLLIDE && LES && q.active) Nu[q.e0] = nu[0];
+        if (COLLIDE && LES && ok_cells) Nu[q.e0] = nu[0];
         return;
     }
-    const bool k_first = q.k0 == 0;
+    const bool j_first = q.j0 == 0;
 #pragma unroll
     for (int s = 0; s < NQ; s++) {
         const int sg = EVEN ? -1 : 1;
         const bool oi = sg * cx_of(s) > 0, oj = sg * cy_of(s) > 0, ok = sg * cz_of(s) > 0;
         const int d = EVEN ? (s ^ 1) : s;      // direction written to slot s
-        const int base = ((oi ? i1 : q.i) * g.ny + (oj ? j1 : q.j)) * g.kp;
-        if (!ok) {
-            if (q.active) pstore<S, V>(Q.p[s], base + q.k0, f[d]);
+        const int base = ((oi ? i1 : q.i) * g.nz + (ok ? k1 : q.k)) * g.jp;
+        if (!oj) {
+            if (PART == 2 && ok_cells != ALL) {
+#pragma unroll
+                for (int e = 0; e < V; e++)
+                    if ((ok_cells >> e) & 1u) pstore1<S>(Q.p[s], base + q.j0 + e, f[d][e]);
+            } else if (ok_cells) {
+                pstore<S, V>(Q.p[s], base + q.j0, f[d]);
+            }
             continue;
         }
         float w[V];
@@ -567,35 +586,47 @@ __device__ __forceinline__ void esotwist_quad(const Planes& Q, float* __restrict
 #pragma unroll
         for (int e = 1; e < V; e++) w[e] = f[d][e - 1];
         if (!q.active) continue;
-        if (lane != 0 && !k_first) {
-            pstore<S, V>(Q.p[s], base + q.k0, w);
+        if (lane != 0 && !j_first && (PART == 0 || (put & ALL) == ALL)) {
+            pstore<S, V>(Q.p[s], base + q.j0, w);
         } else {
+            if (PART != 0 && lane != 0 && !j_first && (put & 1u)) pstore1<S>(Q.p[s], base + q.j0, w[0]);
 #pragma unroll
-            for (int e = 1; e < V; e++) pstore1<S>(Q.p[s], base + q.k0 + e, w[e]);
+            for (int e = 1; e < V; e++)
+                if (PART == 0 || ((put >> e) & 1u)) pstore1<S>(Q.p[s], base + q.j0 + e, w[e]);
         }
-        if (k_last) {                          // the wrap location of k = nz-1
+        if (j_last) {                          // the wrap location of j = ny-1
 #pragma unroll
             for (int e = 0; e < V; e++)
-                if (e == last_e) pstore1<S>(Q.p[s], base, f[d][e]);
-        } else if (lane == 31) {
-            pstore1<S>(Q.p[s], base + q.k0 + V, f[d][V - 1]);
+                if (e == last_e && (PART == 0 || ((ok_cells >> e) & 1u))) pstore1<S>(Q.p[s], base, f[d][e]);
+        } else if (lane == SEG - 1 && (PART == 0 || ((ok_cells >> (V - 1)) & 1u))) {
+            pstore1<S>(Q.p[s], base + q.j0 + V, f[d][V - 1]);
         }
     }
-    if (COLLIDE && LES && q.active) vstore<V>(Nu + q.e0, nu);
+    if (COLLIDE && LES && ok_cells) {
+        if (PART == 2 && ok_cells != ALL) {
+#pragma unroll
+            for (int e = 0; e < V; e++)
+                if ((ok_cells >> e) & 1u) Nu[q.e0 + e] = nu[e];
+        } else {
+            vstore<V>(Nu + q.e0, nu);
+        }
+    }
 }
 
 
-// Split step (one cell per thread). The immersed-boundary pass of a step
-// touches a thin set of cells, so a step can run as two launches over
-// 32-cell chunks of the flat (row, k) index, one warp per listed chunk:
-//   PART 1 (outer): the chunks outside the zone; F is zero there, so these
-//     warps read neither F nor the touched flags;
-//   PART 2 (inner): the chunks of the zone.
+// Split step. The immersed-boundary pass of a step touches a thin set of
+// cells, so a step can run as two launches over the flag words (StepPart):
+//   PART 1 (outer): the words outside the zone; F is zero there, so this
+//     launch reads neither F nor the touched flags. It walks the whole lattice
+//     as PART 0 does, prefetch included, and drops the zone's results at the
+//     store (a few per cent of the cells): the flag is loaded beside the
+//     populations and delays nothing;
+//   PART 2 (inner): the words of the zone, from a list.
 // PART 0 runs every cell. The outer launch of a step depends on the previous
 // step's populations only, so it can run while the previous forcing pass is
 // still in flight.
 // L2 prefetch ahead of a full launch's walk. CTA b covers elements
-// [128 V b, 128 V (b + 1)) of the flat row * kp + k index. Every
+// [128 V b, 128 V (b + 1)) of the flat row * jp + j index. Every
 // kPrefetchTiles-th CTA, as it starts, has NQ + 1 of its threads issue one
 // cp.async.bulk.prefetch.L2 each, for the kPrefetchTiles tiles that begin
 // `ahead` CTAs later: the span of plane d the pull reads (Simple: the tiles
@@ -625,43 +656,27 @@ __device__ __forceinline__ void prefetch_ahead(const Planes& A, const float* Nu,
     if (ahead <= 0 || d >= (LES ? NQ + 1 : NQ) || blockIdx.x % kPrefetchTiles) return;
     constexpr long long tile = 128LL * V;
     const long long e0 = ((long long)blockIdx.x + ahead) * tile, e1 = e0 + kPrefetchTiles * tile;
-    if (e0 >= g.rows() * g.kp) return;
+    if (e0 >= g.rows() * g.jp) return;
     if (d == NQ) return prefetch_span(Nu, 4, g.plane, e0, e1);
-    const long long rs = (long long)g.ny * g.kp;
+    const long long rs = (long long)g.nz * g.jp;
     long long sh;
     if (ESO) {
         const int sg = EVEN ? -1 : 1;
-        sh = (sg * cx_of(d) > 0 ? rs : 0) + (sg * cy_of(d) > 0 ? g.kp : 0);
+        sh = (sg * cx_of(d) > 0 ? rs : 0) + (sg * cz_of(d) > 0 ? g.jp : 0);
     } else {
-        sh = -(cx_of(d) * rs + cy_of(d) * g.kp);
+        sh = -(cx_of(d) * rs + cz_of(d) * g.jp);
     }
-    // one element either side: the k +- 1 neighbours
+    // one element either side: the j +- 1 neighbours
     prefetch_span(A.p[d], (int)sizeof(S), g.plane, e0 + sh - 1, e1 + sh + 1);
 }
 
-template <int PART>
-__device__ __forceinline__ bool part_thread(const StepPart& part, unsigned& t) {
-    t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (PART != 0) {
-        const unsigned w = t >> 5;
-        if (w >= (unsigned)part.count) return false;   // whole warps
-        t = (unsigned)__ldg(part.chunks + w) * kSplitChunk + (threadIdx.x & 31u);
-    }
-    return true;
-}
-
-template <typename S, int V, bool LES, bool FROM_MOMENTS, bool COLLIDE, int PART = 0, int BOX = 0>
+template <typename S, int V, bool LES, bool FROM_MOMENTS, bool COLLIDE, int PART = 0>
 __global__ void __launch_bounds__(128, 4) k_step_simple(Planes A, Planes B, float* __restrict__ Nu,
                                                        const float4* __restrict__ F, const uint32_t* __restrict__ mask,
-                                                       Dims g, CollideParams p, StepPart part, ResidualBox rr,
-                                                       BoxOut out) {
-    static_assert(PART == 0 || V == 1, "split steps run one cell per thread");
-    static_assert(BOX != 2 || PART != 0, "the box path runs a chunk list");
-    if constexpr (PART == 0 && COLLIDE && !FROM_MOMENTS)
+                                                       Dims g, CollideParams p, StepPart part) {
+    if constexpr (PART != 2 && COLLIDE && !FROM_MOMENTS)
         prefetch_ahead<S, V, LES, false, false>(A, Nu, g, part.l2_ahead);
-    unsigned t;
-    if (!part_thread<PART>(part, t)) return;   // whole warps
-    simple_quad<S, V, LES, FROM_MOMENTS, COLLIDE, PART != 1, BOX>(A, B, Nu, F, mask, g, p, t, rr, out);
+    simple_quad<S, V, LES, FROM_MOMENTS, COLLIDE, PART>(A, B, Nu, F, mask, g, p, blockIdx.x * blockDim.x + threadIdx.x, part);
 }
 
 // Resident 128-thread blocks per SM the Esotwist kernel is built for: the
@@ -670,47 +685,64 @@ __global__ void __launch_bounds__(128, 4) k_step_simple(Planes A, Planes B, floa
 template <int V>
 constexpr int kEsotwistBlocksPerSM = V == 1 ? 8 : (V == 2 ? 6 : 4);
 
-template <typename S, int V, bool LES, bool FROM_MOMENTS, bool COLLIDE, bool EVEN, int PART = 0, int BOX = 0>
-__global__ void __launch_bounds__(128, BOX == 2 ? 4 : kEsotwistBlocksPerSM<V>) k_step_esotwist(Planes Q, float* __restrict__ Nu,
+template <typename S, int V, bool LES, bool FROM_MOMENTS, bool COLLIDE, bool EVEN, int PART = 0>
+__global__ void __launch_bounds__(128, kEsotwistBlocksPerSM<V>) k_step_esotwist(Planes Q, float* __restrict__ Nu,
                                                          const float4* __restrict__ F, const uint32_t* __restrict__ mask,
-                                                         Dims g, CollideParams p, StepPart part, ResidualBox rb,
-                                                         BoxOut out) {
-    static_assert(PART == 0 || V == 1, "split steps run one cell per thread");
-    static_assert(BOX != 2 || PART != 0, "the box path runs a chunk list");
-    if constexpr (PART == 0 && COLLIDE && !FROM_MOMENTS)
+                                                         Dims g, CollideParams p, StepPart part) {
+    if constexpr (PART != 2 && COLLIDE && !FROM_MOMENTS)
         prefetch_ahead<S, V, LES, true, EVEN>(Q, Nu, g, part.l2_ahead);
-    unsigned t;
-    if (!part_thread<PART>(part, t)) return;   // whole warps
-    esotwist_quad<S, V, LES, FROM_MOMENTS, COLLIDE, EVEN, PART != 1, BOX>(Q, Nu, F, mask, g, p, t, rb, out);
+    esotwist_quad<S, V, LES, FROM_MOMENTS, COLLIDE, EVEN, PART>(Q, Nu, F, mask, g, p, blockIdx.x * blockDim.x + threadIdx.x, part);
 }
 
-// After the plain launch of a step with a residual box: every cell of the box
-// chunks takes the outputs its box launch computed (entry blockIdx.x * 128 +
-// threadIdx.x of `out`): Simple stores direction d to its own cell of plane d
-// of Q (the destination buffer), Esotwist slot s to the slot's location;
-// the residuals of the locations inside the box (rb: the destination's set)
-// and Nu go with them.
-template <typename S, bool SIMPLE, bool EVEN>
-__global__ void __launch_bounds__(128) k_box_commit(Planes Q, float* __restrict__ Nu, Dims g, StepPart part,
-                                                    ResidualBox rb, BoxOut out, int les) {
-    unsigned t;
-    if (!part_thread<2>(part, t)) return;
-    const Quad q = quad_of<1, true>(g, g.kp, t);
-    if (!q.active) return;
-    const long long o = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    const int i1 = q.i + 1 == g.nx ? 0 : q.i + 1;
-    const int j1 = q.j + 1 == g.ny ? 0 : q.j + 1;
-    const int k1 = q.k0 + 1 == g.nz ? 0 : q.k0 + 1;
+// One cell of the box list per thread: its 18 stored deviations, exact where
+// their locations lie in the box (rr), collided as the one-cell-per-thread
+// step kernels do and written with the residuals of the locations inside the
+// box (rw: the destination's set, the same one for Esotwist). Scattered runs of
+// a few tens of cells: bound by load latency (B200, 160^3 FP16 Simple: it and
+// the commit of a scratch array that it replaces 27.5 us).
+template <typename S, bool SIMPLE, bool LES, bool EVEN>
+__global__ void __launch_bounds__(128) k_box_step(Planes A, Planes B, float* __restrict__ Nu, const float4* __restrict__ F,
+                                                  const uint32_t* __restrict__ mask, Dims g, CollideParams p,
+                                                  const int* __restrict__ cells, int n, ResidualBox rr, ResidualBox rw) {
+    const int t = (int)(blockIdx.x * blockDim.x + threadIdx.x);
+    if (t >= n) return;
+    Quad q;
+    q.e0 = cells[t];
+    q.row = q.e0 / g.jp;
+    q.j0 = q.e0 - q.row * g.jp;
+    q.i = q.row / g.nz;
+    q.k = q.row - q.i * g.nz;
+    q.active = true;
+    const int i1 = q.i + 1 == g.nx ? 0 : q.i + 1, j1 = q.j0 + 1 == g.ny ? 0 : q.j0 + 1, k1 = q.k + 1 == g.nz ? 0 : q.k + 1;
+    float f[NQ][1];
 #pragma unroll
     for (int s = 0; s < NQ; s++) {
-        int li = q.i, lj = q.j, lk = q.k0;
-        if (!SIMPLE) eso_location<EVEN>(s, q.i, q.j, q.k0, i1, j1, k1, li, lj, lk);
-        const float v = out.v[(long long)s * out.n + o];
-        const S enc = Storage<S>::enc(v);
-        reinterpret_cast<S*>(Q.p[s])[((long long)li * g.ny + lj) * g.kp + lk] = enc;
-        if (rb.contains(li, lj, lk)) *rb.at(s, li, lj, lk) = v - Storage<S>::dec(enc);
+        if constexpr (SIMPLE) {
+            const int si = q.i - cx_of(s), sj = q.j0 - cy_of(s), sk = q.k - cz_of(s);
+            const bool in = (unsigned)si < (unsigned)g.nx && (unsigned)sj < (unsigned)g.ny && (unsigned)sk < (unsigned)g.nz;
+            f[s][0] = pload1<S, false>(A.p[s], in ? (int)g.at(si, sj, sk) : q.e0);
+        } else {
+            int li, lj, lk;
+            eso_location<EVEN>(s, q.i, q.j0, q.k, i1, j1, k1, li, lj, lk);
+            f[EVEN ? s : (s ^ 1)][0] = pload1<S, false>(A.p[s], (int)g.at(li, lj, lk));
+        }
     }
-    if (les) Nu[q.e0] = out.v[(long long)NQ * out.n + o];
+    if (rr.near(q.i, q.j0, q.k)) {
+        if constexpr (SIMPLE) box_pull_simple(rr, q.i, q.j0, q.k, g, f);
+        else box_read_eso<EVEN>(rr, q.i, q.j0, q.k, i1, j1, k1, f);
+    }
+    float nu[1];
+    collide_quad<1, LES, true, true, true, SIMPLE>(f, q, Nu, F, mask, g, p, false, nu);
+#pragma unroll
+    for (int s = 0; s < NQ; s++) {
+        int li = q.i, lj = q.j0, lk = q.k;
+        if (!SIMPLE) eso_location<EVEN>(s, q.i, q.j0, q.k, i1, j1, k1, li, lj, lk);
+        const float v = f[SIMPLE ? s : (EVEN ? (s ^ 1) : s)][0];
+        const S enc = Storage<S>::enc(v);
+        reinterpret_cast<S*>((SIMPLE ? B : A).p[s])[g.at(li, lj, lk)] = enc;
+        if (rw.contains(li, lj, lk)) *rw.at(s, li, lj, lk) = v - Storage<S>::dec(enc);
+    }
+    if (LES) Nu[q.e0] = nu[0];
 }
 
 // Moments of the current state at every interior cell (what the reference's
@@ -721,7 +753,7 @@ template <typename S>
 __device__ __forceinline__ void state_moments18(const Planes& A, const Dims& g, int mode, int even, const CollideParams& p,
                                                 int i, int j, int k, float (&m)[NQ],
                                                 const ResidualBox rb = ResidualBox{}) {
-    const int e = (int)(((long long)i * g.ny + j) * g.kp + k);
+    const int e = (int)g.at(i, j, k);
     float q[NQ];
     if (mode <= 1) {
 #pragma unroll
@@ -730,7 +762,7 @@ __device__ __forceinline__ void state_moments18(const Planes& A, const Dims& g, 
             if (mode == 0) {
                 const int si = i - cx_of(d), sj = j - cy_of(d), sk = k - cz_of(d);
                 const bool in = (unsigned)si < (unsigned)g.nx && (unsigned)sj < (unsigned)g.ny && (unsigned)sk < (unsigned)g.nz;
-                if (in) src = (si * g.ny + sj) * g.kp + sk;
+                if (in) src = (int)g.at(si, sj, sk);
                 if (Storage<S>::deviation && rb.on()) {
                     const int li = in ? si : i, lj = in ? sj : j, lk = in ? sk : k;
                     if (rb.contains(li, lj, lk)) {
@@ -748,7 +780,7 @@ __device__ __forceinline__ void state_moments18(const Planes& A, const Dims& g, 
             const int s = even ? d : (d ^ 1);
             const int sg = even ? -1 : 1;
             const bool oi = sg * cx_of(s) > 0, oj = sg * cy_of(s) > 0, ok = sg * cz_of(s) > 0;
-            q[d] = pload1<S, false>(A.p[s], ((oi ? i1 : i) * g.ny + (oj ? j1 : j)) * g.kp + (ok ? k1 : k)) +
+            q[d] = pload1<S, false>(A.p[s], (int)g.at(oi ? i1 : i, oj ? j1 : j, ok ? k1 : k)) +
                    (mode == 2 ? rest_of<S>(d, p) : 0.f);
             if (Storage<S>::deviation && mode == 2 && rb.on() && rb.contains(oi ? i1 : i, oj ? j1 : j, ok ? k1 : k))
                 q[d] += *rb.at(s, oi ? i1 : i, oj ? j1 : j, ok ? k1 : k);
@@ -765,15 +797,12 @@ template <typename S>
 __global__ void __launch_bounds__(256) k_state_moments(Planes A, Planes M, Dims g, int mode, int even, CollideParams p,
                                                        ResidualBox rb) {
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    const long long total = g.rows() * g.nz;
-    if (t >= total) return;
-    const int k = (int)(t % g.nz);
-    const long long row = t / g.nz;
-    const int j = (int)(row % g.ny);
-    const int i = (int)(row / g.ny);
+    if (t >= g.cells()) return;
+    int i, j, k;
+    g.cell(t, i, j, k);
     float m[NQ];
     state_moments18<S>(A, g, mode, even, p, i, j, k, m, rb);
-    const long long e = row * g.kp + k;
+    const long long e = g.at(i, j, k);
 #pragma unroll
     for (int d = 0; d < NQ; d++) M.p[d][e] = m[d];
 }

@@ -59,7 +59,6 @@ void release(tdlb_lattice* h) {
     cudaFree(h->d_plane_lv1);
     cudaFree(h->d_blade_planes);
     cudaFree(h->d_cell_e);
-    cudaFree(h->d_cell_order);
     cudaFree(h->d_plane_cell);
     cudaFree(h->d_prep);
     cudaFree(h->d_cell_m);
@@ -69,17 +68,16 @@ void release(tdlb_lattice* h) {
     cudaFree(h->d_mask_static);
     cudaFree(h->d_plane_list);
     cudaFree(h->d_exclude);
-    cudaFree(h->d_zone_list);
+    tdlb_rt::drop_zone(h);
     cudaFree(h->d_box_list);
-    cudaFree(h->d_box_out);
     for (cudaEvent_t e : h->tev) cudaEventDestroy(e);
     if (h->side) cudaStreamDestroy(h->side);
-    if (h->ibm) cudaStreamDestroy(h->ibm);
+    if (h->bulk) cudaStreamDestroy(h->bulk);
     if (h->ev_fork) cudaEventDestroy(h->ev_fork);
     if (h->ev_join) cudaEventDestroy(h->ev_join);
     if (h->ev_outer) cudaEventDestroy(h->ev_outer);
     if (h->ev_inner) cudaEventDestroy(h->ev_inner);
-    if (h->ev_sync) cudaEventDestroy(h->ev_sync);
+    if (h->ev_fence) cudaEventDestroy(h->ev_fence);
     cudaFree(h->d_red);
     cudaFree(h->d_rot_xz);
     cudaFree(h->d_load);
@@ -122,23 +120,24 @@ tdlb_lattice* build(const tdlb_config& c, int device) {
         h->vec = tdlb_rt::default_cells_per_thread(c);
         h->err.reserve(512);
         TDLB_CK(cudaSetDevice(device));
-        TDLB_CK(cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking));
-        // the forcing pass is the latency-bound critical path of a split
-        // step: its streams get the highest priority, so its blocks are
-        // scheduled ahead of the outer launch's as SMs free up
+        // the forcing pass is the latency-bound path of a split step: its
+        // streams get the highest priority, so its blocks are scheduled ahead
+        // of the outer launch's as SMs free up
         int prio_lo = 0, prio_hi = 0;
         TDLB_CK(cudaDeviceGetStreamPriorityRange(&prio_lo, &prio_hi));
+        TDLB_CK(cudaStreamCreateWithPriority(&h->stream, cudaStreamNonBlocking, prio_hi));
         TDLB_CK(cudaStreamCreateWithPriority(&h->side, cudaStreamNonBlocking, prio_hi));
-        TDLB_CK(cudaStreamCreateWithPriority(&h->ibm, cudaStreamNonBlocking, prio_hi));
+        TDLB_CK(cudaStreamCreateWithPriority(&h->bulk, cudaStreamNonBlocking, prio_lo));
         TDLB_CK(cudaEventCreateWithFlags(&h->ev_fork, cudaEventDisableTiming));
         TDLB_CK(cudaEventCreateWithFlags(&h->ev_join, cudaEventDisableTiming));
         TDLB_CK(cudaEventCreateWithFlags(&h->ev_outer, cudaEventDisableTiming));
         TDLB_CK(cudaEventCreateWithFlags(&h->ev_inner, cudaEventDisableTiming));
-        TDLB_CK(cudaEventCreateWithFlags(&h->ev_sync, cudaEventDisableTiming));
+        TDLB_CK(cudaEventCreateWithFlags(&h->ev_fence, cudaEventDisableTiming));
         Dims& g = h->g;
         g = tdlb::make_dims((int)c.x, (int)c.y, (int)c.z);
-        h->mask_words = round_up((long long)g.nx * g.ny * g.kw, 64);
-        if ((long long)g.nx * g.ny * g.kp >= (1LL << 31) - 64)
+        h->mask_words = round_up(g.rows() * g.jw, 64);
+        // (the limit that the 16-element row granule along z gave)
+        if (c.x * c.y * round_up(c.z, 16) >= tdlb::kMaxPlane || g.rows() * g.jp >= tdlb::kMaxPlane)
             throw Fail{TDLB_EINVAL, "lattice too large: one population plane must stay below 2^31 elements"};
         if (tdlb::ibm_smem_bytes(g, 0) > 200 * 1024)
             throw Fail{TDLB_EINVAL, "x * ceil(z/32) too large for the per-plane IBM flag tile"};
@@ -216,15 +215,16 @@ tdlb_config config_from_json(const char* text) {
     return c;
 }
 
-// Entry points run `fn` after joining the split-step stream (JOIN), so they
-// see every queued step and forcing pass; the step loop's own calls
-// (collision, forcing_resident, rotate_impeller, step) do not join.
-template <bool JOIN = true, typename F>
+// FENCE: what `fn` queues or changes may concern the populations, so the next
+// outer launch of a split step waits for it; the step loop's own calls
+// (collision, forcing_resident, rotate_impeller, set_rotating_markers, step, the
+// impeller load) touch nothing that launch reads or writes.
+template <bool FENCE = true, typename F>
 int guarded(tdlb_lattice* h, F&& fn) {
     if (!h) return TDLB_EINVAL;
     try {
         cudaSetDevice(h->device);
-        if (JOIN) TDLB_CK(tdlb_rt::join_side(h));
+        if (FENCE) tdlb_rt::fence(h);
         fn();
         return TDLB_OK;
     } catch (const Fail& f) {
@@ -256,7 +256,7 @@ tdlb::StepArgs step_args(tdlb_lattice* h, bool collide) {
     a.from_moments = h->holds_moments ? 1 : 0;
     a.collide = collide ? 1 : 0;
     a.even = h->even ? 1 : 0;
-    a.vec = h->vec;
+    a.vec = tdlb::vector_width(h->g, h->vec);
     a.l2_prefetch = h->l2_prefetch;
     a.storage = h->cfg.storage;
     // residual box (16-bit storage): Simple reads the state buffer's
@@ -270,190 +270,193 @@ tdlb::StepArgs step_args(tdlb_lattice* h, bool collide) {
 // Split steps.
 //
 // The forcing pass reads and writes only cells inside the stencils of the
-// markers, and the step reads F only there. The "zone" is a set of 32-element
-// chunks of the flat row*kp + k index that holds every stencil cell of the
-// resident markers at any impeller angle (and, for Esotwist, their 26
-// neighbours: an Esotwist location of a stencil cell is also a location of
-// its neighbours in the other parity). A step then runs as
-//   stream: wait(inner of step s-1), outer chunks of step s
-//   ibm:    forcing pass s-1 ... wait(outer of step s), inner chunks of step s,
-//           forcing pass s
-// so forcing pass s-1 runs concurrently with the outer chunks of step s:
+// markers, and the step reads F only there. The "zone" (zone.cu) is the set of
+// flag words (32 cells of a row) that hold every stencil cell of the resident
+// markers at any impeller angle and, for Esotwist, their 26 neighbours. A step
+// then runs as
+//   bulk:   wait(inner words of step s-1), outer words of step s
+//   stream: forcing pass s-1, inner words of step s, wait(outer words of step
+//           s), forcing pass s
+// so forcing pass s-1 and the inner words run beside the outer words of step s:
 // those cells neither read F nor share a population location with a stencil
-// cell, and every cell computes exactly what the unsplit step computes.
+// cell, and every cell computes exactly what the unsplit step computes. With
+// rows along j the zone of a stirred tank is whole rows (3 to 5 % of a 400^3
+// tank), so the outer launch is the full launch in all but the rows it drops,
+// and a step takes as long as the longer of the two streams.
 // ---------------------------------------------------------------------------
 
-// The split-step stream, ordered after everything queued on `stream` so far.
-cudaStream_t loop_stream(tdlb_lattice* h) {
-    if (!h->pending) {
-        TDLB_CK(cudaEventRecord(h->ev_sync, h->stream));
-        TDLB_CK(cudaStreamWaitEvent(h->ibm, h->ev_sync, 0));
-        h->pending = true;
-    }
-    return h->ibm;
-}
-
-inline void mark_bit(std::vector<uint64_t>& b, long long e) { b[(size_t)(e >> 6)] |= 1ull << (e & 63); }
-inline bool test_bit(const std::vector<uint64_t>& b, long long e) { return (b[(size_t)(e >> 6)] >> (e & 63)) & 1ull; }
-
-// Every stencil cell of markers [b, e) lies in `core`.
-bool stencils_inside(const tdlb_lattice* h, const tdlb_marker* m, size_t n, const std::vector<uint64_t>& core) {
-    const Dims& g = h->g;
+// Every stencil cell of markers [0, n) is set in `core`.
+bool stencils_inside(const Dims& g, const tdlb_marker* m, size_t n, const std::vector<uint32_t>& core) {
     for (size_t q = 0; q < n; q++) {
         int st[9];
         tdlb::MarkerSchedule::stencil(reinterpret_cast<const tdlb::Marker*>(m)[q], g.nx, g.nz, st);
-        for (int c = 0; c < 9; c++) {
-            const long long i = st[c] / g.nz, k = st[c] % g.nz;
-            if (!test_bit(core, (i * g.ny + m[q].j) * g.kp + k)) return false;
-        }
+        const int j = (int)m[q].j;
+        for (int c = 0; c < 9; c++)
+            if (!((core[(size_t)g.word(st[c] / g.nz, j, st[c] % g.nz)] >> (j & 31)) & 1u)) return false;
     }
     return true;
 }
 
-void build_zone(tdlb_lattice* h) {
-    TDLB_CK(tdlb_rt::join_side(h));
-    TDLB_CK(cudaStreamSynchronize(h->stream));   // no launch still reads the old zone
-    const Dims& g = h->g;
-    const long long nel = g.rows() * g.kp;
-    std::vector<uint64_t> core((size_t)((nel + 63) / 64), 0ull);
-    for (int e : h->cells.cell_e) mark_bit(core, e);   // first segment: its stencil cells, exactly
-    const int n1 = h->n_markers - h->n0;
-    const tdlb_marker* rot = h->h_markers.data() + h->n0;
-    if (n1 > 0 && h->impeller_begin >= 0 && h->h_rot_xz.size() == 2 * (size_t)n1) {
-        // Blades turn about (ci, ck). A blade marker at radius r rounds to the
-        // nearest cell, and its stencil cells lie within 1.5 cells of that
-        // position per axis, so within r +- 2.13 of the axis: mark, plane by
-        // plane, the annulus between the smallest and the largest blade radius
-        // widened by 3 cells.
-        std::vector<double> rlo((size_t)g.ny, 1e300), rhi((size_t)g.ny, -1.0);
-        for (int q = 0; q < n1; q++) {
-            const double r = std::sqrt(h->h_rot_xz[2 * q] * h->h_rot_xz[2 * q] + h->h_rot_xz[2 * q + 1] * h->h_rot_xz[2 * q + 1]);
-            const int j = (int)rot[q].j;
-            rlo[(size_t)j] = std::min(rlo[(size_t)j], r);
-            rhi[(size_t)j] = std::max(rhi[(size_t)j], r);
-        }
-        for (int j = 0; j < g.ny; j++) {
-            if (rhi[(size_t)j] < 0) continue;
-            const double lo = rlo[(size_t)j] - 3.0, hi = rhi[(size_t)j] + 3.0;
-            const int i0 = std::max(0, (int)std::floor(h->rot_ci - hi)), i1 = std::min(g.nx - 1, (int)std::ceil(h->rot_ci + hi));
-            const int k0 = std::max(0, (int)std::floor(h->rot_ck - hi)), k1 = std::min(g.nz - 1, (int)std::ceil(h->rot_ck + hi));
-            for (int i = i0; i <= i1; i++)
-                for (int k = k0; k <= k1; k++) {
-                    const double d = std::sqrt((i - h->rot_ci) * (i - h->rot_ci) + (k - h->rot_ck) * (k - h->rot_ck));
-                    if (d >= lo && d <= hi) mark_bit(core, ((long long)i * g.ny + j) * g.kp + k);
-                }
-        }
-    } else {
-        // blades set by the host without an attached impeller: their current cells
-        for (int q = 0; q < n1; q++) {
-            int st[9];
-            tdlb::MarkerSchedule::stencil(reinterpret_cast<const tdlb::Marker*>(rot)[q], g.nx, g.nz, st);
-            for (int c = 0; c < 9; c++) mark_bit(core, ((long long)(st[c] / g.nz) * g.ny + rot[q].j) * g.kp + st[c] % g.nz);
-        }
+// Host blades (tdlb_set_rotating_markers) against the zone's stencil cells.
+bool blades_in_zone(tdlb_lattice* h) {
+    const size_t n1 = (size_t)(h->n_markers - h->n0);
+    if (n1 == 0 || h->rot_device) return true;   // device rotation stays inside the zone's annuli
+    if (h->h_zone_core.empty()) {
+        h->h_zone_core.resize((size_t)(h->g.rows() * h->g.jw));
+        TDLB_CK(cudaMemcpyAsync(h->h_zone_core.data(), h->d_zone_core, h->h_zone_core.size() * sizeof(uint32_t),
+                                cudaMemcpyDeviceToHost, h->stream));
+        TDLB_CK(cudaStreamSynchronize(h->stream));
     }
-    std::vector<uint64_t> zone;
-    if (h->cfg.streaming == TDLB_STREAMING_ESOTWIST) {
-        zone.assign(core.size(), 0ull);
-        for (size_t w = 0; w < core.size(); w++)
-            for (uint64_t b = core[w]; b; b &= b - 1) {
-                const long long e = (long long)w * 64 + __builtin_ctzll(b);
-                const long long row = e / g.kp;
-                const int k = (int)(e - row * g.kp), i = (int)(row / g.ny), j = (int)(row % g.ny);
-                for (int di = -1; di <= 1; di++)
-                    for (int dj = -1; dj <= 1; dj++)
-                        for (int dk = -1; dk <= 1; dk++) {
-                            const int a = (i + di + g.nx) % g.nx, b2 = (j + dj + g.ny) % g.ny, c = (k + dk + g.nz) % g.nz;
-                            mark_bit(zone, ((long long)a * g.ny + b2) * g.kp + c);
-                        }
-            }
-    } else {
-        zone = core;
-    }
-    // 32-element chunks (half a word of `zone`): the inner ones (any element
-    // in the zone), then the outer ones
-    static_assert(tdlb::kSplitChunk == 32, "chunk = half a word of the zone bitset");
-    const long long nchunks = (nel + 31) / 32;
-    std::vector<uint32_t> bits((size_t)((nchunks + 31) / 32), 0u);
-    std::vector<int> list, outer;
-    long long inner_cells = 0;   // interior cells of the inner chunks
-    for (long long c = 0; c < nchunks; c++) {
-        const uint32_t half = (uint32_t)(zone[(size_t)(c >> 1)] >> ((c & 1) * 32));
-        if (half) {
-            bits[(size_t)(c >> 5)] |= 1u << (c & 31);
-            list.push_back((int)c);
-            for (long long e = c * 32; e < std::min(c * 32 + 32, nel); e++) inner_cells += (e % g.kp) < g.nz;
-        } else {
-            outer.push_back((int)c);
-        }
-    }
-    const long long n_in = (long long)list.size();
-    list.insert(list.end(), outer.begin(), outer.end());
-    if ((long long)list.size() > h->zone_list_cap || !h->d_zone_list) {
-        cudaFree(h->d_zone_list);
-        h->d_zone_list = nullptr;
-        TDLB_CK(cudaMalloc(&h->d_zone_list, list.size() * sizeof(int)));
-        h->zone_list_cap = (long long)list.size();
-    }
-    TDLB_CK(cudaMemcpyAsync(h->d_zone_list, list.data(), list.size() * sizeof(int), cudaMemcpyHostToDevice, h->stream));
-    TDLB_CK(cudaStreamSynchronize(h->stream));
-    h->n_zone = (int)n_in;
-    h->n_outer = (int)(nchunks - n_in);
-    h->zone_small = (double)inner_cells <= 0.6 * (double)g.rows() * (double)g.nz;
-    h->h_zone_bits = std::move(bits);
-    h->zone_ok = stencils_inside(h, rot, (size_t)std::max(n1, 0), core);
-    h->h_zone_core = std::move(core);
-    h->zone_gen = h->marker_gen;
+    return stencils_inside(h->g, h->h_markers.data() + h->n0, n1, h->h_zone_core);
 }
 
-// Forcing passes may go to the split-step stream (the next step can split).
+// `all`: every word, whatever the markers (they change with every pass).
+void build_zone(tdlb_lattice* h, bool all) {
+    TDLB_CK(cudaStreamSynchronize(h->stream));   // no launch still reads the old zone
+    const Dims& g = h->g;
+    const long long nw = g.rows() * g.jw;
+    const bool boxed = h->rbox_geom.n > 0;
+    if (h->zone_cap < nw) {
+        tdlb_rt::drop_zone(h);
+        TDLB_CK(cudaMalloc(&h->d_zone_core, (size_t)nw * sizeof(uint32_t)));
+        TDLB_CK(cudaMalloc(&h->d_zone_skip, (size_t)nw));
+        TDLB_CK(cudaMalloc(&h->d_zone_words, (size_t)nw * sizeof(int)));
+        h->zone_cap = nw;
+    }
+    h->h_zone_core.clear();
+    double2* d_ring = nullptr;
+    const int n1 = h->n_markers - h->n0;
+    if (!all && n1 > 0) {
+        // Blades turn about (ci, ck). A blade marker at radius r rounds to the
+        // nearest cell, and its stencil cells lie within 1.5 cells of that
+        // position per axis, so within r +- 2.13 of the axis: plane by plane,
+        // the annulus between the smallest and the largest blade radius
+        // widened by 3 cells.
+        const tdlb_marker* rot = h->h_markers.data() + h->n0;
+        std::vector<double2> ring((size_t)g.ny, make_double2(1e300, -1.0));
+        for (int q = 0; q < n1; q++) {
+            const double r = std::sqrt(h->h_rot_xz[2 * q] * h->h_rot_xz[2 * q] + h->h_rot_xz[2 * q + 1] * h->h_rot_xz[2 * q + 1]);
+            double2& p = ring[(size_t)rot[q].j];
+            p.x = std::min(p.x, r - 3.0);
+            p.y = std::max(p.y, r + 3.0);
+        }
+        TDLB_CK(cudaMalloc(&d_ring, ring.size() * sizeof(double2)));
+        const cudaError_t e = cudaMemcpy(d_ring, ring.data(), ring.size() * sizeof(double2), cudaMemcpyHostToDevice);
+        if (e != cudaSuccess) {
+            cudaFree(d_ring);
+            TDLB_CK(e);
+        }
+    }
+    cudaError_t e = cudaSuccess;
+    if (!all) e = tdlb::launch_zone_core(g, h->d_mask_static, d_ring, h->rot_ci, h->rot_ck, h->d_zone_core, h->stream);
+    if (e == cudaSuccess)
+        e = tdlb::launch_zone_words(g, all ? nullptr : h->d_zone_core, h->cfg.streaming == TDLB_STREAMING_ESOTWIST,
+                                    h->d_zone_skip, h->stream);
+    if (e == cudaSuccess && boxed) {
+        if (!h->d_zone_except) e = cudaMalloc(&h->d_zone_except, (size_t)h->zone_cap * sizeof(uint32_t));
+        if (e == cudaSuccess) e = cudaMemsetAsync(h->d_zone_except, 0, (size_t)nw * sizeof(uint32_t), h->stream);
+        if (e == cudaSuccess) e = tdlb::launch_zone_box(g, h->d_box_list, h->n_box, h->d_zone_except, h->d_zone_skip, h->stream);
+    }
+    h->h_zone_skip.resize((size_t)nw);
+    if (e == cudaSuccess)
+        e = cudaMemcpyAsync(h->h_zone_skip.data(), h->d_zone_skip, (size_t)nw, cudaMemcpyDeviceToHost, h->stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
+    cudaFree(d_ring);
+    TDLB_CK(e);
+    std::vector<int> words;
+    long long inner_cells = 0;
+    for (long long w = 0; w < nw; w++)
+        if (h->h_zone_skip[(size_t)w]) {
+            words.push_back((int)w);
+            inner_cells += std::min(32, g.ny - (int)(w % g.jw) * 32);
+        }
+    if (!words.empty())
+        TDLB_CK(cudaMemcpy(h->d_zone_words, words.data(), words.size() * sizeof(int), cudaMemcpyHostToDevice));
+    h->n_zone = (int)words.size();
+    h->n_outer = (int)(nw - h->n_zone);
+    h->zone_small = (double)inner_cells <= 0.6 * (double)g.cells();
+    h->zone_all = all;
+    h->zone_gen = h->marker_gen;
+    h->zone_box_gen = h->box_gen;
+    h->zone_ok = all || blades_in_zone(h);
+}
+
+// The zone of the resident markers can be built.
+bool zone_known(tdlb_lattice* h) {
+    if (!h->markers_set || !h->resident) return false;
+    const size_t n1 = (size_t)(h->n_markers - h->n0);
+    return n1 == 0 || (h->impeller_begin >= 0 && h->h_rot_xz.size() == 2 * n1);
+}
+
+void build_box_list(tdlb_lattice* h);
+
+void ensure_zone(tdlb_lattice* h, bool all) {
+    build_box_list(h);
+    if (h->zone_gen != h->marker_gen || h->zone_box_gen != h->box_gen || h->zone_all != all || !h->d_zone_skip)
+        build_zone(h, all);
+}
+
+// Smallest lattice whose steps split unasked.
+constexpr long long kAutoSplitCells = 1 << 19;
+
+// The lattice's steps can run split.
 bool split_capable(tdlb_lattice* h) {
-    if (!h->overlap || h->own_stream || h->vec != 1 || !h->markers_set || !h->resident) return false;
-    if (h->zone_gen != h->marker_gen) build_zone(h);
+    if (!h->overlap || h->own_stream || !zone_known(h)) return false;
+    if (h->overlap < 0 && h->g.cells() < kAutoSplitCells) return false;
+    if (h->cfg.storage == TDLB_STORAGE_FP32 && tdlb::vector_width(h->g, h->vec) != 1) return false;
+    ensure_zone(h, false);
     // a zone covering most of the lattice leaves little to overlap with
     return h->zone_ok && (h->zone_small || h->overlap == 2);
 }
 
-// (A step with a residual box runs unsplit: its box launch reads the box
-// chunks' populations and Nu before the plain launch writes them.)
 bool can_split(tdlb_lattice* h) {
-    if (h->rbox_geom.n) return false;
-    return !h->holds_moments && split_capable(h);
+    if (h->holds_moments || !h->overlap) return false;
+    // a captured step stays on the captured stream and its own side stream
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(h->stream, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) return false;
+    return split_capable(h);
 }
 
-// The chunks with a cell near the residual box (ResidualBox::near), which the
-// box launch of a step runs, and that launch's scratch outputs.
+// The cells that the box launch of a step takes, by element (none without a
+// box). Which cells these are is part of the results: the box launch's
+// scalar arithmetic and the plain kernel's packed one differ
+// by FP32 ulps, which 16-bit storage then rounds. They are the cells of every
+// group of 32 along k (groups counted through the lines of constant (i, j),
+// lines padded to 16 cells) that holds a cell near the box.
 void build_box_list(tdlb_lattice* h) {
     if (h->box_list_gen == h->box_gen) return;
-    TDLB_CK(tdlb_rt::join_side(h));
     TDLB_CK(cudaStreamSynchronize(h->stream));   // no launch still reads the old list
     const Dims& g = h->g;
     const tdlb::ResidualBox& b = h->rbox_geom;
-    const long long nchunks = (g.rows() * g.kp + 31) / 32;
-    std::vector<uint8_t> hit((size_t)nchunks, 0);
+    if (b.n == 0) {
+        h->n_box = 0;
+        h->box_list_gen = h->box_gen;
+        return;
+    }
+    const long long line = round_up(g.nz, 16), ngroups = ((long long)g.nx * g.ny * line + 31) / 32;
+    std::vector<uint8_t> hit((size_t)ngroups, 0);
     for (int i = std::max(0, b.i0 - 1); i <= std::min(g.nx - 1, b.i0 + b.bx); i++)
         for (int j = std::max(0, b.j0 - 1); j <= std::min(g.ny - 1, b.j0 + b.by); j++)
             for (int k = std::max(0, b.k0 - 1); k <= std::min(g.nz - 1, b.k0 + b.bz); k++)
-                if (b.around(i, j, k)) hit[(size_t)((((long long)i * g.ny + j) * g.kp + k) >> 5)] = 1;
+                if (b.around(i, j, k)) hit[(size_t)((((long long)i * g.ny + j) * line + k) >> 5)] = 1;
     std::vector<int> list;
-    for (long long c = 0; c < nchunks; c++)
-        if (hit[(size_t)c]) list.push_back((int)c);
+    // in element order; a group may reach into the lines before and after
+    int j0 = b.j0 - 2, j1 = b.j0 + b.by + 2;
+    if (j0 < 0 || j1 > g.ny) {
+        j0 = 0;
+        j1 = g.ny;
+    }
+    for (int i = std::max(0, b.i0 - 2); i < std::min(g.nx, b.i0 + b.bx + 2); i++)
+        for (int k = 0; k < g.nz; k++)
+            for (int j = j0; j < j1; j++)
+                if (hit[(size_t)((((long long)i * g.ny + j) * line + k) >> 5)]) list.push_back((int)g.at(i, j, k));
     if ((long long)list.size() > h->box_list_cap || !h->d_box_list) {
         cudaFree(h->d_box_list);
         h->d_box_list = nullptr;
         h->box_list_cap = 0;
-        TDLB_CK(cudaMalloc(&h->d_box_list, std::max<size_t>(list.size(), 1) * sizeof(int)));
-        h->box_list_cap = (long long)std::max<size_t>(list.size(), 1);
-    }
-    {
-        // one entry per thread of the box launch (128-thread blocks)
-        const long long need = (long long)(tdlb::NQ + 1) * (((long long)list.size() * 32 + 127) / 128 * 128);
-        if (need > h->box_out_cap || !h->d_box_out) {
-            cudaFree(h->d_box_out);
-            h->d_box_out = nullptr;
-            h->box_out_cap = 0;
-            TDLB_CK(cudaMalloc(&h->d_box_out, (size_t)std::max<long long>(need, 1) * sizeof(float)));
-            h->box_out_cap = std::max<long long>(need, 1);
-        }
+        const size_t cap = std::max<size_t>(list.size(), 1);
+        TDLB_CK(cudaMalloc(&h->d_box_list, cap * sizeof(int)));
+        h->box_list_cap = (long long)cap;
     }
     if (!list.empty())
         TDLB_CK(cudaMemcpyAsync(h->d_box_list, list.data(), list.size() * sizeof(int), cudaMemcpyHostToDevice, h->stream));
@@ -489,40 +492,45 @@ void run_step(tdlb_lattice* h, bool collide) {
     auto launch = [&](const tdlb::StepArgs& x, cudaStream_t st) {
         return simple ? tdlb::launch_step_simple(x, st) : tdlb::launch_step_esotwist(x, st);
     };
-    // With a residual box: the box launch (the chunks near the box, with
-    // residuals, into scratch), the plain launch, then the commit of the box
-    // chunks' outputs (step_kernels.cuh). Such a step is never split.
     const bool boxed = a.rr.on();
-    if (boxed) build_box_list(h);
-    tdlb::StepArgs bx = a;
-    bx.box = 2;
-    bx.part = 2;
-    bx.vec = 1;   // the box launches run one cell per thread, whatever the plain launch's variant
-    bx.zone = tdlb::StepPart{h->d_box_list, h->n_box};
-    bx.bout = tdlb::BoxOut{h->d_box_out, ((long long)h->n_box * 32 + 127) / 128 * 128};
-    const bool run_box = boxed && h->n_box > 0;
-    if (collide && can_split(h)) {
-        cudaStream_t side = loop_stream(h);
-        if (h->inner_queued) TDLB_CK(cudaStreamWaitEvent(h->stream, h->ev_inner, 0));
-        if (h->n_outer > 0) {
-            a.part = 1;
-            a.zone = tdlb::StepPart{h->d_zone_list + h->n_zone, h->n_outer};
+    const bool split = collide && can_split(h);
+    auto part = [&](int which, cudaStream_t st) {   // 1: outer words, 2: inner words without the box's cells
+        tdlb::StepArgs x = a;
+        x.part = which;
+        x.zone.skip = h->d_zone_skip;
+        x.zone.words = h->d_zone_words;
+        x.zone.count = h->n_zone;
+        x.zone.except = boxed ? h->d_zone_except : nullptr;
+        if ((which == 1 ? h->n_outer : h->n_zone) > 0) timed_launch(h, st, [&] { return launch(x, st); });
+    };
+    auto box = [&] {
+        a.box_cells = h->d_box_list;
+        a.n_box = h->n_box;
+        if (h->n_box > 0) timed_launch(h, h->stream, [&] { return tdlb::launch_box(a, simple, h->stream); });
+    };
+    if (split) {
+        if (!h->bulk_ok) TDLB_CK(cudaEventRecord(h->ev_fence, h->stream));
+        TDLB_CK(cudaStreamWaitEvent(h->bulk, h->bulk_ok ? h->ev_inner : h->ev_fence, 0));
+        part(1, h->bulk);
+        TDLB_CK(cudaEventRecord(h->ev_outer, h->bulk));
+        if (boxed) box();
+        part(2, h->stream);
+        TDLB_CK(cudaEventRecord(h->ev_inner, h->stream));
+        TDLB_CK(cudaStreamWaitEvent(h->stream, h->ev_outer, 0));
+        h->bulk_ok = true;
+    } else {
+        tdlb_rt::fence(h);
+        if (boxed) {
+            // the box's cells are left out of the plain launches: the outer
+            // words, or none when the zone is not known, then the inner ones
+            ensure_zone(h, !zone_known(h));
+            if (!h->zone_ok) ensure_zone(h, true);
+            part(1, h->stream);
+            box();
+            part(2, h->stream);
+        } else {
             timed_launch(h, h->stream, [&] { return launch(a, h->stream); });
         }
-        TDLB_CK(cudaEventRecord(h->ev_outer, h->stream));
-        TDLB_CK(cudaStreamWaitEvent(side, h->ev_outer, 0));
-        if (h->n_zone > 0) {
-            a.part = 2;
-            a.zone = tdlb::StepPart{h->d_zone_list, h->n_zone};
-            timed_launch(h, side, [&] { return launch(a, side); });
-        }
-        TDLB_CK(cudaEventRecord(h->ev_inner, side));
-        h->inner_queued = true;
-    } else {
-        TDLB_CK(tdlb_rt::join_side(h));
-        if (run_box) timed_launch(h, h->stream, [&] { return launch(bx, h->stream); });
-        timed_launch(h, h->stream, [&] { return launch(a, h->stream); });
-        if (run_box) timed_launch(h, h->stream, [&] { return tdlb::launch_box_commit(bx, simple, h->stream); });
     }
     if (simple) h->cur ^= 1;
     else h->even = !h->even;   // StreamingEsoteric.hpp:15-18
@@ -639,7 +647,7 @@ void upload_markers(tdlb_lattice* h, const tdlb_marker* m, size_t n, size_t n0, 
         h->tail_cap = cap;
     }
     // first segment: unique cells per plane, slot data
-    h->cells.build(mk, h->seg0, g.nx, g.ny, g.nz, g.kp);
+    h->cells.build(mk, h->seg0, g);
     const long long C0 = (long long)h->cells.cell_e.size();
     cudaFree(h->d_cell_e); cudaFree(h->d_plane_cell); cudaFree(h->d_prep); cudaFree(h->d_cell_m); cudaFree(h->d_cell_F);
     h->d_cell_e = nullptr; h->d_plane_cell = nullptr; h->d_prep = nullptr; h->d_cell_m = nullptr; h->d_cell_F = nullptr;
@@ -677,24 +685,10 @@ void upload_markers(tdlb_lattice* h, const tdlb_marker* m, size_t n, size_t n0, 
         h->n_big = (int)big.size();
         h->big_tile_cells = tdlb::big_bulk_bytes(big_max) <= 220 * 1024 ? big_max : 0;
         TDLB_CK(tdlb::ibm_prepare_smem(h->smem_cells, h->n_small, tdlb::big_bulk_bytes(h->big_tile_cells)));
-        // cell order of the pass: the big planes' cells, then the others
-        cudaFree(h->d_cell_order);
-        h->d_cell_order = nullptr;
-        h->ncell_big = 0;
-        if (!big.empty() && C0) {
-            std::vector<char> is_big((size_t)g.ny, 0);
-            for (int j : big) is_big[(size_t)j] = 1;
-            std::vector<int> order;
-            order.reserve((size_t)C0);
-            for (int pass = 1; pass >= 0; pass--)
-                for (int j = 0; j < g.ny; j++)
-                    if (is_big[(size_t)j] == pass)
-                        for (int c = h->cells.plane_cell[(size_t)j]; c < h->cells.plane_cell[(size_t)j + 1]; c++)
-                            order.push_back(c);
-            for (int j : big) h->ncell_big += h->cells.plane_cell[(size_t)j + 1] - h->cells.plane_cell[(size_t)j];
-            TDLB_CK(cudaMalloc(&h->d_cell_order, order.size() * sizeof(int)));
-            TDLB_CK(cudaMemcpy(h->d_cell_order, order.data(), order.size() * sizeof(int), cudaMemcpyHostToDevice));
-        }
+        h->max_big = big_max;
+        h->max_cells = 0;
+        for (int j : small)
+            h->max_cells = std::max(h->max_cells, h->cells.plane_cell[(size_t)j + 1] - h->cells.plane_cell[(size_t)j]);
         small.insert(small.end(), big.begin(), big.end());
         if (!h->d_plane_list) TDLB_CK(cudaMalloc(&h->d_plane_list, (size_t)g.ny * sizeof(int)));
         TDLB_CK(cudaMemcpy(h->d_plane_list, small.data(), (size_t)g.ny * sizeof(int), cudaMemcpyHostToDevice));
@@ -704,8 +698,8 @@ void upload_markers(tdlb_lattice* h, const tdlb_marker* m, size_t n, size_t n0, 
     {
         std::vector<uint32_t> ms((size_t)h->mask_words, 0u);
         for (int e : h->cells.cell_e) {
-            const int row = e / g.kp, k = e - row * g.kp;
-            ms[(size_t)row * g.kw + (k >> 5)] |= 1u << (k & 31);
+            const int row = e / g.jp, j = e - row * g.jp;
+            ms[(size_t)row * g.jw + (j >> 5)] |= 1u << (j & 31);
         }
         if (!h->d_mask_static) TDLB_CK(cudaMalloc(&h->d_mask_static, (size_t)h->mask_words * sizeof(uint32_t)));
         TDLB_CK(cudaMemcpy(h->d_mask_static, ms.data(), ms.size() * sizeof(uint32_t), cudaMemcpyHostToDevice));
@@ -751,8 +745,8 @@ tdlb::IbmArgs ibm_args(tdlb_lattice* h, float alpha, float beta) {
     a.cell_e = h->d_cell_e;
     a.plane_cell = h->d_plane_cell;
     a.ncell = (int)h->cells.cell_e.size();
-    a.cell_order = h->d_cell_order;
-    a.ncell_big = h->ncell_big;
+    a.max_cells = h->max_cells;
+    a.max_big = h->max_big;
     a.prep = h->d_prep;
     a.cell_m = h->d_cell_m;
     a.cell_F = h->d_cell_F;
@@ -787,18 +781,10 @@ tdlb::IbmArgs ibm_args(tdlb_lattice* h, float alpha, float beta) {
     return a;
 }
 
-// Stream of a forcing pass or blade rotation: the split-step stream when the
-// next step can split, else the handle's stream.
-cudaStream_t ibm_stream(tdlb_lattice* h) {
-    if (split_capable(h)) return loop_stream(h);
-    TDLB_CK(tdlb_rt::join_side(h));
-    return h->stream;
-}
-
 void run_forcing(tdlb_lattice* h, float alpha, float beta) {
     if (!h->markers_set) throw Fail{TDLB_ESTATE, "no markers set (tdlb_set_markers / tdlb_forcing)"};
-    TDLB_CK(tdlb::launch_ibm(ibm_args(h, alpha, beta), ibm_stream(h)));
-    h->launches += (h->cells.cell_e.empty() ? 0 : 1) + (h->n_markers > h->n0 ? 1 : 0) + (h->n_small > 0 ? 1 : 0) +
+    TDLB_CK(tdlb::launch_ibm(ibm_args(h, alpha, beta), h->stream));
+    h->launches += (h->max_cells > 0 ? 1 : 0) + (h->n_big > 0 ? 1 : 0) + (h->n_markers > h->n0 ? 1 : 0) + (h->n_small > 0 ? 1 : 0) +
                    (h->n_big > 0 ? 1 : 0) + (h->n_blade > 0 ? 1 : 0);
     h->pass++;
     h->last_beta = beta;
@@ -815,7 +801,7 @@ void planes_to_host_aos(tdlb_lattice* h, const float* dev, int npl, float* out) 
     for (int i = 0; i < g.nx; i++)
         for (int j = 0; j < g.ny; j++)
             for (int k = 0; k < g.nz; k++, c++) {
-                const size_t e = ((size_t)i * g.ny + j) * g.kp + k;
+                const size_t e = (size_t)g.at(i, j, k);
                 for (int l = 0; l < npl; l++) out[c * npl + l] = tmp[(size_t)l * g.plane + e];
             }
 }
@@ -830,7 +816,7 @@ void force_to_host(tdlb_lattice* h, float* out3) {
     for (int i = 0; i < g.nx; i++)
         for (int j = 0; j < g.ny; j++)
             for (int k = 0; k < g.nz; k++, c++) {
-                const size_t e = ((size_t)i * g.ny + j) * g.kp + k;
+                const size_t e = (size_t)g.at(i, j, k);
                 for (int l = 0; l < 3; l++) out3[c * 3 + l] = tmp[4 * e + (size_t)l];
             }
 }
@@ -842,7 +828,7 @@ void host_aos_to_planes(tdlb_lattice* h, const float* in, int npl, float* dev) {
     for (int i = 0; i < g.nx; i++)
         for (int j = 0; j < g.ny; j++)
             for (int k = 0; k < g.nz; k++, c++) {
-                const size_t e = ((size_t)i * g.ny + j) * g.kp + k;
+                const size_t e = (size_t)g.at(i, j, k);
                 for (int l = 0; l < npl; l++) tmp[(size_t)l * g.plane + e] = in[c * npl + l];
             }
     TDLB_CK(cudaMemcpyAsync(dev, tmp.data(), tmp.size() * sizeof(float), cudaMemcpyHostToDevice, h->stream));
@@ -999,9 +985,9 @@ int tdlb_config_from_json(const char* params_json, tdlb_config* out) {
 
 int tdlb_lattice_bytes(const tdlb_config* c, int64_t* bytes) {
     if (!c || !bytes || c->x < 1 || c->y < 1 || c->z < 1) return TDLB_EINVAL;
-    const long long kp = round_up(c->z, tdlb::kRowPitch), kw = (kp + 31) / 32;
-    const long long plane = round_up(c->x * c->y * kp, 64);
-    const long long mask_words = round_up(c->x * c->y * kw, 64);
+    const long long jp = tdlb::row_pitch(c->x, c->y, c->z), jw = (jp + 31) / 32;
+    const long long plane = round_up(c->x * c->z * jp, 64);
+    const long long mask_words = round_up(c->x * c->z * jw, 64);
     const long long esz = c->storage == TDLB_STORAGE_FP32 ? 4 : 2;
     const long long pops = (long long)tdlb::NQ * plane * esz * (c->streaming == TDLB_STREAMING_SIMPLE ? 2 : 1);
     // fields, flags, and the marker buffers of a tank-wall geometry
@@ -1108,9 +1094,8 @@ int tdlb_read_velocity_density(tdlb_handle h, float* rho, float* ux, float* uy, 
         std::vector<uint32_t> words((size_t)h->mask_words);
         TDLB_CK(cudaMemcpy(words.data(), h->mask_cur(), words.size() * 4, cudaMemcpyDeviceToHost));
         for (size_t c = 0; c < ncell; c++) {
-            const int k = (int)(c % g.nz);
-            const size_t row = c / g.nz;
-            const bool on = (words[row * g.kw + (k >> 5)] >> (k & 31)) & 1u;
+            const int k = (int)(c % g.nz), j = (int)(c / g.nz % g.ny), i = (int)(c / g.nz / g.ny);
+            const bool on = (words[(size_t)g.word(i, j, k)] >> (j & 31)) & 1u;
             const float fx = on ? f[c * 3] : 0.f, fy = on ? f[c * 3 + 1] : 0.f, fz = on ? f[c * 3 + 2] : 0.f;
             const float r = m[c * tdlb::NQ];
             // QVec.hpp:385-394, in the reference's precision
@@ -1132,9 +1117,8 @@ int tdlb_read_force(tdlb_handle h, float* f3) {
         TDLB_CK(cudaMemcpy(words.data(), h->mask_cur(), words.size() * 4, cudaMemcpyDeviceToHost));
         const size_t ncell = (size_t)g.nx * g.ny * g.nz;
         for (size_t c = 0; c < ncell; c++) {
-            const int k = (int)(c % g.nz);
-            const size_t row = c / g.nz;
-            if (!((words[row * g.kw + (k >> 5)] >> (k & 31)) & 1u)) f3[c * 3] = f3[c * 3 + 1] = f3[c * 3 + 2] = 0.f;
+            const int k = (int)(c % g.nz), j = (int)(c / g.nz % g.ny), i = (int)(c / g.nz / g.ny);
+            if (!((words[(size_t)g.word(i, j, k)] >> (j & 31)) & 1u)) f3[c * 3] = f3[c * 3 + 1] = f3[c * 3 + 2] = 0.f;
         }
     });
 }
@@ -1157,15 +1141,14 @@ int tdlb_read_touched(tdlb_handle h, uint8_t* flags) {
         TDLB_CK(cudaStreamSynchronize(h->stream));
         const size_t ncell = (size_t)g.nx * g.ny * g.nz;
         for (size_t c = 0; c < ncell; c++) {
-            const int k = (int)(c % g.nz);
-            const size_t row = c / g.nz;
-            flags[c] = (uint8_t)((words[row * g.kw + (k >> 5)] >> (k & 31)) & 1u);
+            const int k = (int)(c % g.nz), j = (int)(c / g.nz % g.ny), i = (int)(c / g.nz / g.ny);
+            flags[c] = (uint8_t)((words[(size_t)g.word(i, j, k)] >> (j & 31)) & 1u);
         }
     });
 }
 
 int tdlb_get_dims(tdlb_handle h, int64_t* x, int64_t* y, int64_t* z) {
-    return guarded(h, [&] {
+    return guarded<false>(h, [&] {
         if (x) *x = h->g.nx;
         if (y) *y = h->g.ny;
         if (z) *z = h->g.nz;
@@ -1173,7 +1156,7 @@ int tdlb_get_dims(tdlb_handle h, int64_t* x, int64_t* y, int64_t* z) {
 }
 
 int tdlb_get_even_step(tdlb_handle h, int* even) {
-    return guarded(h, [&] {
+    return guarded<false>(h, [&] {
         if (!even) throw Fail{TDLB_EINVAL, "out is NULL"};
         *even = h->even ? 1 : 0;
     });
@@ -1207,23 +1190,19 @@ int tdlb_join(tdlb_handle h) {
 int tdlb_read_zone(tdlb_handle h, uint8_t* flags) {
     return guarded(h, [&] {
         if (!flags) throw Fail{TDLB_EINVAL, "out is NULL"};
-        if (!split_capable(h))
+        if (h->overlap < 0 || tdlb::vector_width(h->g, h->vec) != 1 || !split_capable(h))
             throw Fail{TDLB_ESTATE, "no split step (needs resident markers, one cell per thread, overlap on and, in "
                                     "mode 1, inner chunks holding at most 60 % of the lattice)"};
         const Dims& g = h->g;
-        const std::vector<uint32_t>& bits = h->h_zone_bits;
         size_t c = 0;
-        for (long long i = 0; i < g.nx; i++)
-            for (long long j = 0; j < g.ny; j++)
-                for (long long k = 0; k < g.nz; k++, c++) {
-                    const long long chunk = ((i * g.ny + j) * g.kp + k) / tdlb::kSplitChunk;
-                    flags[c] = (uint8_t)((bits[(size_t)(chunk >> 5)] >> (chunk & 31)) & 1u);
-                }
+        for (int i = 0; i < g.nx; i++)
+            for (int j = 0; j < g.ny; j++)
+                for (int k = 0; k < g.nz; k++, c++) flags[c] = h->h_zone_skip[(size_t)g.word(i, j, k)];
     });
 }
 
 int tdlb_kernel_launches(tdlb_handle h, int64_t* n) {
-    return guarded(h, [&] {
+    return guarded<false>(h, [&] {
         if (!n) throw Fail{TDLB_EINVAL, "out is NULL"};
         *n = (int64_t)h->launches;
     });
@@ -1234,7 +1213,7 @@ int tdlb_set_kernel_timing(tdlb_handle h, int on) {
 }
 
 int tdlb_kernel_time(tdlb_handle h, double* total_ms, int64_t* launches) {
-    return guarded(h, [&] {
+    return guarded<false>(h, [&] {
         TDLB_CK(cudaStreamSynchronize(h->stream));
         double ms = 0.0;
         for (size_t q = 0; q + 1 < h->tev.size(); q += 2) {
@@ -1264,14 +1243,14 @@ int tdlb_reduce_fp64(tdlb_handle h, double* out4) {
 }
 
 int tdlb_get_stream(tdlb_handle h, void** stream) {
-    return guarded(h, [&] {
+    return guarded<false>(h, [&] {
         if (!stream) throw Fail{TDLB_EINVAL, "out is NULL"};
         *stream = (void*)h->stream;
     });
 }
 
 int tdlb_synchronize(tdlb_handle h) {
-    return guarded(h, [&] { TDLB_CK(cudaStreamSynchronize(h->stream)); });
+    return guarded<false>(h, [&] { TDLB_CK(cudaStreamSynchronize(h->stream)); });
 }
 
 int tdlb_attach_rushton(tdlb_handle h, const tdlb_rushton* spec, double nonupdating_delta_angle, double angle,
@@ -1340,15 +1319,14 @@ int tdlb_rotate_impeller(tdlb_handle h, double angle, double delta_angle) {
         if (!h->rot_device) throw Fail{TDLB_ESTATE, "no impeller attached (tdlb_attach_rushton)"};
         // after the previous forcing pass, which reads the blades
         TDLB_CK(tdlb::launch_rotate_markers(h->d_rot_xz, h->d_markers + h->n0, h->n_markers - h->n0, std::cos(angle),
-                                            std::sin(angle), delta_angle, h->rot_ci, h->rot_ck, h->g.nx, h->g.nz,
-                                            ibm_stream(h)));
+                                            std::sin(angle), delta_angle, h->rot_ci, h->rot_ck, h->g.nx, h->g.nz, h->stream));
         h->launches++;
         h->angle = angle;
     });
 }
 
 int tdlb_set_rotating_markers(tdlb_handle h, const tdlb_marker* markers, size_t n) {
-    return guarded(h, [&] {
+    return guarded<false>(h, [&] {
         if (h->impeller_begin < 0) throw Fail{TDLB_ESTATE, "no impeller attached (tdlb_attach_rushton)"};
         if (n != (size_t)(h->n_markers - h->n0)) throw Fail{TDLB_EINVAL, "rotating marker count differs from the attached blades"};
         if (n && !markers) throw Fail{TDLB_EINVAL, "markers is NULL"};
@@ -1393,8 +1371,7 @@ int tdlb_set_rotating_markers(tdlb_handle h, const tdlb_marker* markers, size_t 
         TDLB_CK(cudaEventRecord(st.ev, h->stream));
         h->rot_device = false;   // the blades now follow the host's list
         // a split step needs every blade stencil cell inside the zone
-        if (h->zone_gen == h->marker_gen)
-            h->zone_ok = stencils_inside(h, h->h_markers.data() + h->n0, n, h->h_zone_core);
+        if (h->zone_gen == h->marker_gen && !h->zone_all) h->zone_ok = blades_in_zone(h);
     });
 }
 
@@ -1412,14 +1389,14 @@ void queue_impeller_load(tdlb_lattice* h, double* out5) {
 }
 
 int tdlb_impeller_load(tdlb_handle h, double* out5) {
-    return guarded(h, [&] {
+    return guarded<false>(h, [&] {
         queue_impeller_load(h, out5);
         TDLB_CK(cudaStreamSynchronize(h->stream));
     });
 }
 
 int tdlb_impeller_load_async(tdlb_handle h, double* out5) {
-    return guarded(h, [&] { queue_impeller_load(h, out5); });
+    return guarded<false>(h, [&] { queue_impeller_load(h, out5); });
 }
 
 int tdlb_read_markers(tdlb_handle h, tdlb_marker* out, size_t cap, size_t* n) {
@@ -1488,7 +1465,8 @@ void clear_residual_box(tdlb_lattice* h) { ::clear_rbox(h); }
 tdlb::StepArgs step_args(tdlb_lattice* h, bool collide) { return ::step_args(h, collide); }
 tdlb::IbmArgs ibm_args(tdlb_lattice* h, float alpha, float beta) { return ::ibm_args(h, alpha, beta); }
 void borrow_stream(tdlb_lattice* h, cudaStream_t s) {
-    if (join_side(h) == cudaSuccess) cudaStreamSynchronize(h->stream);
+    fence(h);
+    cudaStreamSynchronize(h->stream);
     if (!h->own_stream) h->own_stream = h->stream;
     h->stream = s;
 }
@@ -1499,13 +1477,17 @@ void return_stream(tdlb_lattice* h) {
     h->own_stream = nullptr;
 }
 
-cudaError_t join_side(tdlb_lattice* h) {
-    if (!h->pending) return cudaSuccess;
-    cudaError_t e = cudaEventRecord(h->ev_sync, h->ibm);
-    if (e == cudaSuccess) e = cudaStreamWaitEvent(h->stream, h->ev_sync, 0);
-    if (e != cudaSuccess) return e;
-    h->pending = false;
-    h->inner_queued = false;
-    return cudaSuccess;
+void drop_zone(tdlb_lattice* h) {
+    cudaFree(h->d_zone_core);
+    cudaFree(h->d_zone_skip);
+    cudaFree(h->d_zone_except);
+    cudaFree(h->d_zone_words);
+    h->d_zone_core = nullptr;
+    h->d_zone_skip = nullptr;
+    h->d_zone_except = nullptr;
+    h->d_zone_words = nullptr;
+    h->zone_cap = 0;
+    h->zone_gen = ~0u;
+    h->h_zone_core.clear();
 }
 }  // namespace tdlb_rt

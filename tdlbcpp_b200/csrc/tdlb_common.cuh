@@ -7,17 +7,23 @@
 // Device layout (one lattice = one "tank"):
 //   * interior cells only (the reference's ghost layer is never read by the
 //     step, so it is not stored);
-//   * cell (i, j, k), 0 <= i < nx, 0 <= j < ny, 0 <= k < nz, row r = i*ny + j,
-//     element e = r*kp + k, kp = row pitch = nz rounded up to kRowPitch
-//     elements (16: every FP32 row starts on a 64-byte boundary);
+//   * cell (i, j, k), 0 <= i < nx, 0 <= j < ny, 0 <= k < nz, row r = i*nz + k,
+//     element e = r*jp + j, jp = row pitch (row_pitch below): j, the vertical
+//     axis of a stirred tank, is the contiguous one. The markers of a tank
+//     (wall, baffles, shaft) repeat from plane to plane of j, so that their
+//     stencil cells form whole rows and the forcing pass reads and writes
+//     full lines; with k contiguous a ring crossed each row in 3 to 7 cells
+//     and every one of the 18 planes cost a line per crossing (B200, 400^3:
+//     gather of the static stencil cells 170 us, 506 B of DRAM per cell);
 //   * 18 population planes (SoA), each `plane` elements long and 256-byte
 //     aligned, addressed through an 18-pointer table;
 //   * F as one float4 (Fx, Fy, Fz, unused) per element -- the forcing pass
 //     reads and writes it at scattered stencil cells, where one 16-byte
 //     access replaces three 4-byte ones in three planes --, Nu as one plane,
-//     and the IBM "touched" flags as one bit per cell: word r*kw + k/32,
-//     bit k%32.
+//     and the IBM "touched" flags as one bit per cell: word r*jw + j/32,
+//     bit j%32.
 #pragma once
+#include <algorithm>
 #include <cstdint>
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
@@ -58,26 +64,51 @@ __host__ inline DivU31 make_div_u31(unsigned d) {
     return r;
 }
 
-// Row pitch granule in elements. 16 FP32 elements = 64-byte rows. 32 (every
-// FP32 row on its own 128-byte L2 line) measured 4 % slower on B200 at 400^3
-// (FP32 Simple step kernel 1.600 -> 1.664 ms, Esotwist 1.670 -> 1.737 ms,
-// FP16 alike): the step's time follows the padded row length (416 against
-// 400 elements) and the line alignment buys nothing back. (Build parameter.)
+// Row pitch granule in elements: 4, the widest vector a thread moves. The
+// step's time follows the padded row length and line alignment buys nothing
+// back: 32 elements (every FP32 row on its own 128-byte line) measured 4 %
+// slower than 16 on B200 at 400^3 (416 against 400 elements; FP32 Simple
+// step kernel 1.600 -> 1.664 ms, Esotwist 1.670 -> 1.737 ms, FP16 alike).
+// (Build parameter.)
 #ifndef TDLB_ROW_PITCH
-#define TDLB_ROW_PITCH 16
+#define TDLB_ROW_PITCH 4
 #endif
 constexpr int kRowPitch = TDLB_ROW_PITCH;
-static_assert(kRowPitch % 16 == 0, "the row pitch is a multiple of 16 elements");
+static_assert(kRowPitch % 4 == 0, "the row pitch is a multiple of 4 elements");
 
 struct Dims {
     int nx, ny, nz;     // interior extent
-    int kp;             // row pitch in elements (multiple of kRowPitch)
-    int kw;             // bitmask words per row
+    int jp;             // row pitch in elements (row_pitch)
+    int jw;             // bitmask words per row
     long long plane;    // elements per population plane (multiple of 64)
-    DivU31 by_ny;       // n / ny
-    DivU31 by_kp16;     // n / (kp / 16)
-    __host__ __device__ long long rows() const { return (long long)nx * ny; }
+    DivU31 by_nz;       // n / nz
+    DivU31 by_nq[3];    // n / (jp / V), V = 1, 2, 4 (where V divides jp)
+    __host__ __device__ long long rows() const { return (long long)nx * nz; }
+    __host__ __device__ long long cells() const { return (long long)nx * ny * nz; }
+    __host__ __device__ long long row(int i, int k) const { return (long long)i * nz + k; }
+    __host__ __device__ long long at(int i, int j, int k) const { return row(i, k) * jp + j; }
+    // word and bit of a cell's flag in a bit-per-cell array
+    __host__ __device__ long long word(int i, int j, int k) const { return row(i, k) * jw + (j >> 5); }
+    // cell t of the interior cells counted along j, then k, then i
+    __host__ __device__ void cell(long long t, int& i, int& j, int& k) const {
+        const long long r = t / ny;
+        j = (int)(t - r * ny);
+        i = (int)(r / nz);
+        k = (int)(r - (long long)i * nz);
+    }
 };
+
+// Most cells a row_pitch may round a plane up to (kernels index planes with
+// int; 64 elements of slack for the plane's own rounding).
+constexpr long long kMaxPlane = (1LL << 31) - 64;
+
+// The row pitch of an nx x ny x nz lattice: ny rounded up to the granule;
+// ny itself where rounding would waste most of the memory (ny below the
+// granule) or push the plane over the 2^31-element limit.
+__host__ inline int row_pitch(long long nx, long long ny, long long nz) {
+    const long long jp = (ny + kRowPitch - 1) / kRowPitch * kRowPitch;
+    return (int)(ny < kRowPitch || nx * nz * jp >= kMaxPlane ? ny : jp);
+}
 
 // Extent, row pitch, plane size and divisors of an nx x ny x nz lattice.
 __host__ inline Dims make_dims(int nx, int ny, int nz) {
@@ -85,12 +116,19 @@ __host__ inline Dims make_dims(int nx, int ny, int nz) {
     g.nx = nx;
     g.ny = ny;
     g.nz = nz;
-    g.kp = (nz + kRowPitch - 1) / kRowPitch * kRowPitch;
-    g.kw = (g.kp + 31) / 32;
-    g.plane = ((long long)nx * ny * g.kp + 63) / 64 * 64;
-    g.by_ny = make_div_u31((unsigned)ny);
-    g.by_kp16 = make_div_u31((unsigned)(g.kp / 16));
+    g.jp = row_pitch(nx, ny, nz);
+    g.jw = (g.jp + 31) / 32;
+    g.plane = ((long long)nx * nz * g.jp + 63) / 64 * 64;
+    g.by_nz = make_div_u31((unsigned)nz);
+    for (int v = 0; v < 3; v++) g.by_nq[v] = make_div_u31((unsigned)std::max(1, g.jp >> v));
     return g;
+}
+
+// The widest cells per thread <= v a lattice's rows take (vectors must not
+// straddle rows): v itself unless the row pitch is not a multiple of it.
+__host__ inline int vector_width(const Dims& g, int v) {
+    while (g.jp % v) v >>= 1;
+    return v;
 }
 
 // 18 plane base pointers of one population buffer. With 16-bit storage the
@@ -166,13 +204,6 @@ struct ResidualBox {
     __device__ __forceinline__ float* at(int s, int i, int j, int k) const {
         return res + (long long)s * n + ((long long)(i - i0) * by + (j - j0)) * bz + (k - k0);
     }
-};
-
-// Scratch outputs of an Esotwist box launch: 19 arrays (the 18 slots' values
-// and Nu) of n entries, one entry per thread of the launch.
-struct BoxOut {
-    float* v = nullptr;
-    long long n = 0;
 };
 
 // Collision constants (FlowParams fields the step reads).

@@ -25,7 +25,7 @@ struct tdlb_lattice {
     float* bufB = nullptr;       // 18 planes (Simple only)
     float* Nu = nullptr;
     float* F = nullptr;          // 3 planes: Fx, Fy, Fz
-    uint32_t* mask = nullptr;    // 2 x (rows * kw) words
+    uint32_t* mask = nullptr;    // 2 x (rows * jw) words
     long long mask_words = 0;
 
     // state
@@ -46,8 +46,7 @@ struct tdlb_lattice {
     // first-segment cell lists and per-pass IBM buffers
     tdlb::CellList cells;
     int* d_cell_e = nullptr;
-    int* d_cell_order = nullptr;  // the big planes' cells first (NULL without big planes)
-    int ncell_big = 0;
+    int max_cells = 0, max_big = 0;   // most cells of an ordinary plane, of a big plane
     int* d_plane_cell = nullptr;
     float* d_prep = nullptr;      // PF_STRIDE * n0
     float* d_cell_m = nullptr;    // 4 * C0 (float4 per cell)
@@ -98,36 +97,39 @@ struct tdlb_lattice {
     int pin_cur = 0;
     std::vector<double> h_rot_xz; // host copy of d_rot_xz
 
-    // Split steps: the outer chunks of a step run on `stream` while the
-    // previous forcing pass and the inner chunks run on `ibm`.
-    cudaStream_t ibm = nullptr;
-    cudaEvent_t ev_outer = nullptr, ev_inner = nullptr, ev_sync = nullptr;
-    int overlap = 0;              // split steps: 0 off, 1 when the zone is small, 2 always (tdlb_set_overlap)
-    bool zone_small = false;      // inner chunks hold at most 60 % of the elements
-    bool pending = false;         // `ibm` holds work that `stream` has not waited for
-    bool inner_queued = false;    // ev_inner marks the inner launch of the last step
+    // Split steps: the outer words of a step run on `bulk`, beside the previous
+    // forcing pass and the inner words on `stream`, which then waits for them:
+    // work queued on `stream` after a step sees all of it.
+    cudaStream_t bulk = nullptr;
+    cudaEvent_t ev_outer = nullptr, ev_inner = nullptr, ev_fence = nullptr;
+    int overlap = -1;             // split steps: 0 off, 1 when the zone is small, 2 always (tdlb_set_overlap);
+                                  // -1: as 1, for lattices large enough
+    bool bulk_ok = false;         // nothing but step-loop work queued since ev_inner: the next outer
+                                  // launch waits for that event alone
     bool resident = false;        // markers kept for many passes (set/attach), so a zone pays
-    unsigned zone_gen = ~0u;      // marker_gen the zone was built for
-    bool zone_ok = false;         // every stencil cell of the current markers lies in the zone
-    std::vector<uint64_t> h_zone_core;   // 1 bit per element: the stencil cells the zone covers
-    std::vector<uint32_t> h_zone_bits;   // 1 bit per 32-element chunk, set for the inner chunks
-    int* d_zone_list = nullptr;          // the inner chunks, then the outer chunks, each ascending
-    int n_zone = 0, n_outer = 0;
-    long long zone_list_cap = 0;
+    // the zone (zone.cu), for marker_gen zone_gen and box_gen zone_box_gen
+    unsigned zone_gen = ~0u, zone_box_gen = ~0u;
+    bool zone_all = false;        // every word is in it (markers that change every pass)
+    bool zone_ok = false;         // every stencil cell of the current markers lies in it
+    bool zone_small = false;      // it holds at most 60 % of the cells
+    uint32_t* d_zone_core = nullptr;     // 1 bit per cell: the stencil cells
+    uint8_t* d_zone_skip = nullptr;      // 1 byte per flag word: in the zone
+    uint32_t* d_zone_except = nullptr;   // 1 bit per cell: the residual box's cells (when there is a box)
+    int* d_zone_words = nullptr;         // the zone's words, ascending
+    long long zone_cap = 0;              // words the arrays hold
+    int n_zone = 0, n_outer = 0;         // words inside, outside
+    std::vector<uint8_t> h_zone_skip;
+    std::vector<uint32_t> h_zone_core;   // filled when host blades are checked against it
     // 16-bit storage: the residual box (tdlb::ResidualBox) and its residuals,
     // one set per population buffer (Simple: A and B; Esotwist: one)
     tdlb::ResidualBox rbox_geom{};        // geometry only (res unused)
     float* d_res[2] = {nullptr, nullptr};
     bool rbox_auto = true;                // set from the impeller by tdlb_attach_rushton
     unsigned box_gen = 0;                 // bumped by every change of the box
-    // chunks with a cell near the box (the box launch of a step), ascending,
-    // and the Esotwist box launch's scratch outputs (NQ + 1 floats per
-    // thread of that launch)
+    // elements of the cells the box launch of a step takes, ascending
     int* d_box_list = nullptr;
     int n_box = 0;
     long long box_list_cap = 0;
-    float* d_box_out = nullptr;
-    long long box_out_cap = 0;            // floats
     unsigned box_list_gen = ~0u;          // box_gen the list was built for
     // step-kernel timing (tdlb_set_kernel_timing): start/stop event pairs
     bool timing = false;
@@ -185,9 +187,12 @@ tdlb::IbmArgs ibm_args(tdlb_lattice* h, float alpha, float beta);
 void borrow_stream(tdlb_lattice* h, cudaStream_t s);
 // Undo borrow_stream: h's work goes to its own stream again.
 void return_stream(tdlb_lattice* h);
-// Make `stream` wait for the forcing pass and inner launches queued on the
-// split-step stream (every entry point other than the step loop calls it).
-cudaError_t join_side(tdlb_lattice* h);
+// Work other than the step loop's own is about to be queued on `stream`: the
+// next outer launch of a split step waits for it (every entry point other than
+// the step loop's calls it).
+inline void fence(tdlb_lattice* h) { h->bulk_ok = false; }
+// Free the zone's arrays (the lattice changed size).
+void drop_zone(tdlb_lattice* h);
 // Remove the residual box (a tank joining a batch, whose step kernel keeps
 // none), or set its residuals to zero (after the planes were written
 // without them).

@@ -5,16 +5,19 @@
 
 namespace tdlb {
 
-// Chunks of a split step (32 consecutive elements of the flat row*kp + k
-// index, one warp each): the launch takes chunks[0, count). A full launch
-// (part 0) takes no list; l2_ahead > 0 turns on its L2 prefetch, that many
-// CTAs ahead of the walk (step_kernels.cuh).
+// Which cells a step launch takes (step_kernels.cuh). Cells are told apart by
+// flag words, the 32 cells of a row whose touched flags share a word: part 1
+// takes the words whose `skip` byte is zero, part 2 the words of a list,
+// without the cells whose bit is set in `except` (NULL: all of them). Part 0
+// takes every cell. l2_ahead > 0 turns on the L2 prefetch of parts 0 and 1,
+// that many CTAs ahead of the walk.
 struct StepPart {
-    const int* chunks;
+    const uint8_t* skip;
+    const int* words;
     int count;
+    const uint32_t* except;
     int l2_ahead;
 };
-constexpr int kSplitChunk = 32;
 
 // One wave of resident 128-thread CTAs of kernel K on the current device (the
 // occupancy its register count allows, times the SMs): the L2 prefetch
@@ -52,21 +55,21 @@ struct StepArgs {
     int vec;                // cells per thread: 1, 2 or 4 (float, float2, float4 traffic)
     int l2_prefetch;        // full launches of the population form: L2 prefetch one wave ahead
     int storage;            // StorageKind of the population planes
-    int part;               // 0: every cell; 1: outer chunks; 2: inner chunks (vec == 1, populations)
-    StepPart zone;          // the chunks of part 1 or 2 (box == 2: the chunks near the residual box)
-    ResidualBox rr;         // 16-bit storage, one cell per thread: residuals of the locations read ...
+    int part;               // 0: every cell; 1: outer words; 2: inner words (populations; FP32: vec == 1)
+    StepPart zone;          // the words of part 1 or 2
+    ResidualBox rr;         // 16-bit storage: residuals of the locations read ...
     ResidualBox rw;         // ... and written (Simple: of buffer A and B; Esotwist: the same box)
-    int box;                // 0: no residual box; 2: the box launch over `zone` (the chunks near the box, part 2)
-    BoxOut bout;            // box launch: its scratch outputs
+    const int* box_cells;   // elements of the cells the box launch steps
+    int n_box;
 };
 
-// The StepPart a launch of kernel K takes: the chunk list (parts 1 and 2) or,
-// for a full launch of the population form (FULL) with a.l2_prefetch on, the
-// L2 prefetch distance of one wave of K's resident CTAs.
+// The StepPart a launch of kernel K takes: a.zone, with, for a launch over the
+// whole lattice of the population form (FULL) and a.l2_prefetch on, the L2
+// prefetch distance of one wave of K's resident CTAs.
 template <auto K, bool FULL>
 StepPart launch_walk(const StepArgs& a) {
     StepPart w = a.zone;
-    w.l2_ahead = FULL && a.part == 0 && a.l2_prefetch ? wave_ctas<K>() : 0;
+    w.l2_ahead = FULL && a.part != 2 && a.l2_prefetch ? wave_ctas<K>() : 0;
     return w;
 }
 
@@ -74,9 +77,20 @@ cudaError_t launch_step_simple(const StepArgs& a, cudaStream_t st);
 cudaError_t launch_step_esotwist(const StepArgs& a, cudaStream_t st);
 cudaError_t launch_step_simple_h16(const StepArgs& a, cudaStream_t st);
 cudaError_t launch_step_esotwist_h16(const StepArgs& a, cudaStream_t st);
-// After the plain launch of a step with a residual box: the box launch's
-// outputs (a.bout) to the cells of a.zone (k_box_commit).
-cudaError_t launch_box_commit(const StepArgs& a, bool simple, cudaStream_t st);
+// The box cells of a step with a residual box (the other launches leave them out).
+cudaError_t launch_box(const StepArgs& a, bool simple, cudaStream_t st);
+
+// ---- the zone of a split step (zone.cu) ----
+// core: a bit for every cell in a stencil of the resident markers at any
+// impeller angle: the static flags, and per plane j the annulus
+// [ring[j].x, ring[j].y] about (ci, ck) (none where y < 0).
+cudaError_t launch_zone_core(const Dims& g, const uint32_t* mask_static, const double2* ring, double ci, double ck,
+                             uint32_t* core, cudaStream_t st);
+// skip: a byte per word, 1 where the word holds a core cell or (neighbours) a
+// periodic neighbour of one; core NULL: every word.
+cudaError_t launch_zone_words(const Dims& g, const uint32_t* core, int neighbours, uint8_t* skip, cudaStream_t st);
+// Box cells: their bits in `except` (zeroed by the caller), their words in skip.
+cudaError_t launch_zone_box(const Dims& g, const int* cells, int n, uint32_t* except, uint8_t* skip, cudaStream_t st);
 cudaError_t launch_fill_uniform_moments(Planes Q, const Dims& g, float rho, cudaStream_t st);
 cudaError_t launch_state_moments(Planes A, Planes M, const Dims& g, int mode, int even, cudaStream_t st, int storage,
                                  const CollideParams& p, const ResidualBox& rb = ResidualBox{});
@@ -122,8 +136,7 @@ struct IbmArgs {
     const int* cell_e;          // [C0] element index of each cell
     const int* plane_cell;      // [ny+1] cell range of each plane
     int ncell;                  // C0
-    const int* cell_order;      // [C0] the big planes' cells, then the others (NULL: no big plane)
-    int ncell_big;              // cells of the big planes
+    int max_cells, max_big;     // most cells of an ordinary plane, of a big plane
     const float* prep;          // PF_STRIDE * n0: one row per first-segment slot
     float* cell_m;              // C0 float4: rho, jx, jy, jz of each cell this pass
     float* cell_F;              // 3 * C0: F of each cell at the start of this pass
@@ -157,7 +170,7 @@ cudaError_t launch_ibm(const IbmArgs& a, cudaStream_t st);
 
 // Immersed-boundary passes of many lattices in one set of launches: device
 // IbmArgs per lattice and work lists of (lattice, first index) items --
-// cells: 256 first-segment cells; tails: 128 blade markers; copies: 1024
+// cells: places 8 (y >> 10) .. + 8 of the planes 32 (y & 1023) .. + 32; tails: 128 blade markers; copies: 1024
 // touched-flag words; small / big: one j-plane (128 / 512 threads).
 struct IbmBatch {
     const IbmArgs* args;

@@ -141,17 +141,18 @@ struct MarkerSchedule {
     }
 };
 
-// Unique stencil cells of the first segment, per plane and sorted by
+// Unique stencil cells of the first segment, per plane j and sorted by
 // (i, k), with each slot's 9 plane-local cell indices. The per-pass IBM
 // work is then done once per cell instead of once per (marker, cell): every
 // wall cell is shared by about three markers.
 struct CellList {
-    std::vector<int> cell_e;       // element index (row*kp + k) of each cell
+    std::vector<int> cell_e;       // element index (Dims::at) of each cell
     std::vector<int> plane_cell;   // [ny+1] cell range of each plane
     std::vector<int> mcell;        // [n0][9]: plane-local cell index of stencil cell c of slot p
     int max_plane_cells = 0;
 
-    void build(const Marker* m, const MarkerSchedule& seg0, int nx, int ny, int nz, int kp) {
+    void build(const Marker* m, const MarkerSchedule& seg0, const Dims& g) {
+        const int nx = g.nx, ny = g.ny, nz = g.nz;
         const int n0 = (int)seg0.order.size();
         cell_e.clear();
         mcell.assign((size_t)9 * n0, 0);
@@ -177,7 +178,7 @@ struct CellList {
             for (size_t t = 0; t < cells.size(); t++) {
                 slot[(size_t)cells[t]] = (int)t;
                 const int i = cells[t] / nz, k = cells[t] - i * nz;
-                cell_e.push_back((i * ny + j) * kp + k);
+                cell_e.push_back((int)g.at(i, j, k));
             }
             for (int p = p0; p < p1; p++) {
                 int st[9];
