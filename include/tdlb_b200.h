@@ -157,6 +157,9 @@ int tdlb_read_moments(tdlb_handle h, float* out);
  * interior cell, each array x*y*z in (i, j, k) order. Any pointer may be
  * NULL. */
 int tdlb_read_velocity_density(tdlb_handle h, float* rho, float* ux, float* uy, float* uz);
+/* The same with the velocity interleaved, u3[((i*y + j)*z + k)*3 + c]; rho may
+ * be NULL. */
+int tdlb_read_density_velocity3(tdlb_handle h, float* rho, float* u3);
 
 /* Interior F (3 per cell, AoS; zero where no marker touched the cell), the
  * eddy viscosity Nu (1 per cell) and the touched flags of the last forcing

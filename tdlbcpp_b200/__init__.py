@@ -193,6 +193,7 @@ def load_library() -> ctypes.CDLL:
         "tdlb_step": (i32, [H, f32, f32]),
         "tdlb_read_moments": (i32, [H, vp]),
         "tdlb_read_velocity_density": (i32, [H, vp, vp, vp, vp]),
+        "tdlb_read_density_velocity3": (i32, [H, vp, vp]),
         "tdlb_read_force": (i32, [H, vp]),
         "tdlb_read_nu": (i32, [H, vp]),
         "tdlb_read_touched": (i32, [H, vp]),
@@ -546,9 +547,9 @@ class ComputeUnit:
 
     def read_velocity_density(self):
         shape = (self.x, self.y, self.z)
-        rho, ux, uy, uz = (np.empty(shape, np.float32) for _ in range(4))
-        self._check(self.lib.tdlb_read_velocity_density(self.h, _p(rho), _p(ux), _p(uy), _p(uz)))
-        return rho, np.stack([ux, uy, uz], axis=-1)
+        rho, u = np.empty(shape, np.float32), np.empty(shape + (3,), np.float32)
+        self._check(self.lib.tdlb_read_density_velocity3(self.h, _p(rho), _p(u)))
+        return rho, u
 
     def read_force(self) -> np.ndarray:
         out = np.empty((self.x, self.y, self.z, 3), np.float32)

@@ -139,13 +139,4 @@ cudaError_t launch_fill_uniform_moments(Planes Q, const Dims& g, float rho, cuda
     return cudaGetLastError();
 }
 
-cudaError_t launch_state_moments(Planes A, Planes M, const Dims& g, int mode, int even, cudaStream_t st, int storage,
-                                 const CollideParams& p, const ResidualBox& rb) {
-    const unsigned blocks = blocks_for(g.cells(), 256);
-    with_storage(storage, [&](auto s) {
-        k_state_moments<decltype(s)><<<blocks, 256, 0, st>>>(A, M, g, mode, even, p, rb);
-    });
-    return cudaGetLastError();
-}
-
 }  // namespace tdlb

@@ -745,9 +745,8 @@ __global__ void __launch_bounds__(128) k_box_step(Planes A, Planes B, float* __r
     if (LES) Nu[q.e0] = nu[0];
 }
 
-// Moments of the current state at every interior cell (what the reference's
-// Q holds after moments()), written to 18 FP32 output planes of the same
-// layout. mode: 0 = Simple populations (pull), 1 = moments (own cell),
+// Moments of the current state at an interior cell (what the reference's Q
+// holds after moments()). mode: 0 = Simple populations (pull), 1 = moments (own cell),
 // 2 = Esotwist populations (read map, parity `even`), 3 = Esotwist moments.
 template <typename S>
 __device__ __forceinline__ void state_moments18(const Planes& A, const Dims& g, int mode, int even, const CollideParams& p,
@@ -791,20 +790,6 @@ __device__ __forceinline__ void state_moments18(const Planes& A, const Dims& g, 
 #pragma unroll
         for (int d = 0; d < NQ; d++) m[d] = q[d];
     }
-}
-
-template <typename S>
-__global__ void __launch_bounds__(256) k_state_moments(Planes A, Planes M, Dims g, int mode, int even, CollideParams p,
-                                                       ResidualBox rb) {
-    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= g.cells()) return;
-    int i, j, k;
-    g.cell(t, i, j, k);
-    float m[NQ];
-    state_moments18<S>(A, g, mode, even, p, i, j, k, m, rb);
-    const long long e = g.at(i, j, k);
-#pragma unroll
-    for (int d = 0; d < NQ; d++) M.p[d][e] = m[d];
 }
 
 }  // namespace tdlb

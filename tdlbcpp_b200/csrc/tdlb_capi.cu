@@ -70,6 +70,7 @@ void release(tdlb_lattice* h) {
     cudaFree(h->d_exclude);
     tdlb_rt::drop_zone(h);
     cudaFree(h->d_box_list);
+    cudaFree(h->d_scratch);
     for (cudaEvent_t e : h->tev) cudaEventDestroy(e);
     if (h->side) cudaStreamDestroy(h->side);
     if (h->bulk) cudaStreamDestroy(h->bulk);
@@ -790,37 +791,6 @@ void run_forcing(tdlb_lattice* h, float alpha, float beta) {
     h->last_beta = beta;
 }
 
-// Copy an interior-cell plane set (npl planes of the device layout) to a
-// host AoS array out[cell*npl + l], cells in (i, j, k) order.
-void planes_to_host_aos(tdlb_lattice* h, const float* dev, int npl, float* out) {
-    const Dims& g = h->g;
-    std::vector<float> tmp((size_t)npl * g.plane);
-    TDLB_CK(cudaMemcpyAsync(tmp.data(), dev, tmp.size() * sizeof(float), cudaMemcpyDeviceToHost, h->stream));
-    TDLB_CK(cudaStreamSynchronize(h->stream));
-    size_t c = 0;
-    for (int i = 0; i < g.nx; i++)
-        for (int j = 0; j < g.ny; j++)
-            for (int k = 0; k < g.nz; k++, c++) {
-                const size_t e = (size_t)g.at(i, j, k);
-                for (int l = 0; l < npl; l++) out[c * npl + l] = tmp[(size_t)l * g.plane + e];
-            }
-}
-
-// The force field (one float4 per element) as (Fx, Fy, Fz) per interior cell.
-void force_to_host(tdlb_lattice* h, float* out3) {
-    const Dims& g = h->g;
-    std::vector<float> tmp((size_t)4 * g.plane);
-    TDLB_CK(cudaMemcpyAsync(tmp.data(), h->F, tmp.size() * sizeof(float), cudaMemcpyDeviceToHost, h->stream));
-    TDLB_CK(cudaStreamSynchronize(h->stream));
-    size_t c = 0;
-    for (int i = 0; i < g.nx; i++)
-        for (int j = 0; j < g.ny; j++)
-            for (int k = 0; k < g.nz; k++, c++) {
-                const size_t e = (size_t)g.at(i, j, k);
-                for (int l = 0; l < 3; l++) out3[c * 3 + l] = tmp[4 * e + (size_t)l];
-            }
-}
-
 void host_aos_to_planes(tdlb_lattice* h, const float* in, int npl, float* dev) {
     const Dims& g = h->g;
     std::vector<float> tmp((size_t)npl * g.plane, 0.f);
@@ -834,25 +804,6 @@ void host_aos_to_planes(tdlb_lattice* h, const float* in, int npl, float* dev) {
     TDLB_CK(cudaMemcpyAsync(dev, tmp.data(), tmp.size() * sizeof(float), cudaMemcpyHostToDevice, h->stream));
     TDLB_CK(cudaStreamSynchronize(h->stream));
 }
-
-// Moments of the current state into a temporary 18-plane device buffer.
-float* state_moments(tdlb_lattice* h) {
-    float* M = nullptr;
-    TDLB_CK(cudaMalloc(&M, (size_t)tdlb::NQ * h->g.plane * sizeof(float)));
-    cudaError_t e = tdlb::launch_state_moments(h->planes(h->state_buf()), h->planes32(M), h->g, h->state_mode(),
-                                               h->even ? 1 : 0, h->stream, h->cfg.storage, h->cp,
-                                               h->rbox(h->state_index()));
-    if (e != cudaSuccess) {
-        cudaFree(M);
-        throw Fail{TDLB_ECUDA, std::string("state moments: ") + cudaGetErrorString(e)};
-    }
-    return M;
-}
-
-struct DevBuf {
-    float* p;
-    ~DevBuf() { cudaFree(p); }
-};
 
 // ---------------------------------------------------------------------------
 // Residual box of the 16-bit storage (tdlb::ResidualBox): exact deviations
@@ -1069,81 +1020,6 @@ int tdlb_step(tdlb_handle h, float alpha, float beta) {
         require_init(h);
         run_step(h, true);
         run_forcing(h, alpha, beta);
-    });
-}
-
-int tdlb_read_moments(tdlb_handle h, float* out) {
-    return guarded(h, [&] {
-        require_init(h);
-        if (!out) throw Fail{TDLB_EINVAL, "out is NULL"};
-        DevBuf M{state_moments(h)};
-        planes_to_host_aos(h, M.p, tdlb::NQ, out);
-    });
-}
-
-int tdlb_read_velocity_density(tdlb_handle h, float* rho, float* ux, float* uy, float* uz) {
-    return guarded(h, [&] {
-        require_init(h);
-        const Dims& g = h->g;
-        DevBuf M{state_moments(h)};
-        const size_t ncell = (size_t)g.nx * g.ny * g.nz;
-        std::vector<float> m(ncell * tdlb::NQ), f(ncell * 3);
-        planes_to_host_aos(h, M.p, tdlb::NQ, m.data());
-        force_to_host(h, f.data());
-        std::vector<uint8_t> t(ncell);
-        std::vector<uint32_t> words((size_t)h->mask_words);
-        TDLB_CK(cudaMemcpy(words.data(), h->mask_cur(), words.size() * 4, cudaMemcpyDeviceToHost));
-        for (size_t c = 0; c < ncell; c++) {
-            const int k = (int)(c % g.nz), j = (int)(c / g.nz % g.ny), i = (int)(c / g.nz / g.ny);
-            const bool on = (words[(size_t)g.word(i, j, k)] >> (j & 31)) & 1u;
-            const float fx = on ? f[c * 3] : 0.f, fy = on ? f[c * 3 + 1] : 0.f, fz = on ? f[c * 3 + 2] : 0.f;
-            const float r = m[c * tdlb::NQ];
-            // QVec.hpp:385-394, in the reference's precision
-            if (rho) rho[c] = r;
-            if (ux) ux[c] = (float)((1.0 / r) * (m[c * tdlb::NQ + 1] + 0.5 * fx));
-            if (uy) uy[c] = (float)((1.0 / r) * (m[c * tdlb::NQ + 2] + 0.5 * fy));
-            if (uz) uz[c] = (float)((1.0 / r) * (m[c * tdlb::NQ + 3] + 0.5 * fz));
-        }
-    });
-}
-
-int tdlb_read_force(tdlb_handle h, float* f3) {
-    return guarded(h, [&] {
-        require_init(h);
-        if (!f3) throw Fail{TDLB_EINVAL, "out is NULL"};
-        const Dims& g = h->g;
-        force_to_host(h, f3);
-        std::vector<uint32_t> words((size_t)h->mask_words);
-        TDLB_CK(cudaMemcpy(words.data(), h->mask_cur(), words.size() * 4, cudaMemcpyDeviceToHost));
-        const size_t ncell = (size_t)g.nx * g.ny * g.nz;
-        for (size_t c = 0; c < ncell; c++) {
-            const int k = (int)(c % g.nz), j = (int)(c / g.nz % g.ny), i = (int)(c / g.nz / g.ny);
-            if (!((words[(size_t)g.word(i, j, k)] >> (j & 31)) & 1u)) f3[c * 3] = f3[c * 3 + 1] = f3[c * 3 + 2] = 0.f;
-        }
-    });
-}
-
-int tdlb_read_nu(tdlb_handle h, float* nu) {
-    return guarded(h, [&] {
-        require_init(h);
-        if (!nu) throw Fail{TDLB_EINVAL, "out is NULL"};
-        planes_to_host_aos(h, h->Nu, 1, nu);
-    });
-}
-
-int tdlb_read_touched(tdlb_handle h, uint8_t* flags) {
-    return guarded(h, [&] {
-        require_init(h);
-        if (!flags) throw Fail{TDLB_EINVAL, "out is NULL"};
-        const Dims& g = h->g;
-        std::vector<uint32_t> words((size_t)h->mask_words);
-        TDLB_CK(cudaMemcpyAsync(words.data(), h->mask_cur(), words.size() * 4, cudaMemcpyDeviceToHost, h->stream));
-        TDLB_CK(cudaStreamSynchronize(h->stream));
-        const size_t ncell = (size_t)g.nx * g.ny * g.nz;
-        for (size_t c = 0; c < ncell; c++) {
-            const int k = (int)(c % g.nz), j = (int)(c / g.nz % g.ny), i = (int)(c / g.nz / g.ny);
-            flags[c] = (uint8_t)((words[(size_t)g.word(i, j, k)] >> (j & 31)) & 1u);
-        }
     });
 }
 
@@ -1429,14 +1305,6 @@ int tdlb_schedule_levels(const tdlb_marker* markers, size_t n, int64_t x, int64_
     }
     if (max_levels_per_plane) *max_levels_per_plane = s.max_levels_per_plane;
     return TDLB_OK;
-}
-
-int tdlb_debug_get_state(tdlb_handle h, float* out) {
-    return guarded(h, [&] {
-        if (!out) throw Fail{TDLB_EINVAL, "out is NULL"};
-        if (h->cfg.storage != TDLB_STORAGE_FP32) throw Fail{TDLB_EINVAL, "raw state access needs FP32 storage"};
-        planes_to_host_aos(h, h->state_buf(), tdlb::NQ, out);
-    });
 }
 
 int tdlb_debug_set_state(tdlb_handle h, const float* in, int holds_moments) {

@@ -131,6 +131,9 @@ struct tdlb_lattice {
     int n_box = 0;
     long long box_list_cap = 0;
     unsigned box_list_gen = ~0u;          // box_gen the list was built for
+    // device scratch of the read-back (a slab of output) and the plane dumps
+    void* d_scratch = nullptr;
+    size_t scratch_bytes = 0;
     // step-kernel timing (tdlb_set_kernel_timing): start/stop event pairs
     bool timing = false;
     std::vector<cudaEvent_t> tev;

@@ -92,8 +92,6 @@ cudaError_t launch_zone_words(const Dims& g, const uint32_t* core, int neighbour
 // Box cells: their bits in `except` (zeroed by the caller), their words in skip.
 cudaError_t launch_zone_box(const Dims& g, const int* cells, int n, uint32_t* except, uint8_t* skip, cudaStream_t st);
 cudaError_t launch_fill_uniform_moments(Planes Q, const Dims& g, float rho, cudaStream_t st);
-cudaError_t launch_state_moments(Planes A, Planes M, const Dims& g, int mode, int even, cudaStream_t st, int storage,
-                                 const CollideParams& p, const ResidualBox& rb = ResidualBox{});
 
 // ---- immersed boundary ----
 
