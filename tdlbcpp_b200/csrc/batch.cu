@@ -374,7 +374,7 @@ void build_ibm_work(tdlb_batch_s* b) {
                 for (int jg = 0; jg < h->g.ny; jg += 32) {
                     bool any = false;   // a tile past every plane's cells is left out
                     for (int j = jg; j < std::min(jg + 32, h->g.ny); j++)
-                        any = any || h->cells.plane_cell[(size_t)j + 1] - h->cells.plane_cell[(size_t)j] > p;
+                        any = any || h->plane_cell[(size_t)j + 1] - h->plane_cell[(size_t)j] > p;
                     if (any) cells.push_back(make_int2(t, (p / 8) << 10 | jg / 32));
                 }
             for (int q = 0; q < h->n_markers - h->n0; q += 128) tails.push_back(make_int2(t, q));

@@ -1046,8 +1046,7 @@ cudaError_t ibm_prepare_smem(int small_cells, int n_small, size_t big_bytes) {
     return raise_smem_limit((const void*)k_ibm_spread_bulk<512, 1, false>, big_bytes);
 }
 
-cudaError_t launch_ibm_prepare(const IbmArgs& a, float* prep, const int* mcell, cudaStream_t st) {
-    (void)mcell;
+cudaError_t launch_ibm_prepare(const IbmArgs& a, float* prep, cudaStream_t st) {
     if (a.n0 <= 0) return cudaSuccess;
     k_ibm_prepare<<<(a.n0 + 255) / 256, 256, 0, st>>>(a, prep);
     return cudaGetLastError();

@@ -149,8 +149,13 @@ int tdlb_double_resolution(tdlb_handle h) {
     h->impeller_begin = -1;
     h->n_markers = 0;
     h->n0 = 0;
-    h->h_markers.clear();
-    h->cells = tdlb::CellList{};
+    h->h_blades.clear();
+    h->h_blade_planes.clear();
+    h->n_blade = 0;
+    h->plane_cell.clear();
+    h->ncell = 0;
+    h->n_level0 = 0;
+    drop(h->d_blade_planes);
     drop(h->d_plane_lv0);
     drop(h->d_plane_lv1);
     drop(h->d_plane_cell);

@@ -53,6 +53,8 @@ void release(tdlb_lattice* h) {
     cudaFree(h->F);
     cudaFree(h->mask);
     cudaFree(h->d_markers);
+    cudaFree(h->d_markers_in);
+    cudaFree(h->d_sched_tmp);
     cudaFree(h->d_sched);
     cudaFree(h->d_level_ptr);
     cudaFree(h->d_plane_lv0);
@@ -308,7 +310,7 @@ bool blades_in_zone(tdlb_lattice* h) {
                                 cudaMemcpyDeviceToHost, h->stream));
         TDLB_CK(cudaStreamSynchronize(h->stream));
     }
-    return stencils_inside(h->g, h->h_markers.data() + h->n0, n1, h->h_zone_core);
+    return stencils_inside(h->g, h->h_blades.data(), n1, h->h_zone_core);
 }
 
 // `all`: every word, whatever the markers (they change with every pass).
@@ -333,7 +335,7 @@ void build_zone(tdlb_lattice* h, bool all) {
         // position per axis, so within r +- 2.13 of the axis: plane by plane,
         // the annulus between the smallest and the largest blade radius
         // widened by 3 cells.
-        const tdlb_marker* rot = h->h_markers.data() + h->n0;
+        const tdlb_marker* rot = h->h_blades.data();
         std::vector<double2> ring((size_t)g.ny, make_double2(1e300, -1.0));
         for (int q = 0; q < n1; q++) {
             const double r = std::sqrt(h->h_rot_xz[2 * q] * h->h_rot_xz[2 * q] + h->h_rot_xz[2 * q + 1] * h->h_rot_xz[2 * q + 1]);
@@ -578,7 +580,7 @@ void update_blade_planes(tdlb_lattice* h) {
     const Dims& g = h->g;
     const auto& lv = h->seg1.plane_lv;
     const auto& lp = h->seg1.level_ptr;
-    const int L0 = h->seg0.nlevels;
+    const int L0 = h->n_level0;
     std::vector<int> planes;
     int words = 0;
     for (int j = 0; j < g.ny; j++) {
@@ -601,10 +603,18 @@ void update_blade_planes(tdlb_lattice* h) {
     h->blade_words = std::max(h->blade_words, words);
 }
 
+// Schedule of the second segment (h_blades), slots n0.., levels n_level0...
+void build_blades(tdlb_lattice* h, const double* rot_xz) {
+    const Dims& g = h->g;
+    h->seg1.build(reinterpret_cast<const tdlb::Marker*>(h->h_blades.data()), 0, (int)h->h_blades.size(), g.nx, g.ny, g.nz,
+                  h->n0, h->n_level0, rot_xz);
+    for (int& q : h->seg1.order) q += h->n0;   // list indices
+}
+
 void upload_seg1(tdlb_lattice* h) {
     const Dims& g = h->g;
     update_blade_planes(h);
-    const int L0 = h->seg0.nlevels;
+    const int L0 = h->n_level0;
     ensure_level_cap(h, (long long)L0 + h->seg1.nlevels + 1);
     const int n1 = h->n_markers - h->n0;
     if (n1) TDLB_CK(cudaMemcpyAsync(h->d_sched + h->n0, h->seg1.order.data(), (size_t)n1 * sizeof(int),
@@ -615,29 +625,158 @@ void upload_seg1(tdlb_lattice* h) {
                             cudaMemcpyHostToDevice, h->stream));
 }
 
+// Grow a device buffer to at least `need` elements (contents not kept; the
+// stream's work is waited for by the free).
+template <typename T>
+void grow(T*& p, long long& cap, long long need, long long per) {
+    if (need <= cap && p) return;
+    cudaFree(p);
+    p = nullptr;
+    cap = 0;
+    const long long n = round_up(need + need / 8, 1024);
+    TDLB_CK(cudaMalloc(&p, (size_t)(n * per) * sizeof(T)));
+    cap = n;
+}
+
+// What the host knows of the first segment's cells: the planes' ranges, the
+// launches' shapes and tiles.
+void plan_planes(tdlb_lattice* h, const int* count) {
+    const Dims& g = h->g;
+    h->plane_cell.assign((size_t)g.ny + 1, 0);
+    for (int j = 0; j < g.ny; j++) h->plane_cell[(size_t)j + 1] = h->plane_cell[(size_t)j] + count[j];
+    h->ncell = h->plane_cell[(size_t)g.ny];
+    // F tiles of the ordinary planes' launch: up to 6144 cells (72 KB) of
+    // shared memory; the tile is sized for the most crowded ordinary plane, at
+    // least 4608 cells. Planes with more cells (an impeller disk) go to a
+    // second, 512-thread launch with a tile for the largest of them (global
+    // memory beyond the 227 KB shared-memory limit).
+    int typical = 0;
+    for (int j = 0; j < g.ny; j++)
+        if (count[j] <= 6144) typical = std::max(typical, count[j]);
+    const int small_cap = std::max(4608, round_up(typical, 64) > 6144 ? 6144 : (int)round_up(typical, 64));
+    std::vector<int> small, big;
+    h->max_cells = h->max_big = 0;
+    for (int j = 0; j < g.ny; j++) {
+        if (count[j] > small_cap) { big.push_back(j); h->max_big = std::max(h->max_big, count[j]); }
+        else { small.push_back(j); h->max_cells = std::max(h->max_cells, count[j]); }
+    }
+    h->smem_cells = small_cap;
+    h->n_small = (int)small.size();
+    h->n_big = (int)big.size();
+    h->big_tile_cells = tdlb::big_bulk_bytes(h->max_big) <= 220 * 1024 ? h->max_big : 0;
+    TDLB_CK(tdlb::ibm_prepare_smem(h->smem_cells, h->n_small, tdlb::big_bulk_bytes(h->big_tile_cells)));
+    small.insert(small.end(), big.begin(), big.end());
+    if (!h->d_plane_list) TDLB_CK(cudaMalloc(&h->d_plane_list, (size_t)g.ny * sizeof(int)));
+    TDLB_CK(cudaMemcpyAsync(h->d_plane_list, small.data(), (size_t)g.ny * sizeof(int), cudaMemcpyHostToDevice, h->stream));
+    if (!h->d_plane_cell) TDLB_CK(cudaMalloc(&h->d_plane_cell, (size_t)(g.ny + 1) * sizeof(int)));
+    TDLB_CK(cudaMemcpyAsync(h->d_plane_cell, h->plane_cell.data(), (size_t)(g.ny + 1) * sizeof(int), cudaMemcpyHostToDevice,
+                            h->stream));
+    h->h_plane_list = std::move(small);
+    // 16 elements of padding: the spread's bulk copies and L2 prefetches
+    // round a plane's cell range out to 16-byte boundaries
+    if (h->ncell + 16 > h->cell_cap || !h->d_cell_e) {
+        long long c1 = 0, c2 = 0, c3 = 0;
+        grow(h->d_cell_e, c1, h->ncell + 16, 1);
+        grow(h->d_cell_m, c2, h->ncell + 16, 4);
+        grow(h->d_cell_F, c3, h->ncell + 16, 3);
+        h->cell_cap = c1;
+    }
+}
+
+// The first segment scheduled by the host: lists whose levels the device gave
+// up on (schedule.cu). `m` is the list, already in d_markers.
+void schedule_on_host(tdlb_lattice* h, const tdlb_marker* m, size_t n0) {
+    const Dims& g = h->g;
+    const auto* mk = reinterpret_cast<const tdlb::Marker*>(m);
+    tdlb::MarkerSchedule seg;
+    seg.build(mk, 0, (int)n0, g.nx, g.ny, g.nz, 0, 0);
+    tdlb::CellList cells;
+    cells.build(mk, seg, g);
+    h->n_level0 = seg.nlevels;
+    ensure_level_cap(h, (long long)seg.nlevels + 1);
+    TDLB_CK(cudaMemcpyAsync(h->d_sched, seg.order.data(), n0 * sizeof(int), cudaMemcpyHostToDevice, h->stream));
+    TDLB_CK(cudaMemcpyAsync(h->d_level_ptr, seg.level_ptr.data(), seg.level_ptr.size() * sizeof(int), cudaMemcpyHostToDevice,
+                            h->stream));
+    TDLB_CK(cudaMemcpyAsync(h->d_plane_lv0, seg.plane_lv.data(), (size_t)(g.ny + 1) * sizeof(int), cudaMemcpyHostToDevice,
+                            h->stream));
+    const std::vector<int> lv1((size_t)g.ny + 1, seg.nlevels);   // an empty second segment
+    TDLB_CK(cudaMemcpyAsync(h->d_plane_lv1, lv1.data(), lv1.size() * sizeof(int), cudaMemcpyHostToDevice, h->stream));
+    TDLB_CK(cudaMemcpy2DAsync(h->d_prep + tdlb::PF_CELL, tdlb::PF_STRIDE * sizeof(float), cells.mcell.data(), 9 * sizeof(int),
+                              9 * sizeof(int), n0, cudaMemcpyHostToDevice, h->stream));
+    TDLB_CK(cudaStreamSynchronize(h->stream));   // the host vectors go
+}
+
 // Make `m[0, n)` the resident list: segment 0 = [0, n0) with exact levels,
-// segment 1 = [n0, n), rotation-invariant when rot_xz is given.
+// scheduled on the device (schedule.cu); segment 1 = [n0, n),
+// rotation-invariant when rot_xz is given, scheduled here. A list with a marker
+// outside the lattice leaves the resident one as it is.
 void upload_markers(tdlb_lattice* h, const tdlb_marker* m, size_t n, size_t n0, const double* rot_xz) {
     if (n > 0 && !m) throw Fail{TDLB_EINVAL, "markers is NULL"};
     if (n > (size_t)0x7fffffff) throw Fail{TDLB_EINVAL, "too many markers"};
     const Dims& g = h->g;
-    validate_markers(g, m, n, 0);
     static_assert(sizeof(tdlb_marker) == sizeof(tdlb::Marker), "marker layout");
-    TDLB_CK(cudaStreamSynchronize(h->stream));   // host vectors below are read by queued copies
-    h->h_markers.assign(m, m + n);
-    const auto* mk = reinterpret_cast<const tdlb::Marker*>(h->h_markers.data());
+    if ((long long)n > h->marker_cap || !h->d_markers_in) {
+        // (the resident list stays valid until the new one has been checked)
+        const long long cap = std::max<long long>(round_up((long long)n, 1024), std::max<long long>(h->marker_cap, 1024));
+        TDLB_CK(cudaStreamSynchronize(h->stream));
+        cudaFree(h->d_markers_in);
+        h->d_markers_in = nullptr;
+        TDLB_CK(cudaMalloc(&h->d_markers_in, cap * sizeof(tdlb::Marker)));
+        h->marker_in_cap = cap;
+    }
+    // scratch of the scheduler, one block
+    const size_t ny = (size_t)g.ny, hist = tdlb::sched_hist_ints(g, (long long)n), maps = tdlb::sched_map_words(g);
+    const size_t ints = 4 + hist + n0 + maps + 9 * n0 + n0 + ny + (ny + 1) + ny;
+    if (ints * sizeof(int) > h->sched_tmp_bytes) {
+        TDLB_CK(cudaStreamSynchronize(h->stream));
+        cudaFree(h->d_sched_tmp);
+        h->d_sched_tmp = nullptr;
+        h->sched_tmp_bytes = 0;
+        const size_t bytes = (ints + ints / 8) * sizeof(int);
+        TDLB_CK(cudaMalloc(&h->d_sched_tmp, bytes));
+        h->sched_tmp_bytes = bytes;
+    }
+    int* tmp = (int*)h->d_sched_tmp;
+    auto take = [&](size_t k) { int* p = tmp; tmp += k; return p; };
+    tdlb::SchedArgs a{};
+    a.markers = h->d_markers_in;
+    a.n = (int)n;
+    a.n0 = (int)n0;
+    a.g = g;
+    a.info = take(4);
+    a.plane_count = take(ny);
+    a.plane_slot = take(ny + 1);
+    a.hist = take(hist);
+    a.by_plane = take(n0);
+    a.maps = maps ? (unsigned*)take(maps) : nullptr;
+    a.place = take(9 * n0);
+    a.level_end = take(n0);
+    a.levels = take(ny);
+    if (n) TDLB_CK(cudaMemcpyAsync(h->d_markers_in, m, n * sizeof(tdlb::Marker), cudaMemcpyHostToDevice, h->stream));
+    const int start[4] = {(int)n, 0, 0, 0};
+    TDLB_CK(cudaMemcpyAsync(a.info, start, sizeof start, cudaMemcpyHostToDevice, h->stream));
+    if (hist) TDLB_CK(cudaMemsetAsync(a.hist, 0, hist * sizeof(int), h->stream));
+    TDLB_CK(tdlb::launch_sched_cells(a, h->stream));
+    std::vector<int> got(4 + ny);
+    TDLB_CK(cudaMemcpyAsync(got.data(), a.info, got.size() * sizeof(int), cudaMemcpyDeviceToHost, h->stream));
+    TDLB_CK(cudaStreamSynchronize(h->stream));
+    if (got[0] < (int)n) validate_markers(g, m + got[0], 1, (size_t)got[0]);   // throws
+    // the list is good: it becomes the resident one
+    std::swap(h->d_markers, h->d_markers_in);
+    std::swap(h->marker_cap, h->marker_in_cap);
     h->n_markers = (int)n;
     h->n0 = (int)n0;
-    h->seg0.build(mk, 0, (int)n0, g.nx, g.ny, g.nz, 0, 0);
-    h->seg1.build(mk, (int)n0, (int)n, g.nx, g.ny, g.nz, (int)n0, h->seg0.nlevels, rot_xz);
-    if ((long long)n > h->marker_cap) {
-        cudaFree(h->d_markers); cudaFree(h->d_sched); cudaFree(h->d_sums);
-        h->d_markers = nullptr; h->d_sched = nullptr; h->d_sums = nullptr;
-        const long long cap = std::max<long long>(round_up((long long)n, 1024), 1024);
-        TDLB_CK(cudaMalloc(&h->d_markers, cap * sizeof(tdlb::Marker)));
-        TDLB_CK(cudaMalloc(&h->d_sched, cap * sizeof(int)));
-        TDLB_CK(cudaMalloc(&h->d_sums, (size_t)3 * cap * sizeof(float)));
-        h->marker_cap = cap;
+    h->h_blades.assign(m + n0, m + n);
+    h->markers_set = false;   // until all of this is done
+    if (h->marker_cap > h->slot_cap || !h->d_sched) {
+        cudaFree(h->d_sched);
+        cudaFree(h->d_sums);
+        h->d_sched = nullptr;
+        h->d_sums = nullptr;
+        h->slot_cap = 0;
+        TDLB_CK(cudaMalloc(&h->d_sched, h->marker_cap * sizeof(int)));
+        TDLB_CK(cudaMalloc(&h->d_sums, (size_t)3 * h->marker_cap * sizeof(float)));
+        h->slot_cap = h->marker_cap;
     }
     const long long ntail = (long long)n - (long long)n0;
     if (ntail > h->tail_cap) {
@@ -647,87 +786,39 @@ void upload_markers(tdlb_lattice* h, const tdlb_marker* m, size_t n, size_t n0, 
         TDLB_CK(cudaMalloc(&h->d_tail, (size_t)tdlb::TF_COUNT * cap * sizeof(float)));
         h->tail_cap = cap;
     }
-    // first segment: unique cells per plane, slot data
-    h->cells.build(mk, h->seg0, g);
-    const long long C0 = (long long)h->cells.cell_e.size();
-    cudaFree(h->d_cell_e); cudaFree(h->d_plane_cell); cudaFree(h->d_prep); cudaFree(h->d_cell_m); cudaFree(h->d_cell_F);
-    h->d_cell_e = nullptr; h->d_plane_cell = nullptr; h->d_prep = nullptr; h->d_cell_m = nullptr; h->d_cell_F = nullptr;
-    TDLB_CK(cudaMalloc(&h->d_plane_cell, (size_t)(g.ny + 1) * sizeof(int)));
-    if (C0) {
-        // 16 elements of padding: the spread's bulk copies and L2 prefetches
-        // round a plane's cell range out to 16-byte boundaries
-        TDLB_CK(cudaMalloc(&h->d_cell_e, (C0 + 16) * sizeof(int)));
-        TDLB_CK(cudaMalloc(&h->d_cell_m, (4 * C0 + 16) * sizeof(float)));
-        TDLB_CK(cudaMalloc(&h->d_cell_F, (3 * C0 + 16) * sizeof(float)));
-    }
-    if (n0) TDLB_CK(cudaMalloc(&h->d_prep, ((size_t)tdlb::PF_STRIDE * n0 + 16) * sizeof(float)));
-    {
-        // F tiles of the ordinary planes' launch: up to 6144 cells (72 KB)
-        // of shared memory;
-        // the tile is sized for the most crowded ordinary plane, at least
-        // 4608 cells. Planes with more cells (an impeller disk) go to a
-        // second, 512-thread launch with a tile for the largest of them
-        // (global memory beyond the 227 KB shared-memory limit).
-        int typical = 0;
-        for (int j = 0; j < g.ny; j++) {
-            const int nc = h->cells.plane_cell[(size_t)j + 1] - h->cells.plane_cell[(size_t)j];
-            if (nc <= 6144) typical = std::max(typical, nc);
-        }
-        const int small_cap = std::max(4608, round_up(typical, 64) > 6144 ? 6144 : (int)round_up(typical, 64));
-        std::vector<int> small, big;
-        int big_max = 0;
-        for (int j = 0; j < g.ny; j++) {
-            const int nc = h->cells.plane_cell[(size_t)j + 1] - h->cells.plane_cell[(size_t)j];
-            if (nc > small_cap) { big.push_back(j); big_max = std::max(big_max, nc); }
-            else small.push_back(j);
-        }
-        h->smem_cells = small_cap;
-        h->n_small = (int)small.size();
-        h->n_big = (int)big.size();
-        h->big_tile_cells = tdlb::big_bulk_bytes(big_max) <= 220 * 1024 ? big_max : 0;
-        TDLB_CK(tdlb::ibm_prepare_smem(h->smem_cells, h->n_small, tdlb::big_bulk_bytes(h->big_tile_cells)));
-        h->max_big = big_max;
-        h->max_cells = 0;
-        for (int j : small)
-            h->max_cells = std::max(h->max_cells, h->cells.plane_cell[(size_t)j + 1] - h->cells.plane_cell[(size_t)j]);
-        small.insert(small.end(), big.begin(), big.end());
-        if (!h->d_plane_list) TDLB_CK(cudaMalloc(&h->d_plane_list, (size_t)g.ny * sizeof(int)));
-        TDLB_CK(cudaMemcpy(h->d_plane_list, small.data(), (size_t)g.ny * sizeof(int), cudaMemcpyHostToDevice));
-        h->h_plane_list = small;
-    }
-    // static touched flags of the first segment
-    {
-        std::vector<uint32_t> ms((size_t)h->mask_words, 0u);
-        for (int e : h->cells.cell_e) {
-            const int row = e / g.jp, j = e - row * g.jp;
-            ms[(size_t)row * g.jw + (j >> 5)] |= 1u << (j & 31);
-        }
-        if (!h->d_mask_static) TDLB_CK(cudaMalloc(&h->d_mask_static, (size_t)h->mask_words * sizeof(uint32_t)));
-        TDLB_CK(cudaMemcpy(h->d_mask_static, ms.data(), ms.size() * sizeof(uint32_t), cudaMemcpyHostToDevice));
-    }
+    plan_planes(h, got.data() + 4);
+    if ((long long)n0 > 0) grow(h->d_prep, h->prep_cap, (long long)n0 + 1, tdlb::PF_STRIDE);
+    if (!h->d_mask_static) TDLB_CK(cudaMalloc(&h->d_mask_static, (size_t)h->mask_words * sizeof(uint32_t)));
+    TDLB_CK(cudaMemsetAsync(h->d_mask_static, 0, (size_t)h->mask_words * sizeof(uint32_t), h->stream));
     if (!h->d_plane_lv0) {
         TDLB_CK(cudaMalloc(&h->d_plane_lv0, (size_t)(g.ny + 1) * sizeof(int)));
         TDLB_CK(cudaMalloc(&h->d_plane_lv1, (size_t)(g.ny + 1) * sizeof(int)));
     }
-    ensure_level_cap(h, (long long)h->seg0.nlevels + h->seg1.nlevels + 1);
-    if (n) TDLB_CK(cudaMemcpyAsync(h->d_markers, m, n * sizeof(tdlb::Marker), cudaMemcpyHostToDevice, h->stream));
-    if (n0) TDLB_CK(cudaMemcpyAsync(h->d_sched, h->seg0.order.data(), n0 * sizeof(int), cudaMemcpyHostToDevice, h->stream));
-    TDLB_CK(cudaMemcpyAsync(h->d_level_ptr, h->seg0.level_ptr.data(), h->seg0.level_ptr.size() * sizeof(int),
-                            cudaMemcpyHostToDevice, h->stream));
-    TDLB_CK(cudaMemcpyAsync(h->d_plane_lv0, h->seg0.plane_lv.data(), (size_t)(g.ny + 1) * sizeof(int),
-                            cudaMemcpyHostToDevice, h->stream));
-    upload_seg1(h);
-    TDLB_CK(cudaMemcpyAsync(h->d_plane_cell, h->cells.plane_cell.data(), (size_t)(g.ny + 1) * sizeof(int),
-                            cudaMemcpyHostToDevice, h->stream));
-    if (C0) TDLB_CK(cudaMemcpyAsync(h->d_cell_e, h->cells.cell_e.data(), C0 * sizeof(int), cudaMemcpyHostToDevice, h->stream));
-    if (n0) {
-        // the 9 cell indices of each slot into its prep row
-        TDLB_CK(cudaMemcpy2DAsync(h->d_prep + tdlb::PF_CELL, tdlb::PF_STRIDE * sizeof(float), h->cells.mcell.data(),
-                                  9 * sizeof(int), 9 * sizeof(int), (size_t)n0, cudaMemcpyHostToDevice, h->stream));
-        tdlb::IbmArgs a = ibm_args(h, 0.f, 0.f);
-        TDLB_CK(tdlb::launch_ibm_prepare(a, h->d_prep, nullptr, h->stream));
-    }
+    ensure_level_cap(h, (long long)n0 + 1);   // (never more levels than markers)
+    a.markers = h->d_markers;
+    a.owner = (int*)h->d_cell_F;
+    a.plane_cell = h->d_plane_cell;
+    a.cell_e = h->d_cell_e;
+    a.sched = h->d_sched;
+    a.prep = h->d_prep;
+    a.level_ptr = h->d_level_ptr;
+    a.plane_lv0 = h->d_plane_lv0;
+    a.plane_lv1 = h->d_plane_lv1;
+    a.mask_static = h->d_mask_static;
+    TDLB_CK(tdlb::launch_sched_levels(a, std::max(h->max_cells, h->max_big), h->ncell, h->stream));
+    TDLB_CK(cudaMemcpyAsync(got.data(), a.info, 4 * sizeof(int), cudaMemcpyDeviceToHost, h->stream));
     TDLB_CK(cudaStreamSynchronize(h->stream));
+    h->n_level0 = got[2];
+    if (got[1]) schedule_on_host(h, m, n0);
+    if (n0) TDLB_CK(tdlb::launch_ibm_prepare(ibm_args(h, 0.f, 0.f), h->d_prep, h->stream));
+    // the blades
+    h->h_blade_planes.clear();
+    h->n_blade = 0;
+    if (ntail > 0) {
+        build_blades(h, rot_xz);
+        upload_seg1(h);
+        TDLB_CK(cudaStreamSynchronize(h->stream));   // the host vectors are read by queued copies
+    }
     h->markers_set = true;
     h->rot_device = false;
     h->impeller_begin = -1;
@@ -745,7 +836,7 @@ tdlb::IbmArgs ibm_args(tdlb_lattice* h, float alpha, float beta) {
     a.n0 = h->n0;
     a.cell_e = h->d_cell_e;
     a.plane_cell = h->d_plane_cell;
-    a.ncell = (int)h->cells.cell_e.size();
+    a.ncell = h->ncell;
     a.max_cells = h->max_cells;
     a.max_big = h->max_big;
     a.prep = h->d_prep;
@@ -1211,11 +1302,10 @@ int tdlb_set_rotating_markers(tdlb_handle h, const tdlb_marker* markers, size_t 
         // go through a pinned buffer and are queued after the work already on
         // the stream (the previous forcing pass still reads the old blades),
         // so this call does not wait for the device.
-        std::copy(markers, markers + n, h->h_markers.begin() + h->n0);
-        const auto* mk = reinterpret_cast<const tdlb::Marker*>(h->h_markers.data());
-        h->seg1.build(mk, h->n0, h->n_markers, h->g.nx, h->g.ny, h->g.nz, h->n0, h->seg0.nlevels, nullptr);
+        h->h_blades.assign(markers, markers + n);
+        build_blades(h, nullptr);
         update_blade_planes(h);
-        const int L0 = h->seg0.nlevels;
+        const int L0 = h->n_level0;
         ensure_level_cap(h, (long long)L0 + h->seg1.nlevels + 1);
         const size_t b_mk = n * sizeof(tdlb::Marker);
         const size_t b_order = n * sizeof(int);

@@ -43,8 +43,14 @@ struct tdlb_lattice {
     int* d_level_ptr = nullptr;
     int* d_plane_lv0 = nullptr;
     int* d_plane_lv1 = nullptr;
-    // first-segment cell lists and per-pass IBM buffers
-    tdlb::CellList cells;
+    // first-segment cell lists and per-pass IBM buffers (grown on demand)
+    std::vector<int> plane_cell;  // [ny+1] cell range of each plane (empty: none yet)
+    int ncell = 0;                // unique stencil cells
+    int n_level0 = 0;             // levels of the first segment
+    long long cell_cap = 0, prep_cap = 0;
+    tdlb::Marker* d_markers_in = nullptr;   // the next list, until it has been checked
+    void* d_sched_tmp = nullptr;  // scratch of the scheduler
+    size_t sched_tmp_bytes = 0;
     int* d_cell_e = nullptr;
     int max_cells = 0, max_big = 0;   // most cells of an ordinary plane, of a big plane
     int* d_plane_cell = nullptr;
@@ -69,12 +75,13 @@ struct tdlb_lattice {
     uint32_t* d_exclude = nullptr;       // excluded output points (1 bit per cell), when set
     std::vector<uint32_t> h_exclude;
     double* d_red = nullptr;             // FP64 reduction partials + result
-    long long marker_cap = 0;
+    long long marker_cap = 0, marker_in_cap = 0;   // of d_markers, d_markers_in
+    long long slot_cap = 0;                         // of d_sched, d_sums
     long long level_cap = 0;
     int n_markers = 0;      // list length
     int n0 = 0;             // markers of the first segment (the rest rotate)
-    std::vector<tdlb_marker> h_markers;   // host copy of the resident list
-    tdlb::MarkerSchedule seg0, seg1;
+    std::vector<tdlb_marker> h_blades;    // host copy of the second segment
+    tdlb::MarkerSchedule seg1;
     bool markers_set = false;
     float last_beta = 0.f;        // beta of the last forcing pass (for the load)
     // resident impeller: markers [n0, n_markers) are blades

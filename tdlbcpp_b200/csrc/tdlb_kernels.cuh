@@ -166,6 +166,42 @@ struct IbmArgs {
 
 cudaError_t launch_ibm(const IbmArgs& a, cudaStream_t st);
 
+// ---- the marker scheduler on the device (schedule.cu) ----
+struct SchedArgs {
+    const Marker* markers;      // the list
+    int n, n0;                  // its length, the first segment's
+    Dims g;
+    // scratch
+    int* info;                  // [3] first marker out of range (starts at n), given up (starts at 0), levels
+    int* hist;                  // [sched_hist_ints] zero
+    int* by_plane;              // [n0]
+    unsigned* maps;             // [sched_map_words], NULL when that is 0
+    int* place;                 // [9 n0]
+    int* owner;                 // [cells]
+    int* level_end;             // [n0]
+    int* levels;                // [ny]
+    // results of launch_sched_cells
+    int* plane_slot;            // [ny+1] slots of each plane
+    int* plane_count;           // [ny] unique stencil cells of each plane
+    // inputs and results of launch_sched_levels
+    const int* plane_cell;      // [ny+1] running sum of plane_count
+    int* cell_e;                // [cells]
+    int* sched;                 // [n0]
+    float* prep;                // [PF_STRIDE n0]: the places (PF_CELL)
+    int* level_ptr;             // [levels + 1]
+    int* plane_lv0;             // [ny+1]
+    int* plane_lv1;             // [ny+1]: an empty second segment
+    uint32_t* mask_static;      // zero; touched flags of the cells
+};
+size_t sched_hist_ints(const Dims& g, long long n);
+size_t sched_map_words(const Dims& g);
+// The list checked and sorted by plane, the planes' cells counted.
+cudaError_t launch_sched_cells(const SchedArgs& a, cudaStream_t st);
+// Cells, levels and order; max_cells: the most of a plane, ncell: of all.
+cudaError_t launch_sched_levels(const SchedArgs& a, int max_cells, int ncell, cudaStream_t st);
+// Raise a kernel's dynamic shared-memory limit on the current device (it only grows).
+cudaError_t raise_smem_limit(const void* fn, size_t bytes);
+
 // Immersed-boundary passes of many lattices in one set of launches: device
 // IbmArgs per lattice and work lists of (lattice, first index) items --
 // cells: places 8 (y >> 10) .. + 8 of the planes 32 (y & 1023) .. + 32; tails: 128 blade markers; copies: 1024
@@ -184,7 +220,7 @@ constexpr int kMaskCopyWords = 1024;
 cudaError_t launch_ibm_batch(const IbmBatch& b, cudaStream_t st, cudaStream_t side, cudaEvent_t fork, cudaEvent_t join);
 cudaError_t ibm_batch_prepare_smem(size_t small_bytes, size_t big_bytes);
 // Per-upload preparation of the first segment (weights, velocities).
-cudaError_t launch_ibm_prepare(const IbmArgs& a, float* prep, const int* mcell, cudaStream_t st);
+cudaError_t launch_ibm_prepare(const IbmArgs& a, float* prep, cudaStream_t st);
 // Shared memory the spread kernel needs: the plane's touched-flag tile plus
 // an F tile of `cells` cells.
 size_t ibm_smem_bytes(const Dims& g, int cells);
