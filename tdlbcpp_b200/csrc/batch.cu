@@ -12,10 +12,11 @@
 //                       per item; one block per item or a persistent grid of
 //                       a few blocks per SM looping over the items (block 0
 //                       also advances the step counter);
-//   3-7. the immersed-boundary passes of the group's tanks
-//                       (launch_ibm_batch) on a high-priority stream: cells,
-//                       blade gathers, touched-flag copies, small-plane and
-//                       large-plane spreads, each one launch over the group.
+//   3-5. the immersed-boundary passes of the group's tanks
+//                       (launch_ibm_batch) on a high-priority stream: the
+//                       gather (stencil cells, blades, touched flags), the
+//                       small-plane and the large-plane spreads, each one
+//                       launch over the group.
 // The groups' fused launches take turns, so each group's forcing pass runs
 // while the other group's fused launch streams through HBM. Four step pairs
 // (A/B and parity cycles), and single pairs for the rest of a run, are
@@ -210,7 +211,7 @@ struct BatchGroup {
     WorkList work;                     // fused-step items (tank, first quad)
     WorkList rot_work;                 // (tank, first blade)
     std::vector<int2> rot_items;       // host copy of rot_work
-    WorkList cells, tails, copies, small, big;   // immersed-boundary items
+    WorkList gather, small, big;       // immersed-boundary items
     int small_tile = 0, big_tile = 0;
     cudaStream_t stream = nullptr;     // group 0: the batch's stream
     cudaStream_t side = nullptr;       // large-plane spreads
@@ -364,29 +365,28 @@ void build_ibm_work(tdlb_batch_s* b) {
     TDLB_BCK(quiesce(b));
     int small_all = 0, big_all = 0;
     for (BatchGroup& G : b->grp) {
-        std::vector<int2> cells, tails, copies, small, big;
+        std::vector<int2> gather, small, big;
         int small_tile = 0, big_tile = 0;
         for (int t : G.tanks) {
             const tdlb_lattice* h = b->tanks[(size_t)t];
             if (!h->markers_set) continue;
+            for (int q = 0; q < 9 * (h->n_markers - h->n0); q += 256) gather.push_back(make_int2(t, (q / 256) << 2 | tdlb::GATHER_TAIL));
+            for (long long wd = 0; wd < h->mask_words; wd += tdlb::kMaskCopyWords)
+                gather.push_back(make_int2(t, (int)(wd / tdlb::kMaskCopyWords) << 2 | tdlb::GATHER_FLAGS));
             const int places = std::max(h->max_cells, h->max_big);
             for (int p = 0; p < places; p += 8)
                 for (int jg = 0; jg < h->g.ny; jg += 32) {
                     bool any = false;   // a tile past every plane's cells is left out
                     for (int j = jg; j < std::min(jg + 32, h->g.ny); j++)
                         any = any || h->plane_cell[(size_t)j + 1] - h->plane_cell[(size_t)j] > p;
-                    if (any) cells.push_back(make_int2(t, (p / 8) << 10 | jg / 32));
+                    if (any) gather.push_back(make_int2(t, ((p / 8) << 10 | jg / 32) << 2 | tdlb::GATHER_CELLS));
                 }
-            for (int q = 0; q < h->n_markers - h->n0; q += 128) tails.push_back(make_int2(t, q));
-            for (long long wd = 0; wd < h->mask_words; wd += tdlb::kMaskCopyWords) copies.push_back(make_int2(t, (int)wd));
             for (int s = 0; s < h->n_small; s++) small.push_back(make_int2(t, h->h_plane_list[(size_t)s]));
             for (int s = 0; s < h->n_big; s++) big.push_back(make_int2(t, h->h_plane_list[(size_t)(h->n_small + s)]));
             small_tile = std::max(small_tile, h->smem_cells);
             if (h->n_big) big_tile = std::max(big_tile, h->big_tile_cells);
         }
-        put(G.cells, cells);
-        put(G.tails, tails);
-        put(G.copies, copies);
+        put(G.gather, gather);
         put(G.small, small);
         put(G.big, big);
         G.small_tile = small_tile;
@@ -394,7 +394,7 @@ void build_ibm_work(tdlb_batch_s* b) {
         small_all = std::max(small_all, small_tile);
         big_all = std::max(big_all, big_tile);
     }
-    TDLB_BCK(tdlb::ibm_batch_prepare_smem(tdlb::ibm_smem_bytes(Dims{}, small_all), tdlb::ibm_smem_bytes(Dims{}, big_all)));
+    TDLB_BCK(tdlb::ibm_batch_prepare_smem(small_all, big_all));
     for (size_t t = 0; t < b->tanks.size(); t++) b->ibm_gen[t] = b->tanks[t]->marker_gen;
 }
 
@@ -463,16 +463,14 @@ int queue_step(tdlb_batch_s* b, int k, bool first) {
         TDLB_BCK(cudaStreamWaitEvent(G.ibm, G.ev_fused, 0));
         tdlb::IbmBatch ib{};
         ib.args = b->d_ibm + (size_t)k * n;
-        ib.cells = G.cells.d; ib.n_cells = G.cells.n;
-        ib.tails = G.tails.d; ib.n_tails = G.tails.n;
-        ib.copies = G.copies.d; ib.n_copies = G.copies.n;
+        ib.gather = G.gather.d; ib.n_gather = G.gather.n;
         ib.small = G.small.d; ib.n_small = G.small.n;
         ib.big = G.big.d; ib.n_big = G.big.n;
         ib.small_tile = G.small_tile;
         ib.big_tile = G.big_tile;
         ib.storage = storage_of(b);
         TDLB_BCK(tdlb::launch_ibm_batch(ib, G.ibm, G.side, G.ev_fork, G.ev_join));
-        kernels += (ib.n_cells > 0) + (ib.n_tails > 0) + (ib.n_copies > 0) + (ib.n_small > 0) + (ib.n_big > 0);
+        kernels += (ib.n_gather > 0) + (ib.n_small > 0) + (ib.n_big > 0);
         TDLB_BCK(cudaEventRecord(G.ev_ibm, G.ibm));
         TDLB_BCK(cudaStreamWaitEvent(G.stream, G.ev_ibm, 0));
     }
@@ -708,7 +706,7 @@ std::vector<uintptr_t> graph_key(const tdlb_batch_s* b, int P) {
         k.push_back(G.tanks.size());
         k.push_back((uintptr_t)G.stream);
         k.push_back((uintptr_t)G.side);
-        for (const WorkList* w : {&G.work, &G.rot_work, &G.cells, &G.tails, &G.copies, &G.small, &G.big}) {
+        for (const WorkList* w : {&G.work, &G.rot_work, &G.gather, &G.small, &G.big}) {
             k.push_back((uintptr_t)w->d);
             k.push_back((uintptr_t)w->n);
         }
@@ -846,7 +844,7 @@ void release(tdlb_batch_s* b) {
     cudaFree(b->d_tables);
     drop(b->work);
     for (BatchGroup& G : b->grp) {
-        for (WorkList* w : {&G.work, &G.rot_work, &G.cells, &G.tails, &G.copies, &G.small, &G.big}) drop(*w);
+        for (WorkList* w : {&G.work, &G.rot_work, &G.gather, &G.small, &G.big}) drop(*w);
         if (G.ev_fork) cudaEventDestroy(G.ev_fork);
         if (G.ev_join) cudaEventDestroy(G.ev_join);
         if (G.ev_fused) cudaEventDestroy(G.ev_fused);

@@ -25,12 +25,11 @@
 // Per pass (launch_ibm): k_ibm_cells (moments and starting F of every unique
 // stencil cell of the static markers; it also starts mask_new as the static
 // touched flags), k_ibm_gather_tail (weights and stencil moments of every
-// blade marker, which no marker changes), k_ibm_spread_bulk (one plane per
-// group of threads: the static markers' levels on an F tile in shared
-// memory), then k_ibm_blades (the blade levels of the planes that have
-// blades, on a shared-memory hash table of the plane's blade cells). The
-// batched passes run the same steps per lattice, with the blade levels
-// inside their spread.
+// blade marker, which no marker changes), k_ibm_spread (one plane per block:
+// the static markers' levels on an F tile in shared memory, then the plane's
+// blade levels on a shared-memory hash table of its blade cells); a tank with
+// more blade markers in a plane than the block has threads walks them with
+// k_ibm_blades afterwards. The batched passes run the same steps per lattice.
 #include "tdlb_kernels.cuh"
 #include "tdlb_rotate.hpp"
 
@@ -178,18 +177,6 @@ __device__ __forceinline__ void put_cell(const IbmArgs& a, int c, const float4 m
     a.cell_F[2 * C + c] = f.z;
 }
 
-// The cells of one plane in list order: the big planes (an impeller disk),
-// whose cells fill an (i, k) area of a single j.
-template <typename S>
-__global__ void __launch_bounds__(256) k_ibm_cells_big(IbmArgs a, const int* __restrict__ planes) {
-    const int j = planes[blockIdx.y];
-    const int c = a.plane_cell[j] + (int)(blockIdx.x * blockDim.x + threadIdx.x);
-    if (c >= a.plane_cell[j + 1]) return;
-    float4 m, f;
-    ibm_cell<S>(a, a.cell_e[c], m, f);
-    put_cell(a, c, m, f);
-}
-
 // The cells of 32 consecutive planes, 8 list places of each: place p of plane
 // j is cell plane_cell[j] + p, the places sorted by (i, k). The markers of a
 // tank repeat from plane to plane, so place p is the same (i, k) in
@@ -198,11 +185,11 @@ __global__ void __launch_bounds__(256) k_ibm_cells_big(IbmArgs a, const int* __r
 // so that lanes running over the places write the lists (128 bytes of a list
 // per plane). Any list is right; one that does not repeat reads a sector per
 // cell and row. Bound by DRAM bytes: 72 populations + 16 F + 4 index + 28
-// written per cell. Planes with more than skip_above cells belong to
-// k_ibm_cells_big. copy: the launch's threads also start mask_new as the
-// first segment's touched flags (mask_static, a multiple of 16 bytes), so
-// that the pass needs no separate copy.
+// written per cell (400^3: 64 us for 2.1 M cells). Planes with more than
+// skip_above cells (an impeller disk, whose cells fill an (i, k) area of a single
+// j) are taken in list order instead.
 constexpr int kCellPlaces = 8;
+constexpr int kGatherThreads = 32 * kCellPlaces;
 struct CellTile {
     int e[32][kCellPlaces + 1];
     float4 m[kCellPlaces][33];
@@ -232,54 +219,12 @@ __device__ __forceinline__ void ibm_cell_tile(const IbmArgs& a, CellTile& sm, in
     const int jj = threadIdx.x / kCellPlaces, p = threadIdx.x % kCellPlaces;
     if (sm.e[jj][p] >= 0) put_cell(a, a.plane_cell[j0 + jj] + p0 + p, sm.m[p][jj], sm.f[p][jj]);
 }
+// Second segment (the blades): weight and moments of stencil cell c of blade
+// marker t, u = c * ntail + t (c = 3 (k1 + 1) + (i1 + 1)): the nine cells of a
+// marker are gathered in parallel; c = 0 also writes the marker velocity.
 template <typename S>
-__global__ void __launch_bounds__(32 * kCellPlaces) k_ibm_cells(IbmArgs a, int skip_above, int copy_mask) {
-    __shared__ CellTile sm;
-    if (copy_mask) {
-        const long long n4 = (long long)(a.mask_bytes / 16);
-        const long long t = ((long long)blockIdx.y * gridDim.x + blockIdx.x) * blockDim.x + threadIdx.x;
-        for (long long w = t; w < n4; w += (long long)gridDim.x * gridDim.y * blockDim.x)
-            reinterpret_cast<uint4*>(a.mask_new)[w] = reinterpret_cast<const uint4*>(a.mask_static)[w];
-    }
-    ibm_cell_tile<S>(a, sm, (int)blockIdx.x * 32, (int)blockIdx.y * kCellPlaces, skip_above);
-}
-
-// Second segment (the blades): weights and the moments of the 9 stencil
-// cells of every blade marker.
-template <typename S>
-__device__ __forceinline__ void ibm_tail_marker(const IbmArgs& a, int t) {
-    const Marker mk = a.markers[a.sched[a.n0 + t]];
-    const int i = (int)mk.i, j = (int)mk.j, k = (int)mk.k;
-    float* s = a.tail;
-    const long long cap = a.tail_cap;
-    int c = 0;
-    for (int k1 = -1; k1 <= 1; k1++) {
-        for (int i1 = -1; i1 <= 1; i1++, c++) {
-            const float w = stencil_weight(mk.iCartFraction, mk.kCartFraction, i1, k1);
-            const int i2 = wrap_i(i + i1, a.g.nx), k2 = wrap_i(k + k1, a.g.nz);
-            float m4[4];
-            cell_moments4<S>(a.A, a.state_mode, a.even, a.g, i2, j, k2, a.p, m4, a.rbox);
-            s[(TF_W + c) * cap + t] = w;
-            s[(TF_RHO + c) * cap + t] = m4[0];
-            s[(TF_MX + c) * cap + t] = m4[1];
-            s[(TF_MY + c) * cap + t] = m4[2];
-            s[(TF_MZ + c) * cap + t] = m4[3];
-            s[(TF_CELL + c) * cap + t] = __int_as_float((i2 << 16) | k2);
-        }
-    }
-    s[TF_U * cap + t] = mk.uDelta;
-    s[TF_V * cap + t] = mk.vDelta;
-    s[TF_WV * cap + t] = mk.wDelta;
-}
-
-// One thread per (blade marker t, stencil cell c): thread u takes c = u /
-// ntail, t = u % ntail (c = 3 (k1 + 1) + (i1 + 1), as ibm_tail_marker), so
-// the 9 cells of a marker are gathered in parallel; c = 0 also writes the
-// marker velocity.
-template <typename S>
-__global__ void __launch_bounds__(128) k_ibm_gather_tail(IbmArgs a) {
+__device__ __forceinline__ void ibm_tail_cell(const IbmArgs& a, int u) {
     const int ntail = a.n - a.n0;
-    const int u = blockIdx.x * blockDim.x + threadIdx.x;
     if (u >= 9 * ntail) return;
     const int c = u / ntail, t = u - c * ntail;
     const Marker mk = a.markers[a.sched[a.n0 + t]];
@@ -300,6 +245,33 @@ __global__ void __launch_bounds__(128) k_ibm_gather_tail(IbmArgs a) {
         s[TF_V * cap + t] = mk.vDelta;
         s[TF_WV * cap + t] = mk.wDelta;
     }
+}
+
+// Everything the pass reads from the state, in one launch: the blades' stencils
+// (the first tail_blocks blocks), the big planes' cells (big_blocks blocks of each),
+// the other planes' cell tiles; its threads also start mask_new as the first
+// segment's touched flags (mask_static, a multiple of 16 bytes).
+template <typename S>
+__global__ void __launch_bounds__(kGatherThreads) k_ibm_gather(IbmArgs a, int tail_blocks, int big_blocks, int tiles_j) {
+    __shared__ CellTile sm;
+    {
+        const int n4 = (int)(a.mask_bytes / 16);
+        for (int w = (int)(blockIdx.x * blockDim.x + threadIdx.x); w < n4; w += (int)(gridDim.x * blockDim.x))
+            reinterpret_cast<uint4*>(a.mask_new)[w] = reinterpret_cast<const uint4*>(a.mask_static)[w];
+    }
+    int b = (int)blockIdx.x;
+    if (b < tail_blocks) return ibm_tail_cell<S>(a, b * kGatherThreads + (int)threadIdx.x);
+    b -= tail_blocks;
+    if (b < a.n_big * big_blocks) {
+        const int j = a.plane_list[a.n_small + b / big_blocks];
+        const int c = a.plane_cell[j] + b % big_blocks * kGatherThreads + (int)threadIdx.x;
+        if (c >= a.plane_cell[j + 1]) return;
+        float4 m, f;
+        ibm_cell<S>(a, a.cell_e[c], m, f);
+        return put_cell(a, c, m, f);
+    }
+    b -= a.n_big * big_blocks;
+    ibm_cell_tile<S>(a, sm, b % tiles_j * 32, b / tiles_j * kCellPlaces, a.smem_cells);
 }
 
 // Bulk asynchronous copies global -> shared memory with an mbarrier
@@ -364,56 +336,51 @@ __device__ __forceinline__ void prefetch_l2(const void* base, int c0, int n) {
     const BulkSpan sp = bulk_span(base, c0, n);
     asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(sp.src), "r"(sp.bytes) : "memory");
 }
-// The per-marker and per-cell data a group's walk of plane j reads, into L2
-// while the group fills its tile: the first segment's weights, cells and
-// velocities (markers [pm0, pm1) of the prep arrays), the plane's cell
-// moments and elements, and the blade markers' gathered stencils. One array
-// per lane.
-template <typename GRP>
-__device__ __forceinline__ void prefetch_plane(const IbmArgs& a, int j, int c0, int nc, const GRP grp) {
-    const int lane = grp.tid();
+// The per-marker and per-cell data the walk of plane j reads, into L2 while the
+// block fills its tile: the first segment's rows (slots [p0, p1)), the plane's
+// cell moments and elements, and the blade markers' gathered stencils (slots
+// [q0, q1) of the second segment). One array per lane.
+__device__ __forceinline__ void prefetch_plane(const IbmArgs& a, int c0, int nc, int p0, int p1, int q0, int q1) {
+    const int lane = threadIdx.x;
     if (lane >= 32) return;
-    const int pm0 = a.level_ptr[a.plane_lv0[j]], pm1 = a.level_ptr[a.plane_lv0[j + 1]];
-    const int q0 = a.level_ptr[a.plane_lv1[j]] - a.n0, q1 = a.level_ptr[a.plane_lv1[j + 1]] - a.n0;
     for (int f = lane; f < 3 + TF_COUNT; f += 32) {
-        if (f == 0) prefetch_l2(a.prep, pm0 * PF_STRIDE, (pm1 - pm0) * PF_STRIDE);
+        if (f == 0) prefetch_l2(a.prep, p0 * PF_STRIDE, (p1 - p0) * PF_STRIDE);
         else if (f == 1) prefetch_l2(a.cell_m, 4 * c0, 4 * nc);
         else if (f == 2) prefetch_l2(a.cell_e, c0, nc);
-        else prefetch_l2(a.tail + (size_t)(f - 3) * a.tail_cap, q0, q1 - q0);
+        else prefetch_l2(a.tail + (size_t)(f - 3) * a.tail_cap, q0 - a.n0, q1 - q0);
     }
 }
 
-// A group of NT threads (whole warps) that walks one j-plane. Several groups
-// can share a CTA, each synchronising on its own named barrier (bar.sync id,
-// NT), so that the planes of one CTA advance independently; a group that is
-// the whole CTA uses barrier 0 (__syncthreads).
-template <int NT, bool NAMED = false>
-struct PlaneGroup {
-    int base;  // the group's first thread in the CTA
-    int bar;   // named barrier id (NAMED), else the CTA barrier
-    // thread index within the group (read from threadIdx each time, so that
-    // it occupies no register of the register-bound walks)
-    __device__ __forceinline__ int tid() const { return NAMED ? (int)threadIdx.x - base : (int)threadIdx.x; }
-    __device__ __forceinline__ void sync() const {
-        if constexpr (NAMED) asm volatile("bar.sync %0, %1;" ::"r"(bar), "r"(NT) : "memory");
-        else __syncthreads();
-    }
+// Slot offsets of a plane's levels [lv0, lv1]: the first kLevelSmem staged in
+// shared memory, so that a level starts without a trip to the L2.
+constexpr int kLevelSmem = 64;
+struct Levels {
+    const int* global;   // a.level_ptr + lv0
+    const int* staged;
+    int n;               // levels
+    __device__ __forceinline__ int at(int l) const { return l < kLevelSmem ? staged[l] : __ldg(global + l); }
 };
+template <int NT>
+__device__ __forceinline__ Levels stage_levels(const IbmArgs& a, const int* plane_lv, int j, int* staged) {
+    const int lv0 = plane_lv[j], n = plane_lv[j + 1] - lv0;
+    for (int l = threadIdx.x; l < kLevelSmem && l <= n; l += NT) staged[l] = a.level_ptr[lv0 + l];
+    return Levels{a.level_ptr + lv0, staged, n};
+}
 
 // Blade levels of plane j on global memory: F and the touched flags are
 // read back from L2 (__ldcg), since earlier levels of this CTA wrote them.
 // Used when the plane's blade stencils do not fit the shared-memory table;
 // a called function rather than inlined, so that this rare fallback costs
 // the register-bound walks around it no registers.
-template <int NT, typename GRP>
-__device__ __noinline__ void blade_levels_global(const IbmArgs& a, int j, const GRP grp) {
+template <int NT>
+__device__ __noinline__ void blade_levels_global(const IbmArgs& a, int j) {
     const Dims g = a.g;
     const float* s = a.tail;
     const long long cap = a.tail_cap;
     for (int lv = a.plane_lv1[j]; lv < a.plane_lv1[j + 1]; lv++) {
         const int p0 = a.level_ptr[lv], p1 = a.level_ptr[lv + 1];
 #pragma unroll 1
-        for (int p = p0 + grp.tid(); p < p1; p += NT) {
+        for (int p = p0 + (int)threadIdx.x; p < p1; p += NT) {
             const int t = p - a.n0;
             float rhoSum = 0.f, xSum = 0.f, ySum = 0.f, zSum = 0.f;
 #pragma unroll
@@ -451,9 +418,70 @@ __device__ __noinline__ void blade_levels_global(const IbmArgs& a, int j, const 
                 atomicOr(&a.mask_new[wd], bit);
             }
         }
-        grp.sync();
+        __syncthreads();
     }
 }
+
+// The table of blade_levels_tile and the update of one marker on it.
+struct BladeTable {
+    int* keys;
+    float *hx, *hy, *hz;
+};
+struct BladeMarker {
+    float w[9], rho[9], mx[9], my[9], mz[9], u, v, wv;
+    __device__ __forceinline__ void load(const float* s, long long cap, int t) {
+#pragma unroll
+        for (int c = 0; c < 9; c++) {
+            w[c] = s[(TF_W + c) * cap + t];
+            rho[c] = s[(TF_RHO + c) * cap + t];
+            mx[c] = s[(TF_MX + c) * cap + t];
+            my[c] = s[(TF_MY + c) * cap + t];
+            mz[c] = s[(TF_MZ + c) * cap + t];
+        }
+        u = s[TF_U * cap + t];
+        v = s[TF_V * cap + t];
+        wv = s[TF_WV * cap + t];
+    }
+    // interpolate at the table entries hh, subtract the marker's velocity,
+    // spread; the sums go to slot p
+    __device__ __forceinline__ void apply(const IbmArgs& a, const BladeTable& h, const int (&hh)[9], int p, bool distinct) const {
+        float rhoSum = 0.f, xSum = 0.f, ySum = 0.f, zSum = 0.f;
+        float ox[9], oy[9], oz[9];
+#pragma unroll
+        for (int c = 0; c < 9; c++) {
+            ox[c] = h.hx[hh[c]];
+            oy[c] = h.hy[hh[c]];
+            oz[c] = h.hz[hh[c]];
+            rhoSum = fmaf(w[c], rho[c], rhoSum);
+            xSum = fmaf(w[c], fmaf(0.5f, ox[c], mx[c]), xSum);
+            ySum = fmaf(w[c], fmaf(0.5f, oy[c], my[c]), ySum);
+            zSum = fmaf(w[c], fmaf(0.5f, oz[c], mz[c]), zSum);
+        }
+        xSum = fmaf(-rhoSum, u, xSum);
+        ySum = fmaf(-rhoSum, v, ySum);
+        zSum = fmaf(-rhoSum, wv, zSum);
+        a.sums[p] = xSum;
+        a.sums[a.n + p] = ySum;
+        a.sums[2 * a.n + p] = zSum;
+        if (distinct) {   // 9 different cells: independent updates
+#pragma unroll
+            for (int c = 0; c < 9; c++) {
+                const float bw = a.beta * w[c];
+                h.hx[hh[c]] = fmaf(a.alpha, ox[c], -bw * xSum);
+                h.hy[hh[c]] = fmaf(a.alpha, oy[c], -bw * ySum);
+                h.hz[hh[c]] = fmaf(a.alpha, oz[c], -bw * zSum);
+            }
+        } else {
+#pragma unroll
+            for (int c = 0; c < 9; c++) {   // sequential: a wrapped stencil sees its own update
+                const float bw = a.beta * w[c];
+                h.hx[hh[c]] = fmaf(a.alpha, h.hx[hh[c]], -bw * xSum);
+                h.hy[hh[c]] = fmaf(a.alpha, h.hy[hh[c]], -bw * ySum);
+                h.hz[hh[c]] = fmaf(a.alpha, h.hz[hh[c]], -bw * zSum);
+            }
+        }
+    }
+};
 
 // Blade levels of plane j on a shared-memory table. The plane's 9 x nb
 // stencil references (nb blade markers) go into an open-addressing hash
@@ -463,351 +491,383 @@ __device__ __noinline__ void blade_levels_global(const IbmArgs& a, int j, const 
 // previous one touched it -- the levels run on the table, and the cells go
 // back to F with their touched flags. The walk reads and writes the same
 // values in the same order as blade_levels_global; only the L2 round trips
-// between levels go. Needs 4 H + 9 nb words of `tile`; returns false, having
-// done nothing, when they do not fit.
-template <int THREADS, typename GRP>
-__device__ __forceinline__ bool blade_levels_tile(const IbmArgs& a, int j, float* tile, int tile_words,
-                                                  const GRP grp) {
-    const int lv0 = a.plane_lv1[j], lv1 = a.plane_lv1[j + 1];
-    const int q0 = a.level_ptr[lv0], q1 = a.level_ptr[lv1];
-    const int nref = 9 * (q1 - q0);
+// between levels go. Needs blade_table_words(nb) words of `tile`; returns
+// false, having done nothing, when they do not fit.
+// With a thread for every marker (nb <= NT) a thread holds its marker's data
+// and table entries in registers from the start, and the thread that put a
+// cell into the table loads its F and writes it back, so a level is table
+// reads, the update and a barrier, and the walk one trip to the L2 before
+// them. (Bound by latency. 160^3 tank, 84 markers a plane: 17 us with the data
+// of each level loaded inside it.)
+template <int NT>
+__device__ __forceinline__ bool blade_levels_tile(const IbmArgs& a, int j, float* tile, int tile_words, const Levels lv) {
+    const int q0 = lv.at(0), nb = lv.at(lv.n) - q0, nref = 9 * nb;
     int lg = 5;
     while ((1 << lg) < nref) lg++;
     const int H = 1 << lg;
     if (4LL * H + nref > (long long)tile_words) return false;
-    int* keys = reinterpret_cast<int*>(tile);
-    float* hx = tile + H;
-    float* hy = tile + 2 * H;
-    float* hz = tile + 3 * H;
-    int* ref = reinterpret_cast<int*>(tile + 4 * H);
+    BladeTable h{reinterpret_cast<int*>(tile), tile + H, tile + 2 * H, tile + 3 * H};
     const Dims g = a.g;
     const float* s = a.tail;
     const long long cap = a.tail_cap;
     const bool distinct = g.nx >= 3 && g.nz >= 3;   // the 9 stencil cells of a marker differ
+    const int tid = (int)threadIdx.x;
+    // the entry of `key`; first: this call put it there
+    auto insert = [&](int key, bool& first) {
+        unsigned at = ((unsigned)key * 2654435761u) >> (32 - lg);
+        first = false;
+        for (int probe = 0; probe < H; probe++) {
+            const int prev = atomicCAS(&h.keys[at], -1, key);
+            first = prev == -1;
+            if (first || prev == key) break;
+            at = (at + 1) & (unsigned)(H - 1);
+        }
+        return (int)at;
+    };
+    // F of `key`, zero unless this pass or the previous one touched it
+    auto load_cell = [&](int key, float& x, float& y, float& z) {
+        const int i2 = key >> 16, k2 = key & 0xffff;
+        const long long wd = g.word(i2, j, k2);
+        const uint32_t bit = 1u << (j & 31);
+        const float4 v = __ldcg(a.F4 + g.at(i2, j, k2));   // (a lattice cell whatever the flags say)
+        const bool live = ((__ldcg(a.mask_new + wd) | a.mask_old[wd]) & bit) != 0u;
+        x = live ? v.x : 0.f;
+        y = live ? v.y : 0.f;
+        z = live ? v.z : 0.f;
+    };
+    auto store_cell = [&](int key, int at) {
+        const int i2 = key >> 16, k2 = key & 0xffff;
+        a.F4[g.at(i2, j, k2)] = make_float4(h.hx[at], h.hy[at], h.hz[at], 0.f);
+        atomicOr(&a.mask_new[g.word(i2, j, k2)], 1u << (j & 31));
+    };
 
-    for (int h = grp.tid(); h < H; h += THREADS) keys[h] = -1;
-    grp.sync();
-    // inserts, four references per thread at a time (their keys loaded
-    // together)
-    for (int r0 = grp.tid(); r0 < nref; r0 += 4 * THREADS) {
-        int kk[4];
+    if (nb <= NT) {
+        const bool on = tid < nb;
+        const int t = q0 + tid - a.n0;
+        BladeMarker mk;
+        int key[9], hh[9];
+        if (on) {
 #pragma unroll
-        for (int u = 0; u < 4; u++) {
-            const int r = r0 + u * THREADS;
-            const int m = r / 9, c = r - 9 * m;
-            kk[u] = r < nref ? __float_as_int(s[(TF_CELL + c) * cap + (q0 + m - a.n0)]) : -1;
+            for (int c = 0; c < 9; c++) key[c] = __float_as_int(s[(TF_CELL + c) * cap + t]);
+            mk.load(s, cap, t);
         }
+        for (int e = tid; e < H; e += NT) h.keys[e] = -1;
+        __syncthreads();
+        unsigned mine = 0;
+        if (on) {
+            // every cell's F, so that the loads leave together; the inserts
+            // meanwhile say which of them this thread keeps
+            float x[9], y[9], z[9];
 #pragma unroll
-        for (int u = 0; u < 4; u++) {
-            const int r = r0 + u * THREADS;
-            if (r >= nref) break;
-            const int key = kk[u];
-            unsigned h = ((unsigned)key * 2654435761u) >> (32 - lg);
-            for (int probe = 0; probe < H; probe++) {
-                const int prev = atomicCAS(&keys[h], -1, key);
-                if (prev == -1 || prev == key) break;
-                h = (h + 1) & (unsigned)(H - 1);
-            }
-            ref[r] = (int)h;
-        }
-    }
-    grp.sync();
-    // each table cell's F, four entries per thread at a time: F is read
-    // whatever the flags say (e is a lattice cell), so that the flag and F
-    // loads of the four make one round trip
-    for (int h0 = grp.tid(); h0 < H; h0 += 4 * THREADS) {
-        float vx[4], vy[4], vz[4];
-        bool live[4];
-#pragma unroll
-        for (int u = 0; u < 4; u++) {
-            const int h = h0 + u * THREADS;
-            const int key = h < H ? keys[h] : -1;
-            const int i2 = key >> 16, k2 = key & 0xffff;
-            const long long e = g.at(i2, j, k2), wd = g.word(i2, j, k2);
-            const uint32_t bit = 1u << (j & 31);
-            live[u] = false;
-            vx[u] = vy[u] = vz[u] = 0.f;
-            if (key >= 0) {
-                const float4 v = __ldcg(a.F4 + e);
-                vx[u] = v.x;
-                vy[u] = v.y;
-                vz[u] = v.z;
-                live[u] = (__ldcg(a.mask_new + wd) & bit) || (a.mask_old[wd] & bit);
-            }
-        }
-#pragma unroll
-        for (int u = 0; u < 4; u++) {
-            const int h = h0 + u * THREADS;
-            if (h < H && keys[h] >= 0) {
-                hx[h] = live[u] ? vx[u] : 0.f;
-                hy[h] = live[u] ? vy[u] : 0.f;
-                hz[h] = live[u] ? vz[u] : 0.f;
-            }
-        }
-    }
-    grp.sync();
-    for (int lv = lv0; lv < lv1; lv++) {
-        const int p0 = a.level_ptr[lv], p1 = a.level_ptr[lv + 1];
-#pragma unroll 1
-        for (int p = p0 + grp.tid(); p < p1; p += THREADS) {
-            const int t = p - a.n0;
-            const int* rf = ref + 9 * (p - q0);
-            float rhoSum = 0.f, xSum = 0.f, ySum = 0.f, zSum = 0.f;
-            float w[9], ox[9], oy[9], oz[9];
-            int hh[9];
+            for (int c = 0; c < 9; c++) load_cell(key[c], x[c], y[c], z[c]);
 #pragma unroll
             for (int c = 0; c < 9; c++) {
-                w[c] = s[(TF_W + c) * cap + t];
-                hh[c] = rf[c];
-                ox[c] = hx[hh[c]];
-                oy[c] = hy[hh[c]];
-                oz[c] = hz[hh[c]];
-                rhoSum = fmaf(w[c], s[(TF_RHO + c) * cap + t], rhoSum);
-                xSum = fmaf(w[c], fmaf(0.5f, ox[c], s[(TF_MX + c) * cap + t]), xSum);
-                ySum = fmaf(w[c], fmaf(0.5f, oy[c], s[(TF_MY + c) * cap + t]), ySum);
-                zSum = fmaf(w[c], fmaf(0.5f, oz[c], s[(TF_MZ + c) * cap + t]), zSum);
+                bool first;
+                hh[c] = insert(key[c], first);
+                mine |= first ? 1u << c : 0u;
             }
-            xSum = fmaf(-rhoSum, s[TF_U * cap + t], xSum);
-            ySum = fmaf(-rhoSum, s[TF_V * cap + t], ySum);
-            zSum = fmaf(-rhoSum, s[TF_WV * cap + t], zSum);
-            a.sums[p] = xSum;
-            a.sums[a.n + p] = ySum;
-            a.sums[2 * a.n + p] = zSum;
-            if (distinct) {   // 9 different cells: independent updates
 #pragma unroll
-                for (int c = 0; c < 9; c++) {
-                    const float bw = a.beta * w[c];
-                    hx[hh[c]] = fmaf(a.alpha, ox[c], -bw * xSum);
-                    hy[hh[c]] = fmaf(a.alpha, oy[c], -bw * ySum);
-                    hz[hh[c]] = fmaf(a.alpha, oz[c], -bw * zSum);
+            for (int c = 0; c < 9; c++)
+                if ((mine >> c) & 1u) {
+                    h.hx[hh[c]] = x[c];
+                    h.hy[hh[c]] = y[c];
+                    h.hz[hh[c]] = z[c];
                 }
-            } else {
-#pragma unroll
-                for (int c = 0; c < 9; c++) {   // sequential: a wrapped stencil sees its own update
-                    const float bw = a.beta * w[c];
-                    hx[hh[c]] = fmaf(a.alpha, hx[hh[c]], -bw * xSum);
-                    hy[hh[c]] = fmaf(a.alpha, hy[hh[c]], -bw * ySum);
-                    hz[hh[c]] = fmaf(a.alpha, hz[hh[c]], -bw * zSum);
-                }
-            }
         }
-        grp.sync();
+        __syncthreads();
+        for (int l = 0; l < lv.n; l++) {
+            const int p = q0 + tid;
+            if (p >= lv.at(l) && p < lv.at(l + 1)) mk.apply(a, h, hh, p, distinct);
+            __syncthreads();
+        }
+        if (on) {
+#pragma unroll
+            for (int c = 0; c < 9; c++)
+                if ((mine >> c) & 1u) store_cell(key[c], hh[c]);
+        }
+        return true;
     }
-    for (int h = grp.tid(); h < H; h += THREADS) {
-        const int key = keys[h];
-        if (key < 0) continue;
-        const int i2 = key >> 16, k2 = key & 0xffff;
-        a.F4[g.at(i2, j, k2)] = make_float4(hx[h], hy[h], hz[h], 0.f);
-        atomicOr(&a.mask_new[g.word(i2, j, k2)], 1u << (j & 31));
+    int* ref = reinterpret_cast<int*>(tile + 4 * H);
+    for (int e = tid; e < H; e += NT) h.keys[e] = -1;
+    __syncthreads();
+    for (int r = tid; r < nref; r += NT) {
+        const int m = r / 9, c = r - 9 * m;
+        bool first;
+        ref[r] = insert(__float_as_int(s[(TF_CELL + c) * cap + (q0 + m - a.n0)]), first);
     }
+    __syncthreads();
+    for (int e = tid; e < H; e += NT)
+        if (h.keys[e] >= 0) load_cell(h.keys[e], h.hx[e], h.hy[e], h.hz[e]);
+    __syncthreads();
+    for (int l = 0; l < lv.n; l++) {
+        const int p1 = lv.at(l + 1);
+#pragma unroll 1
+        for (int p = lv.at(l) + tid; p < p1; p += NT) {
+            BladeMarker mk;
+            mk.load(s, cap, p - a.n0);
+            int hh[9];
+#pragma unroll
+            for (int c = 0; c < 9; c++) hh[c] = ref[9 * (p - q0) + c];
+            mk.apply(a, h, hh, p, distinct);
+        }
+        __syncthreads();
+    }
+    for (int e = tid; e < H; e += NT)
+        if (h.keys[e] >= 0) store_cell(h.keys[e], e);
     return true;
 }
 
-// One group per j-plane: the plane's first-segment levels on an F tile in
-// shared memory (planes with more cells than the tile holds work on cell_F
-// in place), write-back to F, then (BLADES) the blade levels, on a
-// shared-memory table when they fit the tile, else on global F. The touched
-// flags of the first segment never change, so each pass starts mask_new as
-// a copy of them (mask_static) and the blade walk adds its cells.
-// BULK: the group's tile is [3][bulk_tile_stride(tile_cells)] words (F x, y,
-// z), filled by bulk copies of the plane's cell range (bar: the group's
-// mbarrier).
-// Otherwise the tile is [3][tile_cells] and filled by plain loads.
-template <int THREADS, bool BULK = false, typename GRP = PlaneGroup<THREADS>, bool PIPE = false, bool BLADES = true>
-__device__ __forceinline__ void ibm_spread_plane(const IbmArgs& a, int j, int tile_cells, float* tile, const GRP grp,
-                                                 uint64_t* bar = nullptr, int* bulk_fail = nullptr) {
+// A first-segment marker's data: its slot row (weights, places, velocity) and,
+// gathered through the row's places, its cells' rho and momentum.
+struct SlotRow {
+    float4 r[PF_STRIDE / 4];
+    __device__ __forceinline__ void load(const float* prep, int p) {
+#pragma unroll
+        for (int u = 0; u < PF_STRIDE / 4; u++) r[u] = __ldg(reinterpret_cast<const float4*>(prep + (size_t)p * PF_STRIDE) + u);
+    }
+    __device__ __forceinline__ float w(int c) const { return f4_lane(r, PF_W + c); }
+    __device__ __forceinline__ int place(int c) const { return __float_as_int(f4_lane(r, PF_CELL + c)); }
+};
+struct SlotMoments {
+    float4 m[9];
+    __device__ __forceinline__ void load(const float4* cm, const SlotRow& row) {
+#pragma unroll
+        for (int c = 0; c < 9; c++) m[c] = cm[row.place(c)];
+    }
+};
+__device__ __forceinline__ void apply_slot(const IbmArgs& a, const SlotRow& row, const SlotMoments& mo, float* fx, float* fy,
+                                           float* fz, int p, bool distinct) {
+    float rhoSum = 0.f, xSum = 0.f, ySum = 0.f, zSum = 0.f;
+    float ox[9], oy[9], oz[9];
+#pragma unroll
+    for (int c = 0; c < 9; c++) {
+        const int li = row.place(c);
+        const float w = row.w(c);
+        ox[c] = fx[li];
+        oy[c] = fy[li];
+        oz[c] = fz[li];
+        rhoSum = fmaf(w, mo.m[c].x, rhoSum);
+        xSum = fmaf(w, fmaf(0.5f, ox[c], mo.m[c].y), xSum);
+        ySum = fmaf(w, fmaf(0.5f, oy[c], mo.m[c].z), ySum);
+        zSum = fmaf(w, fmaf(0.5f, oz[c], mo.m[c].w), zSum);
+    }
+    xSum = fmaf(-rhoSum, f4_lane(row.r, PF_U), xSum);
+    ySum = fmaf(-rhoSum, f4_lane(row.r, PF_V), ySum);
+    zSum = fmaf(-rhoSum, f4_lane(row.r, PF_WV), zSum);
+    a.sums[p] = xSum;
+    a.sums[a.n + p] = ySum;
+    a.sums[2 * a.n + p] = zSum;
+    if (distinct) {
+        // 9 different cells: each update starts from the value read above, so
+        // the 27 stores are independent
+#pragma unroll
+        for (int c = 0; c < 9; c++) {
+            const int li = row.place(c);
+            const float bw = a.beta * row.w(c);
+            fx[li] = fmaf(a.alpha, ox[c], -bw * xSum);
+            fy[li] = fmaf(a.alpha, oy[c], -bw * ySum);
+            fz[li] = fmaf(a.alpha, oz[c], -bw * zSum);
+        }
+    } else {
+#pragma unroll
+        for (int c = 0; c < 9; c++) {   // sequential: a wrapped stencil sees its own update
+            const int li = row.place(c);
+            const float bw = a.beta * row.w(c);
+            fx[li] = fmaf(a.alpha, fx[li], -bw * xSum);
+            fy[li] = fmaf(a.alpha, fy[li], -bw * ySum);
+            fz[li] = fmaf(a.alpha, fz[li], -bw * zSum);
+        }
+    }
+}
+
+// One block per j-plane: the plane's first-segment levels on an F tile in
+// shared memory (planes with more cells than the tile holds work on cell_F in
+// place), write-back to F, then (BLADES) the blade levels, on a shared-memory
+// table when they fit the tile, else on global F. The touched flags of the
+// first segment never change, so each pass starts mask_new as a copy of them
+// (mask_static) and the blade walk adds its cells. The tile is
+// [3][bulk_tile_stride(tile_cells)] words (F x, y, z), filled by bulk copies of
+// the plane's cell range.
+//
+// A level is a chain -- its markers read the F that the levels before it wrote --
+// so the walk is bound by latency, and everything but F is brought in ahead:
+// the level offsets are staged, a thread's next slot row is on its way two
+// slots ahead and the next slot's cell moments one slot ahead (PIPE: 84 more
+// registers, launches of 128 threads; the 512 threads of a big plane hold only
+// their current slot and hide the trips by number). Measured on B200 with the
+// rows one slot ahead and the moments loaded inside the level: 37 us for a
+// 160^3 tank, 85 us at 400^3.
+template <int NT, bool PIPE, bool BLADES>
+__device__ __forceinline__ void ibm_spread_plane(const IbmArgs& a, int j, int tile_cells, float* tile) {
+    __shared__ uint64_t bar;
+    __shared__ int fail;
+    __shared__ int staged0[kLevelSmem], staged1[BLADES ? kLevelSmem : 1];
+    const int tid = (int)threadIdx.x;
     const int c0 = a.plane_cell[j], nc = a.plane_cell[j + 1] - c0;
+    const Levels lv = stage_levels<NT>(a, a.plane_lv0, j, staged0);
+    Levels lb{nullptr, nullptr, 0};
+    if (BLADES) lb = stage_levels<NT>(a, a.plane_lv1, j, staged1);
     const long long C = a.ncell;
     const bool in_smem = nc <= tile_cells;
     float *fx, *fy, *fz;
-    prefetch_plane(a, j, c0, nc, grp);
-    if (BULK && in_smem && nc > 0) {
+    int at_x = 0, at_y = 0, at_z = 0;   // the arrays' first words in the tile
+    if (in_smem && nc > 0) {
         const int tc = bulk_tile_stride(tile_cells);
         const BulkSpan sx = bulk_span(a.cell_F + c0, 0, nc), sy = bulk_span(a.cell_F + C + c0, 0, nc),
                        sz = bulk_span(a.cell_F + 2 * C + c0, 0, nc);
-        if (grp.tid() == 0) {
-            mbar_init(bar);
-            *bulk_fail = 0;
+        if (tid == 0) {
+            mbar_init(&bar);
+            fail = 0;
+            mbar_expect(&bar, sx.bytes + sy.bytes + sz.bytes);
+            bulk_to_smem(tile, sx.src, sx.bytes, &bar);
+            bulk_to_smem(tile + tc, sy.src, sy.bytes, &bar);
+            bulk_to_smem(tile + 2 * tc, sz.src, sz.bytes, &bar);
         }
-        grp.sync();
-        if (grp.tid() == 0) {
-            mbar_expect(bar, sx.bytes + sy.bytes + sz.bytes);
-            bulk_to_smem(tile, sx.src, sx.bytes, bar);
-            bulk_to_smem(tile + tc, sy.src, sy.bytes, bar);
-            bulk_to_smem(tile + 2 * tc, sz.src, sz.bytes, bar);
-        }
-        fx = tile + sx.off; fy = tile + tc + sy.off; fz = tile + 2 * tc + sz.off;
-        // bounded wait; the group decides together whether it gave up, so
-        // that every thread takes the same barriers
-        if (!mbar_wait0(bar, 1 << 20)) *bulk_fail = 1;
-        grp.sync();
-        if (*bulk_fail) {
-            // should not happen: count it, give the copies more time, then
-            // load the tile with plain loads
-            if (grp.tid() == 0) atomicAdd(&g_ibm_bulk_timeouts, 1u);
-            mbar_wait0(bar, 1 << 22);
-            grp.sync();
-            for (int t = grp.tid(); t < nc; t += THREADS) {
-                fx[t] = a.cell_F[c0 + t];
-                fy[t] = a.cell_F[C + c0 + t];
-                fz[t] = a.cell_F[2 * C + c0 + t];
-            }
-        }
-    } else if (in_smem) {
-        fx = tile; fy = tile + tile_cells; fz = tile + 2 * tile_cells;
-#pragma unroll 4
-        for (int t = grp.tid(); t < nc; t += THREADS) {
-            fx[t] = a.cell_F[c0 + t];
-            fy[t] = a.cell_F[C + c0 + t];
-            fz[t] = a.cell_F[2 * C + c0 + t];
-        }
+        __syncthreads();   // the barrier is set up; the staged offsets are in
+        prefetch_plane(a, c0, nc, lv.at(0), lv.at(lv.n), BLADES ? lb.at(0) : a.n0, BLADES ? lb.at(lb.n) : a.n0);
+        at_x = sx.off;
+        at_y = tc + sy.off;
+        at_z = 2 * tc + sz.off;
+        fx = tile + at_x; fy = tile + at_y; fz = tile + at_z;
     } else {
+        __syncthreads();
         fx = a.cell_F + c0; fy = a.cell_F + C + c0; fz = a.cell_F + 2 * C + c0;
     }
-    grp.sync();
-
     // ---- first segment: each marker in list order relative to every marker
     //      it shares a cell with (level walk). With x and z at least 3 the 9
     //      stencil cells of a marker differ (the stencil wraps onto itself
     //      only on a narrower lattice).
     const bool distinct = a.g.nx >= 3 && a.g.nz >= 3;
     const float4* cm = reinterpret_cast<const float4*>(a.cell_m) + c0;   // rho, jx, jy, jz
-    // PIPE: each thread's next slot row (the next slot of this level, else
-    // its first slot of the next level) is loaded while the current slot is
-    // processed, so a level's rounds wait for the cell moments only (it takes
-    // 24 more registers: launches of at most 384 threads).
-    const int lvb = a.plane_lv0[j], lve = a.plane_lv0[j + 1];
-    float4 r[PF_STRIDE / 4];
-    int rp = -1;   // the slot r holds
-    for (int lv = lvb; lv < lve; lv++) {
-        const int p0 = a.level_ptr[lv], p1 = a.level_ptr[lv + 1];
-        const int p2 = lv + 1 < lve ? a.level_ptr[lv + 2] : p1;
-#pragma unroll 1
-        for (int p = p0 + grp.tid(); p < p1; p += THREADS) {
-            float rhoSum = 0.f, xSum = 0.f, ySum = 0.f, zSum = 0.f;
-            float w[9], ox[9], oy[9], oz[9];
-            int li[9];
-            if (rp != p) {
-#pragma unroll
-                for (int u = 0; u < PF_STRIDE / 4; u++) r[u] = reinterpret_cast<const float4*>(a.prep + (size_t)p * PF_STRIDE)[u];
-            }
-            int pn = p + THREADS, pe = p1;
-            if (pn >= p1) {
-                pn = p1 + grp.tid();
-                pe = p2;
-            }
-            float4 rn[PF_STRIDE / 4];
-            if (PIPE && pn < pe) {
-#pragma unroll
-                for (int u = 0; u < PF_STRIDE / 4; u++) rn[u] = reinterpret_cast<const float4*>(a.prep + (size_t)pn * PF_STRIDE)[u];
-            }
-#pragma unroll
-            for (int c = 0; c < 9; c++) {
-                w[c] = f4_lane(r, PF_W + c);
-                li[c] = __float_as_int(f4_lane(r, PF_CELL + c));
-            }
-#pragma unroll
-            for (int c = 0; c < 9; c++) {
-                const float4 m = cm[li[c]];
-                ox[c] = fx[li[c]];
-                oy[c] = fy[li[c]];
-                oz[c] = fz[li[c]];
-                rhoSum = fmaf(w[c], m.x, rhoSum);
-                xSum = fmaf(w[c], fmaf(0.5f, ox[c], m.y), xSum);
-                ySum = fmaf(w[c], fmaf(0.5f, oy[c], m.z), ySum);
-                zSum = fmaf(w[c], fmaf(0.5f, oz[c], m.w), zSum);
-            }
-            xSum = fmaf(-rhoSum, f4_lane(r, PF_U), xSum);
-            ySum = fmaf(-rhoSum, f4_lane(r, PF_V), ySum);
-            zSum = fmaf(-rhoSum, f4_lane(r, PF_WV), zSum);
-            a.sums[p] = xSum;
-            a.sums[a.n + p] = ySum;
-            a.sums[2 * a.n + p] = zSum;
-            if (distinct) {
-                // 9 different cells: each update starts from the value read
-                // above, so the 27 stores are independent
-#pragma unroll
-                for (int c = 0; c < 9; c++) {
-                    const float bw = a.beta * w[c];
-                    fx[li[c]] = fmaf(a.alpha, ox[c], -bw * xSum);
-                    fy[li[c]] = fmaf(a.alpha, oy[c], -bw * ySum);
-                    fz[li[c]] = fmaf(a.alpha, oz[c], -bw * zSum);
-                }
-            } else {
-#pragma unroll
-                for (int c = 0; c < 9; c++) {   // sequential: a wrapped stencil sees its own update
-                    const float bw = a.beta * w[c];
-                    fx[li[c]] = fmaf(a.alpha, fx[li[c]], -bw * xSum);
-                    fy[li[c]] = fmaf(a.alpha, fy[li[c]], -bw * ySum);
-                    fz[li[c]] = fmaf(a.alpha, fz[li[c]], -bw * zSum);
-                }
-            }
-            if constexpr (PIPE) {
-#pragma unroll
-                for (int u = 0; u < PF_STRIDE / 4; u++) r[u] = rn[u];
-                rp = pn < pe ? pn : -1;
-            }
+    // Rounds: the slots [b, b + NT) of a level, one per thread, round after
+    // round, level after level (e: the level's end, where the next one starts).
+    // Row and moment sets take turns (their roles, not their contents, move
+    // on: a copied register would wait for its load).
+    struct Round {
+        int l, b, e;
+    };
+    auto after = [&](Round q) {
+        q.b += NT;
+        if (q.b >= q.e) {
+            q.l++;
+            q.b = q.e;
+            if (q.l < lv.n) q.e = lv.at(q.l + 1);
         }
-        grp.sync();
+        return q;
+    };
+    Round q0{0, 0, 0}, q1 = q0, q2 = q0;   // (no slot: b + tid >= e)
+    SlotRow r0, r1, r2;
+    SlotMoments m0, m1;
+    if (PIPE && lv.n > 0) {
+        q0 = Round{0, lv.at(0), lv.at(1)};
+        if (q0.b + tid < q0.e) r0.load(a.prep, q0.b + tid);
+        q1 = after(q0);
+        if (q1.b + tid < q1.e) r1.load(a.prep, q1.b + tid);
+        q2 = after(q1);
+        if (q0.b + tid < q0.e) m0.load(cm, r0);
+    }
+    if (in_smem && nc > 0) {
+        // bounded wait; the block decides together whether it gave up, so
+        // that every thread takes the same barriers
+        if (!mbar_wait0(&bar, 1 << 20)) fail = 1;
+        __syncthreads();
+        if (fail) {
+            // should not happen: count it, give the copies more time, then
+            // load the tile with plain loads
+            if (tid == 0) atomicAdd(&g_ibm_bulk_timeouts, 1u);
+            mbar_wait0(&bar, 1 << 22);
+            __syncthreads();
+            for (int t = tid; t < nc; t += NT) {
+                fx[t] = a.cell_F[c0 + t];
+                fy[t] = a.cell_F[C + c0 + t];
+                fz[t] = a.cell_F[2 * C + c0 + t];
+            }
+            __syncthreads();
+        }
+    }
+    if (PIPE && in_smem) {
+        float *sx = tile + at_x, *sy = tile + at_y, *sz = tile + at_z;   // shared memory, as the compiler can see
+        // the round of (rc, mc); on the way: the next round's moments, the row after it
+        auto round = [&](const SlotRow& rc, const SlotRow& rn, SlotRow& rnn, const SlotMoments& mc, SlotMoments& mn) {
+            if (q1.b + tid < q1.e) mn.load(cm, rn);
+            if (q2.b + tid < q2.e) rnn.load(a.prep, q2.b + tid);
+            if (q0.b + tid < q0.e) apply_slot(a, rc, mc, sx, sy, sz, q0.b + tid, distinct);
+            if (q1.l != q0.l) __syncthreads();
+            q0 = q1;
+            q1 = q2;
+            q2 = after(q2);
+            return q0.l < lv.n;
+        };
+        bool more = lv.n > 0;
+        while (more) {
+            if (!(more = round(r0, r1, r2, m0, m1))) break;
+            if (!(more = round(r1, r2, r0, m1, m0))) break;
+            if (!(more = round(r2, r0, r1, m0, m1))) break;
+            if (!(more = round(r0, r1, r2, m1, m0))) break;
+            if (!(more = round(r1, r2, r0, m0, m1))) break;
+            more = round(r2, r0, r1, m1, m0);
+        }
+    } else {
+        for (int l = 0; l < lv.n; l++) {
+            const int p1 = lv.at(l + 1);
+#pragma unroll 1
+            for (int q = lv.at(l) + tid; q < p1; q += NT) {
+                r0.load(a.prep, q);
+                m0.load(cm, r0);
+                apply_slot(a, r0, m0, fx, fy, fz, q, distinct);
+            }
+            __syncthreads();
+        }
     }
     // ---- write the plane's cells back to F (eight element loads in flight
     //      per thread)
     {
-        int t = grp.tid();
-        for (; t + 7 * THREADS < nc; t += 8 * THREADS) {
+        int t = tid;
+        for (; t + 7 * NT < nc; t += 8 * NT) {
             int e[8];
 #pragma unroll
-            for (int u = 0; u < 8; u++) e[u] = a.cell_e[c0 + t + u * THREADS];
+            for (int u = 0; u < 8; u++) e[u] = a.cell_e[c0 + t + u * NT];
 #pragma unroll
-            for (int u = 0; u < 8; u++)
-                a.F4[e[u]] = make_float4(fx[t + u * THREADS], fy[t + u * THREADS], fz[t + u * THREADS], 0.f);
+            for (int u = 0; u < 8; u++) a.F4[e[u]] = make_float4(fx[t + u * NT], fy[t + u * NT], fz[t + u * NT], 0.f);
         }
-        for (; t < nc; t += THREADS) {
+        for (; t < nc; t += NT) {
             const int e = a.cell_e[c0 + t];
             a.F4[e] = make_float4(fx[t], fy[t], fz[t], 0.f);
         }
     }
-    grp.sync();
-
     // ---- second segment (blades), unless a separate launch walks them
-    if (!BLADES || a.plane_lv1[j] == a.plane_lv1[j + 1]) return;
-    const int words = BULK ? 3 * bulk_tile_stride(tile_cells) : 3 * tile_cells;
-    if (!blade_levels_tile<THREADS>(a, j, tile, words, grp)) blade_levels_global<THREADS>(a, j, grp);
+    if constexpr (BLADES) {
+        if (lb.n == 0) return;
+        __syncthreads();
+        if (!blade_levels_tile<NT>(a, j, tile, 3 * bulk_tile_stride(tile_cells), lb)) blade_levels_global<NT>(a, j);
+    }
 }
 
-// G planes per CTA: group g (NT threads, its own barrier) walks plane
-// planes[blockIdx.x * G + g] on its own tile, which bulk copies fill with one
-// latency whatever the group's size. The ordinary planes run G = 1..4 groups
-// of 128 threads, so all planes of a large lattice are resident at once; the
-// big planes (an impeller disk) one group of 512.
-template <int NT, int G, bool BLADES = true>
-__global__ void __launch_bounds__(NT * G, 1) k_ibm_spread_bulk(IbmArgs a, const int* __restrict__ planes, int nplanes,
-                                                              int tile_cells) {
-    extern __shared__ __align__(128) float btile[];             // [G][3][bulk_tile_stride(tile_cells)]
-    __shared__ uint64_t bars[G];
-    __shared__ int fails[G];
-    const int g = G == 1 ? 0 : (int)threadIdx.x / NT;
-    const int q = (int)blockIdx.x * G + g;
-    if (q >= nplanes) return;
-    const PlaneGroup<NT, (G > 1)> grp{g * NT, g + 1};
-    ibm_spread_plane<NT, true, PlaneGroup<NT, (G > 1)>, (NT * G <= 384), BLADES>(
-        a, planes[q], tile_cells, btile + (size_t)g * 3 * bulk_tile_stride(tile_cells), grp, &bars[g],
-                               &fails[g]);
+// A plane per block: the ordinary planes with 128 threads, the big ones (an
+// impeller disk) with 512. Two blocks of 128 at most share an SM, which leaves
+// registers and shared memory to the outer launch of a split step beside them
+// (the walk's time is the chain's, not the number of threads').
+template <int NT, bool BLADES>
+__global__ void __launch_bounds__(NT, NT == 128 ? 2 : 1) k_ibm_spread(IbmArgs a, const int* __restrict__ planes,
+                                                                     int tile_cells) {
+    extern __shared__ __align__(128) float btile[];             // [3][bulk_tile_stride(tile_cells)]
+    ibm_spread_plane<NT, NT == 128, BLADES>(a, planes[blockIdx.x], tile_cells, btile);
 }
 
 // The blade levels of the planes that have blades, one plane per CTA of NT
-// threads, after both first-segment spreads have written their planes' F:
-// the blade planes' walks then run wide instead of holding up the
-// 128-thread groups of the ordinary planes' launch. `words` floats of
-// shared memory hold the plane's hash table.
+// threads, after both first-segment spreads have written their planes' F, for
+// planes with more blade markers than an ordinary plane's block has threads.
+// `words` floats of shared memory hold the plane's hash table.
 template <int NT>
 __global__ void __launch_bounds__(NT, 1) k_ibm_blades(IbmArgs a, const int* __restrict__ planes, int nplanes,
                                                       int words) {
     extern __shared__ __align__(16) float btab[];
+    __shared__ int staged[kLevelSmem];
     if ((int)blockIdx.x >= nplanes) return;
     const int j = planes[blockIdx.x];
-    const PlaneGroup<NT> grp{0, 0};
-    if (!blade_levels_tile<NT>(a, j, btab, words, grp)) blade_levels_global<NT>(a, j, grp);
+    const Levels lv = stage_levels<NT>(a, a.plane_lv1, j, staged);
+    __syncthreads();
+    if (!blade_levels_tile<NT>(a, j, btab, words, lv)) blade_levels_global<NT>(a, j);
 }
 
 // Impeller rotation on the device: recomputes the blade markers of the
@@ -835,16 +895,43 @@ cudaError_t launch_rotate_markers(const double* xz, Marker* out, int n, double c
     return cudaGetLastError();
 }
 
-// Deterministic FP64 reduction of the marker forces: fixed grid, fixed
-// per-thread stride, fixed shared-memory tree, then one block sums the
-// partials in order.
-__global__ void __launch_bounds__(256) k_marker_load(IbmArgs a, int begin, double ci, double ck, double* partial) {
-    __shared__ double red[5][256];
+// FP64 sums of five values over a block of 256 threads (fixed order: a warp's
+// lanes by halves, then the warps by halves), in thread 0.
+__device__ __forceinline__ void block_sum5(double (&v)[5]) {
+    __shared__ double part[8][5];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+    for (int w = 16; w > 0; w /= 2)
+#pragma unroll
+        for (int c = 0; c < 5; c++) v[c] += __shfl_down_sync(0xffffffffu, v[c], w);
+    if (lane == 0)
+#pragma unroll
+        for (int c = 0; c < 5; c++) part[warp][c] = v[c];
+    __syncthreads();
+    if (warp == 0) {
+#pragma unroll
+        for (int c = 0; c < 5; c++) v[c] = lane < 8 ? part[lane][c] : 0.0;
+#pragma unroll
+        for (int w = 4; w > 0; w /= 2)
+#pragma unroll
+            for (int c = 0; c < 5; c++) v[c] += __shfl_down_sync(0xffffffffu, v[c], w);
+    }
+    __syncthreads();
+}
+
+// Deterministic FP64 reduction of the marker forces over the impeller's slots
+// (a list built with the schedule: 4 % of a 400^3 tank's markers): fixed grid,
+// fixed strides and trees; the block that finishes last adds the blocks' sums
+// the same way. One launch bound by latency; with a pass over every marker, a
+// second launch and one thread adding 128 blocks' sums it was 26 us at 400^3, 13 us
+// at 24^3. counter: zero before, and again after.
+__global__ void __launch_bounds__(256) k_marker_load(IbmArgs a, const int* __restrict__ slots, int n, double ci, double ck,
+                                                     double* partial, unsigned* counter, double* out) {
+    __shared__ bool last;
     double acc[5] = {0, 0, 0, 0, 0};
-    for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < a.n; p += gridDim.x * blockDim.x) {
-        const int q = a.sched[p];
-        if (q < begin) continue;
-        const Marker mk = a.markers[q];
+    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
+        const int p = slots[t];
+        const Marker mk = a.markers[a.sched[p]];
         const double fx = -(double)a.beta * (double)a.sums[p];
         const double fy = -(double)a.beta * (double)a.sums[a.n + p];
         const double fz = -(double)a.beta * (double)a.sums[2 * a.n + p];
@@ -856,15 +943,52 @@ __global__ void __launch_bounds__(256) k_marker_load(IbmArgs a, int begin, doubl
         acc[3] += dk * fx - di * fz;   // (r x F) along j, r = (di, 0, dk)
         acc[4] += 1.0;
     }
-    for (int c = 0; c < 5; c++) red[c][threadIdx.x] = acc[c];
-    __syncthreads();
-    for (int w = blockDim.x / 2; w > 0; w >>= 1) {
-        if ((int)threadIdx.x < w)
-            for (int c = 0; c < 5; c++) red[c][threadIdx.x] += red[c][threadIdx.x + w];
+    block_sum5(acc);
+    if (gridDim.x > 1) {
+        if (threadIdx.x == 0) {
+#pragma unroll
+            for (int c = 0; c < 5; c++) partial[blockIdx.x * 5 + c] = acc[c];
+            __threadfence();
+            last = atomicAdd(counter, 1u) == gridDim.x - 1;
+        }
         __syncthreads();
+        if (!last) return;
+        __threadfence();
+#pragma unroll
+        for (int c = 0; c < 5; c++) acc[c] = threadIdx.x < gridDim.x ? __ldcg(partial + threadIdx.x * 5 + c) : 0.0;
+        block_sum5(acc);
+        if (threadIdx.x == 0) *counter = 0u;
     }
     if (threadIdx.x == 0)
-        for (int c = 0; c < 5; c++) partial[blockIdx.x * 5 + c] = red[c][0];
+        for (int c = 0; c < 5; c++) out[c] = acc[c];
+}
+
+// The slots whose marker is the impeller's (list index >= begin), in slot
+// order: two passes over 256-slot groups, counts then places.
+__global__ void __launch_bounds__(256) k_impeller_slots(const int* __restrict__ sched, int n, int begin, int* __restrict__ offset,
+                                                        int* __restrict__ slots) {
+    __shared__ int warps[8];
+    const int p = (int)(blockIdx.x * 256 + threadIdx.x), lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const bool in = p < n && sched[p] >= begin;
+    const unsigned vote = __ballot_sync(0xffffffffu, in);
+    if (lane == 0) warps[warp] = __popc(vote);
+    __syncthreads();
+    int before = 0, all = 0;
+    for (int w = 0; w < 8; w++) {
+        if (w < warp) before += warps[w];
+        all += warps[w];
+    }
+    if (!slots) {
+        if (threadIdx.x == 0) offset[blockIdx.x] = all;
+    } else if (in) {
+        slots[offset[blockIdx.x] + before + __popc(vote & ((1u << lane) - 1u))] = p;
+    }
+}
+
+cudaError_t launch_impeller_slots(const int* sched, int n, int begin, int* offset, int* slots, cudaStream_t st) {
+    if (n <= 0) return cudaSuccess;
+    k_impeller_slots<<<(n + 255) / 256, 256, 0, st>>>(sched, n, begin, offset, slots);
+    return cudaGetLastError();
 }
 
 // Ordered sum of the block partials: the warp stages them in shared memory
@@ -887,14 +1011,10 @@ __device__ __forceinline__ void ordered_final(const double* __restrict__ partial
     for (int c = 0; c < NC; c++) out[c] = acc[c];
 }
 
-__global__ void k_marker_load_final(const double* partial, int nblocks, double* out) {
-    ordered_final<5, kLoadBlocks>(partial, nblocks, out);
-}
-
-cudaError_t launch_marker_load(const IbmArgs& a, int begin, double ci, double ck, double* partial, double* out,
-                               cudaStream_t st) {
-    k_marker_load<<<kLoadBlocks, 256, 0, st>>>(a, begin, ci, ck, partial);
-    k_marker_load_final<<<1, 32, 0, st>>>(partial, kLoadBlocks, out);
+cudaError_t launch_marker_load(const IbmArgs& a, const int* slots, int n, double ci, double ck, double* partial,
+                               unsigned* counter, double* out, cudaStream_t st) {
+    const int blocks = n <= 0 ? 1 : std::min(kLoadBlocks, (n + 511) / 512);   // two slots a thread, more in a large tank
+    k_marker_load<<<blocks, 256, 0, st>>>(a, slots, n, ci, ck, partial, counter, out);
     return cudaGetLastError();
 }
 
@@ -963,11 +1083,6 @@ cudaError_t launch_fill_rest(Planes Q, long long plane, float rho, float rho0, i
     return cudaGetLastError();
 }
 
-size_t ibm_smem_bytes(const Dims& g, int cells) {
-    (void)g;
-    return (size_t)3 * cells * sizeof(float);
-}
-
 // The dynamic shared-memory limit is a per-kernel, per-device attribute that
 // every lattice and batch shares: it only ever grows, so that a smaller
 // lattice set up later cannot lower it below what a larger one launches with.
@@ -985,40 +1100,6 @@ cudaError_t raise_smem_limit(const void* fn, size_t bytes) {
     return e;
 }
 
-// Ordinary planes per CTA: as few 128-thread groups as put every plane on
-// the GPU at once (nplanes / SMs, rounded up), at most as many as their F
-// tiles (12 bytes per cell) fit in the 227 KB of shared memory a CTA may use,
-// and at most 4: groups of one CTA share its SM's load/store pipe. (At 400^3
-// the 399 ordinary planes hold 5214 cells each: 3 groups, 133 CTAs.)
-static int sm_count() {
-    static int n[64] = {0};
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 148;
-    if (n[dev] == 0) {
-        int v = 0;
-        n[dev] = cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && v > 0 ? v : 148;
-    }
-    return n[dev];
-}
-int spread_groups(int tile_cells, int nplanes) {
-    const size_t per = (size_t)12 * bulk_tile_stride(tile_cells);
-    int G = (int)((227 * 1024 - 64) / per);
-    G = G < 1 ? 1 : (G > 4 ? 4 : G);
-    const int sms = sm_count();
-    const int want = nplanes > 0 ? (nplanes + sms - 1) / sms : 1;
-    return want < G ? (want < 1 ? 1 : want) : G;
-}
-
-template <int G>
-static const void* spread_bulk_fn() { return (const void*)k_ibm_spread_bulk<128, G, false>; }
-
-template <int G>
-static void spread_small(const IbmArgs& a, cudaStream_t st) {
-    const unsigned grid = (unsigned)((a.n_small + G - 1) / G);
-    const size_t bytes = (size_t)G * 12 * bulk_tile_stride(a.smem_cells);
-    k_ibm_spread_bulk<128, G, false><<<grid, 128 * G, bytes, st>>>(a, a.plane_list, a.n_small, a.smem_cells);
-}
-
 // Shared memory (floats) of the blade launch for a plane of nb blade
 // markers: blade_levels_tile's table of H >= 9 nb entries (a power of two,
 // at least 32) of four words, and 9 nb references.
@@ -1033,17 +1114,16 @@ cudaError_t ibm_prepare_blades(int words) {
     return raise_smem_limit((const void*)k_ibm_blades<512>, (size_t)words * sizeof(float));
 }
 
-// Shared memory of the big planes' launch (one 512-thread group, a bulk
-// tile of big_cells cells; none when the tile does not fit).
+// Shared memory of a plane's bulk tile of `big_cells` cells (none when the tile
+// does not fit).
 size_t big_bulk_bytes(int big_cells) { return big_cells > 0 ? (size_t)12 * bulk_tile_stride(big_cells) : 0; }
 
-cudaError_t ibm_prepare_smem(int small_cells, int n_small, size_t big_bytes) {
-    const int G = spread_groups(small_cells, n_small);
-    const void* fn = G == 4 ? spread_bulk_fn<4>() : G == 3 ? spread_bulk_fn<3>() : G == 2 ? spread_bulk_fn<2>()
-                                                                                       : spread_bulk_fn<1>();
-    cudaError_t e = raise_smem_limit(fn, (size_t)G * 12 * bulk_tile_stride(small_cells));
-    if (e != cudaSuccess) return e;
-    return raise_smem_limit((const void*)k_ibm_spread_bulk<512, 1, false>, big_bytes);
+cudaError_t ibm_prepare_smem(int small_cells, size_t big_bytes) {
+    const size_t small = big_bulk_bytes(small_cells);
+    cudaError_t e = raise_smem_limit((const void*)k_ibm_spread<128, false>, small);
+    if (e == cudaSuccess) e = raise_smem_limit((const void*)k_ibm_spread<128, true>, small);
+    if (e == cudaSuccess) e = raise_smem_limit((const void*)k_ibm_spread<512, false>, big_bytes);
+    return e;
 }
 
 cudaError_t launch_ibm_prepare(const IbmArgs& a, float* prep, cudaStream_t st) {
@@ -1053,75 +1133,44 @@ cudaError_t launch_ibm_prepare(const IbmArgs& a, float* prep, cudaStream_t st) {
 }
 
 cudaError_t launch_ibm(const IbmArgs& a, cudaStream_t st) {
-    bool mask_copied = false;
-    auto cells_small = [&](cudaStream_t cs) {
-        if (a.max_cells <= 0) return;
-        const dim3 grid((unsigned)((a.g.ny + 31) / 32), (unsigned)((a.max_cells + kCellPlaces - 1) / kCellPlaces));
-        with_storage(a.storage, [&](auto s) {
-            k_ibm_cells<decltype(s)><<<grid, 32 * kCellPlaces, 0, cs>>>(a, a.smem_cells, 1);
-        });
-        mask_copied = true;
-    };
-    auto cells_big = [&](cudaStream_t cs) {
-        if (a.n_big <= 0) return;
-        const dim3 grid((unsigned)((a.max_big + 255) / 256), (unsigned)a.n_big);
-        with_storage(a.storage, [&](auto s) {
-            k_ibm_cells_big<decltype(s)><<<grid, 256, 0, cs>>>(a, a.plane_list + a.n_small);
-        });
-    };
-    auto tail = [&](cudaStream_t ts) {
-        if (a.n <= a.n0) return;
-        const unsigned b = (unsigned)((9LL * (a.n - a.n0) + 127) / 128);
-        with_storage(a.storage, [&](auto s) { k_ibm_gather_tail<decltype(s)><<<b, 128, 0, ts>>>(a); });
-    };
-    // mask_new starts as the first segment's (static) touched cells: copied
-    // by the ordinary planes' cells launch, else by a copy; only the blade walk
-    // reads or sets mask_new, at the end of the pass.
-    // Side stream: the blade markers' gather (which reads only the state and
-    // is needed only by the blade walk) and the planes with many cells (an
-    // impeller disk): their cells, then their spread with a full-size tile
-    // and 512 threads, started before the ordinary planes' spread places its
-    // blocks over the SMs. Handle's stream: the other planes' cells and
-    // spread, then, after the side stream, the blade walk.
-    cudaError_t err = cudaSuccess;
-    err = cudaEventRecord(a.ev_fork, st);
+    const int tail_blocks = (int)((9LL * (a.n - a.n0) + kGatherThreads - 1) / kGatherThreads);
+    const int big_blocks = (a.max_big + kGatherThreads - 1) / kGatherThreads;
+    const int tiles_j = (a.g.ny + 31) / 32;
+    const long long blocks = tail_blocks + (long long)a.n_big * big_blocks +
+                             (long long)tiles_j * ((a.max_cells + kCellPlaces - 1) / kCellPlaces);
+    // (an empty list still starts mask_new)
+    with_storage(a.storage, [&](auto s) {
+        k_ibm_gather<decltype(s)><<<(unsigned)std::max(blocks, 1LL), kGatherThreads, 0, st>>>(a, tail_blocks, big_blocks, tiles_j);
+    });
+    cudaError_t err = cudaGetLastError();
     if (err != cudaSuccess) return err;
-    err = cudaStreamWaitEvent(a.side, a.ev_fork, 0);
-    if (err != cudaSuccess) return err;
-    cells_big(a.side);
-    tail(a.side);
+    // Side stream: the planes with many cells (an impeller disk), with a
+    // full-size tile and 512 threads, beside the ordinary planes.
     if (a.n_big > 0) {
-        k_ibm_spread_bulk<512, 1, false><<<a.n_big, 512, big_bulk_bytes(a.big_tile_cells), a.side>>>(
-            a, a.plane_list + a.n_small, a.n_big, a.big_tile_cells);
+        err = cudaEventRecord(a.ev_fork, st);
+        if (err == cudaSuccess) err = cudaStreamWaitEvent(a.side, a.ev_fork, 0);
+        if (err != cudaSuccess) return err;
+        k_ibm_spread<512, false><<<a.n_big, 512, big_bulk_bytes(a.big_tile_cells), a.side>>>(a, a.plane_list + a.n_small,
+                                                                                        a.big_tile_cells);
         err = cudaGetLastError();
+        if (err == cudaSuccess) err = cudaEventRecord(a.ev_join, a.side);
         if (err != cudaSuccess) return err;
     }
-    err = cudaEventRecord(a.ev_join, a.side);
-    if (err != cudaSuccess) return err;
-    cells_small(st);
-    if (!mask_copied) {
-        err = cudaMemcpyAsync(a.mask_new, a.mask_static, a.mask_bytes, cudaMemcpyDeviceToDevice, st);
-        if (err != cudaSuccess) return err;
-    }
+    // A plane's blades are walked by its own block when there is a thread for
+    // every marker and no big plane has any; else by a launch of their own,
+    // once every plane's first segment is in F.
+    const bool own = a.blade_max <= 128 && a.n_big == 0;
     if (a.n_small > 0) {
-        switch (spread_groups(a.smem_cells, a.n_small)) {
-            case 4: spread_small<4>(a, st); break;
-            case 3: spread_small<3>(a, st); break;
-            case 2: spread_small<2>(a, st); break;
-            default: spread_small<1>(a, st); break;
-        }
+        const size_t bytes = big_bulk_bytes(a.smem_cells);
+        if (own && a.n_blade > 0) k_ibm_spread<128, true><<<a.n_small, 128, bytes, st>>>(a, a.plane_list, a.smem_cells);
+        else k_ibm_spread<128, false><<<a.n_small, 128, bytes, st>>>(a, a.plane_list, a.smem_cells);
     }
     err = cudaGetLastError();
-    if (err != cudaSuccess) return err;
-    err = cudaStreamWaitEvent(st, a.ev_join, 0);
-    if (err != cudaSuccess) return err;
-    // the blade levels, once every plane's first segment is in F
-    if (a.n_blade > 0) {
-        k_ibm_blades<512><<<a.n_blade, 512, (size_t)a.blade_words * sizeof(float), st>>>(a, a.blade_planes, a.n_blade,
-                                                                                      a.blade_words);
-        err = cudaGetLastError();
-    }
-    return err;
+    if (err == cudaSuccess && a.n_big > 0) err = cudaStreamWaitEvent(st, a.ev_join, 0);
+    if (err != cudaSuccess || own || a.n_blade == 0) return err;
+    k_ibm_blades<512><<<a.n_blade, 512, (size_t)a.blade_words * sizeof(float), st>>>(a, a.blade_planes, a.n_blade,
+                                                                                  a.blade_words);
+    return cudaGetLastError();
 }
 
 // ---------------------------------------------------------------------------
@@ -1138,127 +1187,51 @@ __device__ __forceinline__ void stage_args(IbmArgs& dst, const IbmArgs* src) {
         reinterpret_cast<unsigned long long*>(&dst)[w] = reinterpret_cast<const unsigned long long*>(src)[w];
 }
 
+// What the pass reads from the states (k_ibm_gather), one work item per block.
 template <typename S>
-__global__ void __launch_bounds__(256) k_ibm_cells_batch(const IbmArgs* __restrict__ args, const int2* __restrict__ work) {
+__global__ void __launch_bounds__(kGatherThreads) k_ibm_gather_batch(const IbmArgs* __restrict__ args,
+                                                                     const int2* __restrict__ work) {
     __shared__ IbmArgs sa;
     __shared__ CellTile sm;
     const int2 w = work[blockIdx.x];
-    stage_args<256>(sa, args + w.x);
+    stage_args<kGatherThreads>(sa, args + w.x);
     __syncthreads();
-    ibm_cell_tile<S>(sa, sm, (w.y & 0x3ff) * 32, (w.y >> 10) * kCellPlaces, 0x7fffffff);
-}
-
-template <typename S>
-__global__ void __launch_bounds__(128) k_ibm_tail_batch(const IbmArgs* __restrict__ args, const int2* __restrict__ work) {
-    __shared__ IbmArgs sa;
-    const int2 w = work[blockIdx.x];
-    stage_args<128>(sa, args + w.x);
-    __syncthreads();
-    const int t = w.y + threadIdx.x;
-    if (t < sa.n - sa.n0) ibm_tail_marker<S>(sa, t);
-}
-
-// mask_new = mask_static, kMaskCopyWords words per work item
-__global__ void __launch_bounds__(256) k_mask_copy_batch(const IbmArgs* __restrict__ args, const int2* __restrict__ work) {
-    const int2 w = work[blockIdx.x];
-    const IbmArgs& a = args[w.x];
-    const long long words = (long long)(a.mask_bytes / sizeof(uint32_t));
-    uint32_t* dst = a.mask_new;
-    const uint32_t* src = a.mask_static;
-    for (int q = threadIdx.x; q < kMaskCopyWords; q += 256) {
-        const long long e = (long long)w.y + q;
-        if (e < words) dst[e] = src[e];
+    const int kind = w.y & 3, q = w.y >> 2;
+    if (kind == GATHER_TAIL) {
+        ibm_tail_cell<S>(sa, q * kGatherThreads + (int)threadIdx.x);
+    } else if (kind == GATHER_FLAGS) {
+        const int n4 = (int)(sa.mask_bytes / 16), v0 = q * (kMaskCopyWords / 4);
+        for (int v = v0 + (int)threadIdx.x; v < min(n4, v0 + kMaskCopyWords / 4); v += kGatherThreads)
+            reinterpret_cast<uint4*>(sa.mask_new)[v] = reinterpret_cast<const uint4*>(sa.mask_static)[v];
+    } else {
+        ibm_cell_tile<S>(sa, sm, (q & 0x3ff) * 32, (q >> 10) * kCellPlaces, 0x7fffffff);
     }
 }
 
-template <int THREADS>
-__global__ void __launch_bounds__(THREADS, THREADS == 128 ? 3 : 1) k_ibm_spread_batch(const IbmArgs* __restrict__ args,
-                                                                             const int2* __restrict__ work, int big) {
-    extern __shared__ float tile[];
+// A work item (lattice, plane) per block, blades included: the ordinary planes
+// with 128 threads, the big ones with 512.
+template <int NT>
+__global__ void __launch_bounds__(NT, NT == 128 ? 2 : 1) k_ibm_spread_batch(const IbmArgs* __restrict__ args,
+                                                                           const int2* __restrict__ work) {
+    extern __shared__ __align__(128) float btile[];
     __shared__ IbmArgs sa;
     const int2 w = work[blockIdx.x];
-    stage_args<THREADS>(sa, args + w.x);
+    stage_args<NT>(sa, args + w.x);
     __syncthreads();
-    const PlaneGroup<THREADS> grp{0, 0};
-    ibm_spread_plane<THREADS>(sa, w.y, big ? sa.big_tile_cells : sa.smem_cells, tile, grp);
+    ibm_spread_plane<NT, NT == 128, true>(sa, w.y, NT == 128 ? sa.smem_cells : sa.big_tile_cells, btile);
 }
 
-// The batch's ordinary planes, G work items (lattice, plane) per CTA: each
-// group stages its lattice's arguments and walks its plane on a tile that
-// bulk copies fill, as k_ibm_spread_bulk does for one lattice. region_cells:
-// the largest tile of the batch's lattices (the group's share of shared
-// memory); each lattice's walk uses its own tile size within it.
-// (One group per CTA: at most 170 registers, so that three such CTAs fit an
-// SM beside the other tank group's fused launch -- 64 tanks: 20,433 -> 21,000
-// MLUPS FP32; 128 registers spill and measured slower.)
-template <int NT, int G>
-__global__ void __launch_bounds__(NT * G, G == 1 ? 3 : 1) k_ibm_spread_batch_bulk(const IbmArgs* __restrict__ args,
-                                                                    const int2* __restrict__ work, int nwork,
-                                                                    int region_cells) {
-    extern __shared__ __align__(128) float btile[];             // [G][3][bulk_tile_stride(region_cells)]
-    __shared__ IbmArgs sa[G];
-    __shared__ uint64_t bars[G];
-    __shared__ int fails[G];
-    const int g = G == 1 ? 0 : (int)threadIdx.x / NT;
-    const int q = (int)blockIdx.x * G + g;
-    if (q >= nwork) return;
-    const PlaneGroup<NT, (G > 1)> grp{g * NT, g + 1};
-    const int2 w = work[q];
-    constexpr int words = sizeof(IbmArgs) / 8;
-    for (int i = grp.tid(); i < words; i += NT)
-        reinterpret_cast<unsigned long long*>(&sa[g])[i] = reinterpret_cast<const unsigned long long*>(args + w.x)[i];
-    grp.sync();
-    ibm_spread_plane<NT, true, PlaneGroup<NT, (G > 1)>, (NT * G <= 384)>(
-        sa[g], w.y, sa[g].smem_cells, btile + (size_t)g * 3 * bulk_tile_stride(region_cells), grp, &bars[g],
-                               &fails[g]);
-}
-
-// Work items per CTA of the batched ordinary-plane spread: one. The batch's
-// forcing pass runs beside the other tank group's fused launch, and a CTA of
-// G groups holds G x 128 threads' registers (128-255 each) for its whole
-// walk; measured on B200 (64 tanks, 20 steps): G <= 4 18,082 MLUPS FP32,
-// G <= 2 19,086, G = 1 19,442 (FP16: 22,863 at G = 1).
-static int batch_spread_groups(int cells) {
-    (void)cells;
-    return 1;
-}
-
-template <int G>
-static const void* batch_bulk_fn() { return (const void*)k_ibm_spread_batch_bulk<128, G>; }
-
-cudaError_t ibm_batch_prepare_smem(size_t small_bytes, size_t big_bytes) {
-    (void)small_bytes;
-    // every variant may be launched (tank groups with smaller tiles take more
-    // work items per CTA): each gets the dynamic shared memory its widest
-    // launch can use
-    const void* fns[4] = {batch_bulk_fn<1>(), batch_bulk_fn<2>(), batch_bulk_fn<3>(), batch_bulk_fn<4>()};
-    for (int G = 1; G <= 4; G++) {
-        const size_t bytes = 227 * 1024 - (size_t)G * (sizeof(IbmArgs) + 16) - 256;
-        cudaError_t e = raise_smem_limit(fns[G - 1], bytes);
-        if (e != cudaSuccess) return e;
-    }
-    return raise_smem_limit((const void*)k_ibm_spread_batch<512>, big_bytes);
-}
-
-template <int G>
-static void batch_spread_small(const IbmBatch& b, cudaStream_t st) {
-    const unsigned grid = (unsigned)((b.n_small + G - 1) / G);
-    const size_t bytes = (size_t)G * 12 * bulk_tile_stride(b.small_tile);
-    k_ibm_spread_batch_bulk<128, G><<<grid, 128 * G, bytes, st>>>(b.args, b.small, b.n_small, b.small_tile);
+cudaError_t ibm_batch_prepare_smem(int small_cells, int big_cells) {
+    const cudaError_t e = raise_smem_limit((const void*)k_ibm_spread_batch<128>, big_bulk_bytes(small_cells));
+    return e != cudaSuccess ? e : raise_smem_limit((const void*)k_ibm_spread_batch<512>, big_bulk_bytes(big_cells));
 }
 
 cudaError_t launch_ibm_batch(const IbmBatch& b, cudaStream_t st, cudaStream_t side, cudaEvent_t fork, cudaEvent_t join) {
-    if (b.n_cells > 0) {
+    if (b.n_gather > 0) {
         with_storage(b.storage, [&](auto s) {
-            k_ibm_cells_batch<decltype(s)><<<b.n_cells, 256, 0, st>>>(b.args, b.cells);
+            k_ibm_gather_batch<decltype(s)><<<b.n_gather, kGatherThreads, 0, st>>>(b.args, b.gather);
         });
     }
-    if (b.n_tails > 0) {
-        with_storage(b.storage, [&](auto s) {
-            k_ibm_tail_batch<decltype(s)><<<b.n_tails, 128, 0, st>>>(b.args, b.tails);
-        });
-    }
-    if (b.n_copies > 0) k_mask_copy_batch<<<b.n_copies, 256, 0, st>>>(b.args, b.copies);
     cudaError_t err = cudaGetLastError();
     if (err != cudaSuccess) return err;
     if (b.n_big > 0) {
@@ -1266,20 +1239,13 @@ cudaError_t launch_ibm_batch(const IbmBatch& b, cudaStream_t st, cudaStream_t si
         if (err != cudaSuccess) return err;
         err = cudaStreamWaitEvent(side, fork, 0);
         if (err != cudaSuccess) return err;
-        k_ibm_spread_batch<512><<<b.n_big, 512, ibm_smem_bytes(Dims{}, b.big_tile), side>>>(b.args, b.big, 1);
+        k_ibm_spread_batch<512><<<b.n_big, 512, big_bulk_bytes(b.big_tile), side>>>(b.args, b.big);
         err = cudaGetLastError();
         if (err != cudaSuccess) return err;
         err = cudaEventRecord(join, side);
         if (err != cudaSuccess) return err;
     }
-    if (b.n_small > 0) {
-        switch (batch_spread_groups(b.small_tile)) {
-            case 4: batch_spread_small<4>(b, st); break;
-            case 3: batch_spread_small<3>(b, st); break;
-            case 2: batch_spread_small<2>(b, st); break;
-            default: batch_spread_small<1>(b, st); break;
-        }
-    }
+    if (b.n_small > 0) k_ibm_spread_batch<128><<<b.n_small, 128, big_bulk_bytes(b.small_tile), st>>>(b.args, b.small);
     err = cudaGetLastError();
     if (err != cudaSuccess) return err;
     if (b.n_big > 0) return cudaStreamWaitEvent(st, join, 0);

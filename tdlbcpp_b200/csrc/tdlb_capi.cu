@@ -84,6 +84,7 @@ void release(tdlb_lattice* h) {
     cudaFree(h->d_red);
     cudaFree(h->d_rot_xz);
     cudaFree(h->d_load);
+    cudaFree(h->d_imp_slots);
     cudaFree(h->d_res[0]);
     cudaFree(h->d_res[1]);
     for (auto& st : h->pin) {
@@ -142,8 +143,6 @@ tdlb_lattice* build(const tdlb_config& c, int device) {
         // (the limit that the 16-element row granule along z gave)
         if (c.x * c.y * round_up(c.z, 16) >= tdlb::kMaxPlane || g.rows() * g.jp >= tdlb::kMaxPlane)
             throw Fail{TDLB_EINVAL, "lattice too large: one population plane must stay below 2^31 elements"};
-        if (tdlb::ibm_smem_bytes(g, 0) > 200 * 1024)
-            throw Fail{TDLB_EINVAL, "x * ceil(z/32) too large for the per-plane IBM flag tile"};
         h->cp = tdlb::make_collide_params(c.nu, c.cs0, c.g3);
         tdlb::set_rest(h->cp, c.initialRho);
 
@@ -583,12 +582,14 @@ void update_blade_planes(tdlb_lattice* h) {
     const int L0 = h->n_level0;
     std::vector<int> planes;
     int words = 0;
+    h->blade_max = 0;
     for (int j = 0; j < g.ny; j++) {
         if (lv[(size_t)j] == lv[(size_t)j + 1]) continue;
         planes.push_back(j);
         // the level ranges are global level indices; seg1's level_ptr starts at level L0
         const int nb = lp[(size_t)(lv[(size_t)j + 1] - L0)] - lp[(size_t)(lv[(size_t)j] - L0)];
         words = std::max(words, tdlb::blade_table_words(nb));
+        h->blade_max = std::max(h->blade_max, nb);
     }
     words = std::min(words, 220 * 1024 / 4);   // a plane beyond this walks its blades on global memory
     if (planes != h->h_blade_planes) {
@@ -664,7 +665,7 @@ void plan_planes(tdlb_lattice* h, const int* count) {
     h->n_small = (int)small.size();
     h->n_big = (int)big.size();
     h->big_tile_cells = tdlb::big_bulk_bytes(h->max_big) <= 220 * 1024 ? h->max_big : 0;
-    TDLB_CK(tdlb::ibm_prepare_smem(h->smem_cells, h->n_small, tdlb::big_bulk_bytes(h->big_tile_cells)));
+    TDLB_CK(tdlb::ibm_prepare_smem(h->smem_cells, tdlb::big_bulk_bytes(h->big_tile_cells)));
     small.insert(small.end(), big.begin(), big.end());
     if (!h->d_plane_list) TDLB_CK(cudaMalloc(&h->d_plane_list, (size_t)g.ny * sizeof(int)));
     TDLB_CK(cudaMemcpyAsync(h->d_plane_list, small.data(), (size_t)g.ny * sizeof(int), cudaMemcpyHostToDevice, h->stream));
@@ -813,7 +814,7 @@ void upload_markers(tdlb_lattice* h, const tdlb_marker* m, size_t n, size_t n0, 
     if (n0) TDLB_CK(tdlb::launch_ibm_prepare(ibm_args(h, 0.f, 0.f), h->d_prep, h->stream));
     // the blades
     h->h_blade_planes.clear();
-    h->n_blade = 0;
+    h->n_blade = h->blade_max = 0;
     if (ntail > 0) {
         build_blades(h, rot_xz);
         upload_seg1(h);
@@ -852,6 +853,7 @@ tdlb::IbmArgs ibm_args(tdlb_lattice* h, float alpha, float beta) {
     a.blade_planes = h->d_blade_planes;
     a.n_blade = h->n_blade;
     a.blade_words = h->blade_words;
+    a.blade_max = h->blade_max;
     a.big_tile_cells = h->big_tile_cells;
     a.side = h->side;
     a.ev_fork = h->ev_fork;
@@ -876,8 +878,8 @@ tdlb::IbmArgs ibm_args(tdlb_lattice* h, float alpha, float beta) {
 void run_forcing(tdlb_lattice* h, float alpha, float beta) {
     if (!h->markers_set) throw Fail{TDLB_ESTATE, "no markers set (tdlb_set_markers / tdlb_forcing)"};
     TDLB_CK(tdlb::launch_ibm(ibm_args(h, alpha, beta), h->stream));
-    h->launches += (h->max_cells > 0 ? 1 : 0) + (h->n_big > 0 ? 1 : 0) + (h->n_markers > h->n0 ? 1 : 0) + (h->n_small > 0 ? 1 : 0) +
-                   (h->n_big > 0 ? 1 : 0) + (h->n_blade > 0 ? 1 : 0);
+    h->launches += 1 + (h->n_small > 0 ? 1 : 0) + (h->n_big > 0 ? 1 : 0) +
+                   (h->n_blade > 0 && (h->n_big > 0 || h->blade_max > 128) ? 1 : 0);
     h->pass++;
     h->last_beta = beta;
 }
@@ -1341,17 +1343,56 @@ int tdlb_set_rotating_markers(tdlb_handle h, const tdlb_marker* markers, size_t 
     });
 }
 
+// The impeller's slots of the resident list. (Its blades keep their slots while
+// they rotate on the device; a host list of blades reorders them within the
+// second segment, which is the impeller's whole.)
+static void find_impeller_slots(tdlb_lattice* h) {
+    if (h->imp_gen == h->marker_gen) return;
+    const int n = h->n_markers, groups = (n + 255) / 256;
+    cudaFree(h->d_imp_slots);
+    h->d_imp_slots = nullptr;
+    h->n_imp = 0;
+    if (n > 0) {
+        struct Tmp {
+            int* p = nullptr;
+            ~Tmp() { cudaFree(p); }
+        } off;
+        std::vector<int> count((size_t)groups);
+        TDLB_CK(cudaMalloc(&off.p, (size_t)groups * sizeof(int)));
+        TDLB_CK(tdlb::launch_impeller_slots(h->d_sched, n, h->impeller_begin, off.p, nullptr, h->stream));
+        TDLB_CK(cudaMemcpyAsync(count.data(), off.p, (size_t)groups * sizeof(int), cudaMemcpyDeviceToHost, h->stream));
+        TDLB_CK(cudaStreamSynchronize(h->stream));
+        int sum = 0;
+        for (int& c : count) {
+            const int v = c;
+            c = sum;
+            sum += v;
+        }
+        TDLB_CK(cudaMalloc(&h->d_imp_slots, (size_t)std::max(sum, 1) * sizeof(int)));
+        TDLB_CK(cudaMemcpyAsync(off.p, count.data(), (size_t)groups * sizeof(int), cudaMemcpyHostToDevice, h->stream));
+        TDLB_CK(tdlb::launch_impeller_slots(h->d_sched, n, h->impeller_begin, off.p, h->d_imp_slots, h->stream));
+        TDLB_CK(cudaStreamSynchronize(h->stream));
+        h->n_imp = sum;
+    }
+    h->imp_gen = h->marker_gen;
+}
+
 // Queue the impeller load of the last forcing pass and its copy into out5.
 void queue_impeller_load(tdlb_lattice* h, double* out5) {
     if (!out5) throw Fail{TDLB_EINVAL, "out is NULL"};
     if (h->impeller_begin < 0) throw Fail{TDLB_ESTATE, "no impeller attached (tdlb_attach_rushton)"};
     if (h->pass == 0) throw Fail{TDLB_ESTATE, "no forcing pass yet"};
-    if (!h->d_load) TDLB_CK(cudaMalloc(&h->d_load, (size_t)(tdlb::kLoadBlocks * 5 + 5) * sizeof(double)));
+    constexpr size_t kDoubles = (size_t)tdlb::kLoadBlocks * 5 + 5 + 1;
+    if (!h->d_load) {
+        TDLB_CK(cudaMalloc(&h->d_load, kDoubles * sizeof(double)));
+        TDLB_CK(cudaMemsetAsync(h->d_load, 0, kDoubles * sizeof(double), h->stream));
+    }
+    find_impeller_slots(h);
     tdlb::IbmArgs a = ibm_args(h, 0.f, h->last_beta);
-    TDLB_CK(tdlb::launch_marker_load(a, h->impeller_begin, h->rot_ci, h->rot_ck, h->d_load,
-                                     h->d_load + tdlb::kLoadBlocks * 5, h->stream));
-    TDLB_CK(cudaMemcpyAsync(out5, h->d_load + tdlb::kLoadBlocks * 5, 5 * sizeof(double), cudaMemcpyDefault,
-                            h->stream));
+    double* out = h->d_load + tdlb::kLoadBlocks * 5;
+    TDLB_CK(tdlb::launch_marker_load(a, h->d_imp_slots, h->n_imp, h->rot_ci, h->rot_ck, h->d_load, (unsigned*)(out + 5), out,
+                                     h->stream));
+    TDLB_CK(cudaMemcpyAsync(out5, out, 5 * sizeof(double), cudaMemcpyDefault, h->stream));
 }
 
 int tdlb_impeller_load(tdlb_handle h, double* out5) {

@@ -68,7 +68,7 @@ struct tdlb_lattice {
     // the planes with blade levels, walked by their own launch
     std::vector<int> h_blade_planes;
     int* d_blade_planes = nullptr;
-    int n_blade = 0, blade_words = 0;
+    int n_blade = 0, blade_words = 0, blade_max = 0;
     cudaStream_t side = nullptr;
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
     uint32_t* d_mask_static = nullptr;   // first segment's touched cells
@@ -92,7 +92,10 @@ struct tdlb_lattice {
     tdlb_rushton rspec{};         // the attached impeller's spec
     double angle = 0.0;           // impeller angle of the last rotation
     unsigned long long rstep = 1; // main-loop step the angle belongs to (main.cpp:336 starts at 1)
-    double* d_load = nullptr;     // kLoadBlocks*5 partials + 5 results
+    double* d_load = nullptr;     // kLoadBlocks*5 partials + 5 results + a counter
+    int* d_imp_slots = nullptr;   // the impeller's slots, ascending, for marker_gen imp_gen
+    int n_imp = 0;
+    unsigned imp_gen = ~0u;
     // pinned staging of the per-step blade upload (markers and their
     // schedule), two buffers used in turn; each buffer's event marks the end
     // of the copies that read it

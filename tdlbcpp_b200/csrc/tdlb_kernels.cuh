@@ -146,6 +146,7 @@ struct IbmArgs {
     int n_small, n_big;         // planes in each launch
     const int* blade_planes;    // the planes with blade levels (the blade launch)
     int n_blade, blade_words;   // their count; shared-memory floats of the blade launch
+    int blade_max, pad0;        // most blade markers of a plane
     int big_tile_cells;         // F tile capacity of the big-plane launch
     cudaStream_t side;          // stream of the big-plane launch
     cudaEvent_t ev_fork, ev_join;
@@ -203,42 +204,45 @@ cudaError_t launch_sched_levels(const SchedArgs& a, int max_cells, int ncell, cu
 cudaError_t raise_smem_limit(const void* fn, size_t bytes);
 
 // Immersed-boundary passes of many lattices in one set of launches: device
-// IbmArgs per lattice and work lists of (lattice, first index) items --
-// cells: places 8 (y >> 10) .. + 8 of the planes 32 (y & 1023) .. + 32; tails: 128 blade markers; copies: 1024
-// touched-flag words; small / big: one j-plane (128 / 512 threads).
+// IbmArgs per lattice and work lists of (lattice, item). gather: 4 q + kind --
+// the places 8 (q >> 10) .. + 8 of the planes 32 (q & 1023) .. + 32, the 256
+// (blade marker, cell) pairs from 256 q, the kMaskCopyWords touched-flag words
+// from kMaskCopyWords q; small / big: one j-plane (128 / 512 threads).
+enum GatherKind { GATHER_CELLS = 0, GATHER_TAIL = 1, GATHER_FLAGS = 2 };
 struct IbmBatch {
     const IbmArgs* args;
-    const int2* cells; int n_cells;
-    const int2* tails; int n_tails;
-    const int2* copies; int n_copies;
+    const int2* gather; int n_gather;
     const int2* small; int n_small;
     const int2* big; int n_big;
     int small_tile, big_tile;   // dynamic F tiles (cells) of the two spread launches
     int storage;
 };
-constexpr int kMaskCopyWords = 1024;
+constexpr int kMaskCopyWords = 8192;
 cudaError_t launch_ibm_batch(const IbmBatch& b, cudaStream_t st, cudaStream_t side, cudaEvent_t fork, cudaEvent_t join);
-cudaError_t ibm_batch_prepare_smem(size_t small_bytes, size_t big_bytes);
+cudaError_t ibm_batch_prepare_smem(int small_cells, int big_cells);
 // Per-upload preparation of the first segment (weights, velocities).
 cudaError_t launch_ibm_prepare(const IbmArgs& a, float* prep, cudaStream_t st);
-// Shared memory the spread kernel needs: the plane's touched-flag tile plus
-// an F tile of `cells` cells.
-size_t ibm_smem_bytes(const Dims& g, int cells);
 // Opt the spread kernels in to the dynamic shared memory of the ordinary
 // planes' launch (tiles of `small_cells` cells) and of the big planes'
 // launch (`big_bytes`).
-cudaError_t ibm_prepare_smem(int small_cells, int n_small, size_t big_bytes);
+cudaError_t ibm_prepare_smem(int small_cells, size_t big_bytes);
 // Shared memory of the big planes' launch for a tile of `big_cells` cells.
 size_t big_bulk_bytes(int big_cells);
 // Shared-memory floats of the blade launch for a plane of nb blade markers,
 // and the opt-in to that many.
 int blade_table_words(int nb);
 cudaError_t ibm_prepare_blades(int words);
-// FP64 force and torque of markers [begin, n) (by list index) of the last
-// forcing pass: out[0..2] = -beta * sum of spread sums, out[3] = torque about
-// the tank axis (ci, ck), out[4] = number of markers summed. `partial` holds
-// kLoadBlocks * 5 doubles.
+// FP64 force and torque of the impeller's slots of the last forcing pass:
+// out[0..2] = -beta * sum of spread sums, out[3] = torque about the tank axis
+// (ci, ck), out[4] = number of markers summed. `partial` holds kLoadBlocks * 5
+// doubles, `counter` is zero between launches.
 constexpr int kLoadBlocks = 128;
+cudaError_t launch_marker_load(const IbmArgs& a, const int* slots, int n, double ci, double ck, double* partial,
+                               unsigned* counter, double* out, cudaStream_t st);
+// Slots of the markers with list index >= begin, ascending: slots NULL: their
+// number in each group of 256 slots to `offset`; else to slots, from each
+// group's offset.
+cudaError_t launch_impeller_slots(const int* sched, int n, int begin, int* offset, int* slots, cudaStream_t st);
 // FP64 mass/momentum reduction: out[0] = sum rho, out[1..3] = sum (j + F/2).
 // `partial` holds kReduceBlocks * 4 doubles.
 constexpr int kReduceBlocks = 592;
@@ -246,8 +250,6 @@ cudaError_t launch_reduce_fp64(const IbmArgs& a, const uint32_t* mask, double* p
 // Rest state at density rho for the 16-bit storage.
 cudaError_t launch_fill_rest(Planes Q, long long plane, float rho, float rho0, int storage, const CollideParams& p,
                              cudaStream_t st);
-cudaError_t launch_marker_load(const IbmArgs& a, int begin, double ci, double ck, double* partial, double* out,
-                               cudaStream_t st);
 // Recompute n rotating markers (offsets xz[2n]) for cos/sin (ca, sa).
 cudaError_t launch_rotate_markers(const double* xz, Marker* out, int n, double ca, double sa, double omega, double ci,
                                   double ck, int nx, int nz, cudaStream_t st);
