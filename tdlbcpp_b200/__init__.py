@@ -456,11 +456,9 @@ class ComputeUnit:
     def plane_xz(self, j: int):
         """savePlaneXZ<float, 4> records: (moments of non-excluded cells, F where non-zero)."""
         nq, nf = ctypes.c_size_t(), ctypes.c_size_t()
-        self._check(self.lib.tdlb_plane_xz(self.h, j, None, 0, ctypes.byref(nq), None, 0, ctypes.byref(nf)))
-        q = np.zeros(nq.value, DISK_GRID4_DTYPE)
-        f = np.zeros(nf.value, DISK_GRID3_DTYPE)
+        q, f = np.empty(self.x * self.z, DISK_GRID4_DTYPE), np.empty(self.x * self.z, DISK_GRID3_DTYPE)
         self._check(self.lib.tdlb_plane_xz(self.h, j, _p(q), len(q), ctypes.byref(nq), _p(f), len(f), ctypes.byref(nf)))
-        return q, f
+        return tuple(a if n.value == len(a) else a[:n.value].copy() for a, n in ((q, nq), (f, nf)))
 
     def set_cells_per_thread(self, v: int):
         """Step-kernel variant (1, 2 or 4 cells per thread)."""

@@ -224,17 +224,10 @@ private:
     std::vector<std::thread> threads_;
 };
 
-// The handle's device scratch, at least `bytes` long.
 char* scratch(tdlb_lattice* h, size_t bytes) {
-    if (bytes > h->scratch_bytes) {
-        TDLB_FCK(cudaStreamSynchronize(h->stream));
-        cudaFree(h->d_scratch);
-        h->d_scratch = nullptr;
-        h->scratch_bytes = 0;
-        TDLB_FCK(cudaMalloc(&h->d_scratch, bytes));
-        h->scratch_bytes = bytes;
-    }
-    return (char*)h->d_scratch;
+    char* p = nullptr;
+    TDLB_FCK(tdlb_rt::scratch(h, bytes, &p));
+    return p;
 }
 
 // Slabs of i of at most about this many bytes of output at a time: enough for

@@ -1476,6 +1476,21 @@ void return_stream(tdlb_lattice* h) {
     h->own_stream = nullptr;
 }
 
+cudaError_t scratch(tdlb_lattice* h, size_t bytes, char** out) {
+    if (bytes > h->scratch_bytes) {
+        cudaError_t e = cudaStreamSynchronize(h->stream);   // (calls wait for their copies, so nothing uses it)
+        if (e != cudaSuccess) return e;
+        cudaFree(h->d_scratch);
+        h->d_scratch = nullptr;
+        h->scratch_bytes = 0;
+        e = cudaMalloc(&h->d_scratch, bytes);
+        if (e != cudaSuccess) return e;
+        h->scratch_bytes = bytes;
+    }
+    *out = (char*)h->d_scratch;
+    return cudaSuccess;
+}
+
 void drop_zone(tdlb_lattice* h) {
     cudaFree(h->d_zone_core);
     cudaFree(h->d_zone_skip);

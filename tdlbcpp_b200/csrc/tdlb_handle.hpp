@@ -204,6 +204,8 @@ void return_stream(tdlb_lattice* h);
 // next outer launch of a split step waits for it (every entry point other than
 // the step loop's calls it).
 inline void fence(tdlb_lattice* h) { h->bulk_ok = false; }
+// The handle's device scratch, at least `bytes` long (kept for the next call).
+cudaError_t scratch(tdlb_lattice* h, size_t bytes, char** out);
 // Free the zone's arrays (the lattice changed size).
 void drop_zone(tdlb_lattice* h);
 // Remove the residual box (a tank joining a batch, whose step kernel keeps
