@@ -121,7 +121,7 @@ __device__ __forceinline__ void prefetch_chunk(const TankStep& ts, unsigned q0) 
 // NULL) is advanced once: this launch runs after the step's rotation, which
 // reads it.
 template <typename S, int V, int NT, bool ESO>
-__global__ void __launch_bounds__(NT, (ESO ? kEsotwistBlocksPerSM<V> : 4) * 128 / NT) k_batch_step(const TankStep* __restrict__ tanks, const int2* __restrict__ work,
+__global__ void __launch_bounds__(NT, (ESO ? kEsotwistBlocksPerSM<S, V> : 4) * 128 / NT) k_batch_step(const TankStep* __restrict__ tanks, const int2* __restrict__ work,
                                                    int nwork, int* counter, int ahead) {
     constexpr bool kFM = sizeof(S) == 4;
     __shared__ TankStep ts;

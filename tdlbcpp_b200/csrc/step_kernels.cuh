@@ -323,9 +323,9 @@ __device__ __forceinline__ void box_read_eso(const ResidualBox& rb, int i, int j
 // together. V = 1 pulls every population directly from x - c_d. V > 1 loads
 // aligned vectors of the upstream rows and moves j-shifted values between
 // lanes with shuffles; the values a lane cannot get from a neighbour (warp
-// edges) and the own values the wall rule needs at row ends come from
-// scalar loads issued in the same batch (in bounds for every lane; the ones
-// a lane does not need hit L1).
+// edges) and the own values the wall rule needs at row ends come from scalar
+// loads of those lanes alone, issued in the same batch. (Issued by every lane,
+// as they were, they doubled the load instructions of the 16-bit kernels.)
 // ---------------------------------------------------------------------------
 template <typename S, int V, bool LES, bool FROM_MOMENTS, bool COLLIDE, int PART = 0>
 __device__ __forceinline__ void simple_quad(const Planes& A, const Planes& B, float* __restrict__ Nu,
@@ -358,7 +358,7 @@ __device__ __forceinline__ void simple_quad(const Planes& A, const Planes& B, fl
             f[d][0] = pload1<S, true>(A.p[d], q.e0 + off);
         }
     } else {
-        float hal[NQ], own[NQ];
+        float ext[NQ];   // what a lane cannot get from its neighbour
         // batch 1: every load
 #pragma unroll
         for (int d = 0; d < NQ; d++) {
@@ -368,13 +368,11 @@ __device__ __forceinline__ void simple_quad(const Planes& A, const Planes& B, fl
             const int src = q.e0 + soff;
             pload<S, V, true>(A.p[d], src, f[d]);
             if (cy > 0) {
-                hal[d] = pload1<S, true>(A.p[d], (lane == 0 && !j_first) ? src - 1 : src);
-                own[d] = (cx != 0 || cz != 0) ? pload1<S, true>(A.p[d], q.e0) : 0.f;
+                ext[d] = (j_first || lane == 0) ? pload1<S, true>(A.p[d], j_first ? q.e0 : src - 1) : 0.f;
             } else if (cy < 0) {
-                hal[d] = pload1<S, true>(A.p[d], (lane == SEG - 1 && !j_last) ? src + V : src);
                 int le = g.ny - 1 - q.j0;
                 le = le < 0 ? 0 : (le > V - 1 ? V - 1 : le);
-                own[d] = (cx != 0 || cz != 0) ? pload1<S, true>(A.p[d], q.e0 + le) : 0.f;
+                ext[d] = (j_last || lane == SEG - 1) ? pload1<S, true>(A.p[d], j_last ? q.e0 + le : src + V) : 0.f;
             }
         }
         // batch 2: shift along j
@@ -383,32 +381,23 @@ __device__ __forceinline__ void simple_quad(const Planes& A, const Planes& B, fl
             const int cx = cx_of(d), cy = cy_of(d), cz = cz_of(d);
             const bool row_ok = !((cx > 0 && i_lo) || (cx < 0 && i_hi) || (cz > 0 && k_lo) || (cz < 0 && k_hi));
             if (cy > 0) {                          // source j - 1
-                float left = __shfl_up_sync(FULL, f[d][V - 1], 1);
-                if (lane == 0) left = hal[d];
-                const float own0 = (cx != 0 || cz != 0) ? own[d] : f[d][0];
+                const float left = __shfl_up_sync(FULL, f[d][V - 1], 1);
                 if (row_ok) {
 #pragma unroll
                     for (int e = V - 1; e > 0; e--) f[d][e] = f[d][e - 1];
-                    f[d][0] = j_first ? own0 : left;
+                    f[d][0] = (j_first || lane == 0) ? ext[d] : left;
                 }
             } else if (cy < 0) {                   // source j + 1
-                float right = __shfl_down_sync(FULL, f[d][0], 1);
-                if (lane == SEG - 1) right = hal[d];
+                const float right = __shfl_down_sync(FULL, f[d][0], 1);
                 const int le = g.ny - 1 - q.j0;   // element of the row's last cell when j_last
-                float ownl = own[d];
-                if (cx == 0 && cz == 0) {
-#pragma unroll
-                    for (int e = 0; e < V; e++)
-                        if (e == le) ownl = f[d][e];
-                }
                 if (row_ok) {
 #pragma unroll
                     for (int e = 0; e < V - 1; e++) f[d][e] = f[d][e + 1];
-                    f[d][V - 1] = right;
+                    f[d][V - 1] = lane == SEG - 1 ? ext[d] : right;
                     if (j_last) {
 #pragma unroll
                         for (int e = 0; e < V; e++)
-                            if (e == le) f[d][e] = ownl;
+                            if (e == le) f[d][e] = ext[d];
                     }
                 }
             }
@@ -499,7 +488,7 @@ __device__ __forceinline__ void esotwist_quad(const Planes& Q, float* __restrict
             }
         }
     } else {
-        float hal[NQ], wrap[NQ];
+        float ext[NQ];   // what a lane cannot get from the next one
 #pragma unroll
         for (int s = 0; s < NQ; s++) {
             const int sg = EVEN ? -1 : 1;
@@ -508,8 +497,7 @@ __device__ __forceinline__ void esotwist_quad(const Planes& Q, float* __restrict
             const int base = ((oi ? i1 : q.i) * g.nz + (ok ? k1 : q.k)) * g.jp;
             pload<S, V, false>(Q.p[s], base + q.j0, f[d]);
             if (oj) {
-                hal[s] = pload1<S, false>(Q.p[s], base + ((lane == SEG - 1 && !j_last) ? q.j0 + V : q.j0));
-                wrap[s] = pload1<S, false>(Q.p[s], base);
+                ext[s] = (j_last || lane == SEG - 1) ? pload1<S, false>(Q.p[s], base + (j_last ? 0 : q.j0 + V)) : 0.f;
             }
         }
 #pragma unroll
@@ -518,15 +506,14 @@ __device__ __forceinline__ void esotwist_quad(const Planes& Q, float* __restrict
             const bool oj = sg * cy_of(s) > 0;
             const int d = EVEN ? s : (s ^ 1);
             if (!oj) continue;
-            float right = __shfl_down_sync(FULL, f[d][0], 1);
-            if (lane == SEG - 1) right = hal[s];
+            const float right = __shfl_down_sync(FULL, f[d][0], 1);
 #pragma unroll
             for (int e = 0; e < V - 1; e++) f[d][e] = f[d][e + 1];
-            f[d][V - 1] = right;
+            f[d][V - 1] = lane == SEG - 1 ? ext[s] : right;
             if (j_last) {                          // j = ny-1 wraps to 0
 #pragma unroll
                 for (int e = 0; e < V; e++)
-                    if (e == last_e) f[d][e] = wrap[s];
+                    if (e == last_e) f[d][e] = ext[s];
             }
         }
     }
@@ -681,12 +668,14 @@ __global__ void __launch_bounds__(128, 4) k_step_simple(Planes A, Planes B, floa
 
 // Resident 128-thread blocks per SM the Esotwist kernel is built for: the
 // register cap that follows (64 at one cell per thread) keeps enough loads in
-// flight; measured on B200 at 400^3, 8 blocks beat 4 by about 5%.
-template <int V>
-constexpr int kEsotwistBlocksPerSM = V == 1 ? 8 : (V == 2 ? 6 : 4);
+// flight; measured on B200 at 400^3, 8 blocks beat 4 by about 5%. 16-bit storage
+// at two cells per thread: 5 blocks 1.287 ms, 6 1.127, 7 1.100, 8 1.071; at four:
+// 3 1.420, 4 1.150, 5 1.183, 6 1.274.
+template <typename S, int V>
+constexpr int kEsotwistBlocksPerSM = V == 1 ? 8 : V == 2 ? (sizeof(S) == 2 ? 8 : 6) : 4;
 
 template <typename S, int V, bool LES, bool FROM_MOMENTS, bool COLLIDE, bool EVEN, int PART = 0>
-__global__ void __launch_bounds__(128, kEsotwistBlocksPerSM<V>) k_step_esotwist(Planes Q, float* __restrict__ Nu,
+__global__ void __launch_bounds__(128, kEsotwistBlocksPerSM<S, V>) k_step_esotwist(Planes Q, float* __restrict__ Nu,
                                                          const float4* __restrict__ F, const uint32_t* __restrict__ mask,
                                                          Dims g, CollideParams p, StepPart part) {
     if constexpr (PART != 2 && COLLIDE && !FROM_MOMENTS)
