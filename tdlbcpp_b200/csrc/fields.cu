@@ -18,6 +18,7 @@
 #endif
 
 #include <algorithm>
+#include <atomic>
 #include <string>
 #include <thread>
 #include <vector>
@@ -190,24 +191,28 @@ struct Out {
 // buffer that cannot be populated, only copy more slowly.
 class Populate {
 public:
-    explicit Populate(const std::vector<std::pair<char*, size_t>>& bufs) {
+    // ranges in the order the copies will take them
+    explicit Populate(const std::vector<std::pair<char*, size_t>>& ranges) {
         size_t total = 0;
-        for (const auto& b : bufs) total += b.second;
+        for (const auto& r : ranges) total += r.second;
         if (total < kLeast) return;
+        // whole huge pages where the caller's memory has them
+        for (const auto& r : ranges) {
+            const uintptr_t page = (uintptr_t)sysconf(_SC_PAGESIZE);
+            const uintptr_t hi = ((uintptr_t)r.first + r.second) / page * page;
+            for (uintptr_t a = ((uintptr_t)r.first + page - 1) / page * page; a < hi;) {
+                const uintptr_t e = std::min(hi, (a / kPiece + 1) * kPiece);
+                pieces_.emplace_back(a, e - a);
+                a = e;
+            }
+        }
         const unsigned hw = std::thread::hardware_concurrency();
-        const int n = (int)std::min<size_t>(std::max(1u, std::min(8u, hw / 2)), total / kLeast + 1);
+        const size_t n = std::min<size_t>(std::max(1u, std::min(8u, hw / 2)), total / kLeast + 1);
         try {
-            for (int t = 0; t < n; t++)
-                threads_.emplace_back([bufs, t, n] {
-                    const uintptr_t page = (uintptr_t)sysconf(_SC_PAGESIZE);
-                    size_t piece = 0;
-                    for (const auto& b : bufs) {
-                        const uintptr_t lo = ((uintptr_t)b.first + page - 1) / page * page;
-                        const uintptr_t hi = ((uintptr_t)b.first + b.second) / page * page;
-                        for (uintptr_t a = lo; a < hi; a += kPiece, piece++)
-                            if (piece % (size_t)n == (size_t)t)
-                                if (madvise((void*)a, std::min<size_t>(kPiece, hi - a), MADV_POPULATE_WRITE) != 0) return;
-                    }
+            for (size_t t = 0; t < n; t++)
+                threads_.emplace_back([this] {
+                    for (size_t q; (q = next_.fetch_add(1)) < pieces_.size();)
+                        if (madvise((void*)pieces_[q].first, pieces_[q].second, MADV_POPULATE_WRITE) != 0) return;
                 });
         } catch (const std::exception&) {
             // no more threads: the copies do without
@@ -220,7 +225,9 @@ public:
     }
 
 private:
-    static constexpr size_t kLeast = (size_t)4 << 20, kPiece = (size_t)1 << 20;
+    static constexpr size_t kLeast = (size_t)4 << 20, kPiece = (size_t)4 << 20;
+    std::vector<std::pair<uintptr_t, size_t>> pieces_;
+    std::atomic<size_t> next_{0};
     std::vector<std::thread> threads_;
 };
 
@@ -242,11 +249,7 @@ void read_out(tdlb_lattice* h, const std::vector<Out>& outs, L&& launch) {
     const Dims& g = h->g;
     const size_t line = (size_t)g.ny * g.nz;
     size_t per = 0;
-    std::vector<std::pair<char*, size_t>> bufs;
-    for (const Out& o : outs) {
-        per += o.per;
-        if (o.dst) bufs.emplace_back((char*)o.dst, o.per * (size_t)g.cells());
-    }
+    for (const Out& o : outs) per += o.per;
     const int ni = (int)std::min<size_t>((size_t)g.nx, std::max<size_t>(1, kSlabBytes / (per * line)));
     std::vector<size_t> at(outs.size());
     size_t bytes = 0;
@@ -255,7 +258,11 @@ void read_out(tdlb_lattice* h, const std::vector<Out>& outs, L&& launch) {
         bytes += (outs[q].per * line * (size_t)ni + 255) / 256 * 256;
     }
     char* base = scratch(h, bytes);
-    Populate populate(bufs);
+    std::vector<std::pair<char*, size_t>> ranges;
+    for (int i0 = 0; i0 < g.nx; i0 += ni)
+        for (const Out& o : outs)
+            if (o.dst) ranges.emplace_back((char*)o.dst + o.per * line * (size_t)i0, o.per * line * (size_t)std::min(ni, g.nx - i0));
+    Populate populate(ranges);
     for (int i0 = 0; i0 < g.nx; i0 += ni) {
         const int n = std::min(ni, g.nx - i0);
         launch(i0, n, base, at);

@@ -78,11 +78,8 @@ extern "C" {
 
 int tdlb_double_resolution(tdlb_handle h) {
     if (!h) return TDLB_EINVAL;
-    float* A = nullptr;
-    float* B = nullptr;
-    float* Nu = nullptr;
-    float* F = nullptr;
-    uint32_t* mask = nullptr;
+    char* block = nullptr;
+    tdlb_rt::LatticeBlock lb{};
     try {
         cudaSetDevice(h->device);
         tdlb_rt::fence(h);
@@ -98,42 +95,31 @@ int tdlb_double_resolution(tdlb_handle h) {
             throw RFail{TDLB_EINVAL, "doubled lattice too large: one plane must stay below 2^31 elements"};
         const long long words = round_up_ll(n.rows() * n.jw, 64);
         const bool simple = h->cfg.streaming == TDLB_STREAMING_SIMPLE;
-        const size_t pop = (size_t)tdlb::NQ * n.plane * sizeof(float);
+        lb = tdlb_rt::lattice_block(n, words, sizeof(float), simple);
         size_t free_b = 0, total_b = 0;
         TDLB_RCK(cudaMemGetInfo(&free_b, &total_b));
-        const size_t need = pop * (simple ? 2 : 1) + (size_t)5 * n.plane * sizeof(float) + 2 * words * sizeof(uint32_t);
-        if (need > free_b)
-            throw RFail{TDLB_ENOMEM, "doubled lattice needs " + std::to_string(need) + " B, " + std::to_string(free_b) +
+        if (lb.bytes > free_b)
+            throw RFail{TDLB_ENOMEM, "doubled lattice needs " + std::to_string(lb.bytes) + " B, " + std::to_string(free_b) +
                                          " B free"};
-        TDLB_RCK(cudaMalloc(&A, pop));
-        if (simple) TDLB_RCK(cudaMalloc(&B, pop));
-        TDLB_RCK(cudaMalloc(&Nu, (size_t)n.plane * sizeof(float)));
-        TDLB_RCK(cudaMalloc(&F, (size_t)4 * n.plane * sizeof(float)));   // one float4 per element
-        TDLB_RCK(cudaMalloc(&mask, (size_t)2 * words * sizeof(uint32_t)));
-        TDLB_RCK(cudaMemsetAsync(A, 0, pop, h->stream));
-        if (B) TDLB_RCK(cudaMemsetAsync(B, 0, pop, h->stream));
-        TDLB_RCK(cudaMemsetAsync(Nu, 0, (size_t)n.plane * sizeof(float), h->stream));
-        TDLB_RCK(cudaMemsetAsync(F, 0, (size_t)4 * n.plane * sizeof(float), h->stream));
-        TDLB_RCK(cudaMemsetAsync(mask, 0, (size_t)2 * words * sizeof(uint32_t), h->stream));
+        TDLB_RCK(cudaMalloc(&block, lb.bytes));
+        TDLB_RCK(cudaMemsetAsync(block, 0, lb.bytes, h->stream));
         Planes dst;
-        for (int d = 0; d < tdlb::NQ; d++) dst.p[d] = A + (size_t)d * n.plane;
+        for (int d = 0; d < tdlb::NQ; d++) dst.p[d] = (float*)(block + lb.a) + (size_t)d * n.plane;
         const long long cells = n.cells();
         tdlb::k_double_resolution<<<(unsigned)((cells + 255) / 256), 256, 0, h->stream>>>(
-            h->planes(h->state_buf()), g, h->state_mode(), h->even ? 1 : 0, h->cp, h->Nu, dst, n, Nu, simple ? 0 : 1);
+            h->planes(h->state_buf()), g, h->state_mode(), h->even ? 1 : 0, h->cp, h->Nu, dst, n, (float*)(block + lb.nu),
+            simple ? 0 : 1);
         TDLB_RCK(cudaGetLastError());
         TDLB_RCK(cudaStreamSynchronize(h->stream));
     } catch (const RFail& f) {
-        cudaFree(A); cudaFree(B); cudaFree(Nu); cudaFree(F); cudaFree(mask);
+        cudaFree(block);
         h->err = f.msg;
         return f.code;
     }
     // swap in the new lattice; the geometry is regenerated by the caller
-    cudaFree(h->bufA); cudaFree(h->bufB); cudaFree(h->Nu); cudaFree(h->F); cudaFree(h->mask);
-    h->bufA = A;
-    h->bufB = B;
-    h->Nu = Nu;
-    h->F = F;
-    h->mask = mask;
+    cudaFree(h->block);
+    h->block = block;
+    lb.place(h);
     Dims& g = h->g;
     g = tdlb::make_dims(g.nx * 2, g.ny * 2, g.nz * 2);
     h->mask_words = round_up_ll(g.rows() * g.jw, 64);

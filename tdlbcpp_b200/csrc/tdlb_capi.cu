@@ -47,11 +47,7 @@ namespace {
 void release(tdlb_lattice* h) {
     if (!h) return;
     cudaSetDevice(h->device);
-    cudaFree(h->bufA);
-    cudaFree(h->bufB);
-    cudaFree(h->Nu);
-    cudaFree(h->F);
-    cudaFree(h->mask);
+    cudaFree(h->block);
     cudaFree(h->d_markers);
     cudaFree(h->d_markers_in);
     cudaFree(h->d_sched_tmp);
@@ -113,10 +109,11 @@ tdlb_lattice* build(const tdlb_config& c, int device) {
     if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev == 0)
         throw Fail{TDLB_ECUDA, "no CUDA device available (this library has no CPU path)"};
     if (device < 0 || device >= ndev) throw Fail{TDLB_EINVAL, "device index out of range"};
-    cudaDeviceProp prop;
-    TDLB_CK(cudaGetDeviceProperties(&prop, device));
-    if (prop.major < 10) throw Fail{TDLB_ECUDA, "this library is built for sm_100a (B200); device is sm_" +
-                                                     std::to_string(prop.major) + std::to_string(prop.minor)};
+    int major = 0, minor = 0;   // (the whole cudaDeviceProp takes 2 to 10 ms to fill)
+    TDLB_CK(cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, device));
+    TDLB_CK(cudaDeviceGetAttribute(&minor, cudaDevAttrComputeCapabilityMinor, device));
+    if (major < 10) throw Fail{TDLB_ECUDA, "this library is built for sm_100a (B200); device is sm_" +
+                                               std::to_string(major) + std::to_string(minor)};
     auto* h = new tdlb_lattice();
     try {
         h->cfg = c;
@@ -146,23 +143,14 @@ tdlb_lattice* build(const tdlb_config& c, int device) {
         h->cp = tdlb::make_collide_params(c.nu, c.cs0, c.g3);
         tdlb::set_rest(h->cp, c.initialRho);
 
-        const size_t pop_bytes = (size_t)tdlb::NQ * g.plane * h->esz();
+        const tdlb_rt::LatticeBlock lb = tdlb_rt::lattice_block(g, h->mask_words, h->esz(), c.streaming == TDLB_STREAMING_SIMPLE);
         size_t free_b = 0, total_b = 0;
         TDLB_CK(cudaMemGetInfo(&free_b, &total_b));
-        const size_t need = pop_bytes * (c.streaming == TDLB_STREAMING_SIMPLE ? 2 : 1) +
-                            (size_t)5 * g.plane * sizeof(float) + 2 * h->mask_words * sizeof(uint32_t);   // F (float4), Nu
-        if (need > free_b) throw Fail{TDLB_ENOMEM, "lattice needs " + std::to_string(need) + " B, " +
-                                                       std::to_string(free_b) + " B free on device"};
-        TDLB_CK(cudaMalloc(&h->bufA, pop_bytes));
-        if (c.streaming == TDLB_STREAMING_SIMPLE) TDLB_CK(cudaMalloc(&h->bufB, pop_bytes));
-        TDLB_CK(cudaMalloc(&h->Nu, (size_t)g.plane * sizeof(float)));
-        TDLB_CK(cudaMalloc(&h->F, (size_t)4 * g.plane * sizeof(float)));
-        TDLB_CK(cudaMalloc(&h->mask, (size_t)2 * h->mask_words * sizeof(uint32_t)));
-        TDLB_CK(cudaMemsetAsync(h->bufA, 0, pop_bytes, h->stream));
-        if (h->bufB) TDLB_CK(cudaMemsetAsync(h->bufB, 0, pop_bytes, h->stream));
-        TDLB_CK(cudaMemsetAsync(h->Nu, 0, (size_t)g.plane * sizeof(float), h->stream));
-        TDLB_CK(cudaMemsetAsync(h->F, 0, (size_t)4 * g.plane * sizeof(float), h->stream));
-        TDLB_CK(cudaMemsetAsync(h->mask, 0, (size_t)2 * h->mask_words * sizeof(uint32_t), h->stream));
+        if (lb.bytes > free_b) throw Fail{TDLB_ENOMEM, "lattice needs " + std::to_string(lb.bytes) + " B, " +
+                                                           std::to_string(free_b) + " B free on device"};
+        TDLB_CK(cudaMalloc(&h->block, lb.bytes));
+        lb.place(h);
+        TDLB_CK(cudaMemsetAsync(h->block, 0, lb.bytes, h->stream));
         TDLB_CK(cudaStreamSynchronize(h->stream));
     } catch (...) {
         release(h);

@@ -21,6 +21,7 @@ struct tdlb_lattice {
     cudaStream_t own_stream = nullptr;   // set when `stream` is borrowed from a batch
     tdlb::CollideParams cp{};
 
+    char* block = nullptr;       // one allocation: the five arrays below (tdlb_rt::LatticeBlock)
     float* bufA = nullptr;       // 18 planes
     float* bufB = nullptr;       // 18 planes (Simple only)
     float* Nu = nullptr;
@@ -193,6 +194,31 @@ namespace tdlb_rt {
 inline int default_cells_per_thread(const tdlb_config& c) {
     if (c.storage == TDLB_STORAGE_FP32) return 1;
     return c.streaming == TDLB_STREAMING_SIMPLE ? 4 : 2;
+}
+// The lattice's arrays in one device allocation, each on a 256-byte boundary:
+// an allocation above a megabyte takes about 0.7 ms and its free as long, four or
+// five times over for every tank that a server builds.
+struct LatticeBlock {
+    size_t a, b, nu, f, mask, bytes;   // offsets; b == a without a second buffer
+    void place(tdlb_lattice* h, char* base) const {
+        h->bufA = (float*)(base + a);
+        h->bufB = b == a ? nullptr : (float*)(base + b);
+        h->Nu = (float*)(base + nu);
+        h->F = (float*)(base + f);
+        h->mask = (uint32_t*)(base + mask);
+    }
+    void place(tdlb_lattice* h) const { place(h, h->block); }
+};
+inline LatticeBlock lattice_block(const Dims& g, long long mask_words, size_t esz, bool simple) {
+    auto up = [](size_t n) { return (n + 255) / 256 * 256; };
+    const size_t pop = up((size_t)tdlb::NQ * g.plane * esz), plane = up((size_t)g.plane * sizeof(float));
+    LatticeBlock l{};
+    l.b = simple ? pop : 0;
+    l.nu = l.b + pop;
+    l.f = l.nu + plane;
+    l.mask = l.f + 4 * plane;          // F: one float4 per element
+    l.bytes = l.mask + up((size_t)2 * mask_words * sizeof(uint32_t));
+    return l;
 }
 tdlb::StepArgs step_args(tdlb_lattice* h, bool collide);
 tdlb::IbmArgs ibm_args(tdlb_lattice* h, float alpha, float beta);
