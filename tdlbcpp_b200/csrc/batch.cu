@@ -7,8 +7,8 @@
 //                       read from a per-step (cos, sin, delta) table indexed
 //                       by a device step counter;
 //   2. k_batch_step     the group's fused collision + streaming: work items
-//                       of eight chunks of 128 or 256 quads of one tank, with
-//                       that tank's step view staged in shared memory once
+//                       of up to eight chunks of 128 or 256 quads of one tank,
+//                       with that tank's step view staged in shared memory once
 //                       per item; one block per item or a persistent grid of
 //                       a few blocks per SM looping over the items (block 0
 //                       also advances the step counter);
@@ -76,9 +76,13 @@ __device__ __forceinline__ void tank_quad(const TankStep& ts, unsigned t) {
     }
 }
 
-// Quads of `NT` threads a work item covers: the tank's view is staged in
-// shared memory once per item.
+// Most chunks of NT quads a work item covers: the tank's view is staged in
+// shared memory once per item. A batch with fewer chunks than fill the SMs that
+// often takes smaller items (chunks_of): six tanks of edge 24 to 56 ran 25 us a
+// step in items of eight, 100 blocks on 148 SMs one chunk after another.
 constexpr int kBatchChunks = 8;
+// Work items per SM a launch should have before its items grow.
+constexpr int kItemsPerSM = 8;
 // How far ahead of the chunk a block starts it prefetches into L2: about this
 // many cells, at least one chunk (a chunk is NT x V cells). Measured on B200:
 // the 64-tank Esotwist batch at its autotuned shapes (FP32 256-cell chunks,
@@ -114,7 +118,7 @@ __device__ __forceinline__ void prefetch_chunk(const TankStep& ts, unsigned q0) 
 }
 
 // Batched step: block b takes work items b, b + grid, ...; an item is
-// kBatchChunks x NT consecutive quads of one tank (fewer at the end of a
+// `chunks` x NT consecutive quads of one tank (fewer at the end of a
 // tank), whose step view is staged in shared memory; as it starts chunk c of
 // an item, the block prefetches chunk c + ahead into L2 (ahead > 0). 16-bit storage
 // never holds moments, so its from-moments bodies are not built. `counter` (may be
@@ -122,7 +126,7 @@ __device__ __forceinline__ void prefetch_chunk(const TankStep& ts, unsigned q0) 
 // reads it.
 template <typename S, int V, int NT, bool ESO>
 __global__ void __launch_bounds__(NT, (ESO ? kEsotwistBlocksPerSM<S, V> : 4) * 128 / NT) k_batch_step(const TankStep* __restrict__ tanks, const int2* __restrict__ work,
-                                                   int nwork, int* counter, int ahead) {
+                                                   int nwork, int* counter, int ahead, int chunks) {
     constexpr bool kFM = sizeof(S) == 4;
     __shared__ TankStep ts;
     if (counter && blockIdx.x == 0 && threadIdx.x == 0) *counter += 1;
@@ -132,10 +136,10 @@ __global__ void __launch_bounds__(NT, (ESO ? kEsotwistBlocksPerSM<S, V> : 4) * 1
         stage<NT>(ts, tanks + wk.x);
         __syncthreads();
         const unsigned nquads = (unsigned)ts.g.nx * (unsigned)ts.g.nz * (unsigned)(ts.g.jp / V);
-        for (int c = 0; c < kBatchChunks; c++) {
+        for (int c = 0; c < chunks; c++) {
             const unsigned t0 = (unsigned)wk.y + (unsigned)(c * NT);
             if (t0 >= nquads) break;   // uniform over the block
-            if (ahead > 0 && c + ahead < kBatchChunks) prefetch_chunk<S, V, NT, ESO>(ts, t0 + (unsigned)(ahead * NT));
+            if (ahead > 0 && c + ahead < chunks) prefetch_chunk<S, V, NT, ESO>(ts, t0 + (unsigned)(ahead * NT));
             const unsigned t = t0 + threadIdx.x;
             if (ts.les) {
                 if (kFM && ts.from_moments) tank_quad<S, V, ESO, true, kFM>(ts, t);
@@ -167,7 +171,7 @@ __global__ void __launch_bounds__(256) k_rotate_batch(const TankRotor* __restric
     o.wDelta = m.wDelta;
 }
 
-using BatchFn = void (*)(const TankStep*, const int2*, int, int*, int);
+using BatchFn = void (*)(const TankStep*, const int2*, int, int*, int, int);
 
 template <typename S, bool ESO>
 BatchFn pick(int v, int nt) {
@@ -195,6 +199,7 @@ namespace {
 struct WorkList {
     int2* d = nullptr;
     int n = 0, cap = 0;
+    int chunks = 1;   // fused-step items: chunks per item
 };
 
 }  // namespace
@@ -341,20 +346,26 @@ cudaError_t quiesce(tdlb_batch_s* b) {
 // for every tank and per group.
 void build_work(tdlb_batch_s* b) {
     const int vec = width_of(b);
-    auto items = [&](const std::vector<int>& ts) {
+    auto fill = [&](WorkList& list, const std::vector<int>& ts) {
         std::vector<int2> w;
-        for (int t : ts) {
+        long long total = 0;   // chunks
+        auto quads = [&](int t) {
             const Dims& g = b->tanks[(size_t)t]->g;
-            const long long nq = g.rows() * (g.jp / vec);
-            for (long long q = 0; q < nq; q += (long long)b->threads * tdlb::kBatchChunks) w.push_back(make_int2(t, (int)q));
-        }
-        return w;
+            return g.rows() * (g.jp / vec);
+        };
+        for (int t : ts) total += (quads(t) + b->threads - 1) / b->threads;
+        const int chunks = (int)std::min<long long>(tdlb::kBatchChunks,
+                                                    std::max(1LL, total / ((long long)std::max(b->sms, 1) * tdlb::kItemsPerSM)));
+        for (int t : ts)
+            for (long long q = 0; q < quads(t); q += (long long)b->threads * chunks) w.push_back(make_int2(t, (int)q));
+        put(list, w);
+        list.chunks = chunks;
     };
     std::vector<int> all(b->tanks.size());
     for (size_t t = 0; t < all.size(); t++) all[t] = (int)t;
     TDLB_BCK(quiesce(b));   // queued launches may still read the old lists
-    put(b->work, items(all));
-    for (BatchGroup& G : b->grp) put(G.work, items(G.tanks));
+    fill(b->work, all);
+    for (BatchGroup& G : b->grp) fill(G.work, G.tanks);
 }
 
 // Immersed-boundary work lists per group; rebuilt when a tank's markers changed.
@@ -432,7 +443,7 @@ void launch_fused(tdlb_batch_s* b, const TankStep* d_views, const WorkList& work
     const tdlb::BatchFn fn = tdlb::batch_kernel(storage_of(b), eso_of(b), vec, b->threads);
     const int grid = b->bps > 0 ? std::min(work.n, b->sms * b->bps) : work.n;
     const int ahead = std::max(1, tdlb::kBatchPrefetchCells / (b->threads * vec));
-    fn<<<grid, b->threads, 0, st>>>(d_views, work.d, work.n, counter, ahead);
+    fn<<<grid, b->threads, 0, st>>>(d_views, work.d, work.n, counter, ahead, work.chunks);
     TDLB_BCK(cudaGetLastError());
 }
 
@@ -709,6 +720,7 @@ std::vector<uintptr_t> graph_key(const tdlb_batch_s* b, int P) {
         for (const WorkList* w : {&G.work, &G.rot_work, &G.gather, &G.small, &G.big}) {
             k.push_back((uintptr_t)w->d);
             k.push_back((uintptr_t)w->n);
+            k.push_back((uintptr_t)w->chunks);
         }
         k.push_back((uintptr_t)G.small_tile);
         k.push_back((uintptr_t)G.big_tile);

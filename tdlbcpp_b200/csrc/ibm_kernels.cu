@@ -888,6 +888,27 @@ __global__ void k_rotate_markers(const double* __restrict__ xz, Marker* __restri
     m.wDelta = r.wDelta;
 }
 
+__global__ void __launch_bounds__(256) k_place_blades(const int* __restrict__ stage, int* __restrict__ markers, int mwords,
+                                                      int* __restrict__ order, int n, int* __restrict__ level_ptr, int nlev,
+                                                      int* __restrict__ plane_lv, int nplane) {
+    int t = (int)(blockIdx.x * blockDim.x + threadIdx.x);
+    const int total = mwords + n + nlev + nplane;
+    if (t >= total) return;
+    const int v = stage[t];
+    if (t < mwords) markers[t] = v;
+    else if ((t -= mwords) < n) order[t] = v;
+    else if ((t -= n) < nlev) level_ptr[t] = v;
+    else plane_lv[t - nlev] = v;
+}
+
+cudaError_t launch_place_blades(const int* stage, Marker* markers, int n, int* order, int* level_ptr, int nlev, int* plane_lv,
+                                int nplane, cudaStream_t st) {
+    const int mwords = (int)(sizeof(Marker) / sizeof(int)) * n;
+    k_place_blades<<<(mwords + n + nlev + nplane + 255) / 256, 256, 0, st>>>(stage, reinterpret_cast<int*>(markers), mwords, order,
+                                                                             n, level_ptr, nlev, plane_lv, nplane);
+    return cudaGetLastError();
+}
+
 cudaError_t launch_rotate_markers(const double* xz, Marker* out, int n, double ca, double sa, double omega, double ci,
                                   double ck, int nx, int nz, cudaStream_t st) {
     if (n <= 0) return cudaSuccess;

@@ -8,7 +8,8 @@
 // 75,000 markers: about 90 ms a call); here every plane is a block's and the
 // list is read twice.
 //
-//   k_sched_count    (a warp per 1024 markers) range check, markers per plane
+//   k_sched_count    (a warp per 256 or 1024 markers) range check, markers per
+//                    plane
 //   k_sched_offsets  per plane: running offsets over the chunks
 //   k_sched_scan     plane offsets
 //   k_sched_scatter  list indices by plane, in list order
@@ -30,9 +31,10 @@
 
 namespace tdlb {
 
-constexpr int kChunk = 1024;       // markers of one warp, in list order
+constexpr int kSteps = 8;           // steps of 32 markers whose loads leave together
 constexpr int kMaxRounds = 4096;
 constexpr unsigned kAll = 0xffffffffu;
+constexpr int kHeld = 3;           // markers of a plane a thread keeps in registers
 
 __device__ __forceinline__ int marker_plane(const SchedArgs& a, int q) {
     const Marker& m = a.markers[q];
@@ -40,19 +42,30 @@ __device__ __forceinline__ int marker_plane(const SchedArgs& a, int q) {
     return in ? (int)m.j : -1;
 }
 
-__global__ void __launch_bounds__(128) k_sched_count(SchedArgs a, int nchunk) {
+// Markers of one warp, in list order: few, so that a short list is many warps
+// (12,900 markers in warps of 1024 took 24 us a pass), more where the offsets of
+// the chunks would be the longer pass.
+static int chunk_of(long long n) { return n <= (1 << 17) ? 32 * kSteps : 128 * kSteps; }
+
+__global__ void __launch_bounds__(128) k_sched_count(SchedArgs a, int nchunk, int per) {
     const int chunk = (int)(blockIdx.x * 4 + threadIdx.x / 32), lane = threadIdx.x & 31;
     if (chunk >= nchunk) return;
-    for (int s = 0; s < kChunk; s += 32) {
-        const long long q = (long long)chunk * kChunk + s + lane;
-        int j = -1;
-        if (q < a.n) {
-            j = marker_plane(a, (int)q);
-            if (j < 0) atomicMin(a.info, (int)q);
-            if (q >= a.n0) j = -1;
+    for (int s = 0; s < per; s += 32 * kSteps) {
+        const long long q0 = (long long)chunk * per + s + lane;
+        int j[kSteps];
+#pragma unroll
+        for (int u = 0; u < kSteps; u++) {
+            const long long q = q0 + 32 * u;
+            j[u] = q < a.n ? marker_plane(a, (int)q) : -2;
         }
-        const unsigned same = __match_any_sync(kAll, j);
-        if (j >= 0 && lane == __ffs(same) - 1) atomicAdd(a.hist + (long long)chunk * a.g.ny + j, __popc(same));
+#pragma unroll
+        for (int u = 0; u < kSteps; u++) {
+            const long long q = q0 + 32 * u;
+            if (j[u] == -1) atomicMin(a.info, (int)q);
+            const int jj = q < a.n0 ? j[u] : -1;
+            const unsigned same = __match_any_sync(kAll, jj);
+            if (jj >= 0 && lane == __ffs(same) - 1) atomicAdd(a.hist + (long long)chunk * a.g.ny + jj, __popc(same));
+        }
     }
 }
 
@@ -110,18 +123,28 @@ __device__ __forceinline__ int block_scan(int* v, int n) {
 
 __global__ void __launch_bounds__(1024) k_sched_scan(SchedArgs a) { block_scan(a.plane_slot, a.g.ny); }
 
-__global__ void __launch_bounds__(128) k_sched_scatter(SchedArgs a, int nchunk) {
+__global__ void __launch_bounds__(128) k_sched_scatter(SchedArgs a, int nchunk, int per) {
     const int chunk = (int)(blockIdx.x * 4 + threadIdx.x / 32), lane = threadIdx.x & 31;
     if (chunk >= nchunk) return;
-    for (int s = 0; s < kChunk; s += 32) {
-        const long long q = (long long)chunk * kChunk + s + lane;
-        const int j = q < a.n0 ? marker_plane(a, (int)q) : -1;
-        const unsigned same = __match_any_sync(kAll, j);
-        const int leader = __ffs(same) - 1;
-        int base = 0;
-        if (j >= 0 && lane == leader) base = a.plane_slot[j] + atomicAdd(a.hist + (long long)chunk * a.g.ny + j, __popc(same));
-        base = __shfl_sync(kAll, base, leader);
-        if (j >= 0) a.by_plane[base + __popc(same & ((1u << lane) - 1u))] = (int)q;
+    for (int s = 0; s < per; s += 32 * kSteps) {
+        const long long q0 = (long long)chunk * per + s + lane;
+        int j[kSteps], first[kSteps];
+#pragma unroll
+        for (int u = 0; u < kSteps; u++) {
+            const long long q = q0 + 32 * u;
+            j[u] = q < a.n0 ? marker_plane(a, (int)q) : -1;
+        }
+#pragma unroll
+        for (int u = 0; u < kSteps; u++) first[u] = j[u] >= 0 ? a.plane_slot[j[u]] : 0;
+#pragma unroll
+        for (int u = 0; u < kSteps; u++) {
+            const unsigned same = __match_any_sync(kAll, j[u]);
+            const int leader = __ffs(same) - 1;
+            int base = 0;
+            if (j[u] >= 0 && lane == leader) base = atomicAdd(a.hist + (long long)chunk * a.g.ny + j[u], __popc(same));
+            base = __shfl_sync(kAll, base, leader);
+            if (j[u] >= 0) a.by_plane[first[u] + base + __popc(same & ((1u << lane) - 1u))] = (int)(q0 + 32 * u);
+        }
     }
 }
 
@@ -177,7 +200,7 @@ __global__ void __launch_bounds__(256) k_sched_cells(SchedArgs a) {
 template <int NT>
 __global__ void __launch_bounds__(NT) k_sched_levels(SchedArgs a, int owner_cap) {
     extern __shared__ unsigned smap[];
-    __shared__ int warps[NT / 32];
+    __shared__ int warps[NT / 32], counts[kHeld][NT / 32];
     __shared__ int placed;
     const int j = (int)blockIdx.x, W = map_words(a.g), lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int p0 = a.plane_slot[j], m = a.plane_slot[j + 1] - p0, c0 = a.plane_cell[j], nc = a.plane_cell[j + 1] - c0;
@@ -228,6 +251,67 @@ __global__ void __launch_bounds__(NT) k_sched_levels(SchedArgs a, int owner_cap)
     }
     __syncthreads();
     int level = 0;
+    if (m <= kHeld * NT) {
+        // every thread holds its markers' places (kHeld sets of nine)
+        int pl[kHeld][9], q[kHeld];
+        bool left[kHeld];
+#pragma unroll
+        for (int u = 0; u < kHeld; u++) {
+            const int p = u * NT + (int)threadIdx.x;
+            left[u] = p < m;
+            q[u] = left[u] ? a.by_plane[p0 + p] : 0;
+#pragma unroll
+            for (int c = 0; c < 9; c++) pl[u][c] = left[u] ? place[9 * p + c] : 0;
+        }
+        int done = 0;
+        for (; level < kMaxRounds; level++) {
+#pragma unroll
+            for (int u = 0; u < kHeld; u++)
+                if (left[u])
+#pragma unroll
+                    for (int c = 0; c < 9; c++) atomicMin(owner + pl[u][c], u * NT + (int)threadIdx.x);
+            __syncthreads();
+            unsigned vote[kHeld];
+            bool ready[kHeld];
+#pragma unroll
+            for (int u = 0; u < kHeld; u++) {
+                ready[u] = left[u];
+                if (left[u])
+#pragma unroll
+                    for (int c = 0; c < 9; c++) ready[u] = ready[u] && *(volatile int*)(owner + pl[u][c]) == u * NT + (int)threadIdx.x;
+                vote[u] = __ballot_sync(kAll, ready[u]);
+                if (lane == 0) counts[u][warp] = __popc(vote[u]);
+            }
+            __syncthreads();
+#pragma unroll
+            for (int u = 0; u < kHeld; u++) {
+                // the counts of the warps before this one, and of all
+                int x = lane < NT / 32 ? counts[u][lane] : 0;
+                const int before = __reduce_add_sync(kAll, lane < warp ? x : 0), all = __reduce_add_sync(kAll, x);
+                if (ready[u]) {
+                    const int slot = p0 + done + before + __popc(vote[u] & ((1u << lane) - 1u));
+                    a.sched[slot] = q[u];
+                    float* prep = a.prep + (size_t)slot * PF_STRIDE + PF_CELL;
+#pragma unroll
+                    for (int c = 0; c < 9; c++) {
+                        prep[c] = __int_as_float(pl[u][c]);
+                        owner[pl[u][c]] = 0x7fffffff;   // (this round's cells of one marker are no other's)
+                    }
+                    left[u] = false;
+                }
+                done += all;
+            }
+            if (threadIdx.x == 0) a.level_end[p0 + level] = p0 + done;
+            // (cells of no placed marker hold the lowest of those that wait, and keep it)
+            __syncthreads();
+            if (done == m) break;
+        }
+        if (threadIdx.x == 0) {
+            a.levels[j] = level + 1;
+            if (level == kMaxRounds) atomicExch(a.info + 1, 1);
+        }
+        return;
+    }
     for (; level < kMaxRounds; level++) {
         for (int p = threadIdx.x; p < m; p += NT) {
             if (place[9 * p] < 0) continue;
@@ -306,18 +390,18 @@ __global__ void __launch_bounds__(256) k_static_flags(Dims g, const int* __restr
 // ---------------------------------------------------------------------------
 constexpr size_t kMapSmem = 160 * 1024;   // shared memory the two maps may take
 
-size_t sched_hist_ints(const Dims& g, long long n) { return (size_t)((n + kChunk - 1) / kChunk) * (size_t)g.ny; }
+size_t sched_hist_ints(const Dims& g, long long n) { return (size_t)((n + chunk_of(n) - 1) / chunk_of(n)) * (size_t)g.ny; }
 size_t sched_map_words(const Dims& g) {
     const size_t W = (size_t)((g.rows() + 31) / 32);
     return W * 8 <= kMapSmem ? 0 : 2 * W * (size_t)g.ny;
 }
 
 cudaError_t launch_sched_cells(const SchedArgs& a, cudaStream_t st) {
-    const int nchunk = (int)((a.n + (long long)kChunk - 1) / kChunk);
-    if (nchunk > 0) k_sched_count<<<(nchunk + 3) / 4, 128, 0, st>>>(a, nchunk);
+    const int per = chunk_of(a.n), nchunk = (int)((a.n + (long long)per - 1) / per);
+    if (nchunk > 0) k_sched_count<<<(nchunk + 3) / 4, 128, 0, st>>>(a, nchunk, per);
     k_sched_offsets<<<(a.g.ny + 127) / 128, 128, 0, st>>>(a, nchunk);
     k_sched_scan<<<1, 1024, 0, st>>>(a);
-    if (nchunk > 0) k_sched_scatter<<<(nchunk + 3) / 4, 128, 0, st>>>(a, nchunk);
+    if (nchunk > 0) k_sched_scatter<<<(nchunk + 3) / 4, 128, 0, st>>>(a, nchunk, per);
     const size_t smem = a.maps ? 0 : (size_t)((a.g.rows() + 31) / 32) * 4;
     cudaError_t e = raise_smem_limit((const void*)k_sched_cells, smem);
     if (e != cudaSuccess) return e;

@@ -81,6 +81,7 @@ void release(tdlb_lattice* h) {
     cudaFree(h->d_rot_xz);
     cudaFree(h->d_load);
     cudaFree(h->d_imp_slots);
+    cudaFree(h->d_blade_stage);
     cudaFree(h->d_res[0]);
     cudaFree(h->d_res[1]);
     for (auto& st : h->pin) {
@@ -1318,13 +1319,21 @@ int tdlb_set_rotating_markers(tdlb_handle h, const tdlb_marker* markers, size_t 
         std::memcpy(q + b_mk, h->seg1.order.data(), b_order);
         std::memcpy(q + b_mk + b_order, h->seg1.level_ptr.data(), b_lv);
         std::memcpy(q + b_mk + b_order + b_lv, h->seg1.plane_lv.data(), b_pl);
-        if (n) {
-            TDLB_CK(cudaMemcpyAsync(h->d_markers + h->n0, q, b_mk, cudaMemcpyHostToDevice, h->stream));
-            TDLB_CK(cudaMemcpyAsync(h->d_sched + h->n0, q + b_mk, b_order, cudaMemcpyHostToDevice, h->stream));
+        // one copy and a launch that puts the four parts in their places (four
+        // copies of a few KB are four trips)
+        if (need > h->blade_stage_cap) {
+            TDLB_CK(cudaStreamSynchronize(h->stream));
+            cudaFree(h->d_blade_stage);
+            h->d_blade_stage = nullptr;
+            h->blade_stage_cap = 0;
+            TDLB_CK(cudaMalloc(&h->d_blade_stage, need + need / 2));
+            h->blade_stage_cap = need + need / 2;
         }
-        TDLB_CK(cudaMemcpyAsync(h->d_level_ptr + L0, q + b_mk + b_order, b_lv, cudaMemcpyHostToDevice, h->stream));
-        TDLB_CK(cudaMemcpyAsync(h->d_plane_lv1, q + b_mk + b_order + b_lv, b_pl, cudaMemcpyHostToDevice, h->stream));
+        TDLB_CK(cudaMemcpyAsync(h->d_blade_stage, q, need, cudaMemcpyHostToDevice, h->stream));
         TDLB_CK(cudaEventRecord(st.ev, h->stream));
+        TDLB_CK(tdlb::launch_place_blades((const int*)h->d_blade_stage, h->d_markers + h->n0, (int)n, h->d_sched + h->n0,
+                                          h->d_level_ptr + L0, (int)h->seg1.level_ptr.size(), h->d_plane_lv1, h->g.ny + 1,
+                                          h->stream));
         h->rot_device = false;   // the blades now follow the host's list
         // a split step needs every blade stencil cell inside the zone
         if (h->zone_gen == h->marker_gen && !h->zone_all) h->zone_ok = blades_in_zone(h);
@@ -1378,9 +1387,17 @@ void queue_impeller_load(tdlb_lattice* h, double* out5) {
     find_impeller_slots(h);
     tdlb::IbmArgs a = ibm_args(h, 0.f, h->last_beta);
     double* out = h->d_load + tdlb::kLoadBlocks * 5;
-    TDLB_CK(tdlb::launch_marker_load(a, h->d_imp_slots, h->n_imp, h->rot_ci, h->rot_ck, h->d_load, (unsigned*)(out + 5), out,
-                                     h->stream));
-    TDLB_CK(cudaMemcpyAsync(out5, out, 5 * sizeof(double), cudaMemcpyDefault, h->stream));
+    // memory the device can write (its own, pinned host, managed) takes the sums
+    // from the kernel; a copy behind it costs 6 us of a small tank's step
+    double* direct = nullptr;
+    cudaPointerAttributes at{};
+    if (cudaPointerGetAttributes(&at, out5) != cudaSuccess) cudaGetLastError();
+    else if (at.type == cudaMemoryTypeHost || ((at.type == cudaMemoryTypeDevice || at.type == cudaMemoryTypeManaged) &&
+                                               at.device == h->device))
+        direct = (double*)at.devicePointer;
+    TDLB_CK(tdlb::launch_marker_load(a, h->d_imp_slots, h->n_imp, h->rot_ci, h->rot_ck, h->d_load, (unsigned*)(out + 5),
+                                     direct ? direct : out, h->stream));
+    if (!direct) TDLB_CK(cudaMemcpyAsync(out5, out, 5 * sizeof(double), cudaMemcpyDefault, h->stream));
 }
 
 int tdlb_impeller_load(tdlb_handle h, double* out5) {

@@ -106,6 +106,8 @@ struct tdlb_lattice {
         cudaEvent_t ev = nullptr;
     } pin[2];
     int pin_cur = 0;
+    char* d_blade_stage = nullptr;   // the upload on the device, before its parts are placed
+    size_t blade_stage_cap = 0;
     std::vector<double> h_rot_xz; // host copy of d_rot_xz
 
     // Split steps: the outer words of a step run on `bulk`, beside the previous

@@ -250,6 +250,10 @@ cudaError_t launch_reduce_fp64(const IbmArgs& a, const uint32_t* mask, double* p
 // Rest state at density rho for the 16-bit storage.
 cudaError_t launch_fill_rest(Planes Q, long long plane, float rho, float rho0, int storage, const CollideParams& p,
                              cudaStream_t st);
+// The parts of a blade upload from `stage`, one after another: n markers, their
+// order, nlev level offsets, nplane plane levels.
+cudaError_t launch_place_blades(const int* stage, Marker* markers, int n, int* order, int* level_ptr, int nlev, int* plane_lv,
+                                int nplane, cudaStream_t st);
 // Recompute n rotating markers (offsets xz[2n]) for cos/sin (ca, sa).
 cudaError_t launch_rotate_markers(const double* xz, Marker* out, int n, double ca, double sa, double omega, double ci,
                                   double ck, int nx, int nz, cudaStream_t st);
