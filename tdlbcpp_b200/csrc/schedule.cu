@@ -69,18 +69,25 @@ __global__ void __launch_bounds__(128) k_sched_count(SchedArgs a, int nchunk, in
     }
 }
 
+// a warp per plane
 __global__ void __launch_bounds__(128) k_sched_offsets(SchedArgs a, int nchunk) {
-    const int j = (int)(blockIdx.x * blockDim.x + threadIdx.x);
+    const int j = (int)(blockIdx.x * 4 + threadIdx.x / 32), lane = threadIdx.x & 31;
     if (j >= a.g.ny) return;
     int sum = 0;
-#pragma unroll 8
-    for (int c = 0; c < nchunk; c++) {
-        int* h = a.hist + (long long)c * a.g.ny + j;
-        const int v = *h;
-        *h = sum;
-        sum += v;
+#pragma unroll 4
+    for (int c0 = 0; c0 < nchunk; c0 += 32) {
+        int* h = a.hist + (long long)(c0 + lane) * a.g.ny + j;
+        const int v = c0 + lane < nchunk ? *h : 0;
+        int s = v;
+#pragma unroll
+        for (int d = 1; d < 32; d *= 2) {
+            const int y = __shfl_up_sync(kAll, s, d);
+            if (lane >= d) s += y;
+        }
+        if (c0 + lane < nchunk) *h = sum + s - v;
+        sum += __shfl_sync(kAll, s, 31);
     }
-    a.plane_slot[j] = sum;
+    if (lane == 0) a.plane_slot[j] = sum;
 }
 
 // Exclusive scan of v[0, n) in place by one block of 1024 threads; v[n] = total.
@@ -399,7 +406,7 @@ size_t sched_map_words(const Dims& g) {
 cudaError_t launch_sched_cells(const SchedArgs& a, cudaStream_t st) {
     const int per = chunk_of(a.n), nchunk = (int)((a.n + (long long)per - 1) / per);
     if (nchunk > 0) k_sched_count<<<(nchunk + 3) / 4, 128, 0, st>>>(a, nchunk, per);
-    k_sched_offsets<<<(a.g.ny + 127) / 128, 128, 0, st>>>(a, nchunk);
+    k_sched_offsets<<<(a.g.ny + 3) / 4, 128, 0, st>>>(a, nchunk);
     k_sched_scan<<<1, 1024, 0, st>>>(a);
     if (nchunk > 0) k_sched_scatter<<<(nchunk + 3) / 4, 128, 0, st>>>(a, nchunk, per);
     const size_t smem = a.maps ? 0 : (size_t)((a.g.rows() + 31) / 32) * 4;

@@ -281,19 +281,27 @@ __device__ __forceinline__ void collide_quad(float (&f)[NQ][V], const Quad& q, f
 // added on reading and kept on writing. The other launches of the step leave
 // those cells out (StepPart::except): a cell's locations are its own alone,
 // so the launches do not meet. f holds the cell's 18 values in direction
-// order.
+// order. The 18 residual loads leave together (a location outside the box reads
+// the first residual instead): behind a branch each, they came one trip to the
+// L2 after the other.
 // ---------------------------------------------------------------------------
 // Simple: add the residuals of the source locations inside the box (x - c_d,
 // or the cell itself where x - c_d is off the lattice).
 __device__ __forceinline__ void box_pull_simple(const ResidualBox& rr, int i, int j, int k, const Dims& g,
                                                 float (&f)[NQ][1]) {
+    float v[NQ];
+    bool on[NQ];
 #pragma unroll
     for (int d = 0; d < NQ; d++) {
         const int si = i - cx_of(d), sj = j - cy_of(d), sk = k - cz_of(d);
         const bool in = (unsigned)si < (unsigned)g.nx && (unsigned)sj < (unsigned)g.ny && (unsigned)sk < (unsigned)g.nz;
         const int li = in ? si : i, lj = in ? sj : j, lk = in ? sk : k;
-        if (rr.contains(li, lj, lk)) f[d][0] += *rr.at(d, li, lj, lk);
+        on[d] = rr.contains(li, lj, lk);
+        v[d] = *(on[d] ? rr.at(d, li, lj, lk) : rr.res);
     }
+#pragma unroll
+    for (int d = 0; d < NQ; d++)
+        if (on[d]) f[d][0] += v[d];
 }
 // Esotwist: slot s of cell (i, j, k) lives at (li, lj, lk); on reading, it
 // holds direction EVEN ? s : s ^ 1, on writing EVEN ? s ^ 1 : s.
@@ -308,12 +316,18 @@ __device__ __forceinline__ void eso_location(int s, int i, int j, int k, int i1,
 template <bool EVEN>
 __device__ __forceinline__ void box_read_eso(const ResidualBox& rb, int i, int j, int k, int i1, int j1, int k1,
                                              float (&f)[NQ][1]) {
+    float v[NQ];
+    bool on[NQ];
 #pragma unroll
     for (int s = 0; s < NQ; s++) {
         int li, lj, lk;
         eso_location<EVEN>(s, i, j, k, i1, j1, k1, li, lj, lk);
-        if (rb.contains(li, lj, lk)) f[EVEN ? s : (s ^ 1)][0] += *rb.at(s, li, lj, lk);
+        on[s] = rb.contains(li, lj, lk);
+        v[s] = *(on[s] ? rb.at(s, li, lj, lk) : rb.res);
     }
+#pragma unroll
+    for (int s = 0; s < NQ; s++)
+        if (on[s]) f[EVEN ? s : (s ^ 1)][0] += v[s];
 }
 // ---------------------------------------------------------------------------
 // Simple (A/B, pull).
