@@ -7,11 +7,11 @@
 //                       read from a per-step (cos, sin, delta) table indexed
 //                       by a device step counter;
 //   2. k_batch_step     the group's fused collision + streaming: work items
-//                       of up to eight chunks of 128 or 256 quads of one tank,
-//                       with that tank's step view staged in shared memory once
-//                       per item; one block per item or a persistent grid of
-//                       a few blocks per SM looping over the items (block 0
-//                       also advances the step counter);
+//                       of 128 or 256 quads of one tank, with that tank's
+//                       view staged in shared memory; one block per item or
+//                       a persistent grid of a few blocks per SM looping
+//                       over the items (block 0 also advances the step
+//                       counter);
 //   3-5. the immersed-boundary passes of the group's tanks
 //                       (launch_ibm_batch) on a high-priority stream: the
 //                       gather (stencil cells, blades, touched flags), the
@@ -76,35 +76,21 @@ __device__ __forceinline__ void tank_quad(const TankStep& ts, unsigned t) {
     }
 }
 
-// Most chunks of NT quads a work item covers: the tank's view is staged in
-// shared memory once per item. A batch with fewer chunks than fill the SMs that
-// often takes smaller items (chunks_of): six tanks of edge 24 to 56 ran 25 us a
-// step in items of eight, 100 blocks on 148 SMs one chunk after another.
-constexpr int kBatchChunks = 8;
-// Work items per SM a launch should have before its items grow.
-constexpr int kItemsPerSM = 8;
-// How far ahead of the chunk a block starts it prefetches into L2: about this
-// many cells, at least one chunk (a chunk is NT x V cells). Measured on B200:
-// the 64-tank Esotwist batch at its autotuned shapes (FP32 256-cell chunks,
-// FP16 1024-cell chunks; fused launch, ms): FP32 1.381 without, 1.267 one
-// chunk ahead, 1.318 two; FP16 1.027, 1.011, 1.016. The server's batches at
-// the default shape (128-cell chunks), the first 64 requests of the serving
-// stream: 20,623 MLUPS without, 20,373 one chunk ahead, 21,243 two. (A
-// prefetch one wave of resident blocks ahead, as in the plain kernels, spans
-// 8-chunk items and overran L2: 1.52 ms.)
-constexpr int kBatchPrefetchCells = 256;
-
-// L2 prefetch of the chunk of NT quads from quad q0 of the staged tank: NQ + 1
-// threads issue one bulk prefetch each (plane d's source span of the chunk's
-// elements, shifted as the pull reads them, and Nu's with LES), as the plain
-// kernels do one wave ahead (prefetch_ahead). The from-moments step reads its
-// own cells and takes the same spans.
+// L2 prefetch, as the plain kernels' (prefetch_ahead): every kPrefetchTiles-th
+// work item, as its block starts it, has NQ + 1 threads issue one bulk prefetch
+// each for the items [w + wave, w + wave + kPrefetchTiles) of the first one's
+// tank, wave = one wave of resident blocks: plane d's source span of their
+// elements, shifted as the pull reads them, and Nu's with LES. The from-moments
+// step reads its own cells and takes the same spans.
 template <typename S, int V, int NT, bool ESO>
-__device__ __forceinline__ void prefetch_chunk(const TankStep& ts, unsigned q0) {
+__device__ __forceinline__ void prefetch_items(const TankStep* __restrict__ tanks, const int2* __restrict__ work, int w, int nwork) {
     const int d = (int)threadIdx.x;
-    if (d > NQ || (d == NQ && !ts.les)) return;
+    if (d > NQ || w >= nwork) return;
+    const int2 wk = work[w];
+    const TankStep& ts = tanks[wk.x];
+    if (d == NQ && !ts.les) return;
     const Dims& g = ts.g;
-    const long long e0 = (long long)q0 * V, e1 = e0 + (long long)NT * V;
+    const long long e0 = (long long)wk.y * V, e1 = e0 + (long long)kPrefetchTiles * NT * V;
     if (d == NQ) return prefetch_span(ts.Nu, 4, g.plane, e0, e1);
     const long long rs = (long long)g.nz * g.jp;
     long long sh;
@@ -117,37 +103,34 @@ __device__ __forceinline__ void prefetch_chunk(const TankStep& ts, unsigned q0) 
     prefetch_span(ts.A.p[d], (int)sizeof(S), g.plane, e0 + sh - 1, e1 + sh + 1);
 }
 
-// Batched step: block b takes work items b, b + grid, ...; an item is
-// `chunks` x NT consecutive quads of one tank (fewer at the end of a
-// tank), whose step view is staged in shared memory; as it starts chunk c of
-// an item, the block prefetches chunk c + ahead into L2 (ahead > 0). 16-bit storage
-// never holds moments, so its from-moments bodies are not built. `counter` (may be
-// NULL) is advanced once: this launch runs after the step's rotation, which
-// reads it.
+// Batched step: block b takes work items b, b + grid, ...; an item is NT
+// consecutive quads of one tank (fewer at its end), whose step view is staged
+// in shared memory. Small items keep the walk in step with the prefetch and fill
+// the SMs for a small batch too. Measured on B200 against items of eight chunks
+// with the next chunk prefetched: six tanks of edge 24 to 56, fused launch 25 ->
+// 5 us (it had 100 blocks); 12 tanks of edge 32 to 128, inside the run 182 -> 159
+// us; 64 tanks, whole step 1.90 -> 1.54 ms FP32, 1.63 -> 1.48 ms FP16. 16-bit storage never holds moments, so its
+// from-moments bodies are not built. `counter` (may be NULL) is advanced once:
+// this launch runs after the step's rotation, which reads it.
 template <typename S, int V, int NT, bool ESO>
 __global__ void __launch_bounds__(NT, (ESO ? kEsotwistBlocksPerSM<S, V> : 4) * 128 / NT) k_batch_step(const TankStep* __restrict__ tanks, const int2* __restrict__ work,
-                                                   int nwork, int* counter, int ahead, int chunks) {
+                                                   int nwork, int* counter, int wave) {
     constexpr bool kFM = sizeof(S) == 4;
     __shared__ TankStep ts;
     if (counter && blockIdx.x == 0 && threadIdx.x == 0) *counter += 1;
     for (int w = blockIdx.x; w < nwork; w += gridDim.x) {
         const int2 wk = work[w];
-        __syncthreads();
+        if (w != (int)blockIdx.x) __syncthreads();   // the last item's view is read no more
         stage<NT>(ts, tanks + wk.x);
+        if (wave > 0 && w % kPrefetchTiles == 0) prefetch_items<S, V, NT, ESO>(tanks, work, w + wave, nwork);
         __syncthreads();
-        const unsigned nquads = (unsigned)ts.g.nx * (unsigned)ts.g.nz * (unsigned)(ts.g.jp / V);
-        for (int c = 0; c < chunks; c++) {
-            const unsigned t0 = (unsigned)wk.y + (unsigned)(c * NT);
-            if (t0 >= nquads) break;   // uniform over the block
-            if (ahead > 0 && c + ahead < chunks) prefetch_chunk<S, V, NT, ESO>(ts, t0 + (unsigned)(ahead * NT));
-            const unsigned t = t0 + threadIdx.x;
-            if (ts.les) {
-                if (kFM && ts.from_moments) tank_quad<S, V, ESO, true, kFM>(ts, t);
-                else tank_quad<S, V, ESO, true, false>(ts, t);
-            } else {
-                if (kFM && ts.from_moments) tank_quad<S, V, ESO, false, kFM>(ts, t);
-                else tank_quad<S, V, ESO, false, false>(ts, t);
-            }
+        const unsigned t = (unsigned)wk.y + threadIdx.x;
+        if (ts.les) {
+            if (kFM && ts.from_moments) tank_quad<S, V, ESO, true, kFM>(ts, t);
+            else tank_quad<S, V, ESO, true, false>(ts, t);
+        } else {
+            if (kFM && ts.from_moments) tank_quad<S, V, ESO, false, kFM>(ts, t);
+            else tank_quad<S, V, ESO, false, false>(ts, t);
         }
     }
 }
@@ -171,7 +154,7 @@ __global__ void __launch_bounds__(256) k_rotate_batch(const TankRotor* __restric
     o.wDelta = m.wDelta;
 }
 
-using BatchFn = void (*)(const TankStep*, const int2*, int, int*, int, int);
+using BatchFn = void (*)(const TankStep*, const int2*, int, int*, int);
 
 template <typename S, bool ESO>
 BatchFn pick(int v, int nt) {
@@ -199,7 +182,6 @@ namespace {
 struct WorkList {
     int2* d = nullptr;
     int n = 0, cap = 0;
-    int chunks = 1;   // fused-step items: chunks per item
 };
 
 }  // namespace
@@ -348,18 +330,12 @@ void build_work(tdlb_batch_s* b) {
     const int vec = width_of(b);
     auto fill = [&](WorkList& list, const std::vector<int>& ts) {
         std::vector<int2> w;
-        long long total = 0;   // chunks
-        auto quads = [&](int t) {
+        for (int t : ts) {
             const Dims& g = b->tanks[(size_t)t]->g;
-            return g.rows() * (g.jp / vec);
-        };
-        for (int t : ts) total += (quads(t) + b->threads - 1) / b->threads;
-        const int chunks = (int)std::min<long long>(tdlb::kBatchChunks,
-                                                    std::max(1LL, total / ((long long)std::max(b->sms, 1) * tdlb::kItemsPerSM)));
-        for (int t : ts)
-            for (long long q = 0; q < quads(t); q += (long long)b->threads * chunks) w.push_back(make_int2(t, (int)q));
+            const long long nq = g.rows() * (g.jp / vec);
+            for (long long q = 0; q < nq; q += b->threads) w.push_back(make_int2(t, (int)q));
+        }
         put(list, w);
-        list.chunks = chunks;
     };
     std::vector<int> all(b->tanks.size());
     for (size_t t = 0; t < all.size(); t++) all[t] = (int)t;
@@ -435,15 +411,14 @@ void advance_step_state(tdlb_lattice* h) {
 // The fused launch over `work`: persistent blocks (bps per SM, each taking
 // items b, b + grid, ...) or, with bps = 0, one block per item, so that the
 // block scheduler fills the SMs the other group's forcing pass leaves free.
-// A block prefetches the chunk about kBatchPrefetchCells cells after the one
-// it starts, within its item.
 void launch_fused(tdlb_batch_s* b, const TankStep* d_views, const WorkList& work, int* counter, cudaStream_t st) {
     if (work.n == 0) return;
     const int vec = width_of(b);
     const tdlb::BatchFn fn = tdlb::batch_kernel(storage_of(b), eso_of(b), vec, b->threads);
     const int grid = b->bps > 0 ? std::min(work.n, b->sms * b->bps) : work.n;
-    const int ahead = std::max(1, tdlb::kBatchPrefetchCells / (b->threads * vec));
-    fn<<<grid, b->threads, 0, st>>>(d_views, work.d, work.n, counter, ahead, work.chunks);
+    int per = 0;
+    TDLB_BCK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, fn, b->threads, 0));
+    fn<<<grid, b->threads, 0, st>>>(d_views, work.d, work.n, counter, per * b->sms);
     TDLB_BCK(cudaGetLastError());
 }
 
@@ -720,7 +695,6 @@ std::vector<uintptr_t> graph_key(const tdlb_batch_s* b, int P) {
         for (const WorkList* w : {&G.work, &G.rot_work, &G.gather, &G.small, &G.big}) {
             k.push_back((uintptr_t)w->d);
             k.push_back((uintptr_t)w->n);
-            k.push_back((uintptr_t)w->chunks);
         }
         k.push_back((uintptr_t)G.small_tile);
         k.push_back((uintptr_t)G.big_tile);
