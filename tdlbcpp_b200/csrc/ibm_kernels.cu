@@ -22,14 +22,16 @@
 // only where the bit is set, and the next pass treats F as zero where neither
 // the previous pass (mask_old) nor the current one has touched the cell.
 //
-// Per pass (launch_ibm): k_ibm_cells (moments and starting F of every unique
-// stencil cell of the static markers; it also starts mask_new as the static
-// touched flags), k_ibm_gather_tail (weights and stencil moments of every
-// blade marker, which no marker changes), k_ibm_spread (one plane per block:
-// the static markers' levels on an F tile in shared memory, then the plane's
-// blade levels on a shared-memory hash table of its blade cells); a tank with
-// more blade markers in a plane than the block has threads walks them with
-// k_ibm_blades afterwards. The batched passes run the same steps per lattice.
+// Per pass (launch_ibm): k_ibm_gather (everything the pass reads from the
+// state: moments and starting F of every unique stencil cell of the static
+// markers, weights and stencil moments of the blade markers; it also starts
+// mask_new as the static touched flags), then k_ibm_spread (one plane per
+// block: the static markers' levels on an F tile in shared memory, then the
+// plane's blade levels on a shared-memory hash table of its blade cells). Planes
+// with many cells (an impeller disk) take a 512-thread launch on the side
+// stream; a tank that has those, or more blade markers in a plane than an
+// ordinary block has threads, walks the blades with k_ibm_blades afterwards.
+// The batched passes run the same steps per lattice.
 #include "tdlb_kernels.cuh"
 #include "tdlb_rotate.hpp"
 
@@ -254,6 +256,7 @@ __device__ __forceinline__ void ibm_tail_cell(const IbmArgs& a, int u) {
 template <typename S>
 __global__ void __launch_bounds__(kGatherThreads) k_ibm_gather(IbmArgs a, int tail_blocks, int big_blocks, int tiles_j) {
     __shared__ CellTile sm;
+    after_previous();
     {
         const int n4 = (int)(a.mask_bytes / 16);
         for (int w = (int)(blockIdx.x * blockDim.x + threadIdx.x); w < n4; w += (int)(gridDim.x * blockDim.x))
@@ -851,7 +854,9 @@ template <int NT, bool BLADES>
 __global__ void __launch_bounds__(NT, NT == 128 ? 2 : 1) k_ibm_spread(IbmArgs a, const int* __restrict__ planes,
                                                                      int tile_cells) {
     extern __shared__ __align__(128) float btile[];             // [3][bulk_tile_stride(tile_cells)]
-    ibm_spread_plane<NT, NT == 128, BLADES>(a, planes[blockIdx.x], tile_cells, btile);
+    int b = (int)blockIdx.x;
+    after_previous(b);
+    ibm_spread_plane<NT, NT == 128, BLADES>(a, planes[b], tile_cells, btile);
 }
 
 // The blade levels of the planes that have blades, one plane per CTA of NT
@@ -875,7 +880,8 @@ __global__ void __launch_bounds__(NT, 1) k_ibm_blades(IbmArgs a, const int* __re
 // re-uploads the whole list every step).
 __global__ void k_rotate_markers(const double* __restrict__ xz, Marker* __restrict__ out, int n, double ca, double sa,
                                  double omega, double ci, double ck, int nx, int nz) {
-    const int q = blockIdx.x * blockDim.x + threadIdx.x;
+    int q = blockIdx.x * blockDim.x + threadIdx.x;
+    after_previous(q);
     if (q >= n) return;
     const RotatedMarker r = rotate_marker(xz[2 * q], xz[2 * q + 1], ca, sa, omega, ci, ck, nx, nz);
     Marker& m = out[q];
@@ -892,6 +898,7 @@ __global__ void __launch_bounds__(256) k_place_blades(const int* __restrict__ st
                                                       int* __restrict__ order, int n, int* __restrict__ level_ptr, int nlev,
                                                       int* __restrict__ plane_lv, int nplane) {
     int t = (int)(blockIdx.x * blockDim.x + threadIdx.x);
+    after_previous(t);
     const int total = mwords + n + nlev + nplane;
     if (t >= total) return;
     const int v = stage[t];
@@ -904,16 +911,14 @@ __global__ void __launch_bounds__(256) k_place_blades(const int* __restrict__ st
 cudaError_t launch_place_blades(const int* stage, Marker* markers, int n, int* order, int* level_ptr, int nlev, int* plane_lv,
                                 int nplane, cudaStream_t st) {
     const int mwords = (int)(sizeof(Marker) / sizeof(int)) * n;
-    k_place_blades<<<(mwords + n + nlev + nplane + 255) / 256, 256, 0, st>>>(stage, reinterpret_cast<int*>(markers), mwords, order,
-                                                                             n, level_ptr, nlev, plane_lv, nplane);
-    return cudaGetLastError();
+    return launch_chained(k_place_blades, (mwords + n + nlev + nplane + 255) / 256, 256, 0, st, stage,
+                          reinterpret_cast<int*>(markers), mwords, order, n, level_ptr, nlev, plane_lv, nplane);
 }
 
 cudaError_t launch_rotate_markers(const double* xz, Marker* out, int n, double ca, double sa, double omega, double ci,
                                   double ck, int nx, int nz, cudaStream_t st) {
     if (n <= 0) return cudaSuccess;
-    k_rotate_markers<<<(n + 255) / 256, 256, 0, st>>>(xz, out, n, ca, sa, omega, ci, ck, nx, nz);
-    return cudaGetLastError();
+    return launch_chained(k_rotate_markers, (n + 255) / 256, 256, 0, st, xz, out, n, ca, sa, omega, ci, ck, nx, nz);
 }
 
 // FP64 sums of five values over a block of 256 threads (fixed order: a warp's
@@ -949,8 +954,10 @@ __device__ __forceinline__ void block_sum5(double (&v)[5]) {
 __global__ void __launch_bounds__(256) k_marker_load(IbmArgs a, const int* __restrict__ slots, int n, double ci, double ck,
                                                      double* partial, unsigned* counter, double* out) {
     __shared__ bool last;
+    int t = (int)(blockIdx.x * blockDim.x + threadIdx.x);
+    after_previous(t);
     double acc[5] = {0, 0, 0, 0, 0};
-    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
+    for (; t < n; t += gridDim.x * blockDim.x) {
         const int p = slots[t];
         const Marker mk = a.markers[a.sched[p]];
         const double fx = -(double)a.beta * (double)a.sums[p];
@@ -1035,8 +1042,7 @@ __device__ __forceinline__ void ordered_final(const double* __restrict__ partial
 cudaError_t launch_marker_load(const IbmArgs& a, const int* slots, int n, double ci, double ck, double* partial,
                                unsigned* counter, double* out, cudaStream_t st) {
     const int blocks = n <= 0 ? 1 : std::min(kLoadBlocks, (n + 511) / 512);   // two slots a thread, more in a large tank
-    k_marker_load<<<blocks, 256, 0, st>>>(a, slots, n, ci, ck, partial, counter, out);
-    return cudaGetLastError();
+    return launch_chained(k_marker_load, blocks, 256, 0, st, a, slots, n, ci, ck, partial, counter, out);
 }
 
 // FP64 mass and momentum over all interior cells, deterministic: a fixed
@@ -1160,10 +1166,11 @@ cudaError_t launch_ibm(const IbmArgs& a, cudaStream_t st) {
     const long long blocks = tail_blocks + (long long)a.n_big * big_blocks +
                              (long long)tiles_j * ((a.max_cells + kCellPlaces - 1) / kCellPlaces);
     // (an empty list still starts mask_new)
+    cudaError_t err = cudaSuccess;
     with_storage(a.storage, [&](auto s) {
-        k_ibm_gather<decltype(s)><<<(unsigned)std::max(blocks, 1LL), kGatherThreads, 0, st>>>(a, tail_blocks, big_blocks, tiles_j);
+        err = launch_chained(k_ibm_gather<decltype(s)>, (unsigned)std::max(blocks, 1LL), kGatherThreads, 0, st, a, tail_blocks,
+                             big_blocks, tiles_j);
     });
-    cudaError_t err = cudaGetLastError();
     if (err != cudaSuccess) return err;
     // Side stream: the planes with many cells (an impeller disk), with a
     // full-size tile and 512 threads, beside the ordinary planes.
@@ -1183,10 +1190,9 @@ cudaError_t launch_ibm(const IbmArgs& a, cudaStream_t st) {
     const bool own = a.blade_max <= 128 && a.n_big == 0;
     if (a.n_small > 0) {
         const size_t bytes = big_bulk_bytes(a.smem_cells);
-        if (own && a.n_blade > 0) k_ibm_spread<128, true><<<a.n_small, 128, bytes, st>>>(a, a.plane_list, a.smem_cells);
-        else k_ibm_spread<128, false><<<a.n_small, 128, bytes, st>>>(a, a.plane_list, a.smem_cells);
+        const auto kernel = own && a.n_blade > 0 ? k_ibm_spread<128, true> : k_ibm_spread<128, false>;
+        err = launch_chained(kernel, a.n_small, 128, bytes, st, a, a.plane_list, a.smem_cells);
     }
-    err = cudaGetLastError();
     if (err == cudaSuccess && a.n_big > 0) err = cudaStreamWaitEvent(st, a.ev_join, 0);
     if (err != cudaSuccess || own || a.n_blade == 0) return err;
     k_ibm_blades<512><<<a.n_blade, 512, (size_t)a.blade_words * sizeof(float), st>>>(a, a.blade_planes, a.n_blade,

@@ -56,11 +56,11 @@ static inline unsigned step_blocks(const StepArgs& a, int V) {
 
 template <int V>
 static cudaError_t launch_simple_v(const StepArgs& a, cudaStream_t st) {
-    const dim3 grid(step_blocks(a, V)), block(128);
+    const unsigned grid = step_blocks(a, V);
+    cudaError_t err = cudaSuccess;
 #define TDLB_SIMPLE(LES, FM, COL, PART)                                                                       \
-    k_step_simple<float, V, LES, FM, COL, PART><<<grid, block, 0, st>>>(                                   \
-        a.A, a.B, a.Nu, a.F, a.mask, a.g, a.p,                                                               \
-        launch_walk<k_step_simple<float, V, LES, FM, COL, PART>, COL && !FM>(a))
+    err = launch_step_kernel<kChained<PART>>(k_step_simple<float, V, LES, FM, COL, PART>, grid, st, a.A, a.B, a.Nu, a.F, a.mask, a.g, a.p, \
+                                   launch_walk<k_step_simple<float, V, LES, FM, COL, PART>, COL && !FM>(a))
     if (!a.collide) TDLB_SIMPLE(false, false, false, 0);
     else if (a.from_moments) { if (a.les) TDLB_SIMPLE(true, true, true, 0); else TDLB_SIMPLE(false, true, true, 0); }
     else if constexpr (V == 1) {
@@ -77,39 +77,39 @@ static cudaError_t launch_simple_v(const StepArgs& a, cudaStream_t st) {
         if (a.les) TDLB_SIMPLE(true, false, true, 0); else TDLB_SIMPLE(false, false, true, 0);
     }
 #undef TDLB_SIMPLE
-    return cudaGetLastError();
+    return err;
 }
 
 template <int V, bool LES, bool FM, bool COL, int PART>
-static void eso_launch(const StepArgs& a, dim3 grid, cudaStream_t st) {
+static cudaError_t eso_launch(const StepArgs& a, unsigned grid, cudaStream_t st) {
     if (a.even)
-        k_step_esotwist<float, V, LES, FM, COL, true, PART><<<grid, 128, 0, st>>>(
-            a.A, a.Nu, a.F, a.mask, a.g, a.p, launch_walk<k_step_esotwist<float, V, LES, FM, COL, true, PART>, COL && !FM>(a));
-    else
-        k_step_esotwist<float, V, LES, FM, COL, false, PART><<<grid, 128, 0, st>>>(
-            a.A, a.Nu, a.F, a.mask, a.g, a.p, launch_walk<k_step_esotwist<float, V, LES, FM, COL, false, PART>, COL && !FM>(a));
+        return launch_step_kernel<kChained<PART>>(k_step_esotwist<float, V, LES, FM, COL, true, PART>, grid, st, a.A, a.Nu, a.F, a.mask, a.g,
+                                        a.p, launch_walk<k_step_esotwist<float, V, LES, FM, COL, true, PART>, COL && !FM>(a));
+    return launch_step_kernel<kChained<PART>>(k_step_esotwist<float, V, LES, FM, COL, false, PART>, grid, st, a.A, a.Nu, a.F, a.mask, a.g,
+                                    a.p, launch_walk<k_step_esotwist<float, V, LES, FM, COL, false, PART>, COL && !FM>(a));
 }
 
 template <int V>
 static cudaError_t launch_esotwist_v(const StepArgs& a, cudaStream_t st) {
-    const dim3 grid(step_blocks(a, V));
-    if (!a.collide) eso_launch<V, false, false, false, 0>(a, grid, st);
+    const unsigned grid = step_blocks(a, V);
+    cudaError_t err = cudaSuccess;
+    if (!a.collide) err = eso_launch<V, false, false, false, 0>(a, grid, st);
     else if (a.from_moments) {
-        if (a.les) eso_launch<V, true, true, true, 0>(a, grid, st); else eso_launch<V, false, true, true, 0>(a, grid, st);
+        if (a.les) err = eso_launch<V, true, true, true, 0>(a, grid, st); else err = eso_launch<V, false, true, true, 0>(a, grid, st);
     } else if constexpr (V == 1) {
         if (a.les) {
-            if (a.part == 1) eso_launch<1, true, false, true, 1>(a, grid, st);
-            else if (a.part == 2) eso_launch<1, true, false, true, 2>(a, grid, st);
-            else eso_launch<1, true, false, true, 0>(a, grid, st);
+            if (a.part == 1) err = eso_launch<1, true, false, true, 1>(a, grid, st);
+            else if (a.part == 2) err = eso_launch<1, true, false, true, 2>(a, grid, st);
+            else err = eso_launch<1, true, false, true, 0>(a, grid, st);
         } else {
-            if (a.part == 1) eso_launch<1, false, false, true, 1>(a, grid, st);
-            else if (a.part == 2) eso_launch<1, false, false, true, 2>(a, grid, st);
-            else eso_launch<1, false, false, true, 0>(a, grid, st);
+            if (a.part == 1) err = eso_launch<1, false, false, true, 1>(a, grid, st);
+            else if (a.part == 2) err = eso_launch<1, false, false, true, 2>(a, grid, st);
+            else err = eso_launch<1, false, false, true, 0>(a, grid, st);
         }
     } else {
-        if (a.les) eso_launch<V, true, false, true, 0>(a, grid, st); else eso_launch<V, false, false, true, 0>(a, grid, st);
+        if (a.les) err = eso_launch<V, true, false, true, 0>(a, grid, st); else err = eso_launch<V, false, false, true, 0>(a, grid, st);
     }
-    return cudaGetLastError();
+    return err;
 }
 
 cudaError_t launch_step_simple(const StepArgs& a, cudaStream_t st) {

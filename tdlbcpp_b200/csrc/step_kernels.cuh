@@ -671,13 +671,20 @@ __device__ __forceinline__ void prefetch_ahead(const Planes& A, const float* Nu,
     prefetch_span(A.p[d], (int)sizeof(S), g.plane, e0 + sh - 1, e1 + sh + 1);
 }
 
+// Step launches that go close behind the one before them (launch_chained): all
+// but part 1, which follows an event on a stream of its own.
+template <int PART>
+constexpr bool kChained = PART != 1;
+
 template <typename S, int V, bool LES, bool FROM_MOMENTS, bool COLLIDE, int PART = 0>
 __global__ void __launch_bounds__(128, 4) k_step_simple(Planes A, Planes B, float* __restrict__ Nu,
                                                        const float4* __restrict__ F, const uint32_t* __restrict__ mask,
                                                        Dims g, CollideParams p, StepPart part) {
     if constexpr (PART != 2 && COLLIDE && !FROM_MOMENTS)
         prefetch_ahead<S, V, LES, false, false>(A, Nu, g, part.l2_ahead);
-    simple_quad<S, V, LES, FROM_MOMENTS, COLLIDE, PART>(A, B, Nu, F, mask, g, p, blockIdx.x * blockDim.x + threadIdx.x, part);
+    unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
+    if constexpr (kChained<PART>) after_previous(t);
+    simple_quad<S, V, LES, FROM_MOMENTS, COLLIDE, PART>(A, B, Nu, F, mask, g, p, t, part);
 }
 
 // Resident 128-thread blocks per SM the Esotwist kernel is built for: the
@@ -694,7 +701,19 @@ __global__ void __launch_bounds__(128, kEsotwistBlocksPerSM<S, V>) k_step_esotwi
                                                          Dims g, CollideParams p, StepPart part) {
     if constexpr (PART != 2 && COLLIDE && !FROM_MOMENTS)
         prefetch_ahead<S, V, LES, true, EVEN>(Q, Nu, g, part.l2_ahead);
-    esotwist_quad<S, V, LES, FROM_MOMENTS, COLLIDE, EVEN, PART>(Q, Nu, F, mask, g, p, blockIdx.x * blockDim.x + threadIdx.x, part);
+    unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
+    if constexpr (kChained<PART>) after_previous(t);
+    esotwist_quad<S, V, LES, FROM_MOMENTS, COLLIDE, EVEN, PART>(Q, Nu, F, mask, g, p, t, part);
+}
+
+template <bool CHAINED, typename... P, typename... A>
+cudaError_t launch_step_kernel(void (*kernel)(P...), unsigned grid, cudaStream_t st, A... args) {
+    if constexpr (CHAINED) {
+        return launch_chained(kernel, grid, 128, 0, st, args...);
+    } else {
+        kernel<<<grid, 128, 0, st>>>(static_cast<P>(args)...);
+        return cudaGetLastError();
+    }
 }
 
 // One cell of the box list per thread: its 18 stored deviations, exact where
@@ -707,7 +726,8 @@ template <typename S, bool SIMPLE, bool LES, bool EVEN>
 __global__ void __launch_bounds__(128) k_box_step(Planes A, Planes B, float* __restrict__ Nu, const float4* __restrict__ F,
                                                   const uint32_t* __restrict__ mask, Dims g, CollideParams p,
                                                   const int* __restrict__ cells, int n, ResidualBox rr, ResidualBox rw) {
-    const int t = (int)(blockIdx.x * blockDim.x + threadIdx.x);
+    int t = (int)(blockIdx.x * blockDim.x + threadIdx.x);
+    after_previous(t);
     if (t >= n) return;
     Quad q;
     q.e0 = cells[t];

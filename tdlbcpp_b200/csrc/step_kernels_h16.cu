@@ -13,48 +13,43 @@ static inline unsigned grid16(const StepArgs& a, int V) {
 }
 
 template <typename S, int V, bool LES, int PART>
-static void simple16_part(const StepArgs& a, cudaStream_t st) {
-    k_step_simple<S, V, LES, false, true, PART><<<grid16(a, V), 128, 0, st>>>(
-        a.A, a.B, a.Nu, a.F, a.mask, a.g, a.p, launch_walk<k_step_simple<S, V, LES, false, true, PART>, true>(a));
+static cudaError_t simple16_part(const StepArgs& a, cudaStream_t st) {
+    return launch_step_kernel<kChained<PART>>(k_step_simple<S, V, LES, false, true, PART>, grid16(a, V), st, a.A, a.B, a.Nu, a.F, a.mask,
+                                    a.g, a.p, launch_walk<k_step_simple<S, V, LES, false, true, PART>, true>(a));
 }
 
 template <typename S, int V, bool LES>
-static void simple16_les(const StepArgs& a, cudaStream_t st) {
+static cudaError_t simple16_les(const StepArgs& a, cudaStream_t st) {
     if (a.part == 1) return simple16_part<S, V, LES, 1>(a, st);
     if (a.part == 2) return simple16_part<S, V, LES, 2>(a, st);
-    simple16_part<S, V, LES, 0>(a, st);
+    return simple16_part<S, V, LES, 0>(a, st);
 }
 
 template <typename S, int V>
 static cudaError_t simple16(const StepArgs& a, cudaStream_t st) {
-    if (a.les) simple16_les<S, V, true>(a, st);
-    else simple16_les<S, V, false>(a, st);
-    return cudaGetLastError();
+    return a.les ? simple16_les<S, V, true>(a, st) : simple16_les<S, V, false>(a, st);
 }
 
 template <typename S, int V, bool LES, int PART>
-static void eso16_part(const StepArgs& a, cudaStream_t st) {
+static cudaError_t eso16_part(const StepArgs& a, cudaStream_t st) {
     const unsigned grid = grid16(a, V);
     if (a.even)
-        k_step_esotwist<S, V, LES, false, true, true, PART><<<grid, 128, 0, st>>>(
-            a.A, a.Nu, a.F, a.mask, a.g, a.p, launch_walk<k_step_esotwist<S, V, LES, false, true, true, PART>, true>(a));
-    else
-        k_step_esotwist<S, V, LES, false, true, false, PART><<<grid, 128, 0, st>>>(
-            a.A, a.Nu, a.F, a.mask, a.g, a.p, launch_walk<k_step_esotwist<S, V, LES, false, true, false, PART>, true>(a));
+        return launch_step_kernel<kChained<PART>>(k_step_esotwist<S, V, LES, false, true, true, PART>, grid, st, a.A, a.Nu, a.F, a.mask, a.g,
+                                        a.p, launch_walk<k_step_esotwist<S, V, LES, false, true, true, PART>, true>(a));
+    return launch_step_kernel<kChained<PART>>(k_step_esotwist<S, V, LES, false, true, false, PART>, grid, st, a.A, a.Nu, a.F, a.mask, a.g,
+                                    a.p, launch_walk<k_step_esotwist<S, V, LES, false, true, false, PART>, true>(a));
 }
 
 template <typename S, int V, bool LES>
-static void eso16_les(const StepArgs& a, cudaStream_t st) {
+static cudaError_t eso16_les(const StepArgs& a, cudaStream_t st) {
     if (a.part == 1) return eso16_part<S, V, LES, 1>(a, st);
     if (a.part == 2) return eso16_part<S, V, LES, 2>(a, st);
-    eso16_part<S, V, LES, 0>(a, st);
+    return eso16_part<S, V, LES, 0>(a, st);
 }
 
 template <typename S, int V>
 static cudaError_t eso16(const StepArgs& a, cudaStream_t st) {
-    if (a.les) eso16_les<S, V, true>(a, st);
-    else eso16_les<S, V, false>(a, st);
-    return cudaGetLastError();
+    return a.les ? eso16_les<S, V, true>(a, st) : eso16_les<S, V, false>(a, st);
 }
 
 cudaError_t launch_step_simple_h16(const StepArgs& a, cudaStream_t st) {
@@ -76,14 +71,9 @@ cudaError_t launch_step_esotwist_h16(const StepArgs& a, cudaStream_t st) {
 }
 
 template <typename S, bool SIMPLE, bool EVEN>
-static void box16(const StepArgs& a, cudaStream_t st) {
-    const unsigned grid = blocks16(a.n_box, 128);
-    if (a.les)
-        k_box_step<S, SIMPLE, true, EVEN><<<grid, 128, 0, st>>>(a.A, a.B, a.Nu, a.F, a.mask, a.g, a.p, a.box_cells, a.n_box,
-                                                                a.rr, a.rw);
-    else
-        k_box_step<S, SIMPLE, false, EVEN><<<grid, 128, 0, st>>>(a.A, a.B, a.Nu, a.F, a.mask, a.g, a.p, a.box_cells, a.n_box,
-                                                                 a.rr, a.rw);
+static cudaError_t box16(const StepArgs& a, cudaStream_t st) {
+    return launch_step_kernel<true>(a.les ? k_box_step<S, SIMPLE, true, EVEN> : k_box_step<S, SIMPLE, false, EVEN>,
+                                     blocks16(a.n_box, 128), st, a.A, a.B, a.Nu, a.F, a.mask, a.g, a.p, a.box_cells, a.n_box, a.rr, a.rw);
 }
 
 cudaError_t launch_box(const StepArgs& a, bool simple, cudaStream_t st) {
@@ -93,10 +83,8 @@ cudaError_t launch_box(const StepArgs& a, bool simple, cudaStream_t st) {
         using S = decltype(s);
         if constexpr (sizeof(S) == 4) return cudaErrorInvalidValue;
         else {
-            if (simple) box16<S, true, true>(a, st);
-            else if (a.even) box16<S, false, true>(a, st);
-            else box16<S, false, false>(a, st);
-            return cudaGetLastError();
+            if (simple) return box16<S, true, true>(a, st);
+            return a.even ? box16<S, false, true>(a, st) : box16<S, false, false>(a, st);
         }
     });
 }

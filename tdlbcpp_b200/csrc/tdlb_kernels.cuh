@@ -39,6 +39,43 @@ int wave_ctas() {
     return v;
 }
 
+// A launch whose blocks are set up while the stream's previous launch drains.
+// Every thread of such a kernel begins with after_previous(), which returns
+// once that launch has ended and its writes are visible: the order on the
+// stream is that of an ordinary launch. In a kernel with read-only loads (const
+// __restrict__ or __ldg) the index that addresses them goes through it, so that
+// none of them can be moved ahead of it (k_ibm_gather has none; there the index
+// through it cost registers: 192^3 BF16 30.5 -> 34.9 us).
+// The step, gather, spread, load and rotation of a small tank are a chain of
+// launches of 2 to 25 us with 1.5 to 3 us between them. B200, runs of 60 steps
+// with forcing, load and rotation, ordinary launches -> these: 24^3 2.86 ->
+// 2.14 ms, 101x83x97 with uploaded blades 5.44 -> 5.03, 160^3 FP16 Simple 9.55
+// -> 9.12, 192^3 BF16 Esotwist 13.06 -> 12.97, 400^3 FP16 Esotwist 64.4 -> 64.6
+// (equal). A captured stream gets ordinary launches.
+template <typename... P, typename... A>
+cudaError_t launch_chained(void (*kernel)(P...), unsigned grid, int block, size_t smem, cudaStream_t st, A... args) {
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &capture) != cudaSuccess) return cudaGetLastError();
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3((unsigned)block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cfg.attrs = &attr;
+    cfg.numAttrs = capture == cudaStreamCaptureStatusNone ? 1 : 0;
+    cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+    return cudaGetLastError();
+}
+__device__ __forceinline__ void after_previous() { asm volatile("griddepcontrol.wait;" : : : "memory"); }
+template <typename T>
+__device__ __forceinline__ void after_previous(T& index) {
+    static_assert(sizeof(T) == 4, "a 32-bit index");
+    asm volatile("griddepcontrol.wait;" : "+r"(index) : : "memory");
+}
+
 // Arguments of one fused step launch.
 struct StepArgs {
     Planes A;               // Simple: source buffer; Esotwist: the single buffer
@@ -102,7 +139,7 @@ struct Marker {
 };
 static_assert(sizeof(Marker) == 48, "Marker layout");
 
-// Blade (second-segment) scratch written by k_ibm_gather_tail, read by the
+// Blade (second-segment) scratch written by k_ibm_gather, read by the
 // spread walk; field-major over the segment's slots.
 enum TailField {
     TF_W = 0,               // 9 stencil weights, (k1, i1) order
