@@ -178,15 +178,11 @@ def run_ours(args, rank, world, device):
     except tb.TdlbError:
         zone = None   # the zone covers most of this lattice: steps are not split
 
-    # ---- value: device-resident steps. The library brackets every step-kernel
-    # launch with CUDA events on the stream it runs on (a split step is two
-    # launches on two streams); t1 follows a join of both streams.
+    # ---- value: device-resident steps; t1 follows a join of the unit's streams.
     t0, t1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
     barrier(world)
     cu.synchronize()
     torch.cuda.synchronize()
-    cu.kernel_time()
-    cu.set_kernel_timing(True)
     launches0 = cu.kernel_launches()
     with ClockSampler(device) as clk:
         t0.record(stream)
@@ -198,12 +194,7 @@ def run_ours(args, rank, world, device):
         torch.cuda.synchronize()
     barrier(world)
     launches = cu.kernel_launches() - launches0
-    kernel_total_ms, kernel_n = cu.kernel_time()
-    cu.set_kernel_timing(False)
-    ms = t0.elapsed_time(t1)
-    kernel_ms = kernel_total_ms / args.steps
-    ms = max_over_ranks(ms, world)
-    kernel_ms_max = max_over_ranks(kernel_ms, world)
+    ms = max_over_ranks(t0.elapsed_time(t1), world)
 
     # ---- e2e: host-driven steps through the C ABI. Per step the host
     # generates the blades at the step's angle into pinned memory and uploads
@@ -268,6 +259,27 @@ def run_ours(args, rank, world, device):
     load_np = loads[-1]
     e2e_s = max_over_ranks(w1 - w0, world)
     red = cu.reduce_fp64()
+
+    # ---- the step kernel alone, for its roofline: the library brackets every
+    # step launch with CUDA events. A split step's launches run beside the
+    # forcing pass and one another, so their sum is no kernel time; these
+    # steps, from rest again, are not split.
+    def step_launches(k=10):
+        cu.initialise(1.0)
+        cu.forcing_resident(ALPHA, BETA)
+        for n in range(3 + k):   # (the blades stay where the run left them)
+            if n == 3:
+                cu.kernel_time()
+                cu.set_kernel_timing(True)
+            cu.collision()
+            cu.forcing_resident(ALPHA, BETA)
+        total_ms, n = cu.kernel_time()
+        cu.set_kernel_timing(False)
+        return total_ms / k, n / k
+
+    launches_per_step = step_launches()[1]
+    cu.set_overlap(False)
+    kernel_ms_max = max_over_ranks(step_launches()[0], world)
     cu.close()
 
     result = {
@@ -290,7 +302,9 @@ def run_ours(args, rank, world, device):
         "mass_drift_timed": float(red_timed[0] / cells - 1.0),
         "mass_drift_end": float(red[0] / cells - 1.0),
         "launches": launches,
-        "step_launches": kernel_n,
+        "step_launches": launches_per_step,
+        # (the library splits the steps of lattices from 2^19 cells by itself)
+        "split_on": zone is not None if args.overlap else cells >= 1 << 19,
         "inner_fraction": None if zone is None else float(zone.mean()),
     }
     return result
@@ -760,6 +774,16 @@ def reference_height(steps, warmup):
     return 16 if steps + warmup <= 100 else 8
 
 
+def cpu_baseline(note=""):
+    """The reference's rate on this host, or why it cannot be had (its library
+    is built from the reference's sources, which may not be there)."""
+    try:
+        r = reference_sample(3, 1, host_threads())
+    except FileNotFoundError as e:
+        return {"unavailable": str(e)}
+    return {"value": r["value"], "unit": "MLUPS", "cores": r["cores"], "kind": "reference", "sample": r["sample"] + note}
+
+
 def reference_sample(steps, warmup, threads, edge=EDGE, height=16):
     """Every thread advances its own reference ComputeUnit (FP32, Simple,
     LES) on an edge x height x edge slab through the impeller plane.
@@ -931,9 +955,7 @@ def report_batched(args, rank, world, local, config):
         "fields_finite": res["fields_finite"],
     }
     if world == 1 and not args.no_cpu_baseline:
-        r = reference_sample(3, 1, host_threads())
-        line["cpu_baseline"] = {"value": r["value"], "unit": "MLUPS", "cores": r["cores"], "kind": "reference",
-                                "sample": r["sample"] + " (per-cell rate of the same step)"}
+        line["cpu_baseline"] = cpu_baseline(" (per-cell rate of the same step)")
     print(json.dumps(line), flush=True)
     return 0
 
@@ -950,7 +972,8 @@ def main():
     ap.add_argument("--edge", type=int, default=EDGE)
     ap.add_argument("--no-cpu-baseline", action="store_true")
     ap.add_argument("--overlap", action="store_true",
-                    help="simple/esotwist: split steps (outer cells overlap the previous forcing pass)")
+                    help="simple/esotwist: split steps (outer cells beside the forcing pass) whatever the lattice's size; "
+                         "the library splits those of a large lattice by itself")
     ap.add_argument("--storage", choices=["fp32", "fp16", "bf16"], default="fp32",
                     help="simple/esotwist: population storage (16-bit forms store deviations from the rest weights)")
     args = ap.parse_args()
@@ -992,7 +1015,11 @@ def main():
         nthr = host_threads()
         steps, warm = args.steps, args.warmup
         h = reference_height(steps, warm)
-        r = reference_sample(steps, warm, nthr, height=h)
+        try:
+            r = reference_sample(steps, warm, nthr, height=h)
+        except FileNotFoundError as e:
+            print(json.dumps({"impl": "reference", "unavailable": str(e)}), flush=True)
+            return 0
         line = {"metric": "MLUPS", "value": r["value"], "unit": "MLUPS", "n_gpus": args.gpus, "steps": steps,
                 "warmup": warm, "ms_per_step": r["seconds"] / steps * 1e3, "higher_is_better": True,
                 "scaling": "weak", "vs_baseline": None, "dtype": "fp32", "data": "synthetic", "config": config,
@@ -1038,17 +1065,15 @@ def main():
         "gpu_launches": res["launches"],
         "clocks": res["clocks"],
         "markers": res["n_markers"],
-        "split_step": {"on": res["inner_fraction"] is not None, "inner_cell_fraction": res["inner_fraction"],
-                       "step_launches_per_step": res["step_launches"] / args.steps},
+        "split_step": {"on": res["split_on"], "inner_cell_fraction": res["inner_fraction"],
+                       "step_launches_per_step": res["step_launches"]},
         # the fields and the FP64 mass after the warm-up and timed steps
         "fields_finite": res["fields_finite_after_timed"],
         "steps_from_rest_at_check": res["steps_before_timed_check"],
         "mass_drift": res["mass_drift_timed"],
     }
     if world == 1 and not args.no_cpu_baseline:
-        r = reference_sample(3, 1, host_threads())
-        line["cpu_baseline"] = {"value": r["value"], "unit": "MLUPS", "cores": r["cores"], "kind": "reference",
-                                "sample": r["sample"]}
+        line["cpu_baseline"] = cpu_baseline()
     print(json.dumps(line), flush=True)
     return 0
 

@@ -480,10 +480,11 @@ class ComputeUnit:
         return tuple(int(v) for v in out)
 
     def set_overlap(self, mode):
-        """Split steps: the outer cells of a step run while the previous
-        forcing pass is in flight; results are identical. False/0 (default):
-        off; True/1: when the inner chunks hold at most 60 % of the lattice;
-        "always"/2: whenever the markers are resident."""
+        """Split steps: the outer cells of a step run while the forcing pass is
+        in flight; results are identical. Without a call the library splits
+        the steps of a large lattice. False/0: off; True/1: when the inner
+        words hold at most 60 % of the lattice; "always"/2: whenever the
+        markers are resident."""
         m = 2 if mode == "always" else int(bool(mode)) if isinstance(mode, bool) else int(mode)
         self._check(self.lib.tdlb_set_overlap(self.h, m))
 
@@ -493,7 +494,7 @@ class ComputeUnit:
         self._check(self.lib.tdlb_join(self.h))
 
     def read_zone(self) -> np.ndarray:
-        """Per-cell flags of the split-step inner chunks."""
+        """Per-cell flags of the split-step inner words."""
         out = np.empty((self.x, self.y, self.z), np.uint8)
         self._check(self.lib.tdlb_read_zone(self.h, _p(out)))
         return out
