@@ -705,12 +705,15 @@ void upload_markers(tdlb_lattice* h, const tdlb_marker* m, size_t n, size_t n0, 
     if (n > (size_t)0x7fffffff) throw Fail{TDLB_EINVAL, "too many markers"};
     const Dims& g = h->g;
     static_assert(sizeof(tdlb_marker) == sizeof(tdlb::Marker), "marker layout");
-    if ((long long)n > h->marker_cap || !h->d_markers_in) {
-        // (the resident list stays valid until the new one has been checked)
+    // The list goes into the buffer that is not the resident one's (which stays
+    // valid until the new list has been checked); the two change places with
+    // every list, so each is held against its own length.
+    if ((long long)n > h->marker_in_cap || !h->d_markers_in) {
         const long long cap = std::max<long long>(round_up((long long)n, 1024), std::max<long long>(h->marker_cap, 1024));
         TDLB_CK(cudaStreamSynchronize(h->stream));
         cudaFree(h->d_markers_in);
         h->d_markers_in = nullptr;
+        h->marker_in_cap = 0;
         TDLB_CK(cudaMalloc(&h->d_markers_in, cap * sizeof(tdlb::Marker)));
         h->marker_in_cap = cap;
     }

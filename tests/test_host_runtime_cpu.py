@@ -1,0 +1,78 @@
+"""The host runtime's bookkeeping without a GPU: the library's own objects on a
+CUDA runtime for the CPU (tests/cpp/fake_cuda.cpp). Kernels do nothing there;
+what is checked is that every buffer a copy or a launch names is allocated and
+long enough, and when the library allocates, waits and orders its streams."""
+import ctypes
+import os
+import subprocess
+
+import numpy as np
+import pytest
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+ALPHA, BETA = 0.97, 1.9
+
+
+@pytest.fixture(scope="module")
+def fake_library():
+    r = subprocess.run(["make", "-C", os.path.join(ROOT, "tests", "cpp"), "fake"], stdout=subprocess.PIPE,
+                       stderr=subprocess.STDOUT, text=True)
+    assert r.returncode == 0, r.stdout[-3000:]
+    return os.path.join(ROOT, "tests", "cpp", "_bin", "libtdlb_fake_cuda.so")
+
+
+@pytest.fixture
+def fake(fake_library, monkeypatch):
+    """The package on the CPU runtime; fake.lib has its fake_* functions."""
+    import tdlbcpp_b200 as tb
+    monkeypatch.setattr(tb, "_lib", None)
+    monkeypatch.setattr(tb, "library_path", lambda: fake_library)
+    lib = tb.load_library()
+    for name in ("mallocs", "waits"):
+        getattr(lib, "fake_" + name).restype = ctypes.c_longlong
+    lib.fake_faults.restype = ctypes.c_char_p
+    lib.fake_fail.argtypes = [ctypes.c_longlong]
+    lib.fake_foreign.argtypes, lib.fake_foreign.restype = [ctypes.c_void_p], ctypes.c_longlong
+    lib.fake_launches.argtypes, lib.fake_launches.restype = [ctypes.c_char_p], ctypes.c_longlong
+    lib.fake_unordered.argtypes = [ctypes.c_char_p, ctypes.c_void_p, ctypes.c_longlong]
+    lib.fake_unordered.restype = ctypes.c_longlong
+    lib.fake_pin.argtypes = [ctypes.c_void_p, ctypes.c_size_t]
+    lib.fake_reset()
+    yield tb
+    lib.fake_reset()
+
+
+def faults(tb):
+    return tb.load_library().fake_faults().decode()
+
+
+def markers(tb, n, dims, seed=1):
+    rng = np.random.default_rng(seed)
+    m = np.zeros(n, tb.MARKER_DTYPE)
+    for name, hi in zip("ijk", dims):
+        m[name] = rng.integers(0, hi, n)
+    return m
+
+
+def test_lists_of_changing_length_stay_in_their_buffers(fake):
+    dims = (20, 24, 18)
+    cu = fake.ComputeUnit(x=dims[0], y=dims[1], z=dims[2], nu=1e-3)
+    cu.initialise(1.0)
+    for n in (500, 1000, 5000, 5000, 3000, 6000, 6000, 0, 2000, 7000, 7000):
+        cu.forcing(markers(fake, n, dims), ALPHA, BETA)
+        assert not faults(fake), f"after {n} markers"
+    bad = markers(fake, 9000, dims)
+    bad["i"][4000] = dims[0]
+    for n in (8000, 9000, 8000, 9000):
+        with pytest.raises(fake.TdlbError, match="marker 4000 at"):
+            cu.set_markers(bad[:n])
+        np.testing.assert_array_equal(cu.read_markers(), markers(fake, 7000, dims))
+        cu.forcing(markers(fake, 7000, dims), ALPHA, BETA)
+        assert not faults(fake)
+    cu.doubleResolutionFullCU()
+    cu.initialise(1.0)
+    for n in (20000, 20000, 20000):
+        cu.forcing(markers(fake, n, dims), ALPHA, BETA)
+        assert not faults(fake), f"after {n} markers on the doubled lattice"
+    cu.close()
+    assert not faults(fake)
