@@ -248,7 +248,7 @@ struct BFail {
 #define TDLB_BCK(call)                                                                          \
     do {                                                                                        \
         cudaError_t e_ = (call);                                                                \
-        if (e_ != cudaSuccess) throw BFail{TDLB_ECUDA, std::string(#call) + ": " + cudaGetErrorString(e_)}; \
+        if (e_ != cudaSuccess) throw BFail{TDLB_ECUDA, tdlb_rt::error_text(#call, e_)};                     \
     } while (0)
 
 thread_local std::string g_batch_create_error = "no error";

@@ -144,7 +144,7 @@ struct CFail {
 #define TDLB_CCK(call)                                                                                      \
     do {                                                                                                    \
         cudaError_t e_ = (call);                                                                            \
-        if (e_ != cudaSuccess) throw CFail{TDLB_ECUDA, std::string(#call) + ": " + cudaGetErrorString(e_)}; \
+        if (e_ != cudaSuccess) throw CFail{TDLB_ECUDA, tdlb_rt::error_text(#call, e_)};                     \
     } while (0)
 
 template <typename F>
@@ -207,7 +207,7 @@ void write_device(const std::string& path, const float* dev, size_t bytes, cudaS
         const cudaError_t s = e == cudaSuccess ? cudaStreamSynchronize(st) : e;
         if (s != cudaSuccess) {
             std::fclose(f);
-            throw CFail{TDLB_ECUDA, std::string("checkpoint copy: ") + cudaGetErrorString(s)};
+            throw CFail{TDLB_ECUDA, tdlb_rt::error_text("checkpoint copy", s)};
         }
         if (std::fwrite(pin, 1, n, f) != n) {
             std::fclose(f);
@@ -237,7 +237,7 @@ void read_device(const std::string& path, float* dev, size_t bytes, cudaStream_t
         const cudaError_t s = e == cudaSuccess ? cudaStreamSynchronize(st) : e;
         if (s != cudaSuccess) {
             std::fclose(f);
-            throw CFail{TDLB_ECUDA, std::string("checkpoint copy: ") + cudaGetErrorString(s)};
+            throw CFail{TDLB_ECUDA, tdlb_rt::error_text("checkpoint copy", s)};
         }
     }
     std::fclose(f);

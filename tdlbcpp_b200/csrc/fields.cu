@@ -151,7 +151,7 @@ struct FFail {
 #define TDLB_FCK(call)                                                                                      \
     do {                                                                                                    \
         cudaError_t e_ = (call);                                                                            \
-        if (e_ != cudaSuccess) throw FFail{TDLB_ECUDA, std::string(#call) + ": " + cudaGetErrorString(e_)}; \
+        if (e_ != cudaSuccess) throw FFail{TDLB_ECUDA, tdlb_rt::error_text(#call, e_)};                     \
     } while (0)
 
 template <bool INIT = true, typename F>

@@ -215,7 +215,7 @@ struct OFail {
 #define TDLB_OCK(call)                                                                                      \
     do {                                                                                                    \
         cudaError_t e_ = (call);                                                                            \
-        if (e_ != cudaSuccess) throw OFail{TDLB_ECUDA, std::string(#call) + ": " + cudaGetErrorString(e_)}; \
+        if (e_ != cudaSuccess) throw OFail{TDLB_ECUDA, tdlb_rt::error_text(#call, e_)};                     \
     } while (0)
 
 template <typename F>

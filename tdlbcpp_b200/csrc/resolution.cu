@@ -60,7 +60,7 @@ struct RFail {
 #define TDLB_RCK(call)                                                                                      \
     do {                                                                                                    \
         cudaError_t e_ = (call);                                                                            \
-        if (e_ != cudaSuccess) throw RFail{TDLB_ECUDA, std::string(#call) + ": " + cudaGetErrorString(e_)}; \
+        if (e_ != cudaSuccess) throw RFail{TDLB_ECUDA, tdlb_rt::error_text(#call, e_)};                     \
     } while (0)
 
 long long round_up_ll(long long a, long long m) { return (a + m - 1) / m * m; }

@@ -33,7 +33,7 @@ struct Fail {
     do {                                                                                       \
         cudaError_t e_ = (call);                                                               \
         if (e_ != cudaSuccess)                                                                 \
-            throw Fail{TDLB_ECUDA, std::string(#call) + ": " + cudaGetErrorString(e_)};        \
+            throw Fail{TDLB_ECUDA, tdlb_rt::error_text(#call, e_)};                            \
     } while (0)
 
 long long round_up(long long a, long long m) { return (a + m - 1) / m * m; }
@@ -929,7 +929,7 @@ void set_rbox(tdlb_lattice* h, long long i0, long long i1, long long j0, long lo
         cudaError_t e = cudaMalloc(&h->d_res[q], bytes);
         if (e != cudaSuccess) {
             drop_rbox(h);
-            throw Fail{TDLB_ENOMEM, "residual box: " + std::string(cudaGetErrorString(e))};
+            throw Fail{TDLB_ENOMEM, tdlb_rt::error_text("residual box", e)};
         }
         TDLB_CK(cudaMemsetAsync(h->d_res[q], 0, bytes, h->stream));
     }

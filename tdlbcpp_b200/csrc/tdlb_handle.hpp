@@ -222,6 +222,13 @@ inline LatticeBlock lattice_block(const Dims& g, long long mask_words, size_t es
     l.bytes = l.mask + up((size_t)2 * mask_words * sizeof(uint32_t));
     return l;
 }
+// The message of a CUDA call that failed. The runtime also keeps the error for
+// cudaGetLastError, where the next call's launch check would find it: an
+// allocation that failed is told of once.
+inline std::string error_text(const char* call, cudaError_t e) {
+    cudaGetLastError();
+    return std::string(call) + ": " + cudaGetErrorString(e);
+}
 tdlb::StepArgs step_args(tdlb_lattice* h, bool collide);
 tdlb::IbmArgs ibm_args(tdlb_lattice* h, float alpha, float beta);
 // Queue h's work on `s` instead of its own stream (batches share one).

@@ -76,3 +76,18 @@ def test_lists_of_changing_length_stay_in_their_buffers(fake):
         assert not faults(fake), f"after {n} markers on the doubled lattice"
     cu.close()
     assert not faults(fake)
+
+
+@pytest.mark.parametrize("call", [lambda cu: cu.read_moments(), lambda cu: cu.plane_xz(3), lambda cu: cu.reduce_fp64(),
+                                  lambda cu: cu.doubleResolutionFullCU()])
+def test_a_failed_allocation_is_told_of_once(fake, call):
+    """A call without memory for its scratch fails; the same call does not then."""
+    cu = fake.ComputeUnit(x=24, y=24, z=24, nu=1e-3)
+    cu.initialise(1.0)
+    fake.load_library().fake_fail(1)
+    with pytest.raises(fake.TdlbError):
+        call(cu)
+    call(cu)
+    cu.collision()
+    cu.close()
+    assert not faults(fake)
