@@ -665,6 +665,7 @@ void plan_planes(tdlb_lattice* h, const int* count) {
     // 16 elements of padding: the spread's bulk copies and L2 prefetches
     // round a plane's cell range out to 16-byte boundaries
     if (h->ncell + 16 > h->cell_cap || !h->d_cell_e) {
+        h->cell_cap = 0;   // until all three are there
         long long c1 = 0, c2 = 0, c3 = 0;
         grow(h->d_cell_e, c1, h->ncell + 16, 1);
         grow(h->d_cell_m, c2, h->ncell + 16, 4);
@@ -754,7 +755,12 @@ void upload_markers(tdlb_lattice* h, const tdlb_marker* m, size_t n, size_t n0, 
     TDLB_CK(cudaMemcpyAsync(got.data(), a.info, got.size() * sizeof(int), cudaMemcpyDeviceToHost, h->stream));
     TDLB_CK(cudaStreamSynchronize(h->stream));
     if (got[0] < (int)n) validate_markers(g, m + got[0], 1, (size_t)got[0]);   // throws
-    // the list is good: it becomes the resident one
+    // the list is good: it becomes the resident one, and nothing that the handle
+    // knows of the one before (its impeller, plans by generation) is its own,
+    // whether the rest of this succeeds or not
+    h->rot_device = false;
+    h->impeller_begin = -1;
+    h->marker_gen++;
     std::swap(h->d_markers, h->d_markers_in);
     std::swap(h->marker_cap, h->marker_in_cap);
     h->n_markers = (int)n;
@@ -775,6 +781,7 @@ void upload_markers(tdlb_lattice* h, const tdlb_marker* m, size_t n, size_t n0, 
     if (ntail > h->tail_cap) {
         cudaFree(h->d_tail);
         h->d_tail = nullptr;
+        h->tail_cap = 0;
         const long long cap = round_up(ntail, 256);
         TDLB_CK(cudaMalloc(&h->d_tail, (size_t)tdlb::TF_COUNT * cap * sizeof(float)));
         h->tail_cap = cap;
@@ -783,10 +790,8 @@ void upload_markers(tdlb_lattice* h, const tdlb_marker* m, size_t n, size_t n0, 
     if ((long long)n0 > 0) grow(h->d_prep, h->prep_cap, (long long)n0 + 1, tdlb::PF_STRIDE);
     if (!h->d_mask_static) TDLB_CK(cudaMalloc(&h->d_mask_static, (size_t)h->mask_words * sizeof(uint32_t)));
     TDLB_CK(cudaMemsetAsync(h->d_mask_static, 0, (size_t)h->mask_words * sizeof(uint32_t), h->stream));
-    if (!h->d_plane_lv0) {
-        TDLB_CK(cudaMalloc(&h->d_plane_lv0, (size_t)(g.ny + 1) * sizeof(int)));
-        TDLB_CK(cudaMalloc(&h->d_plane_lv1, (size_t)(g.ny + 1) * sizeof(int)));
-    }
+    if (!h->d_plane_lv0) TDLB_CK(cudaMalloc(&h->d_plane_lv0, (size_t)(g.ny + 1) * sizeof(int)));
+    if (!h->d_plane_lv1) TDLB_CK(cudaMalloc(&h->d_plane_lv1, (size_t)(g.ny + 1) * sizeof(int)));
     ensure_level_cap(h, (long long)n0 + 1);   // (never more levels than markers)
     a.markers = h->d_markers;
     a.owner = (int*)h->d_cell_F;
@@ -813,9 +818,6 @@ void upload_markers(tdlb_lattice* h, const tdlb_marker* m, size_t n, size_t n0, 
         TDLB_CK(cudaStreamSynchronize(h->stream));   // the host vectors are read by queued copies
     }
     h->markers_set = true;
-    h->rot_device = false;
-    h->impeller_begin = -1;
-    h->marker_gen++;
 }
 
 tdlb::IbmArgs ibm_args(tdlb_lattice* h, float alpha, float beta) {

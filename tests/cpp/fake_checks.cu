@@ -49,6 +49,11 @@ extern "C" void fake_check(const char* w, void** args) {
             fake_need(w, "mask_static", a.mask_static, 4 * a.g.rows() * a.g.jw);
         }
     }
+    if (name.find("k_rotate_markers") != std::string::npos) {
+        const int n = *(const int*)args[2];
+        fake_need(w, "offsets", *(const double* const*)args[0], 16LL * n);
+        fake_need(w, "markers", *(Marker* const*)args[1], (long long)n * sizeof(Marker));
+    }
     if (name.find("k_ibm_gather<") != std::string::npos || name.find("k_ibm_spread<") != std::string::npos) {
         const IbmArgs& a = *(const IbmArgs*)args[0];
         fake_need(w, "markers", a.markers, (long long)a.n * sizeof(Marker));

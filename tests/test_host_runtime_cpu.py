@@ -91,3 +91,62 @@ def test_a_failed_allocation_is_told_of_once(fake, call):
     cu.collision()
     cu.close()
     assert not faults(fake)
+
+
+def _small_list(tb, cu, dims):
+    cu.forcing(markers(tb, 40, dims), ALPHA, BETA)
+
+
+def _large_list(tb, cu, dims):
+    cu.set_markers(markers(tb, 9000, dims, seed=2))
+
+
+def _attach(tb, cu, dims, **turbine):
+    rt = tb.RushtonTurbine(*dims, tip_speed=0.1, startup_steps=0, **turbine)
+    d = rt.increment(1)
+    cu.attach_rushton(rt, d, 0.0, d)
+
+
+def _attach_small(tb, cu, dims):
+    _attach(tb, cu, dims, impeller_diameter=9.0, blade_height=3.0, n_blades=2)
+
+
+@pytest.mark.parametrize("first", [None, _small_list, _attach_small])
+@pytest.mark.parametrize("grow", [_large_list, _attach])
+def test_an_allocation_that_fails_costs_that_call_alone(fake, first, grow):
+    """Every allocation of a list upload fails in turn: the call says so, and the
+    calls after it -- the impeller's, a list that fits what was there before, then the
+    same list again -- find every buffer in place or say that there is none."""
+    dims = (48, 48, 48)
+    lib = fake.load_library()
+    for nth in range(1, 200):
+        cu = fake.ComputeUnit(x=dims[0], y=dims[1], z=dims[2], nu=1e-3)
+        cu.initialise(1.0)
+        if first:
+            first(fake, cu, dims)
+        lib.fake_fail(nth)
+        try:
+            grow(fake, cu, dims)
+            failed = False
+        except fake.TdlbError:
+            failed = True
+        lib.fake_fail(0)
+        if failed:
+            for call in (lambda: cu.rotate_impeller(0.2, 0.1), lambda: cu.forcing_resident(ALPHA, BETA), cu.impeller_load):
+                try:
+                    call()
+                except fake.TdlbError:
+                    pass
+                assert not faults(fake), f"allocation {nth}"
+            for n in (40, 30):
+                cu.forcing(markers(fake, n, dims), ALPHA, BETA)
+                assert not faults(fake), f"allocation {nth}"
+            grow(fake, cu, dims)
+        cu.forcing_resident(ALPHA, BETA)
+        cu.collision()
+        cu.forcing_resident(ALPHA, BETA)
+        assert not faults(fake), f"allocation {nth}"
+        cu.close()
+        if not failed:
+            break
+    assert nth > 1
