@@ -818,7 +818,7 @@ void run(tdlb_batch_s* b, int steps, float alpha, float beta, bool graph) {
     merge_streams(b);
     finish_tables(b, steps);
     for (tdlb_lattice* h : b->tanks)
-        if (h->markers_set) h->last_beta = beta;   // for tdlb_impeller_load
+        if (h->markers_set) tdlb_rt::note_pass(h, beta);
 }
 
 void release(tdlb_batch_s* b) {

@@ -450,6 +450,8 @@ int tdlb_checkpoint_read(tdlb_handle h, const char* dir, const char* unit_name) 
         tdlb::set_rest(h->cp, c.initialRho);
         h->cur = 0;
         h->pass = 0;
+        h->forced = true;   // by markers that the file does not name
+        h->force_gen = ~0u;
         h->even = even;
         h->holds_moments = true;
         h->initialised = true;

@@ -128,6 +128,7 @@ int tdlb_double_resolution(tdlb_handle h) {
     h->cfg.z *= 2;
     h->cur = 0;
     h->pass = 0;
+    h->forced = false;
     h->holds_moments = true;
     // markers, schedules and every per-plane or per-cell buffer belong to the old size
     h->markers_set = false;

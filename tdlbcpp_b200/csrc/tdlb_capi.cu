@@ -379,6 +379,13 @@ bool zone_known(tdlb_lattice* h) {
     return n1 == 0 || (h->impeller_begin >= 0 && h->h_rot_xz.size() == 2 * n1);
 }
 
+// The zone (when there is one for the resident markers) holds every cell that
+// the last forcing pass touched: F is zero outside it. The markers may have been
+// replaced since that pass, and the pass's blades by others.
+bool force_in_zone(const tdlb_lattice* h) {
+    return !h->forced || (h->force_gen == h->marker_gen && h->force_blades_in);
+}
+
 void build_box_list(tdlb_lattice* h);
 
 void ensure_zone(tdlb_lattice* h, bool all) {
@@ -405,7 +412,7 @@ bool can_split(tdlb_lattice* h) {
     // a captured step stays on the captured stream and its own side stream
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(h->stream, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) return false;
-    return split_capable(h);
+    return split_capable(h) && force_in_zone(h);
 }
 
 // The cells that the box launch of a step takes, by element (none without a
@@ -515,7 +522,7 @@ void run_step(tdlb_lattice* h, bool collide) {
             // the box's cells are left out of the plain launches: the outer
             // words, or none when the zone is not known, then the inner ones
             ensure_zone(h, !zone_known(h));
-            if (!h->zone_ok) ensure_zone(h, true);
+            if (!h->zone_ok || !force_in_zone(h)) ensure_zone(h, true);
             part(1, h->stream);
             box();
             part(2, h->stream);
@@ -875,7 +882,7 @@ void run_forcing(tdlb_lattice* h, float alpha, float beta) {
     h->launches += 1 + (h->n_small > 0 ? 1 : 0) + (h->n_big > 0 ? 1 : 0) +
                    (h->n_blade > 0 && (h->n_big > 0 || h->blade_max > 128) ? 1 : 0);
     h->pass++;
-    h->last_beta = beta;
+    tdlb_rt::note_pass(h, beta);
 }
 
 void host_aos_to_planes(tdlb_lattice* h, const float* in, int npl, float* dev) {
@@ -1051,6 +1058,7 @@ int tdlb_initialise(tdlb_handle h, float rho) {
         h->even = true;
         h->holds_moments = true;
         h->pass = 0;
+        h->forced = false;
         if (h->cfg.storage == TDLB_STORAGE_FP32) {
             TDLB_CK(tdlb::launch_fill_uniform_moments(h->planes(h->bufA), g, rho, h->stream));
         } else {
@@ -1473,6 +1481,14 @@ void drop_residual_box(tdlb_lattice* h) { ::drop_rbox(h); }
 void clear_residual_box(tdlb_lattice* h) { ::clear_rbox(h); }
 tdlb::StepArgs step_args(tdlb_lattice* h, bool collide) { return ::step_args(h, collide); }
 tdlb::IbmArgs ibm_args(tdlb_lattice* h, float alpha, float beta) { return ::ibm_args(h, alpha, beta); }
+void note_pass(tdlb_lattice* h, float beta) {
+    h->last_beta = beta;
+    h->forced = true;
+    h->force_gen = h->marker_gen;
+    // blades that turn on the device stay inside the zone's annuli
+    h->force_blades_in = h->n_markers == h->n0 || h->rot_device ||
+                         (h->zone_gen == h->marker_gen && !h->zone_all && h->zone_ok);
+}
 void borrow_stream(tdlb_lattice* h, cudaStream_t s) {
     fence(h);
     cudaStreamSynchronize(h->stream);

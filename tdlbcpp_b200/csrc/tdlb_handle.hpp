@@ -131,6 +131,10 @@ struct tdlb_lattice {
     int* d_zone_words = nullptr;         // the zone's words, ascending
     long long zone_cap = 0;              // words the arrays hold
     int n_zone = 0, n_outer = 0;         // words inside, outside
+    // the last forcing pass, which F and the current flags are of
+    bool forced = false;          // there was one since F was last zero everywhere
+    unsigned force_gen = ~0u;     // marker_gen of its list (~0: not known)
+    bool force_blades_in = false; // its blades lay inside the zone of that list
     std::vector<uint8_t> h_zone_skip;
     std::vector<uint32_t> h_zone_core;   // filled when host blades are checked against it
     // 16-bit storage: the residual box (tdlb::ResidualBox) and its residuals,
@@ -239,6 +243,8 @@ void return_stream(tdlb_lattice* h);
 // next outer launch of a split step waits for it (every entry point other than
 // the step loop's calls it).
 inline void fence(tdlb_lattice* h) { h->bulk_ok = false; }
+// A forcing pass of the resident markers has been queued.
+void note_pass(tdlb_lattice* h, float beta);
 // The handle's device scratch, at least `bytes` long (kept for the next call).
 cudaError_t scratch(tdlb_lattice* h, size_t bytes, char** out);
 // Free the zone's arrays (the lattice changed size).

@@ -1,8 +1,9 @@
 // What the launches of the CPU tests' CUDA runtime (fake_cuda.cpp) are held
 // against: the buffers that the marker scheduler's and the forcing pass's
-// arguments name. k_sched_cells counts the planes' stencil cells, so that the
-// host goes on as with a GPU.
+// arguments name. k_sched_cells counts the planes' stencil cells and k_zone_core
+// marks the blades' annuli, so that the host goes on as with a GPU.
 #include <algorithm>
+#include <cmath>
 #include <set>
 #include <string>
 #include <vector>
@@ -48,6 +49,20 @@ extern "C" void fake_check(const char* w, void** args) {
             fake_need(w, "plane_lv1", a.plane_lv1, 4LL * (a.g.ny + 1));
             fake_need(w, "mask_static", a.mask_static, 4 * a.g.rows() * a.g.jw);
         }
+    }
+    if (name.find("k_zone_core") != std::string::npos && *(const double2* const*)args[2]) {
+        const Dims& g = *(const Dims*)args[0];
+        const double2* ring = *(const double2* const*)args[2];
+        const double ci = *(const double*)args[3], ck = *(const double*)args[4];
+        uint32_t* core = *(uint32_t* const*)args[5];
+        fake_need(w, "core", core, 4 * g.rows() * g.jw);
+        fake_need(w, "ring", ring, 16LL * g.ny);
+        for (int i = 0; i < g.nx && fake_sound(); i++)
+            for (int k = 0; k < g.nz; k++)
+                for (int j = 0; j < g.ny; j++) {
+                    const double d = std::sqrt((i - ci) * (i - ci) + (k - ck) * (k - ck));
+                    if (ring[j].y >= 0.0 && d >= ring[j].x && d <= ring[j].y) core[g.word(i, j, k)] |= 1u << (j & 31);
+                }
     }
     if (name.find("k_rotate_markers") != std::string::npos) {
         const int n = *(const int*)args[2];

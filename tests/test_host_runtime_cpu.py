@@ -150,3 +150,60 @@ def test_an_allocation_that_fails_costs_that_call_alone(fake, first, grow):
         if not failed:
             break
     assert nth > 1
+
+
+def _ball(tb, at):
+    m = np.zeros(27, tb.MARKER_DTYPE)
+    for q, name in enumerate("ijk"):
+        m[name] = at[q] + 3 * (np.arange(27) // 3 ** q % 3)
+    return m
+
+
+def test_steps_read_the_force_of_the_list_that_was_applied(fake):
+    """The outer launch of a split step reads no force: it is only queued when the
+    last forcing pass applied the list whose zone it leaves out."""
+    lib = fake.load_library()
+
+    def outer(step):
+        n = lib.fake_launches(b"k_step_simple<float, 1, false, false, true, 1>")
+        step()
+        return lib.fake_launches(b"k_step_simple<float, 1, false, false, true, 1>") - n
+
+    cu = fake.ComputeUnit(x=96, y=96, z=96, nu=1e-3)
+    cu.initialise(1.0)
+    force = lambda: cu.forcing_resident(ALPHA, BETA)  # noqa: E731
+    cu.set_markers(_ball(fake, (20, 30, 40)))
+    force()
+    cu.collision()                       # from moments
+    force()
+    cu.collision()
+    force()
+    assert outer(cu.collision) == 1
+    force()
+    cu.set_markers(_ball(fake, (60, 30, 40)))
+    assert outer(cu.collision) == 0      # the first ball's force
+    force()
+    cu.collision()
+    force()
+    assert outer(cu.collision) == 1
+    cu.forcing(_ball(fake, (10, 70, 10)), ALPHA, BETA)
+    _attach(fake, cu, (96, 96, 96))
+    assert outer(cu.collision) == 0      # the last ball's force
+    for _ in range(2):
+        force()
+        cu.collision()
+    force()
+    assert outer(cu.collision) == 1
+    # blades outside the impeller's swept volume, then inside again
+    rt = fake.RushtonTurbine(96, 96, 96, tip_speed=0.1, startup_steps=0)
+    inside = rt.rotating(0.1, rt.increment(1))
+    outside = inside.copy()
+    outside["i"] = (outside["i"] + 30) % 96
+    for blades, split in ((inside, 1), (outside, 1), (inside, 0), (inside, 1), (inside, 1)):
+        force()
+        cu.set_rotating_markers(blades)
+        n = outer(cu.collision)
+        assert n <= split, "the force of blades outside the zone"
+    assert n == 1
+    cu.close()
+    assert not faults(fake)
