@@ -144,6 +144,13 @@ def make_unit(tb, workload: str, edge: int, device: int, storage: str = "fp32"):
     return cu, rt, nu
 
 
+def split_large(cu, always=False):
+    """Split steps where the library has them by default, on a unit whose stream
+    the bench takes (which ends the default): it only records events there."""
+    if always or cu.ncell >= 1 << 19:
+        cu.set_overlap(True)
+
+
 def run_ours(args, rank, world, device):
     import torch
     import tdlbcpp_b200 as tb
@@ -168,15 +175,14 @@ def run_ours(args, rank, world, device):
         cu.collision()
         cu.forcing_resident(ALPHA, BETA)
 
-    if args.overlap:
-        cu.set_overlap(True)
+    split_large(cu, args.overlap)
     for _ in range(args.warmup):
         device_step()
     cu.synchronize()
     try:
-        zone = cu.read_zone() if args.overlap else None
+        zone = cu.read_zone()
     except tb.TdlbError:
-        zone = None   # the zone covers most of this lattice: steps are not split
+        zone = None   # a small lattice, or the zone covers most of it: steps are not split
 
     # ---- value: device-resident steps; t1 follows a join of the unit's streams.
     t0, t1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
@@ -303,8 +309,7 @@ def run_ours(args, rank, world, device):
         "mass_drift_end": float(red[0] / cells - 1.0),
         "launches": launches,
         "step_launches": launches_per_step,
-        # (the library splits the steps of lattices from 2^19 cells by itself)
-        "split_on": zone is not None if args.overlap else cells >= 1 << 19,
+        "split_on": zone is not None,
         "inner_fraction": None if zone is None else float(zone.mean()),
     }
     return result
@@ -424,6 +429,7 @@ def run_batched(args, rank, world, device):
         cu = tb.ComputeUnit(device=device, **cfg)
         prepare_tank(cu, rt)
         st = torch.cuda.ExternalStream(cu.stream, device=device)
+        split_large(cu)
         angle, s = rt.increment(1), 1
 
         def plain_step():
@@ -491,6 +497,7 @@ def gpu_precision_run(tb, edge, storage, steps, device, timed=False):
     cu.forcing_resident(ALPHA, BETA)
     mass0 = cu.reduce_fp64()[0]
     st = torch.cuda.ExternalStream(cu.stream, device=device)
+    split_large(cu)
     t0, t1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
     angle = d1
     cu.synchronize()

@@ -301,14 +301,19 @@ int tdlb_get_residual_box(tdlb_handle h, int64_t* box6);
  * bit-identical with and without. mode 0: off; 1: on when the inner words
  * hold at most 60 % of the lattice; 2: on whenever possible. Until this is
  * called, as 1 for lattices of at least 2^19 cells (below, the second launch
- * costs more than it hides). FP32 storage needs one cell per thread; a step
+ * costs more than it hides), until the caller takes the handle's stream
+ * (tdlb_get_stream). FP32 storage needs one cell per thread; a step
  * under stream capture is never split. The handle's stream waits for the
  * outer launch at the end of each step, so work queued there afterwards sees
- * the whole step. */
+ * the whole step. The other way round the outer launch of a step waits for
+ * the previous step's inner cells, not for the stream: with modes 1 and 2, call
+ * tdlb_join before queuing work of your own there that the next step must come
+ * after (a replayed graph of steps, a wait for an event). */
 int tdlb_set_overlap(tdlb_handle h, int mode);
 
 /* Order the handle's stream (tdlb_get_stream) after every queued step and
- * forcing pass, without waiting on the host. */
+ * forcing pass, and the next step after everything queued on that stream by
+ * then, without waiting on the host. */
 int tdlb_join(tdlb_handle h);
 
 /* Per-cell flags (interior cells in (i, j, k) order) of the split-step zone:
@@ -328,7 +333,10 @@ int tdlb_kernel_launches(tdlb_handle h, int64_t* n);
 int tdlb_kernel_time(tdlb_handle h, double* total_ms, int64_t* launches);
 
 /* The cudaStream_t (as void*) all of h's device work is queued on, for
- * callers that time it with CUDA events or order their own work after it. */
+ * callers that time it with CUDA events or order their own work after it, or
+ * before it. Steps do not split unasked from then on; a caller that only
+ * records events, or calls tdlb_join where that is needed, turns split steps on
+ * (tdlb_set_overlap). */
 int tdlb_get_stream(tdlb_handle h, void** stream);
 
 /* ---- Rushton-turbine geometry (host only; no GPU needed) ----

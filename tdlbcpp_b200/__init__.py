@@ -482,7 +482,7 @@ class ComputeUnit:
     def set_overlap(self, mode):
         """Split steps: the outer cells of a step run while the forcing pass is
         in flight; results are identical. Without a call the library splits
-        the steps of a large lattice. False/0: off; True/1: when the inner
+        the steps of a large lattice, until `stream` is read. False/0: off; True/1: when the inner
         words hold at most 60 % of the lattice; "always"/2: whenever the
         markers are resident."""
         m = 2 if mode == "always" else int(bool(mode)) if isinstance(mode, bool) else int(mode)
@@ -527,6 +527,8 @@ class ComputeUnit:
 
     @property
     def stream(self) -> int:
+        """The cudaStream_t of this unit's work. Its steps do not split unasked
+        from then on (set_overlap; join() before work that a step must follow)."""
         s = ctypes.c_void_p()
         self._check(self.lib.tdlb_get_stream(self.h, ctypes.byref(s)))
         return s.value or 0
@@ -705,6 +707,8 @@ class Batch:
         return n.value
 
     def stream(self) -> int:
+        """The cudaStream_t of this unit's work. Its steps do not split unasked
+        from then on (set_overlap; join() before work that a step must follow)."""
         s = ctypes.c_void_p()
         self._check(self.lib.tdlb_batch_get_stream(self.h, ctypes.byref(s)))
         return s.value or 0

@@ -273,7 +273,10 @@ tdlb::StepArgs step_args(tdlb_lattice* h, bool collide) {
 // cell, and every cell computes exactly what the unsplit step computes. With
 // rows along j the zone of a stirred tank is whole rows (3 to 5 % of a 400^3
 // tank), so the outer launch is the full launch in all but the rows it drops,
-// and a step takes as long as the longer of the two streams.
+// and a step takes as long as the longer of the two streams. The outer launch
+// follows the inner words of the step before it, not all of `stream`: what a
+// caller queues there is not waited for, unless a call that fences (tdlb_join)
+// comes first.
 // ---------------------------------------------------------------------------
 
 // Every stencil cell of markers [0, n) is set in `core`.
@@ -400,7 +403,7 @@ constexpr long long kAutoSplitCells = 1 << 19;
 // The lattice's steps can run split.
 bool split_capable(tdlb_lattice* h) {
     if (!h->overlap || h->own_stream || !zone_known(h)) return false;
-    if (h->overlap < 0 && h->g.cells() < kAutoSplitCells) return false;
+    if (h->overlap < 0 && (h->stream_taken || h->g.cells() < kAutoSplitCells)) return false;
     if (h->cfg.storage == TDLB_STORAGE_FP32 && tdlb::vector_width(h->g, h->vec) != 1) return false;
     ensure_zone(h, false);
     // a zone covering most of the lattice leaves little to overlap with
@@ -1217,6 +1220,7 @@ int tdlb_get_stream(tdlb_handle h, void** stream) {
     return guarded<false>(h, [&] {
         if (!stream) throw Fail{TDLB_EINVAL, "out is NULL"};
         *stream = (void*)h->stream;
+        if (!h->own_stream) h->stream_taken = true;
     });
 }
 

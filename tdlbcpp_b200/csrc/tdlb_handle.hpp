@@ -119,6 +119,8 @@ struct tdlb_lattice {
                                   // -1: as 1, for lattices large enough
     bool bulk_ok = false;         // nothing but step-loop work queued since ev_inner: the next outer
                                   // launch waits for that event alone
+    bool stream_taken = false;    // the caller has the stream (tdlb_get_stream) and may queue work there that the
+                                  // next step has to follow: no step splits unasked from then on
     bool resident = false;        // markers kept for many passes (set/attach), so a zone pays
     // the zone (zone.cu), for marker_gen zone_gen and box_gen zone_box_gen
     unsigned zone_gen = ~0u, zone_box_gen = ~0u;

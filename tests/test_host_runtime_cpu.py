@@ -207,3 +207,34 @@ def test_steps_read_the_force_of_the_list_that_was_applied(fake):
     assert n == 1
     cu.close()
     assert not faults(fake)
+
+
+@pytest.mark.parametrize("overlap", [None, True, "always"])
+def test_a_step_follows_what_the_caller_queued_on_the_stream(fake, overlap):
+    """Every launch of a step comes after the caller's own work on the handle's
+    stream (a replayed graph): by itself, or after join() where split steps
+    were asked for."""
+    lib = fake.load_library()
+    cu = fake.ComputeUnit(x=96, y=96, z=96, nu=1e-3, streaming="Esotwist")
+    if overlap is not None:
+        cu.set_overlap(overlap)
+    cu.initialise(1.0)
+    cu.set_markers(_ball(fake, (20, 30, 40)))
+    cu.forcing_resident(ALPHA, BETA)
+    for _ in range(4):
+        cu.step(ALPHA, BETA)
+    assert lib.fake_launches(b"k_step_esotwist<float, 1, false, false, true, true, 1>") > 0
+    stream = cu.stream
+    for _ in range(4):
+        if overlap is not None:
+            cu.join()
+        number = lib.fake_foreign(stream)
+        n = lib.fake_unordered(b"k_step_", stream, number)
+        cu.step(ALPHA, BETA)
+        assert lib.fake_unordered(b"k_step_", stream, number) == n, "a step launch runs beside the caller's work"
+    if overlap is not None:
+        before = lib.fake_launches(b"true, 1>")
+        cu.step(ALPHA, BETA)
+        assert lib.fake_launches(b"true, 1>") == before + 1, "asked for, steps stay split"
+    cu.close()
+    assert not faults(fake)
