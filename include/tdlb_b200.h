@@ -99,8 +99,9 @@ int tdlb_config_from_json(const char* params_json, tdlb_config* out);
 /* Same, from a filled tdlb_config (nu used as given). */
 int tdlb_create_config(const tdlb_config* cfg, int device, tdlb_handle* out);
 
-/* Device bytes a lattice of this config takes (fields, flags, and the marker
- * buffers of a tank-wall geometry; an upper estimate). No counterpart in the
+/* Device bytes a lattice of this config takes (fields, flags, the split steps'
+ * zone, and the marker buffers of a tank-wall geometry; an upper estimate). A
+ * field read also keeps up to 32 MiB of scratch. No counterpart in the
  * reference (its checkEnoughMemory only compares, ComputeUnitGpu.hpp:15-30). */
 int tdlb_lattice_bytes(const tdlb_config* cfg, int64_t* bytes);
 

@@ -234,6 +234,9 @@ void build(tdlb_server_s* s, const Pending& p, long long need) {
     tdlb_handle h = nullptr;
     int rc = tdlb_create_config(&c, s->device, &h);
     const double d1 = tdlb_rushton_impeller_increment(&spec, 1);
+    // (a batch steps it: no split steps and no residual box to plan)
+    if (rc == TDLB_OK) rc = tdlb_set_overlap(h, 0);
+    if (rc == TDLB_OK) rc = tdlb_set_residual_box(h, 0, 0, 0, 0, 0, 0);
     if (rc == TDLB_OK) rc = tdlb_attach_rushton(h, &spec, d1, d1, d1);
     if (rc == TDLB_OK) rc = tdlb_initialise(h, 1.0f);
     if (rc == TDLB_OK) rc = tdlb_forcing_resident(h, s->alpha, s->beta);

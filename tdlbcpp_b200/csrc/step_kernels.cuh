@@ -188,7 +188,8 @@ __device__ __forceinline__ Quad part_quad(const Dims& g, const StepPart& part, u
     } else {
         constexpr unsigned SEG = 32 / V;
         const unsigned lw = t / SEG;
-        const int wd = __ldg(part.words + min(lw, (unsigned)part.count - 1u));
+        const unsigned in = min(lw, (unsigned)part.count - 1u);
+        const int wd = part.words ? __ldg(part.words + in) : (int)in;
         const unsigned ex = part.except ? __ldg(part.except + wd) : 0u;
         Quad q;
         q.row = wd / g.jw;

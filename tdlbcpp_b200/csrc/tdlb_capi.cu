@@ -68,6 +68,7 @@ void release(tdlb_lattice* h) {
     cudaFree(h->d_exclude);
     tdlb_rt::drop_zone(h);
     cudaFree(h->d_box_list);
+    cudaFree(h->d_box_except);
     cudaFree(h->d_scratch);
     for (cudaEvent_t e : h->tev) cudaEventDestroy(e);
     if (h->side) cudaStreamDestroy(h->side);
@@ -304,23 +305,14 @@ bool blades_in_zone(tdlb_lattice* h) {
     return stencils_inside(h->g, h->h_blades.data(), n1, h->h_zone_core);
 }
 
-// `all`: every word, whatever the markers (they change with every pass).
-void build_zone(tdlb_lattice* h, bool all) {
+void build_zone(tdlb_lattice* h) {
     TDLB_CK(cudaStreamSynchronize(h->stream));   // no launch still reads the old zone
     const Dims& g = h->g;
     const long long nw = g.rows() * g.jw;
-    const bool boxed = h->rbox_geom.n > 0;
-    if (h->zone_cap < nw) {
-        tdlb_rt::drop_zone(h);
-        TDLB_CK(cudaMalloc(&h->d_zone_core, (size_t)nw * sizeof(uint32_t)));
-        TDLB_CK(cudaMalloc(&h->d_zone_skip, (size_t)nw));
-        TDLB_CK(cudaMalloc(&h->d_zone_words, (size_t)nw * sizeof(int)));
-        h->zone_cap = nw;
-    }
+    h->zone_gen = ~0u;
     h->h_zone_core.clear();
-    double2* d_ring = nullptr;
     const int n1 = h->n_markers - h->n0;
-    if (!all && n1 > 0) {
+    if (n1 > 0) {
         // Blades turn about (ci, ck). A blade marker at radius r rounds to the
         // nearest cell, and its stencil cells lie within 1.5 cells of that
         // position per axis, so within r +- 2.13 of the axis: plane by plane,
@@ -334,29 +326,15 @@ void build_zone(tdlb_lattice* h, bool all) {
             p.x = std::min(p.x, r - 3.0);
             p.y = std::max(p.y, r + 3.0);
         }
-        TDLB_CK(cudaMalloc(&d_ring, ring.size() * sizeof(double2)));
-        const cudaError_t e = cudaMemcpy(d_ring, ring.data(), ring.size() * sizeof(double2), cudaMemcpyHostToDevice);
-        if (e != cudaSuccess) {
-            cudaFree(d_ring);
-            TDLB_CK(e);
-        }
+        TDLB_CK(cudaMemcpy(h->d_zone_ring, ring.data(), ring.size() * sizeof(double2), cudaMemcpyHostToDevice));
     }
-    cudaError_t e = cudaSuccess;
-    if (!all) e = tdlb::launch_zone_core(g, h->d_mask_static, d_ring, h->rot_ci, h->rot_ck, h->d_zone_core, h->stream);
-    if (e == cudaSuccess)
-        e = tdlb::launch_zone_words(g, all ? nullptr : h->d_zone_core, h->cfg.streaming == TDLB_STREAMING_ESOTWIST,
-                                    h->d_zone_skip, h->stream);
-    if (e == cudaSuccess && boxed) {
-        if (!h->d_zone_except) e = cudaMalloc(&h->d_zone_except, (size_t)h->zone_cap * sizeof(uint32_t));
-        if (e == cudaSuccess) e = cudaMemsetAsync(h->d_zone_except, 0, (size_t)nw * sizeof(uint32_t), h->stream);
-        if (e == cudaSuccess) e = tdlb::launch_zone_box(g, h->d_box_list, h->n_box, h->d_zone_except, h->d_zone_skip, h->stream);
-    }
+    TDLB_CK(tdlb::launch_zone_core(g, h->d_mask_static, n1 > 0 ? h->d_zone_ring : nullptr, h->rot_ci, h->rot_ck, h->d_zone_core,
+                                   h->stream));
+    TDLB_CK(tdlb::launch_zone_words(g, h->d_zone_core, h->cfg.streaming == TDLB_STREAMING_ESOTWIST, h->d_zone_skip, h->stream));
+    TDLB_CK(tdlb::launch_zone_box(g, h->d_box_list, h->n_box, nullptr, h->d_zone_skip, h->stream));
     h->h_zone_skip.resize((size_t)nw);
-    if (e == cudaSuccess)
-        e = cudaMemcpyAsync(h->h_zone_skip.data(), h->d_zone_skip, (size_t)nw, cudaMemcpyDeviceToHost, h->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
-    cudaFree(d_ring);
-    TDLB_CK(e);
+    TDLB_CK(cudaMemcpyAsync(h->h_zone_skip.data(), h->d_zone_skip, (size_t)nw, cudaMemcpyDeviceToHost, h->stream));
+    TDLB_CK(cudaStreamSynchronize(h->stream));
     std::vector<int> words;
     long long inner_cells = 0;
     for (long long w = 0; w < nw; w++)
@@ -369,15 +347,14 @@ void build_zone(tdlb_lattice* h, bool all) {
     h->n_zone = (int)words.size();
     h->n_outer = (int)(nw - h->n_zone);
     h->zone_small = (double)inner_cells <= 0.6 * (double)g.cells();
-    h->zone_all = all;
+    h->zone_ok = blades_in_zone(h);
     h->zone_gen = h->marker_gen;
     h->zone_box_gen = h->box_gen;
-    h->zone_ok = all || blades_in_zone(h);
 }
 
 // The zone of the resident markers can be built.
 bool zone_known(tdlb_lattice* h) {
-    if (!h->markers_set || !h->resident) return false;
+    if (!h->markers_set || !h->resident || !h->zone_block) return false;
     const size_t n1 = (size_t)(h->n_markers - h->n0);
     return n1 == 0 || (h->impeller_begin >= 0 && h->h_rot_xz.size() == 2 * n1);
 }
@@ -389,25 +366,28 @@ bool force_in_zone(const tdlb_lattice* h) {
     return !h->forced || (h->force_gen == h->marker_gen && h->force_blades_in);
 }
 
-void build_box_list(tdlb_lattice* h);
-
-void ensure_zone(tdlb_lattice* h, bool all) {
-    build_box_list(h);
-    if (h->zone_gen != h->marker_gen || h->zone_box_gen != h->box_gen || h->zone_all != all || !h->d_zone_skip)
-        build_zone(h, all);
+// The zone, built where the resident markers' is not there yet, holds every
+// stencil cell of theirs.
+bool zone_holds_markers(tdlb_lattice* h) {
+    if (!zone_known(h)) return false;
+    if (h->zone_gen != h->marker_gen || h->zone_box_gen != h->box_gen) build_zone(h);
+    return h->zone_ok;
 }
 
 // Smallest lattice whose steps split unasked.
 constexpr long long kAutoSplitCells = 1 << 19;
 
-// The lattice's steps can run split.
-bool split_capable(tdlb_lattice* h) {
-    if (!h->overlap || h->own_stream || !zone_known(h)) return false;
+// The lattice's steps may run split, whatever its markers.
+bool split_wanted(const tdlb_lattice* h) {
+    if (!h->overlap || h->own_stream) return false;
     if (h->overlap < 0 && (h->stream_taken || h->g.cells() < kAutoSplitCells)) return false;
-    if (h->cfg.storage == TDLB_STORAGE_FP32 && tdlb::vector_width(h->g, h->vec) != 1) return false;
-    ensure_zone(h, false);
-    // a zone covering most of the lattice leaves little to overlap with
-    return h->zone_ok && (h->zone_small || h->overlap == 2);
+    return h->cfg.storage != TDLB_STORAGE_FP32 || tdlb::vector_width(h->g, h->vec) == 1;
+}
+
+// The lattice's steps can run split. (A zone covering most of the lattice leaves
+// little to overlap with.)
+bool split_capable(tdlb_lattice* h) {
+    return split_wanted(h) && zone_holds_markers(h) && (h->zone_small || h->overlap == 2);
 }
 
 bool can_split(tdlb_lattice* h) {
@@ -416,54 +396,6 @@ bool can_split(tdlb_lattice* h) {
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(h->stream, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) return false;
     return split_capable(h) && force_in_zone(h);
-}
-
-// The cells that the box launch of a step takes, by element (none without a
-// box). Which cells these are is part of the results: the box launch's
-// scalar arithmetic and the plain kernel's packed one differ
-// by FP32 ulps, which 16-bit storage then rounds. They are the cells of every
-// group of 32 along k (groups counted through the lines of constant (i, j),
-// lines padded to 16 cells) that holds a cell near the box.
-void build_box_list(tdlb_lattice* h) {
-    if (h->box_list_gen == h->box_gen) return;
-    TDLB_CK(cudaStreamSynchronize(h->stream));   // no launch still reads the old list
-    const Dims& g = h->g;
-    const tdlb::ResidualBox& b = h->rbox_geom;
-    if (b.n == 0) {
-        h->n_box = 0;
-        h->box_list_gen = h->box_gen;
-        return;
-    }
-    const long long line = round_up(g.nz, 16), ngroups = ((long long)g.nx * g.ny * line + 31) / 32;
-    std::vector<uint8_t> hit((size_t)ngroups, 0);
-    for (int i = std::max(0, b.i0 - 1); i <= std::min(g.nx - 1, b.i0 + b.bx); i++)
-        for (int j = std::max(0, b.j0 - 1); j <= std::min(g.ny - 1, b.j0 + b.by); j++)
-            for (int k = std::max(0, b.k0 - 1); k <= std::min(g.nz - 1, b.k0 + b.bz); k++)
-                if (b.around(i, j, k)) hit[(size_t)((((long long)i * g.ny + j) * line + k) >> 5)] = 1;
-    std::vector<int> list;
-    // in element order; a group may reach into the lines before and after
-    int j0 = b.j0 - 2, j1 = b.j0 + b.by + 2;
-    if (j0 < 0 || j1 > g.ny) {
-        j0 = 0;
-        j1 = g.ny;
-    }
-    for (int i = std::max(0, b.i0 - 2); i < std::min(g.nx, b.i0 + b.bx + 2); i++)
-        for (int k = 0; k < g.nz; k++)
-            for (int j = j0; j < j1; j++)
-                if (hit[(size_t)((((long long)i * g.ny + j) * line + k) >> 5)]) list.push_back((int)g.at(i, j, k));
-    if ((long long)list.size() > h->box_list_cap || !h->d_box_list) {
-        cudaFree(h->d_box_list);
-        h->d_box_list = nullptr;
-        h->box_list_cap = 0;
-        const size_t cap = std::max<size_t>(list.size(), 1);
-        TDLB_CK(cudaMalloc(&h->d_box_list, cap * sizeof(int)));
-        h->box_list_cap = (long long)cap;
-    }
-    if (!list.empty())
-        TDLB_CK(cudaMemcpyAsync(h->d_box_list, list.data(), list.size() * sizeof(int), cudaMemcpyHostToDevice, h->stream));
-    TDLB_CK(cudaStreamSynchronize(h->stream));
-    h->n_box = (int)list.size();
-    h->box_list_gen = h->box_gen;
 }
 
 // Queue one step-kernel launch, bracketed by timing events when enabled.
@@ -495,14 +427,15 @@ void run_step(tdlb_lattice* h, bool collide) {
     };
     const bool boxed = a.rr.on();
     const bool split = collide && can_split(h);
-    auto part = [&](int which, cudaStream_t st) {   // 1: outer words, 2: inner words without the box's cells
+    // 1: outer words, 2: inner words (or every word) without the box's cells
+    auto part = [&](int which, cudaStream_t st, bool every = false) {
         tdlb::StepArgs x = a;
         x.part = which;
         x.zone.skip = h->d_zone_skip;
-        x.zone.words = h->d_zone_words;
-        x.zone.count = h->n_zone;
-        x.zone.except = boxed ? h->d_zone_except : nullptr;
-        if ((which == 1 ? h->n_outer : h->n_zone) > 0) timed_launch(h, st, [&] { return launch(x, st); });
+        x.zone.words = every ? nullptr : h->d_zone_words;
+        x.zone.count = every ? (int)(h->g.rows() * h->g.jw) : h->n_zone;
+        x.zone.except = boxed ? h->d_box_except : nullptr;
+        if ((which == 1 ? h->n_outer : x.zone.count) > 0) timed_launch(h, st, [&] { return launch(x, st); });
     };
     auto box = [&] {
         a.box_cells = h->d_box_list;
@@ -523,12 +456,11 @@ void run_step(tdlb_lattice* h, bool collide) {
         tdlb_rt::fence(h);
         if (boxed) {
             // the box's cells are left out of the plain launches: the outer
-            // words, or none when the zone is not known, then the inner ones
-            ensure_zone(h, !zone_known(h));
-            if (!h->zone_ok || !force_in_zone(h)) ensure_zone(h, true);
-            part(1, h->stream);
+            // words and the inner ones, or one over every word without a zone
+            const bool zone = zone_holds_markers(h) && force_in_zone(h);
+            if (zone) part(1, h->stream);
             box();
-            part(2, h->stream);
+            part(2, h->stream, !zone);
         } else {
             timed_launch(h, h->stream, [&] { return launch(a, h->stream); });
         }
@@ -802,7 +734,7 @@ void upload_markers(tdlb_lattice* h, const tdlb_marker* m, size_t n, size_t n0, 
     TDLB_CK(cudaMemsetAsync(h->d_mask_static, 0, (size_t)h->mask_words * sizeof(uint32_t), h->stream));
     if (!h->d_plane_lv0) TDLB_CK(cudaMalloc(&h->d_plane_lv0, (size_t)(g.ny + 1) * sizeof(int)));
     if (!h->d_plane_lv1) TDLB_CK(cudaMalloc(&h->d_plane_lv1, (size_t)(g.ny + 1) * sizeof(int)));
-    ensure_level_cap(h, (long long)n0 + 1);   // (never more levels than markers)
+    ensure_level_cap(h, (long long)n + 1);   // (never more levels than markers)
     a.markers = h->d_markers;
     a.owner = (int*)h->d_cell_F;
     a.plane_cell = h->d_plane_cell;
@@ -910,8 +842,50 @@ void drop_rbox(tdlb_lattice* h) {
     cudaFree(h->d_res[0]);
     cudaFree(h->d_res[1]);
     h->d_res[0] = h->d_res[1] = nullptr;
+    cudaFree(h->d_box_list);
+    cudaFree(h->d_box_except);
+    h->d_box_list = nullptr;
+    h->d_box_except = nullptr;
+    h->n_box = 0;
     h->rbox_geom = tdlb::ResidualBox{};
     h->box_gen++;
+}
+
+// The cells that the box launch of a step takes, by element, and their bits.
+// Which cells these are is part of the results: the box launch's
+// scalar arithmetic and the plain kernel's packed one differ
+// by FP32 ulps, which 16-bit storage then rounds. They are the cells of every
+// group of 32 along k (groups counted through the lines of constant (i, j),
+// lines padded to 16 cells) that holds a cell near the box.
+void build_box_list(tdlb_lattice* h) {
+    const Dims& g = h->g;
+    const tdlb::ResidualBox& b = h->rbox_geom;
+    const long long line = round_up(g.nz, 16), ngroups = ((long long)g.nx * g.ny * line + 31) / 32;
+    std::vector<uint8_t> hit((size_t)ngroups, 0);
+    for (int i = std::max(0, b.i0 - 1); i <= std::min(g.nx - 1, b.i0 + b.bx); i++)
+        for (int j = std::max(0, b.j0 - 1); j <= std::min(g.ny - 1, b.j0 + b.by); j++)
+            for (int k = std::max(0, b.k0 - 1); k <= std::min(g.nz - 1, b.k0 + b.bz); k++)
+                if (b.around(i, j, k)) hit[(size_t)((((long long)i * g.ny + j) * line + k) >> 5)] = 1;
+    std::vector<int> list;
+    // in element order; a group may reach into the lines before and after
+    int j0 = b.j0 - 2, j1 = b.j0 + b.by + 2;
+    if (j0 < 0 || j1 > g.ny) {
+        j0 = 0;
+        j1 = g.ny;
+    }
+    for (int i = std::max(0, b.i0 - 2); i < std::min(g.nx, b.i0 + b.bx + 2); i++)
+        for (int k = 0; k < g.nz; k++)
+            for (int j = j0; j < j1; j++)
+                if (hit[(size_t)((((long long)i * g.ny + j) * line + k) >> 5)]) list.push_back((int)g.at(i, j, k));
+    const size_t n = std::max<size_t>(list.size(), 1) * sizeof(int), bits = (size_t)(g.rows() * g.jw) * sizeof(uint32_t);
+    TDLB_CK(cudaMalloc(&h->d_box_list, n));
+    TDLB_CK(cudaMalloc(&h->d_box_except, bits));
+    if (!list.empty())
+        TDLB_CK(cudaMemcpyAsync(h->d_box_list, list.data(), list.size() * sizeof(int), cudaMemcpyHostToDevice, h->stream));
+    TDLB_CK(cudaMemsetAsync(h->d_box_except, 0, bits, h->stream));
+    TDLB_CK(tdlb::launch_zone_box(g, h->d_box_list, (int)list.size(), h->d_box_except, nullptr, h->stream));
+    TDLB_CK(cudaStreamSynchronize(h->stream));
+    h->n_box = (int)list.size();
 }
 
 // The box [i0, i1) x [j0, j1) x [k0, k1); an empty one removes the box. The
@@ -930,7 +904,7 @@ void set_rbox(tdlb_lattice* h, long long i0, long long i1, long long j0, long lo
     // lattice (index 0) then never lies in the box
     if (i0 < 1 || j0 < 1 || k0 < 1 || i1 > g.nx || j1 > g.ny || k1 > g.nz)
         throw Fail{TDLB_EINVAL, "the residual box must lie within [1, x) x [1, y) x [1, z)"};
-    drop_rbox(h);
+    drop_rbox(h);   // (the frees wait for the launches that read the old one)
     tdlb::ResidualBox b;
     b.i0 = (int)i0; b.j0 = (int)j0; b.k0 = (int)k0;
     b.bx = (int)(i1 - i0); b.by = (int)(j1 - j0); b.bz = (int)(k1 - k0);
@@ -946,7 +920,14 @@ void set_rbox(tdlb_lattice* h, long long i0, long long i1, long long j0, long lo
         TDLB_CK(cudaMemsetAsync(h->d_res[q], 0, bytes, h->stream));
     }
     h->rbox_geom = b;
+    try {
+        build_box_list(h);
+    } catch (...) {
+        drop_rbox(h);
+        throw;
+    }
     h->box_gen++;
+    tdlb_rt::reserve_zone(h);
 }
 
 // Residuals back to zero, after anything wrote the 16-bit planes without
@@ -1038,10 +1019,11 @@ int tdlb_lattice_bytes(const tdlb_config* c, int64_t* bytes) {
     const long long mask_words = round_up(c->x * c->z * jw, 64);
     const long long esz = c->storage == TDLB_STORAGE_FP32 ? 4 : 2;
     const long long pops = (long long)tdlb::NQ * plane * esz * (c->streaming == TDLB_STREAMING_SIMPLE ? 2 : 1);
-    // fields, flags, and the marker buffers of a tank-wall geometry
-    // (about 8 markers per (i, j) column at most, 256 bytes each with
-    // their schedule, stencil-cell and per-pass data)
-    *bytes = pops + 5 * plane * 4 + 2 * mask_words * 4 + 8 * c->x * c->y * 256;   // F (float4) and Nu: 5 planes
+    // fields, flags, the split steps' zone, and the marker buffers of a
+    // tank-wall geometry (about 8 markers per (i, j) column at most, 360 bytes
+    // each with the next list, the scheduler's scratch, their schedule,
+    // stencil-cell and per-pass data)
+    *bytes = pops + 5 * plane * 4 + (2 * 4 + 9) * mask_words + 8 * c->x * c->y * 360;   // F (float4) and Nu: 5 planes
     return TDLB_OK;
 }
 
@@ -1083,6 +1065,7 @@ int tdlb_set_markers(tdlb_handle h, const tdlb_marker* markers, size_t n) {
     return guarded(h, [&] {
         upload_markers(h, markers, n, n, nullptr);
         h->resident = true;
+        tdlb_rt::reserve_zone(h);
     });
 }
 
@@ -1140,6 +1123,7 @@ int tdlb_set_cells_per_thread(tdlb_handle h, int v) {
     return guarded(h, [&] {
         if (v != 1 && v != 2 && v != 4) throw Fail{TDLB_EINVAL, "cells per thread must be 1, 2 or 4"};
         h->vec = v;
+        tdlb_rt::reserve_zone(h);
     });
 }
 
@@ -1154,6 +1138,7 @@ int tdlb_set_overlap(tdlb_handle h, int mode) {
     return guarded(h, [&] {
         if (mode < 0 || mode > 2) throw Fail{TDLB_EINVAL, "overlap mode must be 0, 1 or 2"};
         h->overlap = mode;
+        tdlb_rt::reserve_zone(h);
     });
 }
 
@@ -1261,6 +1246,16 @@ int tdlb_attach_rushton(tdlb_handle h, const tdlb_rushton* spec, double nonupdat
             TDLB_CK(cudaMalloc(&h->d_rot_xz, xz.size() * sizeof(double)));
             TDLB_CK(cudaMemcpy(h->d_rot_xz, xz.data(), xz.size() * sizeof(double), cudaMemcpyHostToDevice));
         }
+        // tdlb_set_rotating_markers' upload: the blades, their order, at most a
+        // level each and the planes' level offsets
+        const size_t stage = pol.size() * (sizeof(tdlb::Marker) + 2 * sizeof(int)) + sizeof(int) + (size_t)(h->g.ny + 1) * sizeof(int);
+        if (stage > h->blade_stage_cap) {
+            cudaFree(h->d_blade_stage);
+            h->d_blade_stage = nullptr;
+            h->blade_stage_cap = 0;
+            TDLB_CK(cudaMalloc(&h->d_blade_stage, stage));
+            h->blade_stage_cap = stage;
+        }
         h->rot_device = true;
         h->rot_ci = G.ci;
         h->rot_ck = G.ck;
@@ -1269,6 +1264,7 @@ int tdlb_attach_rushton(tdlb_handle h, const tdlb_rushton* spec, double nonupdat
         h->angle = angle;
         h->rstep = 1;
         auto_rbox(h, G, pol, rmax);
+        tdlb_rt::reserve_zone(h);
     });
 }
 
@@ -1338,14 +1334,6 @@ int tdlb_set_rotating_markers(tdlb_handle h, const tdlb_marker* markers, size_t 
         std::memcpy(q + b_mk + b_order + b_lv, h->seg1.plane_lv.data(), b_pl);
         // one copy and a launch that puts the four parts in their places (four
         // copies of a few KB are four trips)
-        if (need > h->blade_stage_cap) {
-            TDLB_CK(cudaStreamSynchronize(h->stream));
-            cudaFree(h->d_blade_stage);
-            h->d_blade_stage = nullptr;
-            h->blade_stage_cap = 0;
-            TDLB_CK(cudaMalloc(&h->d_blade_stage, need + need / 2));
-            h->blade_stage_cap = need + need / 2;
-        }
         TDLB_CK(cudaMemcpyAsync(h->d_blade_stage, q, need, cudaMemcpyHostToDevice, h->stream));
         TDLB_CK(cudaEventRecord(st.ev, h->stream));
         TDLB_CK(tdlb::launch_place_blades((const int*)h->d_blade_stage, h->d_markers + h->n0, (int)n, h->d_sched + h->n0,
@@ -1353,7 +1341,7 @@ int tdlb_set_rotating_markers(tdlb_handle h, const tdlb_marker* markers, size_t 
                                           h->stream));
         h->rot_device = false;   // the blades now follow the host's list
         // a split step needs every blade stencil cell inside the zone
-        if (h->zone_gen == h->marker_gen && !h->zone_all) h->zone_ok = blades_in_zone(h);
+        if (h->zone_gen == h->marker_gen) h->zone_ok = blades_in_zone(h);
     });
 }
 
@@ -1491,7 +1479,7 @@ void note_pass(tdlb_lattice* h, float beta) {
     h->force_gen = h->marker_gen;
     // blades that turn on the device stay inside the zone's annuli
     h->force_blades_in = h->n_markers == h->n0 || h->rot_device ||
-                         (h->zone_gen == h->marker_gen && !h->zone_all && h->zone_ok);
+                         (h->zone_gen == h->marker_gen && h->zone_ok);
 }
 void borrow_stream(tdlb_lattice* h, cudaStream_t s) {
     fence(h);
@@ -1504,6 +1492,7 @@ void return_stream(tdlb_lattice* h) {
     if (!h->own_stream) return;
     h->stream = h->own_stream;
     h->own_stream = nullptr;
+    reserve_zone(h);
 }
 
 cudaError_t scratch(tdlb_lattice* h, size_t bytes, char** out) {
@@ -1521,16 +1510,23 @@ cudaError_t scratch(tdlb_lattice* h, size_t bytes, char** out) {
     return cudaSuccess;
 }
 
+void reserve_zone(tdlb_lattice* h) {
+    if (h->zone_block || !h->resident || h->own_stream || !(split_wanted(h) || h->rbox_geom.n > 0)) return;
+    const size_t nw = (size_t)(h->g.rows() * h->g.jw), ring = (size_t)h->g.ny * sizeof(double2);
+    if (cudaMalloc(&h->zone_block, ring + nw * (2 * sizeof(int) + 1)) != cudaSuccess) {
+        h->zone_block = nullptr;
+        cudaGetLastError();
+        return;
+    }
+    h->d_zone_ring = (double2*)h->zone_block;
+    h->d_zone_core = (uint32_t*)(h->zone_block + ring);
+    h->d_zone_words = (int*)(h->d_zone_core + nw);
+    h->d_zone_skip = (uint8_t*)(h->d_zone_words + nw);
+}
+
 void drop_zone(tdlb_lattice* h) {
-    cudaFree(h->d_zone_core);
-    cudaFree(h->d_zone_skip);
-    cudaFree(h->d_zone_except);
-    cudaFree(h->d_zone_words);
-    h->d_zone_core = nullptr;
-    h->d_zone_skip = nullptr;
-    h->d_zone_except = nullptr;
-    h->d_zone_words = nullptr;
-    h->zone_cap = 0;
+    cudaFree(h->zone_block);
+    h->zone_block = nullptr;
     h->zone_gen = ~0u;
     h->h_zone_core.clear();
 }

@@ -122,16 +122,17 @@ struct tdlb_lattice {
     bool stream_taken = false;    // the caller has the stream (tdlb_get_stream) and may queue work there that the
                                   // next step has to follow: no step splits unasked from then on
     bool resident = false;        // markers kept for many passes (set/attach), so a zone pays
-    // the zone (zone.cu), for marker_gen zone_gen and box_gen zone_box_gen
+    // the zone (zone.cu), for marker_gen zone_gen and box_gen zone_box_gen; its
+    // arrays are one allocation, made where the markers are set (tdlb_rt::
+    // reserve_zone): a step allocates nothing, and without them does not split
     unsigned zone_gen = ~0u, zone_box_gen = ~0u;
-    bool zone_all = false;        // every word is in it (markers that change every pass)
     bool zone_ok = false;         // every stencil cell of the current markers lies in it
     bool zone_small = false;      // it holds at most 60 % of the cells
+    char* zone_block = nullptr;
     uint32_t* d_zone_core = nullptr;     // 1 bit per cell: the stencil cells
-    uint8_t* d_zone_skip = nullptr;      // 1 byte per flag word: in the zone
-    uint32_t* d_zone_except = nullptr;   // 1 bit per cell: the residual box's cells (when there is a box)
     int* d_zone_words = nullptr;         // the zone's words, ascending
-    long long zone_cap = 0;              // words the arrays hold
+    double2* d_zone_ring = nullptr;      // per plane: radii of the blades' annulus
+    uint8_t* d_zone_skip = nullptr;      // 1 byte per flag word: in the zone
     int n_zone = 0, n_outer = 0;         // words inside, outside
     // the last forcing pass, which F and the current flags are of
     bool forced = false;          // there was one since F was last zero everywhere
@@ -145,11 +146,11 @@ struct tdlb_lattice {
     float* d_res[2] = {nullptr, nullptr};
     bool rbox_auto = true;                // set from the impeller by tdlb_attach_rushton
     unsigned box_gen = 0;                 // bumped by every change of the box
-    // elements of the cells the box launch of a step takes, ascending
+    // the cells that the box launch of a step takes: their elements, ascending,
+    // and a bit for each (the other launches leave them out)
     int* d_box_list = nullptr;
     int n_box = 0;
-    long long box_list_cap = 0;
-    unsigned box_list_gen = ~0u;          // box_gen the list was built for
+    uint32_t* d_box_except = nullptr;
     // device scratch of the read-back (a slab of output) and the plane dumps
     void* d_scratch = nullptr;
     size_t scratch_bytes = 0;
@@ -249,6 +250,9 @@ inline void fence(tdlb_lattice* h) { h->bulk_ok = false; }
 void note_pass(tdlb_lattice* h, float beta);
 // The handle's device scratch, at least `bytes` long (kept for the next call).
 cudaError_t scratch(tdlb_lattice* h, size_t bytes, char** out);
+// Memory for the zone, where the handle's steps may use one; without it they
+// do not split.
+void reserve_zone(tdlb_lattice* h);
 // Free the zone's arrays (the lattice changed size).
 void drop_zone(tdlb_lattice* h);
 // Remove the residual box (a tank joining a batch, whose step kernel keeps

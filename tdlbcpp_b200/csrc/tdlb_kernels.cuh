@@ -7,10 +7,10 @@ namespace tdlb {
 
 // Which cells a step launch takes (step_kernels.cuh). Cells are told apart by
 // flag words, the 32 cells of a row whose touched flags share a word: part 1
-// takes the words whose `skip` byte is zero, part 2 the words of a list,
-// without the cells whose bit is set in `except` (NULL: all of them). Part 0
-// takes every cell. l2_ahead > 0 turns on the L2 prefetch of parts 0 and 1,
-// that many CTAs ahead of the walk.
+// takes the words whose `skip` byte is zero, part 2 the words of a list (NULL:
+// the first `count`), without the cells whose bit is set in `except` (NULL: all
+// of them). Part 0 takes every cell. l2_ahead > 0 turns on the L2 prefetch of
+// parts 0 and 1, that many CTAs ahead of the walk.
 struct StepPart {
     const uint8_t* skip;
     const int* words;
@@ -124,9 +124,10 @@ cudaError_t launch_box(const StepArgs& a, bool simple, cudaStream_t st);
 cudaError_t launch_zone_core(const Dims& g, const uint32_t* mask_static, const double2* ring, double ci, double ck,
                              uint32_t* core, cudaStream_t st);
 // skip: a byte per word, 1 where the word holds a core cell or (neighbours) a
-// periodic neighbour of one; core NULL: every word.
+// periodic neighbour of one.
 cudaError_t launch_zone_words(const Dims& g, const uint32_t* core, int neighbours, uint8_t* skip, cudaStream_t st);
-// Box cells: their bits in `except` (zeroed by the caller), their words in skip.
+// Box cells: their bits in `except` (zeroed by the caller), their words in skip;
+// either may be NULL.
 cudaError_t launch_zone_box(const Dims& g, const int* cells, int n, uint32_t* except, uint8_t* skip, cudaStream_t st);
 cudaError_t launch_fill_uniform_moments(Planes Q, const Dims& g, float rho, cudaStream_t st);
 

@@ -31,8 +31,8 @@ __global__ void __launch_bounds__(256) k_zone_words(Dims g, const uint32_t* __re
                                                     uint8_t* __restrict__ skip) {
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= g.rows() * g.jw) return;
-    if (!core || !neighbours) {
-        skip[t] = !core || core[t] != 0u;
+    if (!neighbours) {
+        skip[t] = core[t] != 0u;
         return;
     }
     const long long row = t / g.jw;
@@ -57,8 +57,8 @@ __global__ void __launch_bounds__(256) k_zone_box(Dims g, const int* __restrict_
     if (t >= n) return;
     const int e = cells[t], row = e / g.jp, j = e - row * g.jp;
     const long long w = (long long)row * g.jw + (j >> 5);
-    atomicOr(except + w, 1u << (j & 31));
-    skip[w] = 1;
+    if (except) atomicOr(except + w, 1u << (j & 31));
+    if (skip) skip[w] = 1;
 }
 
 static unsigned words_grid(const Dims& g) { return (unsigned)((g.rows() * g.jw + 255) / 256); }

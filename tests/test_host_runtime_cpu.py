@@ -238,3 +238,69 @@ def test_a_step_follows_what_the_caller_queued_on_the_stream(fake, overlap):
         assert lib.fake_launches(b"true, 1>") == before + 1, "asked for, steps stay split"
     cu.close()
     assert not faults(fake)
+
+
+CASES = [("Simple", "fp32"), ("Esotwist", "fp32"), ("Simple", "fp16"), ("Esotwist", "bf16")]
+
+
+def _loop(tb, cu, steps, rt=None):
+    for s in range(steps):
+        if rt is None:
+            cu.rotate_impeller(0.1 * s, 0.1)
+        else:
+            cu.set_rotating_markers(rt.rotating(0.1 * s, 0.1))
+        cu.collision()
+        cu.forcing_resident(ALPHA, BETA)
+
+
+@pytest.mark.parametrize("streaming,storage", CASES)
+@pytest.mark.parametrize("blades", ["device", "host"])
+def test_the_step_loop_allocates_nothing(fake, streaming, storage, blades):
+    """After an attach, also another one on the same handle, split steps and
+    residual box included. (Host blades: two pinned buffers on the first two calls.)"""
+    lib = fake.load_library()
+    dims = (96, 96, 96)
+    cu = fake.ComputeUnit(x=96, y=96, z=96, nu=1e-3, streaming=streaming, storage=storage)
+    for _ in range(2):
+        _attach(fake, cu, dims)
+        rt = fake.RushtonTurbine(*dims, tip_speed=0.1, startup_steps=0) if blades == "host" else None
+        for q in range(2):
+            if rt is not None:
+                cu.set_rotating_markers(rt.rotating(0.3 * q, 0.1))
+        before = lib.fake_mallocs()
+        cu.initialise(1.0)
+        cu.forcing_resident(ALPHA, BETA)
+        _loop(fake, cu, 6, rt)
+        assert lib.fake_mallocs() == before
+        assert lib.fake_launches(b", 1>(") > 0, "the steps split"
+    cu.close()
+    assert not faults(fake)
+
+
+@pytest.mark.parametrize("streaming,storage", CASES)
+def test_without_memory_for_the_zone_steps_do_not_split(fake, streaming, storage):
+    """Each allocation of an attach fails in turn: the attach says so, or the
+    steps run, split or not."""
+    lib = fake.load_library()
+    dims = (96, 96, 96)
+    unsplit = 0
+    for nth in range(1, 60):
+        cu = fake.ComputeUnit(x=96, y=96, z=96, nu=1e-3, streaming=streaming, storage=storage)
+        cu.initialise(1.0)
+        before = lib.fake_mallocs()
+        lib.fake_fail(nth)
+        try:
+            _attach(fake, cu, dims)
+            lib.fake_fail(0)
+            cu.forcing_resident(ALPHA, BETA)
+            n = lib.fake_launches(b", 1>(")
+            _loop(fake, cu, 4)
+            unsplit += lib.fake_launches(b", 1>(") == n
+        except fake.TdlbError:
+            pass
+        lib.fake_fail(0)
+        cu.close()
+        assert not faults(fake), f"allocation {nth}"
+        if lib.fake_mallocs() - before < nth:
+            break
+    assert unsplit == (storage == "fp32")   # (with a residual box the zone is asked for twice)
