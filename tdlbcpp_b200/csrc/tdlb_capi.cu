@@ -366,12 +366,25 @@ bool force_in_zone(const tdlb_lattice* h) {
     return !h->forced || (h->force_gen == h->marker_gen && h->force_blades_in);
 }
 
-// The zone, built where the resident markers' is not there yet, holds every
-// stencil cell of theirs.
-bool zone_holds_markers(tdlb_lattice* h) {
+// A zone is planned (a wait and a pass over the flag words, 1.4 ms at 400^3) once
+// the list has been through this many passes, for lattices whose steps were not
+// asked to split: markers set anew with every step, before the collision or after
+// it, go through one.
+constexpr int kSettledPasses = 2;
+
+// The resident markers' zone is there, or is built now.
+bool zone_built(tdlb_lattice* h, bool may_build) {
     if (!zone_known(h)) return false;
-    if (h->zone_gen != h->marker_gen || h->zone_box_gen != h->box_gen) build_zone(h);
-    return h->zone_ok;
+    if (h->zone_gen == h->marker_gen && h->zone_box_gen == h->box_gen) return true;
+    if (!may_build || (h->overlap <= 0 && h->list_passes < kSettledPasses)) return false;
+    build_zone(h);
+    return true;
+}
+
+// The coming step may leave F out of the words outside the zone.
+bool zone_serves(tdlb_lattice* h, bool may_build) {
+    if (h->forced && h->force_gen != h->marker_gen) return false;   // (and no zone is built for such a step)
+    return zone_built(h, may_build) && h->zone_ok && force_in_zone(h);
 }
 
 // Smallest lattice whose steps split unasked.
@@ -384,18 +397,12 @@ bool split_wanted(const tdlb_lattice* h) {
     return h->cfg.storage != TDLB_STORAGE_FP32 || tdlb::vector_width(h->g, h->vec) == 1;
 }
 
-// The lattice's steps can run split. (A zone covering most of the lattice leaves
-// little to overlap with.)
-bool split_capable(tdlb_lattice* h) {
-    return split_wanted(h) && zone_holds_markers(h) && (h->zone_small || h->overlap == 2);
-}
+// A zone covering most of the lattice leaves little to overlap with.
+bool zone_pays(const tdlb_lattice* h) { return h->zone_small || h->overlap == 2; }
 
-bool can_split(tdlb_lattice* h) {
-    if (h->holds_moments || !h->overlap) return false;
-    // a captured step stays on the captured stream and its own side stream
+bool under_capture(tdlb_lattice* h) {
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(h->stream, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) return false;
-    return split_capable(h) && force_in_zone(h);
+    return cudaStreamIsCapturing(h->stream, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone;
 }
 
 // Queue one step-kernel launch, bracketed by timing events when enabled.
@@ -426,7 +433,12 @@ void run_step(tdlb_lattice* h, bool collide) {
         return simple ? tdlb::launch_step_simple(x, st) : tdlb::launch_step_esotwist(x, st);
     };
     const bool boxed = a.rr.on();
-    const bool split = collide && can_split(h);
+    // a captured step stays on the captured stream and its own side stream, and
+    // takes the zone as it is
+    const bool wanted = collide && !h->holds_moments && split_wanted(h);
+    const bool captured = (wanted || boxed) && under_capture(h);
+    const bool zone = ((wanted && !captured) || boxed) && zone_serves(h, !captured);
+    const bool split = wanted && !captured && zone && zone_pays(h);
     // 1: outer words, 2: inner words (or every word) without the box's cells
     auto part = [&](int which, cudaStream_t st, bool every = false) {
         tdlb::StepArgs x = a;
@@ -457,7 +469,6 @@ void run_step(tdlb_lattice* h, bool collide) {
         if (boxed) {
             // the box's cells are left out of the plain launches: the outer
             // words and the inner ones, or one over every word without a zone
-            const bool zone = zone_holds_markers(h) && force_in_zone(h);
             if (zone) part(1, h->stream);
             box();
             part(2, h->stream, !zone);
@@ -703,6 +714,7 @@ void upload_markers(tdlb_lattice* h, const tdlb_marker* m, size_t n, size_t n0, 
     h->rot_device = false;
     h->impeller_begin = -1;
     h->marker_gen++;
+    h->list_passes = 0;
     std::swap(h->d_markers, h->d_markers_in);
     std::swap(h->marker_cap, h->marker_in_cap);
     h->n_markers = (int)n;
@@ -1149,7 +1161,8 @@ int tdlb_join(tdlb_handle h) {
 int tdlb_read_zone(tdlb_handle h, uint8_t* flags) {
     return guarded(h, [&] {
         if (!flags) throw Fail{TDLB_EINVAL, "out is NULL"};
-        if (h->overlap < 0 || tdlb::vector_width(h->g, h->vec) != 1 || !split_capable(h))
+        if (h->overlap < 0 || tdlb::vector_width(h->g, h->vec) != 1 || !split_wanted(h) || !zone_built(h, true) || !h->zone_ok ||
+            !zone_pays(h))
             throw Fail{TDLB_ESTATE, "no split step (needs resident markers, one cell per thread, overlap on and, in "
                                     "mode 1, inner chunks holding at most 60 % of the lattice)"};
         const Dims& g = h->g;
@@ -1477,6 +1490,7 @@ void note_pass(tdlb_lattice* h, float beta) {
     h->last_beta = beta;
     h->forced = true;
     h->force_gen = h->marker_gen;
+    if (h->list_passes < kSettledPasses) h->list_passes++;
     // blades that turn on the device stay inside the zone's annuli
     h->force_blades_in = h->n_markers == h->n0 || h->rot_device ||
                          (h->zone_gen == h->marker_gen && h->zone_ok);

@@ -134,6 +134,7 @@ struct tdlb_lattice {
     double2* d_zone_ring = nullptr;      // per plane: radii of the blades' annulus
     uint8_t* d_zone_skip = nullptr;      // 1 byte per flag word: in the zone
     int n_zone = 0, n_outer = 0;         // words inside, outside
+    int list_passes = 0;          // forcing passes (or batch runs) of the resident list so far
     // the last forcing pass, which F and the current flags are of
     bool forced = false;          // there was one since F was last zero everywhere
     unsigned force_gen = ~0u;     // marker_gen of its list (~0: not known)

@@ -304,3 +304,92 @@ def test_without_memory_for_the_zone_steps_do_not_split(fake, streaming, storage
         if lib.fake_mallocs() - before < nth:
             break
     assert unsplit == (storage == "fp32")   # (with a residual box the zone is asked for twice)
+
+
+def _zone_builds(tb):
+    return tb.load_library().fake_launches(b"k_zone_words")
+
+
+@pytest.mark.parametrize("streaming,storage", CASES)
+@pytest.mark.parametrize("order", ["before", "after", "list"])
+def test_markers_that_change_every_step_have_no_zone(fake, streaming, storage, order):
+    """A zone is planned for a list that stays, not for each list of a geometry that
+    is set anew before or after the collision, or handed to forcing()."""
+    lib = fake.load_library()
+    cu = fake.ComputeUnit(x=96, y=96, z=96, nu=1e-3, streaming=streaming, storage=storage)
+    if storage != "fp32":
+        cu.set_residual_box(30, 50, 30, 50, 30, 50)
+    cu.initialise(1.0)
+    for s in range(6):
+        ball = _ball(fake, (20 + 5 * s, 30, 40))
+        if order == "before":
+            cu.set_markers(ball)
+        if s:
+            cu.collision()
+        if order == "after":
+            cu.set_markers(ball)
+        if order == "list":
+            cu.forcing(ball, ALPHA, BETA)
+        else:
+            cu.forcing_resident(ALPHA, BETA)
+    assert _zone_builds(fake) == 0
+    if order != "list":                  # and now it stays
+        waits = None
+        for s in range(6):
+            if s == 3:
+                waits = lib.fake_waits()
+            cu.step(ALPHA, BETA)
+        assert _zone_builds(fake) == 1 and lib.fake_waits() == waits
+        assert lib.fake_launches(b", 1>(") > 0
+    cu.close()
+    assert not faults(fake)
+
+
+@pytest.mark.parametrize("streaming,storage", CASES)
+def test_blades_outside_the_zone_do_not_rebuild_it(fake, streaming, storage):
+    lib = fake.load_library()
+    dims = (96, 96, 96)
+    cu = fake.ComputeUnit(x=96, y=96, z=96, nu=1e-3, streaming=streaming, storage=storage)
+    _attach(fake, cu, dims)
+    rt = fake.RushtonTurbine(*dims, tip_speed=0.1, startup_steps=0)
+    cu.initialise(1.0)
+    cu.forcing_resident(ALPHA, BETA)
+    for s in range(10):
+        blades = rt.rotating(0.1 * s, 0.1)
+        if s % 5 > 1:
+            blades["i"] = (blades["i"] + 30) % 96
+        cu.set_rotating_markers(blades)
+        if s == 4:
+            waits = lib.fake_waits()
+        cu.collision()
+        cu.forcing_resident(ALPHA, BETA)
+    assert _zone_builds(fake) == 1 and lib.fake_waits() == waits
+    cu.close()
+    assert not faults(fake)
+
+
+@pytest.mark.parametrize("streaming,storage", CASES)
+@pytest.mark.parametrize("overlap", [None, False, "always"])
+def test_steps_are_captured_after_the_markers_changed(fake, streaming, storage, overlap):
+    """A captured step neither waits nor allocates, whatever changed before it."""
+    lib = fake.load_library()
+    cu = fake.ComputeUnit(x=96, y=96, z=96, nu=1e-3, streaming=streaming, storage=storage)
+    if overlap is not None:
+        cu.set_overlap(overlap)
+    cu.initialise(1.0)
+    for s in range(3):
+        _attach(fake, cu, (96, 96, 96))
+        if storage != "fp32" and s:
+            cu.set_residual_box(30, 50 + s, 30, 50, 30, 50)
+        cu.forcing_resident(ALPHA, BETA)
+        for _ in range(s):
+            cu.step(ALPHA, BETA)
+        if s == 0 and storage == "fp32":
+            cu.collision()               # (the moment form's step)
+        lib.fake_capture(1)
+        for _ in range(3):
+            cu.rotate_impeller(0.1, 0.1)
+            cu.step(ALPHA, BETA)
+        lib.fake_capture(0)
+        assert not faults(fake), f"after attach {s}"
+    cu.close()
