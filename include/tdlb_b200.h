@@ -401,8 +401,8 @@ int tdlb_impeller_load(tdlb_handle h, double* out5);
  * (pinned host memory or device memory), without waiting: out5 holds it once
  * the stream has reached this point (tdlb_synchronize, or an event recorded
  * on the stream after this call). Lets a caller prepare the next step on the
- * host while the device finishes this one. The first call allocates the
- * reduction's device scratch. */
+ * host while the device finishes this one. Nothing is allocated: the
+ * reduction's scratch comes with tdlb_attach_rushton. */
 int tdlb_impeller_load_async(tdlb_handle h, double* out5);
 
 /* The same FP64 impeller load for callers that cannot allocate device

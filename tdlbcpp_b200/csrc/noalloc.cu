@@ -5,8 +5,8 @@
 // its own pool up front (a cudaMalloc from the library would fail or escape
 // the pool's accounting), or a real-time loop with a no-allocation rule after
 // start-up (cudaMalloc can synchronise the device and has no time bound).
-// The allocating entry point, tdlb_impeller_load, creates its reduction
-// buffer with cudaMalloc on its first call; this variant keeps that buffer
+// tdlb_impeller_load uses a reduction buffer of the handle's that
+// tdlb_attach_rushton allocates with cudaMalloc; this variant keeps that buffer
 // in a fixed-size array compiled into the library instead.
 //
 // The scratch: g_load_partials below, a file-scope __device__ array of

@@ -846,6 +846,45 @@ void host_aos_to_planes(tdlb_lattice* h, const float* in, int npl, float* dev) {
     TDLB_CK(cudaStreamSynchronize(h->stream));
 }
 
+// What the impeller load needs: its scratch and the impeller's slots of the
+// resident list, the markers from list index `begin`. (Its blades keep their slots
+// while they rotate on the device; a host list of blades reorders them within the
+// second segment, which is the impeller's whole.) Made with the impeller, so that
+// a load neither allocates nor waits.
+constexpr size_t kLoadDoubles = (size_t)tdlb::kLoadBlocks * 5 + 5 + 1;
+void prepare_load(tdlb_lattice* h, int begin) {
+    if (!h->d_load) {
+        TDLB_CK(cudaMalloc(&h->d_load, kLoadDoubles * sizeof(double)));
+        TDLB_CK(cudaMemsetAsync(h->d_load, 0, kLoadDoubles * sizeof(double), h->stream));
+    }
+    const int n = h->n_markers, groups = (n + 255) / 256;
+    cudaFree(h->d_imp_slots);
+    h->d_imp_slots = nullptr;
+    h->n_imp = 0;
+    if (n > 0) {
+        struct Tmp {
+            int* p = nullptr;
+            ~Tmp() { cudaFree(p); }
+        } off;
+        std::vector<int> count((size_t)groups);
+        TDLB_CK(cudaMalloc(&off.p, (size_t)groups * sizeof(int)));
+        TDLB_CK(tdlb::launch_impeller_slots(h->d_sched, n, begin, off.p, nullptr, h->stream));
+        TDLB_CK(cudaMemcpyAsync(count.data(), off.p, (size_t)groups * sizeof(int), cudaMemcpyDeviceToHost, h->stream));
+        TDLB_CK(cudaStreamSynchronize(h->stream));
+        int sum = 0;
+        for (int& c : count) {
+            const int v = c;
+            c = sum;
+            sum += v;
+        }
+        TDLB_CK(cudaMalloc(&h->d_imp_slots, (size_t)std::max(sum, 1) * sizeof(int)));
+        TDLB_CK(cudaMemcpyAsync(off.p, count.data(), (size_t)groups * sizeof(int), cudaMemcpyHostToDevice, h->stream));
+        TDLB_CK(tdlb::launch_impeller_slots(h->d_sched, n, begin, off.p, h->d_imp_slots, h->stream));
+        TDLB_CK(cudaStreamSynchronize(h->stream));
+        h->n_imp = sum;
+    }
+}
+
 // ---------------------------------------------------------------------------
 // Residual box of the 16-bit storage (tdlb::ResidualBox): exact deviations
 // for every population location inside a box of cells.
@@ -1269,6 +1308,7 @@ int tdlb_attach_rushton(tdlb_handle h, const tdlb_rushton* spec, double nonupdat
             TDLB_CK(cudaMalloc(&h->d_blade_stage, stage));
             h->blade_stage_cap = stage;
         }
+        prepare_load(h, n_fixed);
         h->rot_device = true;
         h->rot_ci = G.ci;
         h->rot_ck = G.ck;
@@ -1358,51 +1398,11 @@ int tdlb_set_rotating_markers(tdlb_handle h, const tdlb_marker* markers, size_t 
     });
 }
 
-// The impeller's slots of the resident list. (Its blades keep their slots while
-// they rotate on the device; a host list of blades reorders them within the
-// second segment, which is the impeller's whole.)
-static void find_impeller_slots(tdlb_lattice* h) {
-    if (h->imp_gen == h->marker_gen) return;
-    const int n = h->n_markers, groups = (n + 255) / 256;
-    cudaFree(h->d_imp_slots);
-    h->d_imp_slots = nullptr;
-    h->n_imp = 0;
-    if (n > 0) {
-        struct Tmp {
-            int* p = nullptr;
-            ~Tmp() { cudaFree(p); }
-        } off;
-        std::vector<int> count((size_t)groups);
-        TDLB_CK(cudaMalloc(&off.p, (size_t)groups * sizeof(int)));
-        TDLB_CK(tdlb::launch_impeller_slots(h->d_sched, n, h->impeller_begin, off.p, nullptr, h->stream));
-        TDLB_CK(cudaMemcpyAsync(count.data(), off.p, (size_t)groups * sizeof(int), cudaMemcpyDeviceToHost, h->stream));
-        TDLB_CK(cudaStreamSynchronize(h->stream));
-        int sum = 0;
-        for (int& c : count) {
-            const int v = c;
-            c = sum;
-            sum += v;
-        }
-        TDLB_CK(cudaMalloc(&h->d_imp_slots, (size_t)std::max(sum, 1) * sizeof(int)));
-        TDLB_CK(cudaMemcpyAsync(off.p, count.data(), (size_t)groups * sizeof(int), cudaMemcpyHostToDevice, h->stream));
-        TDLB_CK(tdlb::launch_impeller_slots(h->d_sched, n, h->impeller_begin, off.p, h->d_imp_slots, h->stream));
-        TDLB_CK(cudaStreamSynchronize(h->stream));
-        h->n_imp = sum;
-    }
-    h->imp_gen = h->marker_gen;
-}
-
 // Queue the impeller load of the last forcing pass and its copy into out5.
 void queue_impeller_load(tdlb_lattice* h, double* out5) {
     if (!out5) throw Fail{TDLB_EINVAL, "out is NULL"};
     if (h->impeller_begin < 0) throw Fail{TDLB_ESTATE, "no impeller attached (tdlb_attach_rushton)"};
     if (h->pass == 0) throw Fail{TDLB_ESTATE, "no forcing pass yet"};
-    constexpr size_t kDoubles = (size_t)tdlb::kLoadBlocks * 5 + 5 + 1;
-    if (!h->d_load) {
-        TDLB_CK(cudaMalloc(&h->d_load, kDoubles * sizeof(double)));
-        TDLB_CK(cudaMemsetAsync(h->d_load, 0, kDoubles * sizeof(double), h->stream));
-    }
-    find_impeller_slots(h);
     tdlb::IbmArgs a = ibm_args(h, 0.f, h->last_beta);
     double* out = h->d_load + tdlb::kLoadBlocks * 5;
     // memory the device can write (its own, pinned host, managed) takes the sums

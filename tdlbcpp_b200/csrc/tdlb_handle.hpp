@@ -94,9 +94,8 @@ struct tdlb_lattice {
     double angle = 0.0;           // impeller angle of the last rotation
     unsigned long long rstep = 1; // main-loop step the angle belongs to (main.cpp:336 starts at 1)
     double* d_load = nullptr;     // kLoadBlocks*5 partials + 5 results + a counter
-    int* d_imp_slots = nullptr;   // the impeller's slots, ascending, for marker_gen imp_gen
+    int* d_imp_slots = nullptr;   // the impeller's slots, ascending
     int n_imp = 0;
-    unsigned imp_gen = ~0u;
     // pinned staging of the per-step blade upload (markers and their
     // schedule), two buffers used in turn; each buffer's event marks the end
     // of the copies that read it

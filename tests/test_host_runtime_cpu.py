@@ -393,3 +393,24 @@ def test_steps_are_captured_after_the_markers_changed(fake, streaming, storage, 
         lib.fake_capture(0)
         assert not faults(fake), f"after attach {s}"
     cu.close()
+
+
+def test_the_impeller_load_is_captured_after_another_attach(fake):
+    """The load's slots and scratch come with the impeller: no load allocates or waits."""
+    lib = fake.load_library()
+    dims = (48, 48, 48)
+    out = np.zeros(5)
+    lib.fake_pin(out.ctypes.data, out.nbytes)
+    cu = fake.ComputeUnit(x=48, y=48, z=48, nu=1e-3)
+    cu.initialise(1.0)
+    for s in range(3):
+        _attach(fake, cu, dims)
+        cu.forcing_resident(ALPHA, BETA)
+        before = lib.fake_mallocs()
+        lib.fake_capture(1)
+        cu.impeller_load_async(out.ctypes.data)
+        lib.fake_capture(0)
+        cu.impeller_load()
+        assert lib.fake_mallocs() == before
+        assert not faults(fake), f"attach {s}"
+    cu.close()
