@@ -1398,6 +1398,26 @@ int tdlb_set_rotating_markers(tdlb_handle h, const tdlb_marker* markers, size_t 
     });
 }
 
+// The device's address of p[0, bytes) where a kernel may store there: both ends lie
+// in one piece of its own, pinned or managed memory, and the address is aligned.
+// NULL where only a copy can go.
+static void* device_address(const tdlb_lattice* h, void* p, size_t bytes, size_t align) {
+    if ((uintptr_t)p % align) return nullptr;
+    char* at[2];
+    for (int end = 0; end < 2; end++) {
+        cudaPointerAttributes a{};
+        if (cudaPointerGetAttributes(&a, (char*)p + (end ? bytes - 1 : 0)) != cudaSuccess) {
+            cudaGetLastError();
+            return nullptr;
+        }
+        const bool writes = a.type == cudaMemoryTypeHost ||
+                            ((a.type == cudaMemoryTypeDevice || a.type == cudaMemoryTypeManaged) && a.device == h->device);
+        if (!writes || !a.devicePointer) return nullptr;
+        at[end] = (char*)a.devicePointer;
+    }
+    return at[1] - at[0] == (ptrdiff_t)bytes - 1 ? at[0] : nullptr;
+}
+
 // Queue the impeller load of the last forcing pass and its copy into out5.
 void queue_impeller_load(tdlb_lattice* h, double* out5) {
     if (!out5) throw Fail{TDLB_EINVAL, "out is NULL"};
@@ -1407,12 +1427,7 @@ void queue_impeller_load(tdlb_lattice* h, double* out5) {
     double* out = h->d_load + tdlb::kLoadBlocks * 5;
     // memory the device can write (its own, pinned host, managed) takes the sums
     // from the kernel; a copy behind it costs 6 us of a small tank's step
-    double* direct = nullptr;
-    cudaPointerAttributes at{};
-    if (cudaPointerGetAttributes(&at, out5) != cudaSuccess) cudaGetLastError();
-    else if (at.type == cudaMemoryTypeHost || ((at.type == cudaMemoryTypeDevice || at.type == cudaMemoryTypeManaged) &&
-                                               at.device == h->device))
-        direct = (double*)at.devicePointer;
+    double* direct = (double*)device_address(h, out5, 5 * sizeof(double), alignof(double));
     TDLB_CK(tdlb::launch_marker_load(a, h->d_imp_slots, h->n_imp, h->rot_ci, h->rot_ck, h->d_load, (unsigned*)(out + 5),
                                      direct ? direct : out, h->stream));
     if (!direct) TDLB_CK(cudaMemcpyAsync(out5, out, 5 * sizeof(double), cudaMemcpyDefault, h->stream));

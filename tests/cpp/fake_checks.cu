@@ -13,6 +13,7 @@
 void fake_need(const char* who, const char* what, const void* p, long long n);
 void fake_fault(const char* who, const char* what);
 bool fake_sound();
+bool fake_writable(const void* p, long long n);   // pinned or device memory
 
 extern "C" void fake_check(const char* w, void** args) {
     using namespace tdlb;
@@ -63,6 +64,11 @@ extern "C" void fake_check(const char* w, void** args) {
                     const double d = std::sqrt((i - ci) * (i - ci) + (k - ck) * (k - ck));
                     if (ring[j].y >= 0.0 && d >= ring[j].x && d <= ring[j].y) core[g.word(i, j, k)] |= 1u << (j & 31);
                 }
+    }
+    if (name.find("k_marker_load(") != std::string::npos) {
+        const double* out = *(double* const*)args[7];
+        if ((uintptr_t)out % 8) fake_fault(w, "the load's address is not a multiple of 8");
+        if (!fake_writable(out, 40)) fake_fault(w, "the load does not lie in memory that the device can write");
     }
     if (name.find("k_rotate_markers") != std::string::npos) {
         const int n = *(const int*)args[2];

@@ -34,7 +34,7 @@ struct Launch {
 };
 
 std::recursive_mutex mu;
-std::map<char*, size_t> device, pinned;
+std::map<char*, size_t> device, pinned, registered;   // (registered: the test's own pinned memory)
 std::map<const void*, std::string>& names() {   // filled by static constructors
     static std::map<const void*, std::string> m;
     return m;
@@ -119,6 +119,7 @@ cudaError_t launch(const void* fn, void** args, cudaStream_t st) {
 // for fake_checks.cu
 void fake_need(const char* who, const char* what, const void* p, long long n) { need(who, what, p, n); }
 void fake_fault(const char* who, const char* what) { fault(std::string(who) + ": " + what); }
+bool fake_writable(const void* p, long long n) { return inside(pinned, p, (size_t)n) || inside(registered, p, (size_t)n) || inside(device, p, (size_t)n); }
 bool fake_sound() { return faults.empty(); }
 
 extern "C" {
@@ -127,6 +128,7 @@ extern "C" {
 void fake_reset() {
     std::lock_guard<std::recursive_mutex> lk(mu);
     launches.clear();
+    registered.clear();
     faults.clear();
     mallocs = waits = fail_in = 0;
     capturing = false;
@@ -134,7 +136,7 @@ void fake_reset() {
 }
 void fake_fail(long long nth) { fail_in = nth; }   // the nth allocation from here fails
 void fake_capture(int on) { capturing = on != 0; }
-void fake_pin(void* p, size_t n) { pinned[(char*)p] = n; }
+void fake_pin(void* p, size_t n) { registered[(char*)p] = n; }
 long long fake_mallocs() { return mallocs; }
 long long fake_waits() { return waits; }
 const char* fake_faults() { return faults.c_str(); }
@@ -239,7 +241,7 @@ cudaError_t cudaEventSynchronize(cudaEvent_t) { not_in_capture("cudaEventSynchro
 cudaError_t cudaEventElapsedTime(float* ms, cudaEvent_t, cudaEvent_t) { *ms = 0.f; return cudaSuccess; }
 cudaError_t cudaPointerGetAttributes(cudaPointerAttributes* a, const void* p) {
     *a = cudaPointerAttributes{};
-    a->type = inside(pinned, p, 1) ? cudaMemoryTypeHost : inside(device, p, 1) ? cudaMemoryTypeDevice : cudaMemoryTypeUnregistered;
+    a->type = inside(pinned, p, 1) || inside(registered, p, 1) ? cudaMemoryTypeHost : inside(device, p, 1) ? cudaMemoryTypeDevice : cudaMemoryTypeUnregistered;
     a->devicePointer = a->type == cudaMemoryTypeUnregistered ? nullptr : const_cast<void*>(p);
     return cudaSuccess;
 }

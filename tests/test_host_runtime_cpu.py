@@ -414,3 +414,20 @@ def test_the_impeller_load_is_captured_after_another_attach(fake):
         assert lib.fake_mallocs() == before
         assert not faults(fake), f"attach {s}"
     cu.close()
+
+
+@pytest.mark.parametrize("at,pinned", [(0, 40), (4, 80), (8, 48), (8, 40), (0, 8), (0, 0)])
+def test_the_load_goes_to_any_address(fake, at, pinned):
+    """5 doubles at an address that is no multiple of 8, or that leave the pinned
+    range, are copied there; the kernel writes only what it can."""
+    lib = fake.load_library()
+    buf = np.zeros(16)
+    if pinned:
+        lib.fake_pin(buf.ctypes.data, pinned)
+    cu = fake.ComputeUnit(x=48, y=48, z=48, nu=1e-3)
+    cu.initialise(1.0)
+    _attach(fake, cu, (48, 48, 48))
+    cu.forcing_resident(ALPHA, BETA)
+    cu.impeller_load_async(buf.ctypes.data + at)
+    cu.close()
+    assert not faults(fake)
