@@ -50,7 +50,7 @@ static inline unsigned blocks_for(long long n, int threads) { return (unsigned)(
 
 // Grid of a launch: every quad (parts 0 and 1) or those of the listed words.
 static inline unsigned step_blocks(const StepArgs& a, int V) {
-    if (a.part == 2) return blocks_for((long long)a.zone.count * (32 / V), 128);
+    if (a.part == 2) return listed_blocks(a.zone.count, V);
     return blocks_for(a.g.rows() * (a.g.jp / V), 128);
 }
 

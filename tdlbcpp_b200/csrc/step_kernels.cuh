@@ -173,6 +173,12 @@ __device__ __forceinline__ Quad quad_of(const Dims& g, int nq, unsigned t) {
     return q;
 }
 
+// The number of a launch's thread: its quad (parts 0 and 1) or its word of the list.
+template <int V, int PART>
+__device__ __forceinline__ unsigned part_number() {
+    return PART == 2 ? listed_word(blockIdx.x, threadIdx.x, V) : blockIdx.x * blockDim.x + threadIdx.x;
+}
+
 // The quad of thread t of a launch (StepPart) and, per cell, whether this launch
 // stores it (ok, V bits). PART 2: SEG = 32 / V consecutive lanes share a word of
 // the list; lanes past the row's end take its last quad, inactive.
@@ -187,18 +193,17 @@ __device__ __forceinline__ Quad part_quad(const Dims& g, const StepPart& part, u
         return q;
     } else {
         constexpr unsigned SEG = 32 / V;
-        const unsigned lw = t / SEG;
-        const unsigned in = min(lw, (unsigned)part.count - 1u);
+        const unsigned in = min(t, (unsigned)part.count - 1u);
         const int wd = part.words ? __ldg(part.words + in) : (int)in;
         const unsigned ex = part.except ? __ldg(part.except + wd) : 0u;
         Quad q;
         q.row = wd / g.jw;
-        const int j = (wd - q.row * g.jw) * 32 + (int)(t % SEG) * V;
+        const int j = (wd - q.row * g.jw) * 32 + (int)(threadIdx.x % SEG) * V;
         q.i = q.row / g.nz;
         q.k = q.row - q.i * g.nz;
         q.j0 = min(j, g.jp - V);
         q.e0 = q.row * g.jp + q.j0;
-        q.active = lw < (unsigned)part.count && j < g.ny;
+        q.active = t < (unsigned)part.count && j < g.ny;
         unsigned live = 0u;
 #pragma unroll
         for (int e = 0; e < V; e++) live |= j + e < g.ny ? 1u << e : 0u;
@@ -683,7 +688,7 @@ __global__ void __launch_bounds__(128, 4) k_step_simple(Planes A, Planes B, floa
                                                        Dims g, CollideParams p, StepPart part) {
     if constexpr (PART != 2 && COLLIDE && !FROM_MOMENTS)
         prefetch_ahead<S, V, LES, false, false>(A, Nu, g, part.l2_ahead);
-    unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
+    unsigned t = part_number<V, PART>();
     if constexpr (kChained<PART>) after_previous(t);
     simple_quad<S, V, LES, FROM_MOMENTS, COLLIDE, PART>(A, B, Nu, F, mask, g, p, t, part);
 }
@@ -702,7 +707,7 @@ __global__ void __launch_bounds__(128, kEsotwistBlocksPerSM<S, V>) k_step_esotwi
                                                          Dims g, CollideParams p, StepPart part) {
     if constexpr (PART != 2 && COLLIDE && !FROM_MOMENTS)
         prefetch_ahead<S, V, LES, true, EVEN>(Q, Nu, g, part.l2_ahead);
-    unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
+    unsigned t = part_number<V, PART>();
     if constexpr (kChained<PART>) after_previous(t);
     esotwist_quad<S, V, LES, FROM_MOMENTS, COLLIDE, EVEN, PART>(Q, Nu, F, mask, g, p, t, part);
 }

@@ -8,7 +8,7 @@ namespace tdlb {
 static inline unsigned blocks16(long long n, int threads) { return (unsigned)((n + threads - 1) / threads); }
 
 static inline unsigned grid16(const StepArgs& a, int V) {
-    if (a.part == 2) return blocks16((long long)a.zone.count * (32 / V), 128);
+    if (a.part == 2) return listed_blocks(a.zone.count, V);
     return blocks16(a.g.rows() * (a.g.jp / V), 128);
 }
 

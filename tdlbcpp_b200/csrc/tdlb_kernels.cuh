@@ -19,6 +19,14 @@ struct StepPart {
     int l2_ahead;
 };
 
+// Part 2: 32 / V lanes of a 128-thread block share a word of the list. Words are
+// counted, not threads: a lattice of a few cells along y has a word per row, up
+// to 2^30 of them, and 32 threads a word pass 2^32.
+__host__ __device__ inline unsigned listed_word(unsigned block, unsigned thread, unsigned V) {
+    return block * (4u * V) + thread * V / 32u;
+}
+inline unsigned listed_blocks(long long words, unsigned V) { return (unsigned)((words + 4u * V - 1) / (4u * V)); }
+
 // One wave of resident 128-thread CTAs of kernel K on the current device (the
 // occupancy its register count allows, times the SMs): the L2 prefetch
 // distance of a full launch. Queried once per kernel; 0 (prefetch off) if the

@@ -91,3 +91,7 @@ extern "C" void fake_check(const char* w, void** args) {
         fake_need(w, "plane_list", a.plane_list, 4LL * a.g.ny);
     }
 }
+
+// index arithmetic that kernels and launches share
+extern "C" long long fake_listed_word(unsigned block, unsigned thread, unsigned V) { return tdlb::listed_word(block, thread, V); }
+extern "C" long long fake_listed_blocks(long long words, unsigned V) { return tdlb::listed_blocks(words, V); }

@@ -431,3 +431,20 @@ def test_the_load_goes_to_any_address(fake, at, pinned):
     cu.impeller_load_async(buf.ctypes.data + at)
     cu.close()
     assert not faults(fake)
+
+
+@pytest.mark.parametrize("V", [1, 2, 4])
+@pytest.mark.parametrize("words", [1, 3, 4, 17, 134217728, 134217729, 268435457, 2 ** 29, 32767 * 32767])
+def test_every_listed_word_has_its_lanes(fake, V, words):
+    """The inner launch: 32 / V lanes of 128-thread blocks for each of up to 2^30 words
+    (x * z rows of few cells along y)."""
+    lib = fake.load_library()
+    lib.fake_listed_word.restype = lib.fake_listed_blocks.restype = ctypes.c_longlong
+    lib.fake_listed_blocks.argtypes = [ctypes.c_longlong, ctypes.c_uint]
+    blocks = lib.fake_listed_blocks(words, V)
+    lanes = 32 // V
+    assert blocks < 2 ** 31 and (blocks - 1) * 128 < words * lanes <= blocks * 128
+    for w in {0, words // 3, words // 2, words - 1}:
+        for lane in (0, lanes - 1):
+            thread = w * lanes + lane
+            assert lib.fake_listed_word(thread // 128, thread % 128, V) == w
