@@ -190,7 +190,6 @@ __device__ __forceinline__ void put_cell(const IbmArgs& a, int c, const float4 m
 // written per cell (400^3: 64 us for 2.1 M cells). Planes with more than
 // skip_above cells (an impeller disk, whose cells fill an (i, k) area of a single
 // j) are taken in list order instead.
-constexpr int kCellPlaces = 8;
 constexpr int kGatherThreads = 32 * kCellPlaces;
 struct CellTile {
     int e[32][kCellPlaces + 1];
@@ -1220,18 +1219,17 @@ __global__ void __launch_bounds__(kGatherThreads) k_ibm_gather_batch(const IbmAr
                                                                      const int2* __restrict__ work) {
     __shared__ IbmArgs sa;
     __shared__ CellTile sm;
-    const int2 w = work[blockIdx.x];
-    stage_args<kGatherThreads>(sa, args + w.x);
+    const GatherItem w = GatherItem::of(work[blockIdx.x]);
+    stage_args<kGatherThreads>(sa, args + w.tank);
     __syncthreads();
-    const int kind = w.y & 3, q = w.y >> 2;
-    if (kind == GATHER_TAIL) {
-        ibm_tail_cell<S>(sa, q * kGatherThreads + (int)threadIdx.x);
-    } else if (kind == GATHER_FLAGS) {
-        const int n4 = (int)(sa.mask_bytes / 16), v0 = q * (kMaskCopyWords / 4);
+    if (w.kind == GATHER_TAIL) {
+        ibm_tail_cell<S>(sa, w.number * kGatherThreads + (int)threadIdx.x);
+    } else if (w.kind == GATHER_FLAGS) {
+        const int n4 = (int)(sa.mask_bytes / 16), v0 = w.number * (kMaskCopyWords / 4);
         for (int v = v0 + (int)threadIdx.x; v < min(n4, v0 + kMaskCopyWords / 4); v += kGatherThreads)
             reinterpret_cast<uint4*>(sa.mask_new)[v] = reinterpret_cast<const uint4*>(sa.mask_static)[v];
     } else {
-        ibm_cell_tile<S>(sa, sm, (q & 0x3ff) * 32, (q >> 10) * kCellPlaces, 0x7fffffff);
+        ibm_cell_tile<S>(sa, sm, w.j0(sa.g.ny), w.p0(sa.g.ny), 0x7fffffff);
     }
 }
 

@@ -250,11 +250,23 @@ cudaError_t launch_sched_levels(const SchedArgs& a, int max_cells, int ncell, cu
 cudaError_t raise_smem_limit(const void* fn, size_t bytes);
 
 // Immersed-boundary passes of many lattices in one set of launches: device
-// IbmArgs per lattice and work lists of (lattice, item). gather: 4 q + kind --
-// the places 8 (q >> 10) .. + 8 of the planes 32 (q & 1023) .. + 32, the 256
-// (blade marker, cell) pairs from 256 q, the kMaskCopyWords touched-flag words
-// from kMaskCopyWords q; small / big: one j-plane (128 / 512 threads).
+// IbmArgs per lattice and work lists. gather: GatherItem's; small / big:
+// (lattice, j-plane), 128 / 512 threads.
 enum GatherKind { GATHER_CELLS = 0, GATHER_TAIL = 1, GATHER_FLAGS = 2 };
+// A block's work of the gather: the kind beside the lattice, and a number: of
+// the tile of 32 planes and kCellPlaces places (CELLS: planes first), of 256
+// (blade marker, cell) pairs, of kMaskCopyWords touched-flag words. (A number
+// with the plane group packed into it ran out of bits at 2^22 cells a plane.)
+constexpr int kCellPlaces = 8;
+struct GatherItem {
+    int tank, kind, number;
+    __host__ __device__ static int2 pack(int tank, int kind, int number) { return make_int2(tank << 2 | kind, number); }
+    __host__ __device__ static GatherItem of(int2 w) { return GatherItem{w.x >> 2, w.x & 3, w.y}; }
+    // CELLS: the tile of planes from j0 and places from p0, of `ny` planes
+    __host__ __device__ static int tile(int j0, int p0, int ny) { return p0 / kCellPlaces * ((ny + 31) / 32) + j0 / 32; }
+    __host__ __device__ int j0(int ny) const { return number % ((ny + 31) / 32) * 32; }
+    __host__ __device__ int p0(int ny) const { return number / ((ny + 31) / 32) * kCellPlaces; }
+};
 struct IbmBatch {
     const IbmArgs* args;
     const int2* gather; int n_gather;

@@ -95,3 +95,11 @@ extern "C" void fake_check(const char* w, void** args) {
 // index arithmetic that kernels and launches share
 extern "C" long long fake_listed_word(unsigned block, unsigned thread, unsigned V) { return tdlb::listed_word(block, thread, V); }
 extern "C" long long fake_listed_blocks(long long words, unsigned V) { return tdlb::listed_blocks(words, V); }
+extern "C" void fake_gather_item(int tank, int j0, int p0, int ny, int* out4) {
+    const int2 w = tdlb::GatherItem::pack(tank, tdlb::GATHER_CELLS, tdlb::GatherItem::tile(j0, p0, ny));
+    const tdlb::GatherItem g = tdlb::GatherItem::of(w);
+    out4[0] = g.tank;
+    out4[1] = g.kind;
+    out4[2] = g.j0(ny);
+    out4[3] = g.p0(ny);
+}

@@ -448,3 +448,14 @@ def test_every_listed_word_has_its_lanes(fake, V, words):
         for lane in (0, lanes - 1):
             thread = w * lanes + lane
             assert lib.fake_listed_word(thread // 128, thread % 128, V) == w
+
+
+@pytest.mark.parametrize("nx,ny,nz", [(3, 1, 3), (400, 400, 400), (2100, 33, 2100), (8000, 32, 8000), (32767, 2, 32767),
+                                      (256, 32767, 255)])
+def test_gather_items_of_the_largest_planes(fake, nx, ny, nz):
+    """The batched gather's work items name every tile of planes and stencil cells."""
+    out = (ctypes.c_int * 4)()
+    for p0 in {0, 8, nx * nz // 16 * 8, (nx * nz - 1) // 8 * 8}:
+        for j0 in {0, (ny - 1) // 32 * 32, (ny - 1) // 64 * 32}:
+            fake.load_library().fake_gather_item(61, j0, p0, ny, out)
+            assert list(out) == [61, 0, j0, p0]
