@@ -152,7 +152,7 @@ int tdlb_double_resolution(tdlb_handle h) {
     drop(h->d_exclude);
     h->h_exclude.clear();
     h->h_plane_list.clear();
-    drop(h->d_rot_xz);
+    h->d_rot_xz = nullptr;   // (in the impeller's block)
     h->marker_gen++;
     h->resident = false;
     tdlb_rt::drop_zone(h);

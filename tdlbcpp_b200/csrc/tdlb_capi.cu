@@ -79,10 +79,7 @@ void release(tdlb_lattice* h) {
     if (h->ev_inner) cudaEventDestroy(h->ev_inner);
     if (h->ev_fence) cudaEventDestroy(h->ev_fence);
     cudaFree(h->d_red);
-    cudaFree(h->d_rot_xz);
-    cudaFree(h->d_load);
-    cudaFree(h->d_imp_slots);
-    cudaFree(h->d_blade_stage);
+    cudaFree(h->imp_block);
     cudaFree(h->d_res[0]);
     cudaFree(h->d_res[1]);
     for (auto& st : h->pin) {
@@ -846,43 +843,55 @@ void host_aos_to_planes(tdlb_lattice* h, const float* in, int npl, float* dev) {
     TDLB_CK(cudaStreamSynchronize(h->stream));
 }
 
-// What the impeller load needs: its scratch and the impeller's slots of the
-// resident list, the markers from list index `begin`. (Its blades keep their slots
-// while they rotate on the device; a host list of blades reorders them within the
-// second segment, which is the impeller's whole.) Made with the impeller, so that
-// a load neither allocates nor waits.
+// The impeller's arrays, one allocation kept for the next impeller: its blades'
+// offsets, the load's scratch and the impeller's slots of the resident list (the
+// markers from list index `begin`), the staging of a blade upload (the blades,
+// their order, at most a level each, the planes' level offsets). Made with the
+// impeller, so that neither a load nor a blade upload allocates or waits. (The
+// blades keep their slots while they rotate on the device; a host list of blades
+// reorders them within the second segment, which is the impeller's whole.)
 constexpr size_t kLoadDoubles = (size_t)tdlb::kLoadBlocks * 5 + 5 + 1;
-void prepare_load(tdlb_lattice* h, int begin) {
-    if (!h->d_load) {
-        TDLB_CK(cudaMalloc(&h->d_load, kLoadDoubles * sizeof(double)));
-        TDLB_CK(cudaMemsetAsync(h->d_load, 0, kLoadDoubles * sizeof(double), h->stream));
-    }
+void prepare_impeller(tdlb_lattice* h, const std::vector<double>& xz, int begin) {
     const int n = h->n_markers, groups = (n + 255) / 256;
-    cudaFree(h->d_imp_slots);
-    h->d_imp_slots = nullptr;
-    h->n_imp = 0;
-    if (n > 0) {
-        struct Tmp {
-            int* p = nullptr;
-            ~Tmp() { cudaFree(p); }
-        } off;
-        std::vector<int> count((size_t)groups);
-        TDLB_CK(cudaMalloc(&off.p, (size_t)groups * sizeof(int)));
-        TDLB_CK(tdlb::launch_impeller_slots(h->d_sched, n, begin, off.p, nullptr, h->stream));
-        TDLB_CK(cudaMemcpyAsync(count.data(), off.p, (size_t)groups * sizeof(int), cudaMemcpyDeviceToHost, h->stream));
+    const size_t blades = xz.size() / 2;
+    size_t at = 0;
+    auto take = [&](size_t bytes) {
+        const size_t here = at;
+        at += (bytes + 255) / 256 * 256;
+        return here;
+    };
+    const size_t o_xz = take(xz.size() * sizeof(double)), o_load = take(kLoadDoubles * sizeof(double)),
+                 o_slots = take((size_t)(n - begin) * sizeof(int)), o_off = take((size_t)groups * sizeof(int)),
+                 o_stage = take(blades * (sizeof(tdlb::Marker) + 2 * sizeof(int)) + (size_t)(h->g.ny + 2) * sizeof(int));
+    if (at > h->imp_block_cap) {
         TDLB_CK(cudaStreamSynchronize(h->stream));
-        int sum = 0;
-        for (int& c : count) {
-            const int v = c;
-            c = sum;
-            sum += v;
-        }
-        TDLB_CK(cudaMalloc(&h->d_imp_slots, (size_t)std::max(sum, 1) * sizeof(int)));
-        TDLB_CK(cudaMemcpyAsync(off.p, count.data(), (size_t)groups * sizeof(int), cudaMemcpyHostToDevice, h->stream));
-        TDLB_CK(tdlb::launch_impeller_slots(h->d_sched, n, begin, off.p, h->d_imp_slots, h->stream));
-        TDLB_CK(cudaStreamSynchronize(h->stream));
-        h->n_imp = sum;
+        cudaFree(h->imp_block);
+        h->imp_block = nullptr;
+        h->imp_block_cap = 0;
+        TDLB_CK(cudaMalloc(&h->imp_block, at));
+        h->imp_block_cap = at;
     }
+    h->d_rot_xz = (double*)(h->imp_block + o_xz);
+    h->d_load = (double*)(h->imp_block + o_load);
+    h->d_imp_slots = (int*)(h->imp_block + o_slots);
+    h->d_blade_stage = h->imp_block + o_stage;
+    h->n_imp = n - begin;
+    int* off = (int*)(h->imp_block + o_off);
+    std::vector<int> count((size_t)groups);
+    if (!xz.empty())
+        TDLB_CK(cudaMemcpyAsync(h->d_rot_xz, xz.data(), xz.size() * sizeof(double), cudaMemcpyHostToDevice, h->stream));
+    TDLB_CK(cudaMemsetAsync(h->d_load, 0, kLoadDoubles * sizeof(double), h->stream));
+    TDLB_CK(tdlb::launch_impeller_slots(h->d_sched, n, begin, off, nullptr, h->stream));
+    if (n) TDLB_CK(cudaMemcpyAsync(count.data(), off, (size_t)groups * sizeof(int), cudaMemcpyDeviceToHost, h->stream));
+    TDLB_CK(cudaStreamSynchronize(h->stream));
+    int sum = 0;
+    for (int& c : count) {
+        const int v = c;
+        c = sum;
+        sum += v;
+    }
+    if (n) TDLB_CK(cudaMemcpyAsync(off, count.data(), (size_t)groups * sizeof(int), cudaMemcpyHostToDevice, h->stream));
+    TDLB_CK(tdlb::launch_impeller_slots(h->d_sched, n, begin, off, h->d_imp_slots, h->stream));
 }
 
 // ---------------------------------------------------------------------------
@@ -1292,23 +1301,7 @@ int tdlb_attach_rushton(tdlb_handle h, const tdlb_rushton* spec, double nonupdat
         upload_markers(h, all.data(), all.size(), n0, xz.data());
         h->resident = true;
         h->h_rot_xz = xz;
-        cudaFree(h->d_rot_xz);
-        h->d_rot_xz = nullptr;
-        if (!xz.empty()) {
-            TDLB_CK(cudaMalloc(&h->d_rot_xz, xz.size() * sizeof(double)));
-            TDLB_CK(cudaMemcpy(h->d_rot_xz, xz.data(), xz.size() * sizeof(double), cudaMemcpyHostToDevice));
-        }
-        // tdlb_set_rotating_markers' upload: the blades, their order, at most a
-        // level each and the planes' level offsets
-        const size_t stage = pol.size() * (sizeof(tdlb::Marker) + 2 * sizeof(int)) + sizeof(int) + (size_t)(h->g.ny + 1) * sizeof(int);
-        if (stage > h->blade_stage_cap) {
-            cudaFree(h->d_blade_stage);
-            h->d_blade_stage = nullptr;
-            h->blade_stage_cap = 0;
-            TDLB_CK(cudaMalloc(&h->d_blade_stage, stage));
-            h->blade_stage_cap = stage;
-        }
-        prepare_load(h, n_fixed);
+        prepare_impeller(h, xz, n_fixed);
         h->rot_device = true;
         h->rot_ci = G.ci;
         h->rot_ck = G.ck;

@@ -86,6 +86,8 @@ struct tdlb_lattice {
     bool markers_set = false;
     float last_beta = 0.f;        // beta of the last forcing pass (for the load)
     // resident impeller: markers [n0, n_markers) are blades
+    char* imp_block = nullptr;    // one allocation: the impeller's arrays (d_rot_xz, d_load, d_imp_slots, d_blade_stage)
+    size_t imp_block_cap = 0;
     double* d_rot_xz = nullptr;   // their impeller-frame offsets (device rotation)
     bool rot_device = false;
     double rot_ci = 0, rot_ck = 0;
@@ -106,7 +108,6 @@ struct tdlb_lattice {
     } pin[2];
     int pin_cur = 0;
     char* d_blade_stage = nullptr;   // the upload on the device, before its parts are placed
-    size_t blade_stage_cap = 0;
     std::vector<double> h_rot_xz; // host copy of d_rot_xz
 
     // Split steps: the outer words of a step run on `bulk`, beside the previous
