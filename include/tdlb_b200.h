@@ -300,11 +300,13 @@ int tdlb_get_residual_box(tdlb_handle h, int64_t* box6);
  * The outer cells of a step then run beside the previous step's forcing
  * pass. Every cell computes what the single launch computes, so results are
  * bit-identical with and without. mode 0: off; 1: on when the inner words
- * hold at most 60 % of the lattice; 2: on whenever possible. Until this is
- * called, as 1 for lattices of at least 2^19 cells (below, the second launch
- * costs more than it hides), until the caller takes the handle's stream
- * (tdlb_get_stream). FP32 storage needs one cell per thread; a step
- * under stream capture is never split. The handle's stream waits for the
+ * hold at most 60 % of the lattice; 2: on whenever possible; -1 (the default):
+ * as 1, for lattices of at least 2^19 cells (below, the second launch costs
+ * more than it hides) whose markers have been through two forcing passes,
+ * until the caller takes the handle's stream (tdlb_get_stream). A step runs
+ * split while the last forcing pass applied the resident markers. FP32
+ * storage needs one cell per thread; a step under stream capture is never
+ * split. The handle's stream waits for the
  * outer launch at the end of each step, so work queued there afterwards sees
  * the whole step. The other way round the outer launch of a step waits for
  * the previous step's inner cells, not for the stream: with modes 1 and 2, call
@@ -318,9 +320,8 @@ int tdlb_set_overlap(tdlb_handle h, int mode);
 int tdlb_join(tdlb_handle h);
 
 /* Per-cell flags (interior cells in (i, j, k) order) of the split-step zone:
- * 1 where the cell belongs to an inner word. TDLB_ESTATE when tdlb_set_overlap
- * has not turned split steps on, the handle cannot split them, or the step
- * kernel takes several cells per thread. */
+ * 1 where the cell belongs to an inner word. TDLB_ESTATE where the handle does
+ * not split its steps (tdlb_set_overlap). */
 int tdlb_read_zone(tdlb_handle h, uint8_t* flags);
 
 /* Step-kernel timing: when on, every step-kernel launch (both launches of a

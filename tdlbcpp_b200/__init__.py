@@ -481,11 +481,11 @@ class ComputeUnit:
 
     def set_overlap(self, mode):
         """Split steps: the outer cells of a step run while the forcing pass is
-        in flight; results are identical. Without a call the library splits
-        the steps of a large lattice, until `stream` is read. False/0: off; True/1: when the inner
+        in flight; results are identical. False/0: off; True/1: when the inner
         words hold at most 60 % of the lattice; "always"/2: whenever the
-        markers are resident."""
-        m = 2 if mode == "always" else int(bool(mode)) if isinstance(mode, bool) else int(mode)
+        markers are resident; "auto"/-1 (the default): as 1 for a large lattice
+        whose markers stay, until `stream` is read."""
+        m = int({"always": 2, "auto": -1}.get(mode, mode))
         self._check(self.lib.tdlb_set_overlap(self.h, m))
 
     def join(self):

@@ -1196,7 +1196,7 @@ int tdlb_set_l2_prefetch(tdlb_handle h, int on) {
 
 int tdlb_set_overlap(tdlb_handle h, int mode) {
     return guarded(h, [&] {
-        if (mode < 0 || mode > 2) throw Fail{TDLB_EINVAL, "overlap mode must be 0, 1 or 2"};
+        if (mode < -1 || mode > 2) throw Fail{TDLB_EINVAL, "overlap mode must be -1, 0, 1 or 2"};
         h->overlap = mode;
         tdlb_rt::reserve_zone(h);
     });
@@ -1209,10 +1209,10 @@ int tdlb_join(tdlb_handle h) {
 int tdlb_read_zone(tdlb_handle h, uint8_t* flags) {
     return guarded(h, [&] {
         if (!flags) throw Fail{TDLB_EINVAL, "out is NULL"};
-        if (h->overlap < 0 || tdlb::vector_width(h->g, h->vec) != 1 || !split_wanted(h) || !zone_built(h, true) || !h->zone_ok ||
-            !zone_pays(h))
-            throw Fail{TDLB_ESTATE, "no split step (needs resident markers, one cell per thread, overlap on and, in "
-                                    "mode 1, inner chunks holding at most 60 % of the lattice)"};
+        if (!split_wanted(h) || !zone_built(h, true) || !h->zone_ok || !zone_pays(h))
+            throw Fail{TDLB_ESTATE, "no split step (needs split steps on, resident markers that, unasked, have been through "
+                                    "two forcing passes, one cell per thread with FP32 storage and, unless mode 2, inner "
+                                    "words holding at most 60 % of the lattice)"};
         const Dims& g = h->g;
         size_t c = 0;
         for (int i = 0; i < g.nx; i++)

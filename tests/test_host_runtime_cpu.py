@@ -459,3 +459,39 @@ def test_gather_items_of_the_largest_planes(fake, nx, ny, nz):
         for j0 in {0, (ny - 1) // 32 * 32, (ny - 1) // 64 * 32}:
             fake.load_library().fake_gather_item(61, j0, p0, ny, out)
             assert list(out) == [61, 0, j0, p0]
+
+
+@pytest.mark.parametrize("streaming,storage", CASES)
+def test_the_automatic_mode_comes_back_and_shows_its_zone(fake, streaming, storage):
+    lib = fake.load_library()
+    cu = fake.ComputeUnit(x=96, y=96, z=96, nu=1e-3, streaming=streaming, storage=storage)
+    cu.initialise(1.0)
+    _attach(fake, cu, (96, 96, 96))
+
+    def split():
+        n = lib.fake_launches(b", 1>(")
+        cu.step(ALPHA, BETA)
+        return lib.fake_launches(b", 1>(") > n
+
+    cu.forcing_resident(ALPHA, BETA)
+    with pytest.raises(fake.TdlbError):
+        cu.read_zone()                   # not planned yet
+    for _ in range(3):
+        cu.step(ALPHA, BETA)
+    assert split() and cu.read_zone().shape == (96, 96, 96)
+    if storage == "fp32":                # (a boxed step has an outer launch in any mode)
+        cu.set_overlap(False)
+        assert not split()
+        with pytest.raises(fake.TdlbError):
+            cu.read_zone()
+        cu.set_overlap("auto")
+        assert split() and cu.read_zone().shape == (96, 96, 96)
+        cu.set_cells_per_thread(2)
+        assert not split()
+        with pytest.raises(fake.TdlbError):
+            cu.read_zone()
+    for bad in (-2, 3):
+        with pytest.raises(fake.TdlbError):
+            cu.set_overlap(bad)
+    cu.close()
+    assert not faults(fake)
