@@ -91,16 +91,7 @@ __device__ __forceinline__ void prefetch_items(const TankStep* __restrict__ tank
     if (d == NQ && !ts.les) return;
     const Dims& g = ts.g;
     const long long e0 = (long long)wk.y * V, e1 = e0 + (long long)kPrefetchTiles * NT * V;
-    if (d == NQ) return prefetch_span(ts.Nu, 4, g.plane, e0, e1);
-    const long long rs = (long long)g.nz * g.jp;
-    long long sh;
-    if (ESO) {
-        const int sg = ts.even ? -1 : 1;
-        sh = (sg * cx_of(d) > 0 ? rs : 0) + (sg * cz_of(d) > 0 ? g.jp : 0);
-    } else {
-        sh = -(cx_of(d) * rs + cz_of(d) * g.jp);
-    }
-    prefetch_span(ts.A.p[d], (int)sizeof(S), g.plane, e0 + sh - 1, e1 + sh + 1);
+    prefetch_span(d == NQ ? ts.Nu : ts.A.p[d], pull_span(g, d, d == NQ ? 4 : (int)sizeof(S), ESO, ts.even, e0, e1));
 }
 
 // Batched step: block b takes work items b, b + grid, ...; an item is NT

@@ -648,14 +648,35 @@ __device__ __forceinline__ void esotwist_quad(const Planes& Q, float* __restrict
 // 16-byte aligned and hold a multiple of 64 elements); a prefetch changes no
 // result.
 constexpr int kPrefetchTiles = 8;
-__device__ __forceinline__ void prefetch_span(const void* base, int es, long long plane, long long e0,
-                                              long long e1) {
+// What the cells of elements [e0, e1) read of population plane d (d == NQ: of Nu,
+// their own elements), as bytes from the plane's base; empty where lo >= hi.
+struct PrefetchSpan {
+    long long lo, hi;
+};
+__host__ __device__ __forceinline__ PrefetchSpan pull_span(const Dims& g, int d, int es, bool eso, bool even, long long e0,
+                                                           long long e1) {
+    if (d < NQ) {
+        const long long rs = (long long)g.nz * g.jp;
+        long long sh;
+        if (eso) {
+            const int sg = even ? -1 : 1;
+            sh = (sg * cx_of(d) > 0 ? rs : 0) + (sg * cz_of(d) > 0 ? g.jp : 0);
+        } else {
+            sh = -(cx_of(d) * rs + cz_of(d) * g.jp);
+        }
+        // one element either side: the j +- 1 neighbours
+        e0 += sh - 1;
+        e1 += sh + 1;
+    }
     e0 = e0 < 0 ? 0 : e0;
-    e1 = e1 > plane ? plane : e1;
-    if (e0 >= e1) return;
-    const uintptr_t lo = (reinterpret_cast<uintptr_t>(base) + (uintptr_t)(e0 * es)) & ~(uintptr_t)15;
-    const uintptr_t hi = (reinterpret_cast<uintptr_t>(base) + (uintptr_t)(e1 * es) + 15) & ~(uintptr_t)15;
-    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(lo), "r"((unsigned)(hi - lo)) : "memory");
+    e1 = e1 > g.plane ? g.plane : e1;
+    if (e0 >= e1) return PrefetchSpan{0, 0};
+    return PrefetchSpan{e0 * es & ~15LL, (e1 * es + 15) & ~15LL};
+}
+__device__ __forceinline__ void prefetch_span(const void* base, PrefetchSpan s) {
+    if (s.lo >= s.hi) return;
+    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"((const char*)base + s.lo), "r"((unsigned)(s.hi - s.lo))
+                 : "memory");
 }
 template <typename S, int V, bool LES, bool ESO, bool EVEN>
 __device__ __forceinline__ void prefetch_ahead(const Planes& A, const float* Nu, const Dims& g, int ahead) {
@@ -664,17 +685,7 @@ __device__ __forceinline__ void prefetch_ahead(const Planes& A, const float* Nu,
     constexpr long long tile = 128LL * V;
     const long long e0 = ((long long)blockIdx.x + ahead) * tile, e1 = e0 + kPrefetchTiles * tile;
     if (e0 >= g.rows() * g.jp) return;
-    if (d == NQ) return prefetch_span(Nu, 4, g.plane, e0, e1);
-    const long long rs = (long long)g.nz * g.jp;
-    long long sh;
-    if (ESO) {
-        const int sg = EVEN ? -1 : 1;
-        sh = (sg * cx_of(d) > 0 ? rs : 0) + (sg * cz_of(d) > 0 ? g.jp : 0);
-    } else {
-        sh = -(cx_of(d) * rs + cz_of(d) * g.jp);
-    }
-    // one element either side: the j +- 1 neighbours
-    prefetch_span(A.p[d], (int)sizeof(S), g.plane, e0 + sh - 1, e1 + sh + 1);
+    prefetch_span(d == NQ ? Nu : A.p[d], pull_span(g, d, d == NQ ? 4 : (int)sizeof(S), ESO, EVEN, e0, e1));
 }
 
 // Step launches that go close behind the one before them (launch_chained): all

@@ -8,7 +8,7 @@
 #include <string>
 #include <vector>
 
-#include "tdlb_kernels.cuh"
+#include "step_kernels.cuh"
 
 void fake_need(const char* who, const char* what, const void* p, long long n);
 void fake_fault(const char* who, const char* what);
@@ -103,3 +103,10 @@ extern "C" void fake_gather_item(int tank, int j0, int p0, int ny, int* out4) {
     out4[2] = g.j0(ny);
     out4[3] = g.p0(ny);
 }
+extern "C" void fake_pull_span(int nx, int ny, int nz, int d, int es, int eso, int even, long long e0, long long e1, long long* out2) {
+    const tdlb::PrefetchSpan s = tdlb::pull_span(tdlb::make_dims(nx, ny, nz), d, es, eso != 0, even != 0, e0, e1);
+    out2[0] = s.lo;
+    out2[1] = s.hi;
+}
+extern "C" int fake_prefetch_tiles() { return tdlb::kPrefetchTiles; }
+extern "C" int fake_row_pitch(int nx, int ny, int nz) { return tdlb::make_dims(nx, ny, nz).jp; }

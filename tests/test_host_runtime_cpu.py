@@ -495,3 +495,46 @@ def test_the_automatic_mode_comes_back_and_shows_its_zone(fake, streaming, stora
             cu.set_overlap(bad)
     cu.close()
     assert not faults(fake)
+
+
+CX = [1, -1, 0, 0, 0, 0, 1, -1, 1, -1, 0, 0, 1, -1, 1, -1, 0, 0]
+CY = [0, 0, 1, -1, 0, 0, 1, -1, 0, 0, 1, -1, -1, 1, 0, 0, 1, -1]
+CZ = [0, 0, 0, 0, 1, -1, 0, 0, 1, -1, 1, -1, 0, 0, -1, 1, -1, 1]
+
+
+@pytest.mark.parametrize("shape", [(40, 96, 36), (45, 38, 51), (17, 5, 3), (9, 2, 64), (31, 3, 30)])
+@pytest.mark.parametrize("cells,es", [(128, 4), (512, 4), (128, 2), (256, 2), (1024, 2)])
+@pytest.mark.parametrize("ahead", [0, 1, 61])
+@pytest.mark.parametrize("eso,even", [(False, False), (True, True), (True, False)])
+def test_prefetch_spans_of_the_step_kernels(fake, shape, cells, es, ahead, eso, even):
+    """Every span that a block's prefetch names -- `cells` elements a block or work
+    item, from `ahead` of them further on -- starts and ends on 16 bytes inside its
+    plane (a multiple of 64 elements) and holds what the cells away from the faces
+    pull from it."""
+    lib = fake.load_library()
+    lib.fake_pull_span.argtypes = [ctypes.c_int] * 7 + [ctypes.c_longlong] * 2 + [ctypes.c_void_p]
+    nx, ny, nz = shape
+    jp, tiles = lib.fake_row_pitch(nx, ny, nz), lib.fake_prefetch_tiles()
+    total = nx * nz * jp
+    plane = (total + 63) // 64 * 64
+    out = np.zeros(2, np.int64)
+    for e0 in range(ahead * cells, total, tiles * cells):
+        e1 = e0 + tiles * cells
+        e = np.arange(e0, min(e1, total))
+        row, j = np.divmod(e, jp)
+        i, k = np.divmod(row, nz)
+        inner = (i >= 1) & (i < nx - 1) & (j >= 1) & (j < ny - 1) & (k >= 1) & (k < nz - 1)
+        for d in range(19):
+            size = es if d < 18 else 4
+            lib.fake_pull_span(nx, ny, nz, d, size, eso, even, e0, e1, out.ctypes.data)
+            lo, hi = int(out[0]), int(out[1])
+            assert lo % 16 == 0 and hi % 16 == 0 and 0 <= lo <= hi <= plane * size
+            if d == 18:
+                src = e
+            elif eso:
+                sg = -1 if even else 1
+                src = e + (nz * jp if sg * CX[d] > 0 else 0) + (jp if sg * CZ[d] > 0 else 0) + (1 if sg * CY[d] > 0 else 0)
+            else:
+                src = e - (CX[d] * nz + CZ[d]) * jp - CY[d]
+            src = src[inner] * size
+            assert ((src >= lo) & (src + size <= hi)).all(), d
