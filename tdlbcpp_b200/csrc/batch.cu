@@ -348,16 +348,16 @@ void build_ibm_work(tdlb_batch_s* b) {
         for (int t : G.tanks) {
             const tdlb_lattice* h = b->tanks[(size_t)t];
             if (!h->markers_set) continue;
-            for (int q = 0; q < 9 * (h->n_markers - h->n0); q += 256) gather.push_back(tdlb::GatherItem::pack(t, tdlb::GATHER_TAIL, q / 256));
+            for (int q = 0; q < 9 * (h->n_markers - h->n0); q += 256) gather.push_back(tdlb::GatherItem::other(t, tdlb::GATHER_TAIL, q / 256));
             for (long long wd = 0; wd < h->mask_words; wd += tdlb::kMaskCopyWords)
-                gather.push_back(tdlb::GatherItem::pack(t, tdlb::GATHER_FLAGS, (int)(wd / tdlb::kMaskCopyWords)));
+                gather.push_back(tdlb::GatherItem::other(t, tdlb::GATHER_FLAGS, (int)(wd / tdlb::kMaskCopyWords)));
             const int places = std::max(h->max_cells, h->max_big);
             for (int p = 0; p < places; p += tdlb::kCellPlaces)
                 for (int jg = 0; jg < h->g.ny; jg += 32) {
                     bool any = false;   // a tile past every plane's cells is left out
                     for (int j = jg; j < std::min(jg + 32, h->g.ny); j++)
                         any = any || h->plane_cell[(size_t)j + 1] - h->plane_cell[(size_t)j] > p;
-                    if (any) gather.push_back(tdlb::GatherItem::pack(t, tdlb::GATHER_CELLS, tdlb::GatherItem::tile(jg, p, h->g.ny)));
+                    if (any) gather.push_back(tdlb::GatherItem::cells(t, jg, p));
                 }
             for (int s = 0; s < h->n_small; s++) small.push_back(make_int2(t, h->h_plane_list[(size_t)s]));
             for (int s = 0; s < h->n_big; s++) big.push_back(make_int2(t, h->h_plane_list[(size_t)(h->n_small + s)]));

@@ -1223,13 +1223,13 @@ __global__ void __launch_bounds__(kGatherThreads) k_ibm_gather_batch(const IbmAr
     stage_args<kGatherThreads>(sa, args + w.tank);
     __syncthreads();
     if (w.kind == GATHER_TAIL) {
-        ibm_tail_cell<S>(sa, w.number * kGatherThreads + (int)threadIdx.x);
+        ibm_tail_cell<S>(sa, w.y * kGatherThreads + (int)threadIdx.x);
     } else if (w.kind == GATHER_FLAGS) {
-        const int n4 = (int)(sa.mask_bytes / 16), v0 = w.number * (kMaskCopyWords / 4);
+        const int n4 = (int)(sa.mask_bytes / 16), v0 = w.y * (kMaskCopyWords / 4);
         for (int v = v0 + (int)threadIdx.x; v < min(n4, v0 + kMaskCopyWords / 4); v += kGatherThreads)
             reinterpret_cast<uint4*>(sa.mask_new)[v] = reinterpret_cast<const uint4*>(sa.mask_static)[v];
     } else {
-        ibm_cell_tile<S>(sa, sm, w.j0(sa.g.ny), w.p0(sa.g.ny), 0x7fffffff);
+        ibm_cell_tile<S>(sa, sm, w.j0(), w.p0(), 0x7fffffff);
     }
 }
 

@@ -95,13 +95,12 @@ extern "C" void fake_check(const char* w, void** args) {
 // index arithmetic that kernels and launches share
 extern "C" long long fake_listed_word(unsigned block, unsigned thread, unsigned V) { return tdlb::listed_word(block, thread, V); }
 extern "C" long long fake_listed_blocks(long long words, unsigned V) { return tdlb::listed_blocks(words, V); }
-extern "C" void fake_gather_item(int tank, int j0, int p0, int ny, int* out4) {
-    const int2 w = tdlb::GatherItem::pack(tank, tdlb::GATHER_CELLS, tdlb::GatherItem::tile(j0, p0, ny));
-    const tdlb::GatherItem g = tdlb::GatherItem::of(w);
+extern "C" void fake_gather_item(int tank, int j0, int p0, int* out4) {
+    const tdlb::GatherItem g = tdlb::GatherItem::of(tdlb::GatherItem::cells(tank, j0, p0));
     out4[0] = g.tank;
     out4[1] = g.kind;
-    out4[2] = g.j0(ny);
-    out4[3] = g.p0(ny);
+    out4[2] = g.j0();
+    out4[3] = g.p0();
 }
 extern "C" void fake_pull_span(int nx, int ny, int nz, int d, int es, int eso, int even, long long e0, long long e1, long long* out2) {
     const tdlb::PrefetchSpan s = tdlb::pull_span(tdlb::make_dims(nx, ny, nz), d, es, eso != 0, even != 0, e0, e1);

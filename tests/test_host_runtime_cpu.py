@@ -457,7 +457,7 @@ def test_gather_items_of_the_largest_planes(fake, nx, ny, nz):
     out = (ctypes.c_int * 4)()
     for p0 in {0, 8, nx * nz // 16 * 8, (nx * nz - 1) // 8 * 8}:
         for j0 in {0, (ny - 1) // 32 * 32, (ny - 1) // 64 * 32}:
-            fake.load_library().fake_gather_item(61, j0, p0, ny, out)
+            fake.load_library().fake_gather_item(61, j0, p0, out)
             assert list(out) == [61, 0, j0, p0]
 
 
