@@ -11,8 +11,8 @@
 // Cells no marker touched end with F = 0 (:162-174).
 //
 // Parallel form with the same result: a marker only interacts with markers
-// of the same j-plane that share a stencil cell. The host scheduler assigns
-// each marker a level = 1 + the highest level of an earlier marker sharing a
+// of the same j-plane that share a stencil cell. The scheduler (schedule.cu, for
+// the blades tdlb_runtime.hpp) assigns each marker a level = 1 + the highest level of an earlier marker sharing a
 // cell, so markers of one level touch disjoint cells and every pair that
 // shares a cell keeps its list order. One CTA per j-plane walks its levels
 // with a barrier between them.

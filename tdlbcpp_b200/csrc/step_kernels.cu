@@ -26,9 +26,6 @@
 
 namespace tdlb {
 
-
-__device__ __forceinline__ int wrap_up(int a, int n) { return a + 1 == n ? 0 : a + 1; }
-
 // ---------------------------------------------------------------------------
 // Moment-form state after initialise(rho): slot 0 = rho, others 0 at every
 // cell (QVec.hpp:406-411). For Esotwist with evenStep = true the reference's

@@ -628,7 +628,8 @@ __device__ __forceinline__ void esotwist_quad(const Planes& Q, float* __restrict
 //     as PART 0 does, prefetch included, and drops the zone's results at the
 //     store (a few per cent of the cells): the flag is loaded beside the
 //     populations and delays nothing;
-//   PART 2 (inner): the words of the zone, from a list.
+//   PART 2 (inner): the words of the zone, from a list, or, for a step with a
+//     residual box and no zone, every word.
 // PART 0 runs every cell. The outer launch of a step depends on the previous
 // step's populations only, so it can run while the previous forcing pass is
 // still in flight.
@@ -641,9 +642,9 @@ __device__ __forceinline__ void esotwist_quad(const Planes& Q, float* __restrict
 // Nu's span (LES). With `ahead` one wave of resident CTAs, the populations
 // are in L2 when those CTAs load them, so the loads -- whose latency bounds
 // the kernels at their occupancy -- wait for the L2, not for the DRAM.
-// Measured on B200 at 400^3 (step kernel alone, ms): FP32 Simple 1.530 ->
-// 1.483, FP32 Esotwist 1.677 -> 1.496, 16-bit Simple (four cells per thread)
-// 1.26 -> 1.08, 16-bit Esotwist (two cells per thread) 1.55 -> 1.35.
+// Measured on B200 at 400^3 (step kernel alone, ms): FP32 Simple 1.558 ->
+// 1.462, FP32 Esotwist 1.741 -> 1.483, 16-bit Simple (four cells per thread)
+// 1.110 -> 0.905, 16-bit Esotwist (two cells per thread) 1.169 -> 1.057.
 // Spans are clamped to the plane and rounded out to 16 bytes (planes start
 // 16-byte aligned and hold a multiple of 64 elements); a prefetch changes no
 // result.
@@ -737,8 +738,9 @@ cudaError_t launch_step_kernel(void (*kernel)(P...), unsigned grid, cudaStream_t
 // their locations lie in the box (rr), collided as the one-cell-per-thread
 // step kernels do and written with the residuals of the locations inside the
 // box (rw: the destination's set, the same one for Esotwist). Scattered runs of
-// a few tens of cells: bound by load latency (B200, 160^3 FP16 Simple: it and
-// the commit of a scratch array that it replaces 27.5 us).
+// a few tens of cells: bound by load latency (B200, beside the outer words: 160^3
+// FP16 Simple 20 us, 400^3 FP16 Esotwist 114; stepping into a scratch array and
+// committing it afterwards took 27.5 and 136).
 template <typename S, bool SIMPLE, bool LES, bool EVEN>
 __global__ void __launch_bounds__(128) k_box_step(Planes A, Planes B, float* __restrict__ Nu, const float4* __restrict__ F,
                                                   const uint32_t* __restrict__ mask, Dims g, CollideParams p,

@@ -511,7 +511,6 @@ void ensure_level_cap(tdlb_lattice* h, long long need) {
     h->level_cap = cap;
 }
 
-// Device copy of the second segment's schedule (slots n0.., levels L0..).
 // The planes whose second segment (blades) has levels, for the blade launch
 // of the forcing pass, and its shared memory; uploaded when they change.
 void update_blade_planes(tdlb_lattice* h) {
@@ -551,6 +550,7 @@ void build_blades(tdlb_lattice* h, const double* rot_xz) {
     for (int& q : h->seg1.order) q += h->n0;   // list indices
 }
 
+// Device copy of the second segment's schedule (slots n0.., levels L0..).
 void upload_seg1(tdlb_lattice* h) {
     const Dims& g = h->g;
     update_blade_planes(h);

@@ -25,7 +25,7 @@ struct tdlb_lattice {
     float* bufA = nullptr;       // 18 planes
     float* bufB = nullptr;       // 18 planes (Simple only)
     float* Nu = nullptr;
-    float* F = nullptr;          // 3 planes: Fx, Fy, Fz
+    float* F = nullptr;          // a float4 (Fx, Fy, Fz, unused) per element
     uint32_t* mask = nullptr;    // 2 x (rows * jw) words
     long long mask_words = 0;
 
@@ -197,10 +197,10 @@ struct tdlb_lattice {
 // Runtime helpers shared by the C-ABI translation units (tdlb_capi.cu).
 namespace tdlb_rt {
 // Default cells per thread of a lattice's step kernel. Measured on B200 at
-// 400^3 with the L2 prefetch on (step kernel alone): FP32 storage is fastest
-// with one cell per thread; 16-bit storage with packed FP32x2 arithmetic,
-// Simple with four (1.08 ms), Esotwist with two (1.35 ms; one: 1.48, four:
-// 1.39).
+// 400^3 with the L2 prefetch on (step kernel alone, one, two, four cells): FP32
+// Simple 1.462, 1.475, 1.575 ms, Esotwist 1.483, 1.522, 1.582; 16-bit storage with
+// packed FP32x2 arithmetic, Simple 1.176, 1.072, 0.905, Esotwist 1.326, 1.057,
+// 1.142.
 inline int default_cells_per_thread(const tdlb_config& c) {
     if (c.storage == TDLB_STORAGE_FP32) return 1;
     return c.streaming == TDLB_STREAMING_SIMPLE ? 4 : 2;
