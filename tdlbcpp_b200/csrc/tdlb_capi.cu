@@ -314,12 +314,12 @@ void build_zone(tdlb_lattice* h) {
         // nearest cell, and its stencil cells lie within 1.5 cells of that
         // position per axis, so within r +- 2.13 of the axis: plane by plane,
         // the annulus between the smallest and the largest blade radius
-        // widened by 3 cells.
-        const tdlb_marker* rot = h->h_blades.data();
+        // widened by 3 cells. (Blades that the host has set since are held
+        // against it, blades_in_zone.)
         std::vector<double2> ring((size_t)g.ny, make_double2(1e300, -1.0));
         for (int q = 0; q < n1; q++) {
             const double r = std::sqrt(h->h_rot_xz[2 * q] * h->h_rot_xz[2 * q] + h->h_rot_xz[2 * q + 1] * h->h_rot_xz[2 * q + 1]);
-            double2& p = ring[(size_t)rot[q].j];
+            double2& p = ring[(size_t)h->h_rot_j[(size_t)q]];
             p.x = std::min(p.x, r - 3.0);
             p.y = std::max(p.y, r + 3.0);
         }
@@ -1301,6 +1301,8 @@ int tdlb_attach_rushton(tdlb_handle h, const tdlb_rushton* spec, double nonupdat
         upload_markers(h, all.data(), all.size(), n0, xz.data());
         h->resident = true;
         h->h_rot_xz = xz;
+        h->h_rot_j.assign(rot.size(), 0);
+        for (size_t q = 0; q < rot.size(); q++) h->h_rot_j[q] = (int)rot[q].j;
         prepare_impeller(h, xz, n_fixed);
         h->rot_device = true;
         h->rot_ci = G.ci;

@@ -109,6 +109,7 @@ struct tdlb_lattice {
     int pin_cur = 0;
     char* d_blade_stage = nullptr;   // the upload on the device, before its parts are placed
     std::vector<double> h_rot_xz; // host copy of d_rot_xz
+    std::vector<int> h_rot_j;     // and the planes of those blades
 
     // Split steps: the outer words of a step run on `bulk`, beside the previous
     // forcing pass and the inner words on `stream`, which then waits for them:

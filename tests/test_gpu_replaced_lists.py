@@ -134,3 +134,40 @@ def test_host_blades_that_come_back_into_the_swept_volume(gpu, streaming, storag
     for early in (True, False):
         for overlap in (None, False, "always"):
             same(run(early, overlap), want)
+
+
+@pytest.mark.parametrize("streaming", ["Simple", "Esotwist"])
+@pytest.mark.parametrize("first", [0, 1, 2, 3, 4])
+def test_host_blades_in_other_planes(gpu, streaming, first):
+    """Blades that the host moves to other planes at step `first`, before or after
+    the zone of the attached ones was planned."""
+    tb = gpu
+    rt = tb.RushtonTurbine(EDGE, EDGE, EDGE, tip_speed=0.1, startup_steps=0)
+    d = rt.increment(1)
+
+    def run(early, overlap):
+        cu = unit(tb, streaming, "fp32", overlap)
+        cu.attach_rushton(rt, d, 0.0, d)
+        cu.initialise(1.0)
+        cu.forcing_resident(ALPHA, BETA)
+        for s in range(8):
+            def blades():
+                if s < first:
+                    cu.rotate_impeller(d * s, d)
+                else:
+                    moved = rt.rotating(d * s, d)
+                    if s % 3 == first % 3:
+                        moved["j"] = (moved["j"] + 30) % EDGE
+                    cu.set_rotating_markers(moved)
+            if early:
+                blades()
+            cu.collision()
+            if not early:
+                blades()
+            cu.forcing_resident(ALPHA, BETA)
+        return outputs(cu)
+
+    want = run(False, False)
+    for early in (True, False):
+        for overlap in (None, "always"):
+            same(run(early, overlap), want)

@@ -538,3 +538,27 @@ def test_prefetch_spans_of_the_step_kernels(fake, shape, cells, es, ahead, eso, 
                 src = e - (CX[d] * nz + CZ[d]) * jp - CY[d]
             src = src[inner] * size
             assert ((src >= lo) & (src + size <= hi)).all(), d
+
+
+@pytest.mark.parametrize("streaming", ["Simple", "Esotwist"])
+def test_the_zone_holds_the_attached_blades_planes(fake, streaming):
+    """Blades that the host moves to other planes before the zone is planned: the
+    last pass's blades are the attached ones."""
+    lib = fake.load_library()
+    dims = (96, 96, 96)
+    cu = fake.ComputeUnit(x=96, y=96, z=96, nu=1e-3, streaming=streaming)
+    cu.set_overlap("always")
+    _attach(fake, cu, dims)
+    rt = fake.RushtonTurbine(*dims, tip_speed=0.1, startup_steps=0)
+    cu.initialise(1.0)
+    cu.forcing_resident(ALPHA, BETA)
+    cu.collision()                       # from moments
+    cu.forcing_resident(ALPHA, BETA)
+    moved = rt.rotating(0.1, rt.increment(1))
+    moved["j"] = (moved["j"] + 30) % 96
+    cu.set_rotating_markers(moved)
+    n = lib.fake_launches(b", 1>(")
+    cu.collision()
+    assert lib.fake_launches(b", 1>(") == n, "the force of the attached blades' planes"
+    cu.close()
+    assert not faults(fake)
