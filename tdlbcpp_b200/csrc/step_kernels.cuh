@@ -644,7 +644,7 @@ __device__ __forceinline__ void esotwist_quad(const Planes& Q, float* __restrict
 // the kernels at their occupancy -- wait for the L2, not for the DRAM.
 // Measured on B200 at 400^3 (step kernel alone, ms): FP32 Simple 1.558 ->
 // 1.462, FP32 Esotwist 1.741 -> 1.483, 16-bit Simple (four cells per thread)
-// 1.110 -> 0.905, 16-bit Esotwist (two cells per thread) 1.169 -> 1.057.
+// 1.110 -> 0.905, 16-bit Esotwist (two cells per thread) 1.252 -> 1.081.
 // Spans are clamped to the plane and rounded out to 16 bytes (planes start
 // 16-byte aligned and hold a multiple of 64 elements); a prefetch changes no
 // result.

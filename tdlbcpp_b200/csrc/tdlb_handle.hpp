@@ -200,8 +200,8 @@ namespace tdlb_rt {
 // Default cells per thread of a lattice's step kernel. Measured on B200 at
 // 400^3 with the L2 prefetch on (step kernel alone, one, two, four cells): FP32
 // Simple 1.462, 1.475, 1.575 ms, Esotwist 1.483, 1.522, 1.582; 16-bit storage with
-// packed FP32x2 arithmetic, Simple 1.176, 1.072, 0.905, Esotwist 1.326, 1.057,
-// 1.142.
+// packed FP32x2 arithmetic, Simple 1.176, 1.072, 0.905, Esotwist 1.335, 1.081,
+// 1.143.
 inline int default_cells_per_thread(const tdlb_config& c) {
     if (c.storage == TDLB_STORAGE_FP32) return 1;
     return c.streaming == TDLB_STREAMING_SIMPLE ? 4 : 2;
